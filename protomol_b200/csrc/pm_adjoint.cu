@@ -179,4 +179,38 @@ int launch_pair_adjoint(const AdjArgs& a, int fp64, cudaStream_t s, long long* l
     return (int)cudaGetLastError();
 }
 
+// ---------------------------------------------------------------- LJ gradient
+// The nonzero entries of the LJ-table gradient (index, value), in no
+// particular order: most type pairs of a system with a type per chain atom
+// never meet inside the cutoff, and the dense table is most of what a
+// backward pass would move to the host (25.6 MB at 894 types, against about
+// 1 MB of entries).  HBM-bound: the table read once.
+__global__ void __launch_bounds__(256) k_lj_entries(const double* __restrict__ g, unsigned n, unsigned* __restrict__ idx,
+                                                    double* __restrict__ val, unsigned* __restrict__ count)
+{
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned stride = gridDim.x * blockDim.x;
+    // whole warps run the same number of rounds (n is a multiple of 4; a tail lane sees a zero)
+    for (unsigned base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < n; base += stride) {
+        const unsigned k = base + lane;
+        const double v = k < n ? g[k] : 0.0;
+        const unsigned m = __ballot_sync(0xffffffffu, !(v == 0.0));       // NaN is an entry
+        if (m == 0) continue;
+        unsigned at = 0;
+        if (lane == 0) at = atomicAdd(count, (unsigned)__popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (!(v == 0.0)) { idx[at] = k; val[at] = v; }
+    }
+}
+
+int launch_lj_entries(const double* g, unsigned n, unsigned* idx, double* val, unsigned* count, cudaStream_t s,
+                      long long* launches)
+{
+    if (n == 0) return 0;
+    const unsigned blocks = (n + 255) / 256;
+    k_lj_entries<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, s>>>(g, n, idx, val, count);
+    *launches += 1;
+    return (int)cudaGetLastError();
+}
+
 }  // namespace pm

@@ -47,6 +47,12 @@ __device__ __forceinline__ void bin_cell_of(const Pbc& b, const CellGrid& g, dou
     cz = (int)floor(dmul(vz, g.rcsz));
 }
 
+__device__ __forceinline__ unsigned fix32(double u)
+{
+    const double f = u - floor(u);                        // [0, 1)
+    return (unsigned)(__double2ull_rn(f * 4294967296.0) & 0xffffffffull);
+}
+
 // Single-block exclusive scans of the per-cell atom counts (-> start) and
 // cluster counts ceil(count / 8) (-> cstart), by the calling block.
 __device__ void scan_counts(const int* counts, int* start, int* cstart, int ncell)
@@ -162,7 +168,8 @@ __device__ __forceinline__ float3 write_atom(const BinArgs& a, int i, int dst)
     a.slo[dst] = make_float4((float)(rx - (double)hx), (float)(ry - (double)hy), (float)(rz - (double)hz),
                              (float)(qi - (double)hq));
     a.smeta[dst] = make_int4(i, a.type[i], a.mol[i], 0);
-    if (a.spos64) a.spos64[dst] = make_double4(x, y, z, qi);
+    a.spos64[dst] = make_double4(x, y, z, qi);
+    a.sfix[dst] = make_int4((int)fix32(x * a.pbc.e1rx), (int)fix32(y * a.pbc.e2ry), (int)fix32(z * a.pbc.e3rz), a.mol[i]);
     return make_float3(hx, hy, hz);
 }
 
@@ -241,12 +248,6 @@ __global__ void __launch_bounds__(128) k_bin_cells(BinArgs a)
 // padded (original index -1).  The reference cell of every atom is computed
 // here too (bit-exact, for pmgpu_get_cells).
 
-__device__ __forceinline__ unsigned fix32(double u)
-{
-    const double f = u - floor(u);                        // [0, 1)
-    return (unsigned)(__double2ull_rn(f * 4294967296.0) & 0xffffffffull);
-}
-
 __global__ void __launch_bounds__(kBinThreads) k_col_count(ColBinArgs a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -295,10 +296,28 @@ __global__ void __launch_bounds__(kBinThreads) k_col_scatter(ColBinArgs a)
 constexpr int kColStage = 2048;      // atoms of a column ordered in shared memory
 constexpr int kColThreads = 128;
 
+// the slot data of atom i at slot dst (a padding slot takes atom i's place
+// in the fixed-point box, no molecule and no charge)
+__device__ __forceinline__ void write_slot(const ColBinArgs& a, int i, bool valid, size_t dst)
+{
+    const double qi = a.q[i];
+    const float qh = (float)qi;
+    a.cq[dst] = make_int4((int)a.qfix[3 * i], (int)a.qfix[3 * i + 1], (int)a.qfix[3 * i + 2], valid ? a.mol[i] : -1);
+    a.cm[dst] = valid ? make_int4(__float_as_int(qh), __float_as_int((float)(qi - (double)qh)), a.type[i], i)
+                      : make_int4(0, 0, 0, -1);
+    if (a.c64)
+        a.c64[dst] = make_double4(a.pos[3 * (size_t)i], a.pos[3 * (size_t)i + 1], a.pos[3 * (size_t)i + 2],
+                                  valid ? qi : 0.0);
+    if (valid) a.slot_of[i] = (int)dst;
+}
+
 // one block per column: z order (a bitonic sort of the (z, index) keys in
-// shared memory), slot data, padding, cluster boxes and the clusters' virial
-// origins.  The sorted atoms' fixed-point coordinates and the j-cluster boxes
-// stay in shared memory for the box passes (no global round trips there).
+// shared memory), slot data, padding and cluster boxes (center, half extent).
+// The sorted atoms' fixed-point coordinates and the j-cluster boxes stay in
+// shared memory for the box passes (no global round trips there).  A column
+// of more atoms than that refuses the system (the mixed forces' cell layout
+// takes it) or, for FP64 forces alone, stays in the order it came in: its
+// boxes are right, and the list takes the column as a whole.
 __global__ void __launch_bounds__(kColThreads) k_col_sort(ColBinArgs a)
 {
     pdl_wait();
@@ -314,102 +333,114 @@ __global__ void __launch_bounds__(kColThreads) k_col_sort(ColBinArgs a)
     const int c = blockIdx.x;
     const int b = a.colstart[c], m = a.colstart[c + 1] - b;
     const int cl0 = a.ccstart[c], ncl = (m + 7) / 8;
-    if (m > kColStage || cl0 + ncl > a.ncl_cap) {            // block-uniform: the cell layout takes this system
+    const size_t slot0 = 8 * (size_t)cl0;
+    const bool large = m > kColStage;
+    // a row of padding atoms past the last: the entries that fill up a list
+    if (c == 0 && t < 8) {
+        a.cq[8 * (size_t)a.ncl_cap + t] = make_int4(0, 0, 0, -1);
+        a.cm[8 * (size_t)a.ncl_cap + t] = make_int4(0, 0, 0, -1);
+        if (a.c64) a.c64[8 * (size_t)a.ncl_cap + t] = make_double4(0.0, 0.0, 0.0, 0.0);
+    }
+    if ((large && a.refuse) || cl0 + ncl > a.ncl_cap) {      // block-uniform: the cell layout takes this system
         if (t == 0) atomicOr(a.status, kStatusColumns);
         return;
     }
-    int n2 = 32;                                            // keys padded to a power of two
-    while (n2 < m) n2 <<= 1;
-    for (int k = t; k < n2; k += kColThreads) {
-        unsigned long long key = ~0ull;
-        if (k < m) {
-            const int i = a.tmp[b + k];
-            key = ((unsigned long long)a.qfix[3 * i + 2] << 32) | (unsigned)i;
-        }
-        s_key[k] = key;
-    }
-    __syncthreads();
-    for (int k = 2; k <= n2; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = t; i < n2; i += kColThreads) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long u = s_key[i], v = s_key[ixj];
-                    if (((i & k) == 0) ? (u > v) : (u < v)) { s_key[i] = v; s_key[ixj] = u; }
-                }
+    if (!large) {
+        int n2 = 32;                                        // keys padded to a power of two
+        while (n2 < m) n2 <<= 1;
+        for (int k = t; k < n2; k += kColThreads) {
+            unsigned long long key = ~0ull;
+            if (k < m) {
+                const int i = a.tmp[b + k];
+                key = ((unsigned long long)a.qfix[3 * i + 2] << 32) | (unsigned)i;
             }
-            __syncthreads();
+            s_key[k] = key;
         }
-    for (int k = t; k < m; k += kColThreads) s_ord[k] = (int)(s_key[k] & 0xffffffffull);
-    __syncthreads();                                        // the keys' space becomes the coordinates'
-    const size_t slot0 = 8 * (size_t)cl0;
+        __syncthreads();
+        for (int k = 2; k <= n2; k <<= 1)
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                for (int i = t; i < n2; i += kColThreads) {
+                    const int ixj = i ^ j;
+                    if (ixj > i) {
+                        const unsigned long long u = s_key[i], v = s_key[ixj];
+                        if (((i & k) == 0) ? (u > v) : (u < v)) { s_key[i] = v; s_key[ixj] = u; }
+                    }
+                }
+                __syncthreads();
+            }
+        for (int k = t; k < m; k += kColThreads) s_ord[k] = (int)(s_key[k] & 0xffffffffull);
+        __syncthreads();                                    // the keys' space becomes the coordinates'
+    }
     for (int r = t; r < 8 * ncl; r += kColThreads) {
         const bool valid = r < m;
-        const int i = s_ord[valid ? r : (r & ~7)];          // padding: the cluster's first atom's place
-        const double qi = a.q[i];
-        const float qh = valid ? (float)qi : 0.f;
-        const float ql = valid ? (float)(qi - (double)qh) : 0.f;
-        const unsigned fx = a.qfix[3 * i], fy = a.qfix[3 * i + 1], fz = a.qfix[3 * i + 2];
-        const int4 qv = make_int4((int)fx, (int)fy, (int)fz, __float_as_int(qh));
-        a.cq[slot0 + r] = qv;
-        a.cm[slot0 + r] = valid ? make_int4(i, a.type[i], a.mol[i], __float_as_int(ql)) : make_int4(-1, 0, -2, 0);
-        if (valid) {
-            a.slot_of[i] = (int)(slot0 + r);
-            s_qf[3 * r] = fx; s_qf[3 * r + 1] = fy; s_qf[3 * r + 2] = fz;
+        const int k = valid ? r : (r & ~7);                 // padding: the cluster's first atom's place
+        const int i = large ? a.tmp[b + k] : s_ord[k];
+        write_slot(a, i, valid, slot0 + r);
+        if (valid && !large) {
+            s_qf[3 * r] = a.qfix[3 * i]; s_qf[3 * r + 1] = a.qfix[3 * i + 1]; s_qf[3 * r + 2] = a.qfix[3 * i + 2];
         }
-        if ((r & 7) == 0) a.corg[cl0 + (r >> 3)] = make_int4(qv.x, qv.y, qv.z, 0);
     }
     __syncthreads();
     // boxes of the j-clusters (4 slots each, the halves of the i-clusters)
     // and of the i-clusters; an empty half gets a box beyond every window
+    // (the z order of the column's boxes stays monotone)
     const double kx = g.lx * (1.0 / 4294967296.0), ky = g.ly * (1.0 / 4294967296.0), kz = g.lz * (1.0 / 4294967296.0);
-    for (int q = t; q < 2 * ncl; q += kColThreads) {
-        const int r0 = 4 * q, r1 = min(m, r0 + 4);
-        // empty: lo.w = 1, both corners at +3e38 (the z order of the column's
-        // boxes stays monotone, and no window reaches it)
-        float4 lo = make_float4(3e38f, 3e38f, 3e38f, 1.f), hi = make_float4(3e38f, 3e38f, 3e38f, 0.f);
-        if (r0 < r1) { lo.w = 0.f; hi = make_float4(-3e38f, -3e38f, -3e38f, 0.f); }
-        for (int r = r0; r < r1; ++r) {
-            const float x = (float)(s_qf[3 * r] * kx), y = (float)(s_qf[3 * r + 1] * ky),
-                        z = (float)(s_qf[3 * r + 2] * kz);
-            lo.x = fminf(lo.x, x); lo.y = fminf(lo.y, y); lo.z = fminf(lo.z, z);
-            hi.x = fmaxf(hi.x, x); hi.y = fmaxf(hi.y, y); hi.z = fmaxf(hi.z, z);
-        }
-        const size_t jc = 2 * (size_t)cl0 + q;
-        a.jbox[2 * jc] = lo;
-        a.jbox[2 * jc + 1] = hi;
-        s_jb[2 * q] = lo;
-        s_jb[2 * q + 1] = hi;
-    }
-    __syncthreads();
     for (int q = t; q < ncl; q += kColThreads) {
-        const float4 l0 = s_jb[4 * q], h0 = s_jb[4 * q + 1];
-        const float4 l1 = s_jb[4 * q + 2], h1 = s_jb[4 * q + 3];
-        const bool e1 = l1.w != 0.f;                        // empty second half
-        a.ibox[2 * (cl0 + q)] = e1 ? l0 : make_float4(fminf(l0.x, l1.x), fminf(l0.y, l1.y), fminf(l0.z, l1.z), 0.f);
-        a.ibox[2 * (cl0 + q) + 1] = e1 ? h0 : make_float4(fmaxf(h0.x, h1.x), fmaxf(h0.y, h1.y), fmaxf(h0.z, h1.z), 0.f);
+        float4 ilo = make_float4(3e38f, 3e38f, 3e38f, 0.f), ihi = make_float4(-3e38f, -3e38f, -3e38f, 0.f);
+        for (int h = 0; h < 2; ++h) {
+            const int r0 = 8 * q + 4 * h, r1 = min(m, r0 + 4);
+            float4 lo = make_float4(3e38f, 3e38f, 3e38f, 0.f), hi = make_float4(-3e38f, -3e38f, -3e38f, 0.f);
+            for (int r = r0; r < r1; ++r) {
+                unsigned ux, uy, uz;
+                if (large) {
+                    const int i = a.tmp[b + r];
+                    ux = a.qfix[3 * i]; uy = a.qfix[3 * i + 1]; uz = a.qfix[3 * i + 2];
+                } else {
+                    ux = s_qf[3 * r]; uy = s_qf[3 * r + 1]; uz = s_qf[3 * r + 2];
+                }
+                const float x = (float)(ux * kx), y = (float)(uy * ky), z = (float)(uz * kz);
+                lo.x = fminf(lo.x, x); lo.y = fminf(lo.y, y); lo.z = fminf(lo.z, z);
+                hi.x = fmaxf(hi.x, x); hi.y = fmaxf(hi.y, y); hi.z = fmaxf(hi.z, z);
+            }
+            const bool empty = r0 >= r1;
+            const size_t jc = 2 * (size_t)(cl0 + q) + h;
+            a.jbox[2 * jc] = empty ? make_float4(0.f, 0.f, 3e38f, 0.f)
+                                   : make_float4(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z), 0.f);
+            a.jbox[2 * jc + 1] = empty ? make_float4(0.f, 0.f, 0.f, 1.f)
+                                       : make_float4(0.5f * (hi.x - lo.x), 0.5f * (hi.y - lo.y), 0.5f * (hi.z - lo.z), 0.f);
+            if (!large) s_jb[2 * q + h] = make_float4(empty ? 3e38f : lo.z, empty ? 3e38f : hi.z, 0.f, 0.f);
+            ilo.x = fminf(ilo.x, lo.x); ilo.y = fminf(ilo.y, lo.y); ilo.z = fminf(ilo.z, lo.z);
+            ihi.x = fmaxf(ihi.x, hi.x); ihi.y = fmaxf(ihi.y, hi.y); ihi.z = fmaxf(ihi.z, hi.z);
+        }
+        a.ibox[2 * (cl0 + q)] = make_float4(0.5f * (ilo.x + ihi.x), 0.5f * (ilo.y + ihi.y), 0.5f * (ilo.z + ihi.z), 0.f);
+        a.ibox[2 * (cl0 + q) + 1] = make_float4(0.5f * (ihi.x - ilo.x), 0.5f * (ihi.y - ilo.y), 0.5f * (ihi.z - ilo.z), 0.f);
         a.ccol[cl0 + q] = c;
     }
+    __syncthreads();
     // the column's z index for the list kernel's window searches: per bin
     // edge z_b = b L_z / kZBins the first j-cluster whose box ends at or
     // above z_b, and the first whose box starts above it (both corners are
     // monotone along the column; empty halves sit at +3e38, at the end)
     const float binw = g.lzf / kZBins;
     int* zi = a.zidx + (size_t)c * kZIndex;
-    for (int b = t; b <= kZBins; b += kColThreads) {
-        const float zb = b * binw;
+    if (large) {
+        if (t == 0) zi[0] = -1;
+        return;
+    }
+    for (int k = t; k <= kZBins; k += kColThreads) {
+        const float zb = k * binw;
         int lo = 0, hi = 2 * ncl;
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (s_jb[2 * mid + 1].z < zb) lo = mid + 1; else hi = mid;
+            if (s_jb[mid].y < zb) lo = mid + 1; else hi = mid;
         }
         int lo2 = 0, hi2 = 2 * ncl;
         while (lo2 < hi2) {
             const int mid = (lo2 + hi2) >> 1;
-            if (s_jb[2 * mid].z > zb) hi2 = mid; else lo2 = mid + 1;
+            if (s_jb[mid].x > zb) hi2 = mid; else lo2 = mid + 1;
         }
-        zi[b] = 2 * cl0 + lo;
-        zi[kZBins + 1 + b] = 2 * cl0 + lo2;
+        zi[k] = 2 * cl0 + lo;
+        zi[kZBins + 1 + k] = 2 * cl0 + lo2;
     }
 }
 
@@ -441,8 +472,8 @@ __global__ void __launch_bounds__(kBinThreads) k_col_refresh(ColBinArgs a, doubl
     const double uz = (double)(int)(qz - a.qfix[3 * i + 2]) * (g.lz * (1.0 / 4294967296.0));
     if (ux * ux + uy * uy + uz * uz > half_skin2) atomicOr(a.status, kStatusListStale);
     const int sl = a.slot_of[i];
-    const int4 old = a.cq[sl];
-    a.cq[sl] = make_int4((int)qx, (int)qy, (int)qz, old.w);
+    a.cq[sl] = make_int4((int)qx, (int)qy, (int)qz, a.cq[sl].w);
+    if (a.c64) a.c64[sl] = make_double4(x, y, z, a.q[i]);
 }
 
 }  // namespace

@@ -23,6 +23,7 @@ constexpr int kMaxDeltas = 1024;
 constexpr int kExclWindow = 32;        // exclusion bitmask window (index delta 1..32)
 constexpr double kScaleMixed = 4294967296.0;        // 2^32
 constexpr double kScaleFp64 = 1099511627776.0;      // 2^40
+constexpr double kScaleRowJ = 17592186044416.0;     // 2^44: the fine sums of the FP64 rows
 constexpr double kFixedLimit = 4.0e18;               // |value * scale| bound before int64 overflow
 
 // status bits written by kernels

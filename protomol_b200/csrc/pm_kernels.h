@@ -28,7 +28,8 @@ struct BinArgs {
     float4* spos;               // N: FP32 (hi) cell-relative x, y, z and charge
     float4* slo;                // N: FP32 remainders (lo) of the same four values
     int4* smeta;                // N
-    double4* spos64;            // N (raw FP64 position + charge) or null
+    double4* spos64;            // N (raw FP64 position + charge)
+    int4* sfix;                 // N (fixed-point position x / L 2^32 mod 2^32 per axis, molecule)
     int* skey;                  // N: Morton key of the cell-relative position
     int* cstart;                // ncell + 1: first cluster of each cell
     int* ccell;                 // cluster -> cell
@@ -56,7 +57,7 @@ struct ColGrid {
     float sx, sy;                // column side
     float lxf, lyf, lzf;         // box edges (FP32)
     float sch[3], scl[3];        // L / 2^32 per axis, FP32 hi + lo
-    float zext;                  // largest z extent of an i-cluster that keeps every tile's image unique
+    float zext;                  // largest z extent of an i-cluster of the mixed path (taller ones prune too little)
 };
 
 // z index of a column's j-clusters: kZBins bins of L_z / kZBins; per column
@@ -82,14 +83,15 @@ struct ColBinArgs {
     int* colstart;               // ncol + 1: first atom of each column (compact order)
     int* ccstart;                // ncol + 1: first i-cluster of each column
     int* tmp;                    // N
-    int4* cq;                    // slot: qx, qy, qz, charge (FP32 hi, as bits)
-    int4* cm;                    // slot: original index (-1: padding), type, molecule, charge (FP32 lo, as bits)
+    int4* cq;                    // slot: qx, qy, qz, molecule (-1: padding)
+    int4* cm;                    // slot: charge (FP32 hi, lo, as bits), type, original index (-1: padding)
+    double4* c64;                // slot: raw position and charge (FP64 row kernels), or null
     int* slot_of;                // N: slot of every atom
-    float4* ibox;                // 2 per i-cluster: lo, hi (A, box frame [0, L))
-    float4* jbox;                // 2 per j-cluster
+    float4* ibox;                // 2 per i-cluster: center, half extent (A, box frame [0, L))
+    float4* jbox;                // 2 per j-cluster (half extent .w = 1: empty)
     int* ccol;                   // i-cluster -> column
-    int4* corg;                  // i-cluster -> fixed-point position of its first atom (virial origin)
-    int* zidx;                   // kZIndex per column: the z index of its j-clusters
+    int* zidx;                   // kZIndex per column: the z index of its j-clusters (first int < 0: unsorted column)
+    int refuse;                  // a column of more atoms than the sort holds: 1 the system is refused, 0 left unsorted
     int ncl_cap;                 // i-cluster capacity
     int* status;
 };
@@ -153,6 +155,8 @@ struct PairArgs {
     const float4* slo;
     const int4* smeta;
     const double4* spos64;
+    const int4* sfix;            // fixed-point position, molecule
+    int rows_split;              // FP64 row kernels: shares a row is cut into
     const double* pos;           // raw positions, original order (exact rechecks)
     // exclusions (check() classes), window masks + CSR for larger deltas
     const uint32_t* xfull;
@@ -199,6 +203,7 @@ struct PairArgs {
     int virial;
     // outputs
     unsigned long long* facc;    // 3 per sorted slot
+    unsigned long long* faccj;   // FP64 rows over the columns: the fine sums (2^44), 3 per slot
     double scale;
     double* erec;                // energy records (component-major, see kERec)
     int erec_stride;
@@ -228,9 +233,12 @@ struct PairArgs {
     const int* zidx;             // kZIndex per column (ColBinArgs::zidx)
     const int* ccstart;          // ncol + 1
     const int* ccol;
-    const int4* corg;            // virial origin of every i-cluster
-    int4* clist;                 // column-path entries (the plist buffer): {jc | flags << 25, o.x, o.y, o.z};
-                                 // o = O_c(j) - O_c(i) + t L (FP32 bits), the tile's virial offset
+    const double4* c64;          // raw position and charge per slot
+    int* clist;                  // column-path entries (the plist buffer): j-clusters, a row's contiguous
+    int2* rowent;                // per row: first entry (< 0: not listed) and entries
+    int col_none;                // a j-cluster of padding atoms (the last row's, written by the binning)
+    int col_half;                // the list names every unordered pair once (mixed forces), or every ordered one
+    int col_refuse;              // 1: a list that does not fit (or a row too tall) is an error status (mixed forces)
     int icl_cap;                 // i-clusters the list kernel's grid covers
     ColGrid cg;
     const double* qorig;         // charges, types in atom order (FP64 near-pair energies)
@@ -264,11 +272,16 @@ int launch_pair_col_batch(const BatchPairArgs& b, int combo, cudaStream_t s, lon
 int launch_near_energy_col(const PairArgs& a, int combo, int n_atoms, cudaStream_t s, long long* launches);
 long long col_list_estimate(int n_atoms, const ColGrid& g, double volume, double cutoff);
 long long col_chunk_estimate(long long entries, int n_atoms, const ColGrid& g, int chunk);
-int launch_pair_fp64(const PairArgs& a, int combo, int blocks, cudaStream_t s, long long* launches);
+int col_chunk_entries(int n_atoms, const ColGrid& g, double volume, double cutoff, int most, bool half);
+int col_rows_split(int n_atoms, const ColGrid& g, double cutoff);
+int col_row_blocks(int n_atoms, const ColGrid& g, double cutoff);
+int launch_pair_fp64(const PairArgs& a, int combo, bool col, int blocks, cudaStream_t s, long long* launches);
 // the molecular virial records (kMRec) of a cutoff force over the cell-sorted
 // order, one per block (blocks as launch_pair_fp64), no forces or energies
-int launch_pair_molvir(const PairArgs& a, int combo, int blocks, cudaStream_t s, long long* launches);
-int pair_blocks(const CellGrid& g, int nd);
+int launch_pair_molvir(const PairArgs& a, int combo, bool col, int blocks, cudaStream_t s, long long* launches);
+// shares of a row and blocks of the FP64 row kernels (records: one per block)
+int rows_split(int n_atoms, const CellGrid& g, int nd);
+int pair_blocks(int n_atoms, const CellGrid& g, int nd);
 // blocks of the mixed kernel (4 warps, one energy record per warp)
 // estimated cluster-pair list entries and chunks of a system
 long long plist_estimate(int n_atoms, const CellGrid& g, int nh);
@@ -314,11 +327,15 @@ struct AdjArgs {
     int virial;
 };
 int launch_pair_adjoint(const AdjArgs& a, int fp64, cudaStream_t s, long long* launches);
-// the same backward pass for a cutoff force over the cell list (the cell
-// pairs and pair set of launch_pair_fp64; p holds the cell-sorted order):
+// the same backward pass for a cutoff force over the rows of the column list
+// (col) or the cell-sorted clusters, with the pair set of launch_pair_fp64:
 // dq, dlj, hv and energy of a (facc, hess and erec are not written)
-int launch_pair_adjoint_cells(const PairArgs& p, const AdjArgs& a, int fp64, int blocks, cudaStream_t s,
-                              long long* launches);
+int launch_pair_adjoint_rows(const PairArgs& p, const AdjArgs& a, int fp64, bool col, int blocks, cudaStream_t s,
+                             long long* launches);
+// the nonzero entries of an LJ-table gradient of n doubles (n < 2^31): idx and
+// val hold n, *count starts at zero
+int launch_lj_entries(const double* g, unsigned n, unsigned* idx, double* val, unsigned* count, cudaStream_t s,
+                      long long* launches);
 // records (blocks) of one launch_pair_adjoint
 int adjoint_blocks(int n);
 
@@ -452,14 +469,13 @@ struct FinArgs {
     const float4* spos;
     const float4* slo;
     int pair_virial;
-    // column-cluster pair forces (2^32) per slot, gathered through slot_of;
-    // their virial from the fixed-point positions (cq) times L / 2^32
+    // column-cluster pair forces per slot (mixed 2^32, FP64 2^40), gathered
+    // through slot_of
     const unsigned long long* c32;
+    const unsigned long long* c40;
+    const unsigned long long* c44;       // the FP64 rows' fine sums, 2^44
     const int* c_slot_of;
-    int c_slots;                         // slots of c32 / cq (an out-of-range slot_of adds nothing)
-    const int4* cq;
-    const int4* corg;                    // virial origin of each i-cluster (slot / 8)
-    double cscale[3];
+    int c_slots;                         // slots of c32 / c40 (an out-of-range slot_of adds nothing)
     double* fout;
     double* erec;
     int erec_stride;

@@ -1,0 +1,169 @@
+// pm_pair_col.cu -- K2' and K11: launches of the pair list and the
+// mixed-precision pair kernels over column clusters.
+#include "pm_pair_math.cuh"
+
+namespace pm {
+
+#include "pm_pair_mixed.cuh"
+#include "pm_pair_col.cuh"
+
+// ---------------------------------------------------------------- column path
+long long col_list_estimate(int n_atoms, const ColGrid& g, double volume, double cutoff)
+{
+    // the 4-atom j-clusters within the cutoff plus 1.5 column sides of each
+    // row, with 30% slack
+    const double rho = volume > 0.0 ? n_atoms / volume : 0.0;
+    const double r = cutoff + 1.5 * std::max(g.sx, g.sy);
+    const double rows = (double)n_atoms / kCluster + g.ncol + 1;
+    const double per = std::min(rho * (4.0 / 3.0) * 3.14159265358979 * r * r * r / 4.0, 2.0 * rows);
+    return (long long)(1.3 * rows * per) + 4096;
+}
+
+// Entries per chunk of the pair kernel: about four chunks for every resident
+// warp (148 SMs x 16), so that the last wave is short, but no more than
+// most (six tuned chunk units) or a block: every chunk ends with partly filled
+// rings.
+int col_chunk_entries(int n_atoms, const ColGrid& g, double volume, double cutoff, int most, bool half)
+{
+    const double rho = volume > 0.0 ? n_atoms / volume : 0.0;
+    const double r = cutoff + 0.75 * std::max(g.sx, g.sy);
+    const double rows = (double)n_atoms / kCluster + 0.5 * g.ncol + 1;
+    const double per = std::min(rho * (4.0 / 3.0) * 3.14159265358979 * r * r * r / 4.0, 2.0 * rows);
+    const double want = rows * per * (half ? 0.5 : 1.0) / (4.0 * 148 * 16);
+    return std::max(16, std::min(std::min(most, kColBlock), 2 * (int)(0.5 * std::min(want, 1e6) + 1.0)));
+}
+
+long long col_chunk_estimate(long long entries, int n_atoms, const ColGrid& g, int chunk)
+{
+    return entries / std::max(1, chunk) + (long long)n_atoms / kCluster + g.ncol + 1024;
+}
+
+int launch_col_list(const PairArgs& a, cudaStream_t s, long long* launches)
+{
+    const int blocks = std::max(1, (a.icl_cap + 3) / 4);    // one warp per i-cluster
+    launch_pdl(k_col_list, blocks, 128, 0, s, a);
+    *launches += 1;
+    return (int)cudaGetLastError();
+}
+
+template <int NT, int P0, int S0, int P1, int S1>
+static int run_col(const PairArgs& a, cudaStream_t s, long long* launches)
+{
+    static int sms = 0, per_sm = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_col<NT, P0, S0, P1, S1>, 128, 0);
+        if (sms <= 0) sms = 148;
+        if (per_sm <= 0) per_sm = 1;
+    }
+    const int bps = a.blocks_per_sm > 0 ? std::min(per_sm, a.blocks_per_sm) : per_sm;
+    launch_pdl(k_pair_col<NT, P0, S0, P1, S1>, sms * bps, 128, 0, s, a);
+    *launches += 1;
+    return (int)cudaGetLastError();
+}
+
+int launch_pair_col(const PairArgs& a, int combo, cudaStream_t s, long long* launches)
+{
+    switch (combo) {
+#define PM_COL_CASE(ID, ...) case ID: return run_col<__VA_ARGS__>(a, s, launches);
+    PM_COL_CASE(0, 1, CO, SC1, NP, SUN)
+    PM_COL_CASE(1, 1, CO, SC2, NP, SUN)
+    PM_COL_CASE(2, 1, CO, SCUT, NP, SUN)
+    PM_COL_CASE(3, 1, CO, SSH, NP, SUN)
+    PM_COL_CASE(4, 1, EW, SCUT, NP, SUN)
+    PM_COL_CASE(5, 1, LJ, SC1, NP, SUN)
+    PM_COL_CASE(6, 1, LJ, SC2, NP, SUN)
+    PM_COL_CASE(7, 1, LJ, SCUT, NP, SUN)
+    PM_COL_CASE(8, 1, LJ, SSH, NP, SUN)
+    PM_COL_CASE(9, 2, LJ, SC1, EW, SCUT)
+    PM_COL_CASE(10, 2, LJ, SC1, CO, SSH)
+    PM_COL_CASE(11, 2, LJ, SC2, CO, SC1)
+    PM_COL_CASE(12, 2, LJ, SC2, EW, SCUT)
+    PM_COL_CASE(13, 2, LJ, SC2, CO, SCUT)
+    PM_COL_CASE(14, 2, LJ, SC2, CO, SSH)
+    PM_COL_CASE(15, 2, LJ, SCUT, EW, SCUT)
+    PM_COL_CASE(16, 2, LJ, SC2, CO, SC2)
+    PM_COL_CASE(17, 1, LJT, SUN, NP, SUN)
+    PM_COL_CASE(18, 1, COT, SUN, NP, SUN)
+    PM_COL_CASE(19, 1, EWT, SUN, NP, SUN)
+    PM_COL_CASE(20, 2, LJ, SC1, EWT, SUN)
+    PM_COL_CASE(21, 2, LJ, SC2, EWT, SUN)
+    PM_COL_CASE(22, 2, LJ, SCUT, EWT, SUN)
+    PM_COL_CASE(23, 2, LJT, SUN, EWT, SUN)
+    PM_COL_CASE(24, 2, LJT, SUN, COT, SUN)
+#undef PM_COL_CASE
+    default: return (int)cudaErrorInvalidValue;
+    }
+}
+
+template <int NT, int P0, int S0, int P1, int S1>
+static int run_col_batch(const BatchPairArgs& b, cudaStream_t s, long long* launches)
+{
+    static int sms = 0, per_sm = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_col_batch<NT, P0, S0, P1, S1>, 128, 0);
+        if (sms <= 0) sms = 148;
+        if (per_sm <= 0) per_sm = 1;
+    }
+    k_pair_col_batch<NT, P0, S0, P1, S1><<<sms * per_sm, 128, 0, s>>>(b);
+    *launches += 1;
+    return (int)cudaGetLastError();
+}
+
+int launch_pair_col_batch(const BatchPairArgs& b, int combo, cudaStream_t s, long long* launches)
+{
+    if (b.n < 1 || b.n > kBatchPairMax) return (int)cudaErrorInvalidValue;
+    switch (combo) {
+#define PM_COLB_CASE(ID, ...) case ID: return run_col_batch<__VA_ARGS__>(b, s, launches);
+    PM_COLB_CASE(0, 1, CO, SC1, NP, SUN)
+    PM_COLB_CASE(1, 1, CO, SC2, NP, SUN)
+    PM_COLB_CASE(2, 1, CO, SCUT, NP, SUN)
+    PM_COLB_CASE(3, 1, CO, SSH, NP, SUN)
+    PM_COLB_CASE(4, 1, EW, SCUT, NP, SUN)
+    PM_COLB_CASE(5, 1, LJ, SC1, NP, SUN)
+    PM_COLB_CASE(6, 1, LJ, SC2, NP, SUN)
+    PM_COLB_CASE(7, 1, LJ, SCUT, NP, SUN)
+    PM_COLB_CASE(8, 1, LJ, SSH, NP, SUN)
+    PM_COLB_CASE(9, 2, LJ, SC1, EW, SCUT)
+    PM_COLB_CASE(10, 2, LJ, SC1, CO, SSH)
+    PM_COLB_CASE(11, 2, LJ, SC2, CO, SC1)
+    PM_COLB_CASE(12, 2, LJ, SC2, EW, SCUT)
+    PM_COLB_CASE(13, 2, LJ, SC2, CO, SCUT)
+    PM_COLB_CASE(14, 2, LJ, SC2, CO, SSH)
+    PM_COLB_CASE(15, 2, LJ, SCUT, EW, SCUT)
+    PM_COLB_CASE(16, 2, LJ, SC2, CO, SC2)
+    PM_COLB_CASE(17, 1, LJT, SUN, NP, SUN)
+    PM_COLB_CASE(18, 1, COT, SUN, NP, SUN)
+    PM_COLB_CASE(19, 1, EWT, SUN, NP, SUN)
+    PM_COLB_CASE(20, 2, LJ, SC1, EWT, SUN)
+    PM_COLB_CASE(21, 2, LJ, SC2, EWT, SUN)
+    PM_COLB_CASE(22, 2, LJ, SCUT, EWT, SUN)
+    PM_COLB_CASE(23, 2, LJT, SUN, EWT, SUN)
+    PM_COLB_CASE(24, 2, LJT, SUN, COT, SUN)
+#undef PM_COLB_CASE
+    default: return (int)cudaErrorInvalidValue;
+    }
+}
+
+int launch_near_energy_col(const PairArgs& a, int combo, int n_atoms, cudaStream_t s, long long* launches)
+{
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (sms <= 0) sms = 148;
+    }
+    long long want = (30LL * n_atoms + 127) / 128;
+    const int blocks = (int)std::max(1LL, std::min<long long>(want, 16LL * sms));
+    PM_COMBO_SWITCH(k_near_energy_col)
+    *launches += 1;
+    return (int)cudaGetLastError();
+}
+
+}  // namespace pm

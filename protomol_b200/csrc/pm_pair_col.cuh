@@ -1,6 +1,6 @@
-// pm_pair_col.cuh -- K2a' / K2b' / K2c': the mixed-precision pair force over
-// column clusters (included by pm_pair.cu after pm_pair_mixed.cuh, whose
-// helpers it shares).
+// pm_pair_col.cuh -- K2a' / K2b' / K2c', K9', K10', K11: the pair kernels over
+// column clusters (included after pm_pair_mixed.cuh, whose helpers the mixed
+// kernel shares).
 //
 // Layout (K1c, pm_cells.cu): every atom holds an unsigned 32-bit fixed-point
 // coordinate of the periodic box per axis, q = round(frac((x - min) / L) 2^32).
@@ -9,126 +9,135 @@
 // shared by the pairs of an atom or of a cell pair enters the pair vector.
 // The only roundings are the conversion of that integer to FP32 and its
 // product with the FP32 hi + lo of L / 2^32, both unbiased, so the FP32 pair
-// energies carry no systematic error into the sums (cell-relative FP32
-// coordinates with FP32 cell offsets lose the offsets' and the atoms' FP32
-// remainders in the last addition, a bias of ~1e-8 of every distance).
+// energies carry no systematic error into the sums.
 //
 // Clusters: the atoms of one column of an x-y grid (~4 A side), sorted by z,
-// cut into runs of 8 (i-clusters); each half of an i-cluster is a 4-atom
-// j-cluster.  A warp's tile is one i-cluster against one j-cluster: 8 x 4
-// pairs, one per lane (lane l: i-atom l % 8, j-atom l / 8).
+// cut into runs of 8; each run is a row (the i side), each half of it a 4-atom
+// j-cluster.
 //
-// K2a' k_col_list: one warp per i-cluster, one lane per candidate column of
-// the half neighbourhood.  A j-cluster is listed when its bounding box, in
-// the periodic image the column and the z window select, comes within the
-// cutoff (plus the FP32 guard band) of the i-cluster's box.  Every unordered
-// pair of atoms is visited once: a pair of columns from the one whose offset
-// to the other is in the positive half (ox > 0, or ox = 0 < oy), the own
-// column from the own cluster on, and in the own cluster (diag tiles) only
-// j > i.  The box edges are more
-// than (2 rx + 1) columns wide and the z windows shorter than the box, so no
-// j-cluster is reached twice, and every pair inside the cutoff lies in the
-// tile's image (t, the entry's shift), which the virial's shift form needs.
+// K2a' k_col_list: one warp per row lists the j-clusters whose bounding box
+// comes within the cutoff (plus the FP32 guard band) of the row's box by the
+// nearest image.  Boxes are center and half extent; the gap of the nearest
+// centers is a bound in any box.  Two forms: the full list (FP64 kernels: every
+// ordered pair of atoms once) and the half list (mixed kernel, molecular
+// virial: every unordered pair once).  In the half list a pair of columns
+// belongs to the one whose offset to the other is in the positive half plane
+// and, within a column, a pair of rows to the lower one; where the reach covers
+// the box (an offset is no longer unique) a pair of rows r < s belongs to r
+// when r + s is even, else to s.  The own row's clusters come with the sign bit
+// set: only j > i of them.
 //
-// K2b' k_pair_col: persistent warps over chunks of one i-cluster's entries,
-// two tiles per iteration.  i-forces stay in registers for the chunk;
-// j-forces are reduce-scattered over the 8 lanes of a j-atom and added in
-// int64 fixed point.  The exact FP64 decisions near a cutoff, the exclusion
-// classes, the near pairs' FP64 energies and the fixed-point sums are those
-// of K2b.
+// The pair kernels take chunks of one row's entries and alternate between two
+// phases (col_entries):
 //
-// Virial in the shift form, with each atom's position taken from its
-// i-cluster's origin O_c (the cluster's first atom), so that the lever arm
-// of the per-atom term is a cluster's size, not the box's:
-// sum_pairs d (x) f = sum_atoms (x - O_c(a)) (x) F + sum_tiles o (x) F_tile,
-// o = O_c(j) - O_c(i) + t L.  The finalize kernel adds the first sum from
-// the fixed-point positions and forces; the list kernel stores each tile's
-// o in FP32 (a rounding of the tile's own) and the pair kernel sums o (x)
-// F_tile in FP64.
+//   test   two entries (2 x 32 candidates) per step: lane l holds row atom
+//          l % 8 and candidate l / 8 of the cluster; distance in FP32, the
+//          exact FP64 decision inside a cutoff's guard band and the exclusion
+//          class of a pair of one molecule behind a warp vote.  Pairs inside
+//          the cutoff go to the row atom's ring in shared memory.
+//   pairs  the lanes of a row atom take the next pairs of its ring: the pair
+//          terms run on full warps.
+//
+// What bounds the mixed kernel: issue slots.  The pair terms are ~150 warp
+// instructions (LJ C2 + Ewald real) and 40% of an 8 x 4 tile's pairs lie inside
+// the cutoff; evaluated tile by tile they were two thirds of the kernel's 106 M
+// instructions on the 14,281-atom box.  The rings fill the lanes of the pair
+// phase (a tile's test is ~40 instructions).
+// Measured against the tile-by-tile kernel (each pair list's kernel alone): 106
+// -> 86 M instructions and 141 -> 139 us on the 14,281-atom box (894 atom types:
+// its Lennard-Jones table is an L2 gather, which neither form hides), 360 ->
+// 308 us for 61,233 atoms of water at 10 A, 8.10 -> 6.53 ms for 1,000,000 at
+// 12 A.  Tried: the full list with the rings and no j side (152 M
+// instructions, 217 us: the terms run twice); five blocks per SM (spills, 146
+// us); chunks twice and four times as long (within 1% from 61,233 atoms on,
+// 5% slower at 14,281).
 
-__device__ __forceinline__ int col_entry_y(int tx, int ty, int tz, bool diag)
+constexpr int kEnergyFlush = 8;          // pair-phase steps per FP32 partial sum
+constexpr int kColRing = 64;             // ring places per row atom
+constexpr int kColStageEntries = 1024;   // entries of one row staged in shared memory
+constexpr int kColBlock = 96;            // most entries of a chunk (and of a block of a longer row)
+constexpr int kColNear = 256;            // near pairs a warp queues for FP64 energies
+constexpr int kCodeSlot = (1 << 27) - 1; // ring code: j (a slot, or 4 x entry + atom of the chunk) | flags
+constexpr int kCodeIn0 = 1 << 28, kCodeIn1 = 1 << 29, kCodeMod = 1 << 30;
+
+// gap of two intervals (center distance d, half extents summed h) by the
+// nearest image
+__device__ __forceinline__ float image_gap(float d, float len, float inv, float h)
 {
-    return (tx + 1) | ((ty + 1) << 2) | ((tz + 1) << 4) | ((diag ? 1 : 0) << 6);
+    d = fmaf(-len, rintf(d * inv), d);
+    return fmaxf(0.f, fabsf(d) - h);
 }
 
-// the j-cluster range [jb, je) of column colj's image tz whose boxes may meet
-// the window [zlo, zhi] (in the box frame): j-boxes are sorted by z in a
-// column (both corners monotone), so the column's z index gives a start at
-// or before each end of the range, and a short forward scan finds it
-__device__ __forceinline__ int2 col_zrange(const PairArgs& p, int colj, int jb, int je, float zlo, float zhi,
-                                           float sz)
+// the j-clusters [lo, hi) of column c whose boxes may meet the z window
+// [zlo, zhi] (within [0, L)): j-boxes are sorted by z in a column (both corners
+// monotone), so the column's z index gives a start at or before each end of
+// the range, and a short forward scan finds it
+__device__ __forceinline__ int2 col_zrange(const PairArgs& p, const int* zi, int jb, int je, float zlo, float zhi)
 {
-    const float plo = zlo - sz, phi = zhi - sz;          // the window in the column's frame [0, L)
-    if (phi < 0.f || plo >= p.cg.lzf) return make_int2(jb, 0);
-    const int* zi = p.zidx + (size_t)colj * kZIndex;
     const float inv = kZBins / p.cg.lzf;
-    // first j-cluster ending at or above plo, from the bin edge one below
-    // plo's (the FP32 bin of plo may round up by one)
-    const int b0 = plo <= 0.f ? 0 : max(0, min(kZBins, (int)(plo * inv)) - 1);
+    // first j-cluster ending at or above zlo, from the bin edge one below
+    // zlo's (the FP32 bin of zlo may round up by one)
+    const int b0 = zlo <= 0.f ? 0 : max(0, min(kZBins, (int)(zlo * inv)) - 1);
     int lo = max(jb, __ldg(zi + b0));
-    while (lo < je && p.jbox[2 * lo + 1].z < plo) ++lo;
-    // first j-cluster starting above phi, likewise from one bin edge below
-    const int b1 = max(0, min(kZBins, (int)(phi * inv)) - 1);
-    int lo2 = max(lo, __ldg(zi + kZBins + 1 + b1));
-    while (lo2 < je && p.jbox[2 * lo2].z <= phi) ++lo2;
-    return make_int2(lo, lo2 - lo);
+    while (lo < je && p.jbox[2 * lo].z + p.jbox[2 * lo + 1].z < zlo) ++lo;
+    // first j-cluster starting above zhi, likewise from one bin edge below
+    const int b1 = max(0, min(kZBins, (int)(zhi * inv)) - 1);
+    int hi = max(lo, __ldg(zi + kZBins + 1 + b1));
+    while (hi < je && p.jbox[2 * hi].z - p.jbox[2 * hi + 1].z <= zhi) ++hi;
+    return make_int2(lo, hi);
 }
 
-constexpr int kColStageEntries = 512;    // entries of one i-cluster staged in shared memory
-constexpr int kEnergyFlush = 8;          // pair-kernel iterations per FP32 energy partial sum
-
-// The list of i-cluster ic (one warp): every candidate column of the half
-// neighbourhood -- the column offsets (ox, oy) with ox > 0 or ox = 0 < oy,
-// and the own column from the own cluster on -- in rounds of 32, one lane per
-// column (x-y gap, z window, the j-cluster ranges of its z images), then the
-// round's j-clusters flattened over the lanes for the box tests.  Entries
-// are written in a fixed order to out[0 .. cap); returns how many there are
-// (also when more than cap).
-__device__ int col_gather(const PairArgs& p, int ic, int col_i, const float4& ilo, const float4& ihi,
-                          const int4& Oi, float lim, int4* out, int cap, int4 (*s_part)[3], int* s_pre)
+// The list of one row (one warp): the columns around its own (all of them
+// where the reach covers the box), in rounds of 32, one lane per column (x-y
+// gap, z window, at most two ranges of j-clusters), then the round's j-clusters
+// flattened over the lanes for the box tests.  Entries (j-clusters) are
+// written in a fixed order to out[0 .. cap); returns how many there are (also
+// when more than cap).
+static __device__ int col_gather(const PairArgs& p, int row, int col_i, const float4& ic, const float4& ih, float lim, int* out, int cap,
+                          int4* s_part, int* s_pre)
 {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const ColGrid& g = p.cg;
-    const double ux = g.lx * (1.0 / 4294967296.0), uy = g.ly * (1.0 / 4294967296.0), uz = g.lz * (1.0 / 4294967296.0);
-    const int nyo = 2 * g.ry + 1;
-    const int ncand = (g.rx + 1) * nyo;                  // ox = 0 .. rx
-    const int cxi = col_i / g.ncy, cyi = col_i % g.ncy;
+    const float ilx = 1.0f / g.lxf, ily = 1.0f / g.lyf, ilz = 1.0f / g.lzf;
+    const int nxo = min(2 * g.rx + 1, g.ncx), nyo = min(2 * g.ry + 1, g.ncy);
+    const int ncand = nxo * nyo;
+    const bool half = p.col_half, plane = half && nxo == 2 * g.rx + 1 && nyo == 2 * g.ry + 1;
+    const int cxi = col_i / g.ncy, cyi = col_i - cxi * g.ncy;
     int ne = 0;
     for (int k0 = 0; k0 < ncand; k0 += 32) {
         const int k = k0 + lane;
-        int cnt = 0;
-        int4 part[3];
-#pragma unroll
-        for (int z = 0; z < 3; ++z) part[z] = make_int4(0, 0, 0, 0);
-        const int ox = k / nyo, oy = k % nyo - g.ry;
-        if (k < ncand && (ox > 0 || oy >= 0)) {
-            int jx = cxi + ox, jy = cyi + oy, tx = 0, ty = 0;
-            if (jx >= g.ncx) { jx -= g.ncx; tx = 1; }
-            if (jy < 0) { jy += g.ncy; ty = -1; } else if (jy >= g.ncy) { jy -= g.ncy; ty = 1; }
-            const int colj = jx * g.ncy + jy;
-            const float sx = tx * g.lxf, sy = ty * g.lyf;
-            const float x0 = jx * g.sx + sx, y0 = jy * g.sy + sy;
-            const float gx = fmaxf(0.f, fmaxf(x0 - ihi.x, ilo.x - (x0 + g.sx)));
-            const float gy = fmaxf(0.f, fmaxf(y0 - ihi.y, ilo.y - (y0 + g.sy)));
+        int4 part = make_int4(0, 0, 0, 0);            // {first, count} of up to two ranges
+        if (k < ncand) {
+            const int ox = k / nyo - nxo / 2, oy = k % nyo - nyo / 2;
+            const bool other = ox < 0 || (ox == 0 && oy < 0);     // the other column's, in the half plane rule
+            int jx = cxi + ox, jy = cyi + oy;
+            jx += jx < 0 ? g.ncx : 0; jx -= jx >= g.ncx ? g.ncx : 0;
+            jy += jy < 0 ? g.ncy : 0; jy -= jy >= g.ncy ? g.ncy : 0;
+            const int c = jx * g.ncy + jy;
+            const float gx = image_gap((jx + 0.5f) * g.sx - ic.x, g.lxf, ilx, 0.5f * g.sx + ih.x);
+            const float gy = image_gap((jy + 0.5f) * g.sy - ic.y, g.lyf, ily, 0.5f * g.sy + ih.y);
             const float rem = lim - (gx * gx + gy * gy);
-            if (rem >= 0.f) {
-                const float wz = sqrtf(rem);
-                const bool own = ox == 0 && oy == 0;
-                const int jb = own ? 2 * ic : 2 * p.ccstart[colj];
-                const int je = 2 * p.ccstart[colj + 1];
-#pragma unroll
-                for (int z = 0; z < 3; ++z) {
-                    const int tz = z - 1;
-                    const int2 r = col_zrange(p, colj, jb, je, ilo.z - wz, ihi.z + wz, tz * g.lzf);
-                    part[z] = make_int4(r.x, r.y, col_entry_y(tx, ty, tz, false) | (own ? 1 << 7 : 0), 0);
-                    cnt += r.y;
+            const int jb = 2 * (plane && c == col_i ? row : p.ccstart[c]), je = 2 * p.ccstart[c + 1];
+            if (rem >= 0.f && je > jb && !(plane && other)) {
+                const int* zi = p.zidx + (size_t)c * kZIndex;
+                const float w = sqrtf(rem) + ih.z + 1e-3f;
+                const float lo = ic.z - w, hi = ic.z + w;
+                if (__ldg(zi) < 0 || 2.f * w >= g.lzf) {          // an unsorted column, or a window as high as the box
+                    part = make_int4(jb, je - jb, 0, 0);
+                } else if (lo < 0.f || hi > g.lzf) {              // the window wraps: its low part, then its high one
+                    const int2 a = col_zrange(p, zi, jb, je, 0.f, lo < 0.f ? hi : hi - g.lzf);
+                    const int2 b = col_zrange(p, zi, jb, je, lo < 0.f ? lo + g.lzf : lo, g.lzf);
+                    const int b0 = max(b.x, a.y);                 // no cluster twice
+                    part = make_int4(a.x, a.y - a.x, b0, max(0, b.y - b0));
+                } else {
+                    const int2 a = col_zrange(p, zi, jb, je, lo, hi);
+                    part = make_int4(a.x, a.y - a.x, 0, 0);
                 }
             }
         }
-#pragma unroll
-        for (int z = 0; z < 3; ++z) s_part[lane][z] = part[z];
-        int incl = cnt;
+        int incl = part.y + part.w;
+        s_part[lane] = part;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int v = __shfl_up_sync(FULL, incl, o);
@@ -141,43 +150,28 @@ __device__ int col_gather(const PairArgs& p, int ic, int col_i, const float4& il
         for (int f0 = 0; f0 < total; f0 += 32) {
             const int f = f0 + lane;
             bool take = false;
-            int4 ent = make_int4(0, 0, 0, 0);
+            int jc = 0;
             if (f < total) {
-                int lo = 0, hi = 32;                      // owner lane: s_pre[o] <= f < s_pre[o + 1]
+                int lo = 0, hi = 32;                      // owner lane: s_pre[lo] <= f < s_pre[lo + 1]
                 while (hi - lo > 1) {
                     const int mid = (lo + hi) >> 1;
                     if (s_pre[mid] <= f) lo = mid; else hi = mid;
                 }
-                int u = f - s_pre[lo];
-                int4 pt = s_part[lo][0];
-                if (u >= pt.y) { u -= pt.y; pt = s_part[lo][1]; if (u >= pt.y) { u -= pt.y; pt = s_part[lo][2]; } }
-                const int jc = pt.x + u;
-                const int fl = pt.z & 0x3f;
-                const float sx = ((fl & 3) - 1) * g.lxf, sy = (((fl >> 2) & 3) - 1) * g.lyf,
-                            sz = (((fl >> 4) & 3) - 1) * g.lzf;
-                const float4 jl = p.jbox[2 * jc], jh = p.jbox[2 * jc + 1];
-                const float bx = fmaxf(0.f, fmaxf((jl.x + sx) - ihi.x, ilo.x - (jh.x + sx)));
-                const float by = fmaxf(0.f, fmaxf((jl.y + sy) - ihi.y, ilo.y - (jh.y + sy)));
-                const float bz = fmaxf(0.f, fmaxf((jl.z + sz) - ihi.z, ilo.z - (jh.z + sz)));
-                take = bx * bx + by * by + bz * bz <= lim;
-                if (take) {
-                    // the tile's virial offset O_c(j) - O_c(i) + t L, exact in
-                    // fixed point, then FP32 (a rounding of its own per tile)
-                    const bool diag = (pt.z >> 7) && (jc >> 1) == ic;
-                    const int4 Oj = p.corg[jc >> 1];
-                    const long long qx = (long long)(unsigned)Oj.x - (long long)(unsigned)Oi.x +
-                                         (long long)((fl & 3) - 1) * 4294967296LL;
-                    const long long qy = (long long)(unsigned)Oj.y - (long long)(unsigned)Oi.y +
-                                         (long long)(((fl >> 2) & 3) - 1) * 4294967296LL;
-                    const long long qz = (long long)(unsigned)Oj.z - (long long)(unsigned)Oi.z +
-                                         (long long)(((fl >> 4) & 3) - 1) * 4294967296LL;
-                    ent = make_int4(jc | ((fl | (diag ? 1 << 6 : 0)) << 25), __float_as_int((float)((double)qx * ux)),
-                                    __float_as_int((float)((double)qy * uy)), __float_as_int((float)((double)qz * uz)));
-                }
+                const int u = f - s_pre[lo];
+                const int4 pt = s_part[lo];
+                jc = u < pt.y ? pt.x + u : pt.z + (u - pt.y);
+                const float4 bc = __ldg(p.jbox + 2 * jc), bh = __ldg(p.jbox + 2 * jc + 1);
+                const float bx = image_gap(bc.x - ic.x, g.lxf, ilx, bh.x + ih.x);
+                const float by = image_gap(bc.y - ic.y, g.lyf, ily, bh.y + ih.y);
+                const float bz = image_gap(bc.z - ic.z, g.lzf, ilz, bh.z + ih.z);
+                take = bh.w == 0.f && bx * bx + by * by + bz * bz <= lim;
+                const int rj = jc >> 1;
+                if (half && !plane && rj != row) take = take && (((row + rj) & 1) == 0) == (row < rj);
+                if (half && rj == row) jc |= 1 << 31;
             }
             const unsigned b = __ballot_sync(FULL, take);
             const int at = ne + __popc(b & ((1u << lane) - 1u));
-            if (take && at < cap) out[at] = ent;
+            if (take && at < cap) out[at] = jc;
             ne += __popc(b);
         }
         __syncwarp();                                     // s_part / s_pre are rewritten next round
@@ -185,353 +179,511 @@ __device__ int col_gather(const PairArgs& p, int ic, int col_i, const float4& il
     return ne;
 }
 
-__global__ void __launch_bounds__(128) k_col_list(PairArgs p)
+// box distance^2 within which a j-cluster is listed; a reused list holds the
+// pairs within the cutoff plus the skin
+__device__ __forceinline__ float col_list_lim(const PairArgs& p)
+{
+    const float rl = sqrtf(p.cut2f) + p.list_skin;
+    return rl * rl * (1.0f + 8.0f * p.guard) + 1e-3f;
+}
+
+static __global__ void __launch_bounds__(128) k_col_list(const __grid_constant__ PairArgs p)
 {
     pdl_wait();
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __shared__ int4 s_ent[4][kColStageEntries];
-    __shared__ int4 s_part[4][32][3];                    // per lane and z image: {first j, count, flags, 0}
+    __shared__ int s_ent[4][kColStageEntries];
+    __shared__ int4 s_part[4][32];
     __shared__ int s_pre[4][33];
-    const int ic = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-    if (ic >= p.icl_cap) return;                                 // warp-uniform
+    const int row = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
+    if (row >= p.icl_cap) return;                                // warp-uniform
     // a refused system leaves a mark in the list's need count, which a
     // reused list keeps (the status word starts at zero every evaluation)
     if (*p.status & kStatusColumns) {
-        if (ic == 0 && lane == 0) atomicMax(p.plist_need, 1);
+        if (row == 0 && lane == 0) atomicMax(p.plist_need, 1);
         return;
     }
     const ColGrid& g = p.cg;
-    if (ic >= p.ccstart[g.ncol]) return;
-    const int col_i = p.ccol[ic];
-    const float4 ilo = p.ibox[2 * ic], ihi = p.ibox[2 * ic + 1];
-    if (ihi.z - ilo.z > g.zext) {                                // a tile's image could be ambiguous
+    if (row >= p.ccstart[g.ncol]) return;
+    const float4 ic = p.ibox[2 * row], ih = p.ibox[2 * row + 1];
+    if (p.col_refuse && 2.f * ih.z > g.zext) {                   // too tall to prune by: the cell layout
         if (lane == 0) { atomicOr(p.status, kStatusColumns); atomicMax(p.plist_need, 1); }
         return;
     }
-    const int4 Oi = p.corg[ic];
-    // a reused list holds the pairs within the cutoff plus the skin
-    const float rl = sqrtf(p.cut2f) + p.list_skin;
-    const float lim = rl * rl * (1.0f + 8.0f * p.guard) + 1e-3f;
-    const int ne = col_gather(p, ic, col_i, ilo, ihi, Oi, lim, s_ent[w], kColStageEntries, s_part[w], s_pre[w]);
-    if (ne == 0) return;
-    const int nch = (ne + p.chunk - 1) / p.chunk;
+    const float lim = col_list_lim(p);
+    const int col_i = p.ccol[row];
+    const int ne = col_gather(p, row, col_i, ic, ih, lim, s_ent[w], kColStageEntries, s_part[w], s_pre[w]);
+    if (ne == 0) {                                               // not even its own cluster: cannot be
+        if (lane == 0) p.rowent[row] = make_int2(0, 0);
+        return;
+    }
+    // equal chunks of a row, an even number of entries each
+    const int nch = (ne + p.chunk - 1) / p.chunk, per = ((ne + nch - 1) / nch + 1) & ~1;
     int b0 = 0, b1 = 0;
     if (lane == 0) {
-        // the entries take two int2 places each of the list buffer (plist_cap
-        // and plist_need count int2)
         b0 = atomicAdd(p.plist_count, ne);
         b1 = atomicAdd(p.chunk_count, nch);
-        if (2 * (b0 + ne) > p.plist_cap) { atomicOr(p.status, kStatusListFull); atomicMax(p.plist_need, 2 * (b0 + ne)); }
-        if (b1 + nch > p.chunk_cap) { atomicOr(p.status, kStatusListFull); atomicMax(p.chunk_need, b1 + nch); }
+        // the FP64 kernels take a row that did not fit without its entries
+        const bool full = b0 > p.plist_cap - ne || b1 > p.chunk_cap - nch;
+        p.rowent[row] = full ? make_int2(-1, 0) : make_int2(b0, ne);
+        if (full && p.col_refuse) {
+            atomicOr(p.status, kStatusListFull);
+            // the list buffer is counted in int2: two entries each
+            if (b0 > p.plist_cap - ne) atomicMax(p.plist_need, (b0 + ne) / 2 + 1);
+            if (b1 > p.chunk_cap - nch) atomicMax(p.chunk_need, b1 + nch);
+        }
     }
     const int ebase = __shfl_sync(FULL, b0, 0), cbase = __shfl_sync(FULL, b1, 0);
-    if (2 * (ebase + ne) > p.plist_cap || cbase + nch > p.chunk_cap) return;   // warp-uniform
+    if (ebase > p.plist_cap - ne || cbase > p.chunk_cap - nch) return;         // warp-uniform
     if (ne <= kColStageEntries) {
         for (int t = lane; t < ne; t += 32) p.clist[ebase + t] = s_ent[w][t];
     } else {                                              // more than the staging holds: list again, into place
-        col_gather(p, ic, col_i, ilo, ihi, Oi, lim, p.clist + ebase, ne, s_part[w], s_pre[w]);
+        col_gather(p, row, col_i, ic, ih, lim, p.clist + ebase, ne, s_part[w], s_pre[w]);
     }
     for (int t = lane; t < nch; t += 32)
-        p.chunks[cbase + t] = make_int4(ic, 0, ebase + t * p.chunk, min(p.chunk, ne - t * p.chunk));
+        p.chunks[cbase + t] = make_int4(row, 0, ebase + t * per, max(0, min(per, ne - t * per)));
 }
 
-// geometry and the FP32 within-cutoff decision of one pair of the 8 x 4 tile
-template <int NT, int S0, int S1>
-__device__ __forceinline__ PairGeo col_geo(const PairArgs& p, const int4& pi, const int4& pj, bool valid,
-                                           int mol_i, int mol_j)
-{
-    PairGeo g;
-    const float g_lo = 1.0f - p.guard, g_hi = 1.0f + p.guard;
-    const float t0c2 = p.tf[0].cut2, t1c2 = NT > 1 ? p.tf[1].cut2 : 0.f;
-    // minimal image in fixed point, exact; one rounding to FP32, then the
-    // compensated unit L / 2^32
-    const float qx = (float)(int)((unsigned)pj.x - (unsigned)pi.x);
-    const float qy = (float)(int)((unsigned)pj.y - (unsigned)pi.y);
-    const float qz = (float)(int)((unsigned)pj.z - (unsigned)pi.z);
-    const float dx = fmaf(qx, p.cg.sch[0], qx * p.cg.scl[0]);
-    const float dy = fmaf(qy, p.cg.sch[1], qy * p.cg.scl[1]);
-    const float dz = fmaf(qz, p.cg.sch[2], qz * p.cg.scl[2]);
-    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-    const bool far = r2 > p.cut2f * g_hi;
-    bool near = !far && r2 >= p.cut2f * g_lo;
-    if (S0 == SCUT && t0c2 != p.cut2f) near |= (r2 >= t0c2 * g_lo && r2 <= t0c2 * g_hi);
-    if (NT > 1 && S1 == SCUT && t1c2 != p.cut2f) near |= (r2 >= t1c2 * g_lo && r2 <= t1c2 * g_hi);
-    g.near = near && valid;
-    g.in0 = r2 <= t0c2;
-    g.in1 = NT > 1 ? r2 <= t1c2 : false;
-    g.act = valid && !far;
-    g.same = mol_i == mol_j;
-    g.excl = PMGPU_EXCL_NONE;
-    g.dx = dx; g.dy = dy; g.dz = dz; g.r2 = r2;
-    return g;
-}
-
-// the tile of one list entry, decoded, with its j-atom for this lane
-struct ColTile {
-    int jc;                      // j-cluster
-    bool diag;
-    float ox, oy, oz;            // virial offset
-    int4 P, M;                   // j-atom: fixed-point position + charge hi; original index, type, molecule, charge lo
+// ---------------------------------------------------------------- rows
+// The test phase's cutoffs: pairs up to far2 are looked at, from band2 on (and
+// around the smaller of two cutoffs) their decisions are taken in FP64
+struct ColTest {
+    float sx, sy, sz;            // L / 2^32
+    float far2, band2;
+    float c0, c1;                // the terms' own cutoffs^2
+    float g_lo, g_hi;
+    bool two;                    // they differ
 };
 
-// the tile of entry c (has: the entry exists), with its j-atom for lane jj
-__device__ __forceinline__ void col_tile_of(const PairArgs& p, const int4& c, bool has, int jj, ColTile& t)
+__device__ __forceinline__ ColTest col_test(const PairArgs& p)
 {
-    t.jc = c.x & 0x1ffffff;
-    t.diag = has && (((unsigned)c.x >> 31) & 1u);
-    t.ox = __int_as_float(c.y); t.oy = __int_as_float(c.z); t.oz = __int_as_float(c.w);
-    if (has) {                                   // read-only during the pair kernel
-        t.P = __ldg(p.cq + 4 * (size_t)t.jc + jj);
-        t.M = __ldg(p.cm + 4 * (size_t)t.jc + jj);
-    } else {
-        t.P = make_int4(0, 0, 0, 0);
-        t.M = make_int4(-1, 0, -2, 0);
+    ColTest t;
+    t.sx = p.cg.sch[0]; t.sy = p.cg.sch[1]; t.sz = p.cg.sch[2];
+    t.g_lo = 1.0f - p.guard; t.g_hi = 1.0f + p.guard;
+    t.far2 = p.cut2f * t.g_hi;
+    t.band2 = p.cut2f * t.g_lo;
+    t.c0 = p.tf[0].cut2;
+    t.c1 = p.n_terms > 1 ? p.tf[1].cut2 : p.tf[0].cut2;
+    t.two = t.c0 != t.c1;
+    return t;
+}
+
+// A row's atom of the calling lane and its ring
+struct ColRow {
+    int si;                      // slot
+    int4 P;                      // fixed-point position, molecule
+    bool vi;
+    float far2;                  // the test's limit (below zero for a padding atom)
+    int head, tail;              // places of its ring taken / filled (the same in its four lanes)
+};
+
+// the exact decisions of one candidate (cutoff in the guard band, exclusion
+// class within a molecule, j > i in the own row of a half list); code keeps
+// the flags of a pair inside
+template <bool DIFFMOL, bool TWO>
+__device__ __forceinline__ void col_resolve(const PairArgs& p, const ColTest& t, int si, int j, bool own, float r2,
+                                            bool same, bool& in, int& code)
+{
+    if (!in) return;
+    if (own ? j <= si : j == si) { in = false; return; }
+    const int oi = p.cm[si].w, oj = p.cm[j].w;
+    bool band = r2 >= t.band2;
+    if (TWO && t.two) band |= r2 >= fminf(t.c0, t.c1) * t.g_lo && r2 <= fminf(t.c0, t.c1) * t.g_hi;
+    if (band) {
+        const double d2 = exact_d2(p, oi, oj);
+        if (d2 > p.cut2d) { in = false; return; }
+        if (TWO) {
+            code &= ~(kCodeIn0 | kCodeIn1);
+            if (!(d2 > p.td[0].cut2)) code |= kCodeIn0;
+            if (!(d2 > p.td[1].cut2)) code |= kCodeIn1;
+        }
+    }
+    if (same) {
+        if (DIFFMOL) { in = false; return; }
+        const int x = excl_class(p, oi, oj);
+        if (x == PMGPU_EXCL_FULL) in = false;
+        if (x == PMGPU_EXCL_MODIFIED) code |= kCodeMod;
     }
 }
 
-template <bool SH>
-__device__ __forceinline__ int4 col_entry(const int4* ents, int e, int e_end)
-{
-    if (e >= e_end) return make_int4(0, 0, 0, 0);
-    return SH ? ents[e] : __ldg(ents + e);
-}
-
-__device__ __forceinline__ JAtom col_atom(const int4& P, const int4& M)
-{
-    JAtom a;
-    a.p = make_float4(0.f, 0.f, 0.f, __int_as_float(P.w));
-    a.l = make_float4(0.f, 0.f, 0.f, __int_as_float(M.w));
-    a.m = make_int4(M.x, M.y, M.z, 0);
-    return a;
-}
-
-// One i-cluster's run of list entries [e_begin, e_end) of ents (the global
-// list, or entries in shared memory: SH), two tiles per iteration: the tile
-// loop of K2b'.  Adds the j-forces and, at the end, the i-forces; queues the
-// near pairs (flushed at the end) and adds the run's energies and tile virial
-// to the lane's int64 sums acc.
-template <bool SH, int NT, int P0, int S0, int P1, int S1>
-__device__ __forceinline__ void col_run(const PairArgs& p, int ic, const int4* ents, int e_begin, int e_end,
-                                        int2* s_near, long long (&acc)[5], bool& bad)
+// One block of up to kColBlock entries of a row, in shared memory and followed
+// by three empty ones (p.col_none, a cluster of padding atoms): tested two at
+// a time; op.drain runs when a ring may overflow, and to the end after the
+// last block of a chunk (last).  There is one copy of it in the loop: the pair
+// phase is most of the kernel's code, and a second copy (or an unrolled loop)
+// did not fit the instruction cache (271 us against 150 on the 14,281-atom box,
+// 8.6 of 12.8 stall cycles per instruction waiting for instructions).
+// Op::kLocal: ring codes name the entry and its atom, not the slot.
+template <bool DIFFMOL, bool TWO, class Op>
+__device__ __forceinline__ void col_entries(const PairArgs& p, const ColTest& t, ColRow& r, int* ring, const int* ent,
+                                            int n, bool last, Op& op)
 {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, il = lane & 7, jj = lane >> 3;
-    // after the reduce-scatter lane il (< 6) holds component il % 3 of the
-    // j-force of tile A's (il < 3) or tile B's (il >= 3) j-atom jj
-    const bool holds = il < 6, onB = il >= 3;
-    const int comp = il < 3 ? il : il - 3;
-    const int si = 8 * ic + il;
-    const int4 Pi = p.cq[si], Mi = p.cm[si];
-    const JAtom ia = col_atom(Pi, Mi);
-    const bool vi = Mi.x >= 0;
-    float fix = 0.f, fiy = 0.f, fiz = 0.f;
-    double el = 0.0, ec = 0.0;
-    // the far pairs' FP32 energies summed over up to kEnergyFlush
-    // iterations in FP32, then into the FP64 sums
-    float elf = 0.f, ecf = 0.f;
-    int nacc = 0;
-    double wv[3] = {0.0, 0.0, 0.0};
-    int nq = 0;
-    // software pipeline: the entries two iterations ahead, the j-atoms of
-    // the next iteration's tiles one ahead
-    ColTile nA, nB;
-    col_tile_of(p, col_entry<SH>(ents, e_begin, e_end), true, jj, nA);
-    col_tile_of(p, col_entry<SH>(ents, e_begin + 1, e_end), e_begin + 1 < e_end, jj, nB);
-    int4 qA = col_entry<SH>(ents, e_begin + 2, e_end), qB = col_entry<SH>(ents, e_begin + 3, e_end);
-    for (int e = e_begin; e < e_end; e += 2) {
-        if (nq > kNearCap - 64) {                  // room for one more pair of tiles
-            append_near(p, s_near, nq, lane);
-            nq = 0;
+    const unsigned below = (1u << (8 * jj)) - 1u;
+    const int4* base = p.cq + jj;
+    int2 e = *reinterpret_cast<const int2*>(ent);
+    int4 A = __ldg(base + 4 * (size_t)(e.x & 0x7fffffff)), B = __ldg(base + 4 * (size_t)(e.y & 0x7fffffff));
+    int* const mine = ring + il;
+    for (int k = 0;; k += 2) {
+        const bool done = k >= n;
+        if ((done && last) || __any_sync(FULL, r.tail - r.head > kColRing - 8)) {
+            __syncwarp();
+            op.drain(r, ring, done && last ? 0 : Op::kKeep);
+            __syncwarp();
         }
-        const ColTile tA = nA, tB = nB;
-        const bool hasB = e + 1 < e_end;           // warp-uniform
-        if (e + 2 < e_end) {
-            col_tile_of(p, qA, true, jj, nA);
-            col_tile_of(p, qB, e + 3 < e_end, jj, nB);
-            qA = col_entry<SH>(ents, e + 4, e_end);
-            qB = col_entry<SH>(ents, e + 5, e_end);
+        if (done) break;
+        // the next two, while these are tested
+        const int2 en = *reinterpret_cast<const int2*>(ent + k + 2);
+        const int4 nA = __ldg(base + 4 * (size_t)(en.x & 0x7fffffff)), nB = __ldg(base + 4 * (size_t)(en.y & 0x7fffffff));
+        const float ax = (float)(int)((unsigned)A.x - (unsigned)r.P.x) * t.sx;
+        const float ay = (float)(int)((unsigned)A.y - (unsigned)r.P.y) * t.sy;
+        const float az = (float)(int)((unsigned)A.z - (unsigned)r.P.z) * t.sz;
+        const float bx = (float)(int)((unsigned)B.x - (unsigned)r.P.x) * t.sx;
+        const float by = (float)(int)((unsigned)B.y - (unsigned)r.P.y) * t.sy;
+        const float bz = (float)(int)((unsigned)B.z - (unsigned)r.P.z) * t.sz;
+        const float ra = fmaf(az, az, fmaf(ay, ay, ax * ax));
+        const float rb = fmaf(bz, bz, fmaf(by, by, bx * bx));
+        bool inA = (A.w >= 0) & (ra <= r.far2);
+        bool inB = (B.w >= 0) & (rb <= r.far2);
+        const bool sameA = A.w == r.P.w, sameB = B.w == r.P.w;
+        int codeA = Op::kLocal ? 4 * k + jj : 4 * (e.x & 0x7fffffff) + jj;
+        int codeB = Op::kLocal ? 4 * k + jj + 4 : 4 * (e.y & 0x7fffffff) + jj;
+        bool rare = (inA & (sameA | (ra >= t.band2))) | (inB & (sameB | (rb >= t.band2))) | ((e.x | e.y) < 0);
+        if (TWO && t.two) {                           // two cutoffs: which terms the pair is inside of
+            codeA |= (ra <= t.c0 ? kCodeIn0 : 0) | (ra <= t.c1 ? kCodeIn1 : 0);
+            codeB |= (rb <= t.c0 ? kCodeIn0 : 0) | (rb <= t.c1 ? kCodeIn1 : 0);
+            const float lo = fminf(t.c0, t.c1);
+            rare |= (ra >= lo * t.g_lo && ra <= lo * t.g_hi) || (rb >= lo * t.g_lo && rb <= lo * t.g_hi);
         }
-        const JAtom ja = col_atom(tA.P, tA.M), jb = col_atom(tB.P, tB.M);
-        const bool va = vi && ja.m.x >= 0 && (!tA.diag || 4 * (tA.jc & 1) + jj > il);
-        const bool vb = hasB && vi && jb.m.x >= 0 && (!tB.diag || 4 * (tB.jc & 1) + jj > il);
-        PairGeo ga = col_geo<NT, S0, S1>(p, Pi, tA.P, va, ia.m.z, ja.m.z);
-        PairGeo gb = col_geo<NT, S0, S1>(p, Pi, tB.P, vb, ia.m.z, jb.m.z);
-        if (__any_sync(FULL, is_rare(ga) || is_rare(gb))) {   // warp-uniform, rare
-            resolve_rare<NT>(p, ga, ia, ja);
-            resolve_rare<NT>(p, gb, ia, jb);
-        }
-        const bool any_a = __any_sync(FULL, ga.act), any_b = __any_sync(FULL, gb.act);
-        if (!(any_a || any_b)) continue;
-        float fta = 0.f, ela = 0.f, eca = 0.f, ftb = 0.f, elb = 0.f, ecb = 0.f;
-        if (any_a && any_b) {
-            pair_math<NT, P0, S0, P1, S1>(p, ga, ia, ja, fta, ela, eca);
-            pair_math<NT, P0, S0, P1, S1>(p, gb, ia, jb, ftb, elb, ecb);
-        } else {
-            float ft, e1, e2;
-            pair_math<NT, P0, S0, P1, S1>(p, any_a ? ga : gb, ia, any_a ? ja : jb, ft, e1, e2);
-            if (any_a) { fta = ft; ela = e1; eca = e2; } else { ftb = ft; elb = e1; ecb = e2; }
-        }
-        const float xa = ga.dx * fta, ya = ga.dy * fta, za = ga.dz * fta;
-        const float xb = gb.dx * ftb, yb = gb.dy * ftb, zb = gb.dz * ftb;
-        fix -= xa + xb; fiy -= ya + yb; fiz -= za + zb;
-        // near pairs: queued (original indices) for FP64 energies in place of the FP32 ones
-        {
-            const bool na = ga.act && ga.r2 < p.near2, nb = gb.act && gb.r2 < p.near2;   // near2 = 0: none
-            if (__any_sync(FULL, na || nb)) {
-                const unsigned ba = __ballot_sync(FULL, na), bb = __ballot_sync(FULL, nb);
-                const unsigned lt = (1u << lane) - 1u;
-                if (na) {
-                    s_near[nq + __popc(ba & lt)] =
-                        make_int2(ia.m.x, ja.m.x | (ga.excl == PMGPU_EXCL_MODIFIED ? 1 << 30 : 0));
-                    ela = 0.f; eca = 0.f;
-                }
-                nq += __popc(ba);
-                if (nb) {
-                    s_near[nq + __popc(bb & lt)] =
-                        make_int2(ia.m.x, jb.m.x | (gb.excl == PMGPU_EXCL_MODIFIED ? 1 << 30 : 0));
-                    elb = 0.f; ecb = 0.f;
-                }
-                nq += __popc(bb);
+        if (__any_sync(FULL, rare)) {
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const int eh = h ? e.y : e.x;
+                bool in = h ? inB : inA;
+                int code = h ? codeB : codeA;
+                col_resolve<DIFFMOL, TWO>(p, t, r.si, 4 * (eh & 0x7fffffff) + jj, eh < 0, h ? rb : ra, h ? sameB : sameA,
+                                          in, code);
+                if (h) { inB = in; codeB = code; } else { inA = in; codeA = code; }
             }
         }
-        elf += ela + elb;
-        ecf += eca + ecb;
-        if (++nacc == kEnergyFlush) {
-            el += (double)elf;
-            ec += (double)ecf;
-            elf = 0.f; ecf = 0.f; nacc = 0;
+        const unsigned mA = (__ballot_sync(FULL, inA) >> il) & 0x01010101u;
+        const unsigned mB = (__ballot_sync(FULL, inB) >> il) & 0x01010101u;
+        const int tb = r.tail + __popc(mA);
+        if (inA) mine[((r.tail + __popc(mA & below)) & (kColRing - 1)) * kCluster] = codeA;
+        if (inB) mine[((tb + __popc(mB & below)) & (kColRing - 1)) * kCluster] = codeB;
+        r.tail = tb + __popc(mB);
+        e = en; A = nA; B = nB;
+    }
+}
+
+// the row's atom for this lane
+__device__ __forceinline__ void col_row_begin(const PairArgs& p, const ColTest& t, int row, ColRow& r)
+{
+    r.si = kCluster * row + (threadIdx.x & 7);
+    r.P = p.cq[r.si];
+    r.vi = r.P.w >= 0;
+    r.far2 = r.vi ? t.far2 : -1.f;
+    r.head = r.tail = 0;
+}
+
+// the warp's copy of n <= kColBlock entries, followed by three empty ones
+__device__ __forceinline__ void col_stage(const PairArgs& p, const int* src, int n, int* ent)
+{
+    __syncwarp();
+    for (int k = threadIdx.x & 31; k < n + 3; k += 32) ent[k] = k < n ? __ldg(src + k) : p.col_none;
+    __syncwarp();
+}
+
+// sum over the four lanes of a row atom
+__device__ __forceinline__ double row_sum(double v)
+{
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    return v + __shfl_xor_sync(0xffffffffu, v, 16);
+}
+
+// ---------------------------------------------------------------- K2b': FP32 pairs
+// A warp's shared memory in the mixed kernel
+struct ColShared32 {
+    int ring[kColRing * kCluster];
+    int ent[kColBlock + 4];
+    int fj[3][4 * kColBlock];            // the chunk's j-forces (2^22 per kcal/mol/A), zero between chunks
+    int2 near[kColNear];
+    long long acc[8];                    // sums: LJ, Coulomb, virial xx xy xz yy yz zz
+};
+constexpr float kScaleJ = 4194304.0f;    // 2^22
+constexpr float kLimitJ = 60.0f;         // a j-force component this large is added in 64 bits at once (8 x 60 2^22 < 2^31)
+
+// Two pairs per lane and step (their instructions interleave).  i-forces, far
+// pairs' energies and virial in FP32 over kEnergyFlush steps, then in FP64 for
+// the chunk, then int64 fixed point.  j-forces are added up over the row's
+// atoms in shared memory as 32-bit integers of 2^-22 (as fine as FP32 holds a
+// component of 1; each atom gets at most eight per chunk), and added to the
+// atoms' int64 sums once per chunk: everything is independent of the
+// chunk-to-warp assignment.  Near pairs (r < 5 A) go to the warp's queue for
+// K2c'; their FP32 energies and virial are left out.
+template <int NT, int P0, int S0, int P1, int S1>
+struct ColForce32 {
+    static constexpr int kKeep = 16;     // a drain leaves rings below this (longer ones share the idle lanes)
+    static constexpr bool kLocal = true;
+    static constexpr bool kTwo = NT > 1 && (S0 == SCUT || S1 == SCUT);
+    const PairArgs& p;
+    ColShared32& sh;
+    int nq;
+    JAtom ia;
+    float f[3], e[2], v[6];              // FP32 partial sums
+    double fd[3], ed[2], vd[6];
+    int steps;
+
+    __device__ __forceinline__ void init()
+    {
+        const int lane = threadIdx.x & 31;
+        if (lane < 8) sh.acc[lane] = 0;
+        for (int k = lane; k < 12 * kColBlock; k += 32) (&sh.fj[0][0])[k] = 0;
+        nq = 0;
+    }
+    __device__ __forceinline__ JAtom atom(int slot) const
+    {
+        const int4 m = __ldg(p.cm + slot);           // charge hi, lo, type, original index
+        JAtom a;
+        a.p = make_float4(0.f, 0.f, 0.f, __int_as_float(m.x));
+        a.l = make_float4(0.f, 0.f, 0.f, __int_as_float(m.y));
+        a.m = make_int4(m.w, m.z, 0, 0);
+        return a;
+    }
+    __device__ __forceinline__ void begin(const ColRow& r)
+    {
+        ia = atom(r.si);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { f[k] = 0.f; fd[k] = 0.0; }
+        e[0] = e[1] = 0.f;
+        ed[0] = ed[1] = 0.0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) { v[k] = 0.f; vd[k] = 0.0; }
+        steps = 0;
+    }
+    __device__ __forceinline__ void flush()
+    {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { fd[k] += (double)f[k]; f[k] = 0.f; }
+        ed[0] += (double)e[0]; ed[1] += (double)e[1];
+        e[0] = e[1] = 0.f;
+        if (p.virial) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) { vd[k] += (double)v[k]; v[k] = 0.f; }
         }
-        // j-forces of both tiles: lane il < 6 ends with one component
-        const float v = j_reduce_scatter(xa, ya, za, xb, yb, zb, il);
-        if (holds && v != 0.f)
-            fixed_addf(p.facc + 3 * (4 * (size_t)(onB ? tB.jc : tA.jc) + jj) + comp, v, p.status);
-        if (p.virial && holds) {                       // o (x) F_tile, column comp
-            const float ox = onB ? tB.ox : tA.ox, oy = onB ? tB.oy : tA.oy, oz = onB ? tB.oz : tA.oz;
-            wv[0] += (double)(ox * v);
-            wv[1] += (double)(oy * v);
-            wv[2] += (double)(oz * v);
+        steps = 0;
+    }
+    __device__ __forceinline__ int slot(int code) const
+    {
+        const int k = code & kCodeSlot;
+        return 4 * (sh.ent[k >> 2] & 0x7fffffff) + (k & 3);
+    }
+    __device__ __forceinline__ PairGeo geo(const ColRow& r, int code, int slot, bool valid) const
+    {
+        PairGeo g;
+        const int4 P = __ldg(p.cq + slot);
+        const float qx = (float)(int)((unsigned)P.x - (unsigned)r.P.x);
+        const float qy = (float)(int)((unsigned)P.y - (unsigned)r.P.y);
+        const float qz = (float)(int)((unsigned)P.z - (unsigned)r.P.z);
+        g.dx = fmaf(qx, p.cg.sch[0], qx * p.cg.scl[0]);
+        g.dy = fmaf(qy, p.cg.sch[1], qy * p.cg.scl[1]);
+        g.dz = fmaf(qz, p.cg.sch[2], qz * p.cg.scl[2]);
+        g.r2 = fmaf(g.dz, g.dz, fmaf(g.dy, g.dy, g.dx * g.dx));
+        g.act = valid;
+        const bool two = kTwo && p.tf[0].cut2 != p.tf[1].cut2;
+        g.in0 = !two || (code & kCodeIn0);
+        g.in1 = !two || (code & kCodeIn1);
+        g.excl = (code & kCodeMod) ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE;
+        g.near = g.same = false;
+        return g;
+    }
+    // the j-force of one pair
+    __device__ __forceinline__ void add_j(int code, int slot, bool big, bool valid, float x, float y, float z)
+    {
+        if (!valid) return;
+        const int k = code & kCodeSlot;
+        if (!big) {
+            atomicAdd(&sh.fj[0][k], __float2int_rn(x * kScaleJ));
+            atomicAdd(&sh.fj[1][k], __float2int_rn(y * kScaleJ));
+            atomicAdd(&sh.fj[2][k], __float2int_rn(z * kScaleJ));
+        } else {
+            unsigned long long* to = p.facc + 3 * (size_t)slot;
+            fixed_addf(to, x, p.status);
+            fixed_addf(to + 1, y, p.status);
+            fixed_addf(to + 2, z, p.status);
         }
+    }
+    // the pairs from places at and at + 4 of the lane's ring
+    __device__ __forceinline__ void step(const ColRow& r, const int* ring, int at, bool va, bool vb)
+    {
+        const unsigned FULL = 0xffffffffu;
+        const int lane = threadIdx.x & 31, il = lane & 7;
+        const int ca = va ? ring[(at & (kColRing - 1)) * kCluster + il] : 0;
+        const int cb = vb ? ring[((at + 4) & (kColRing - 1)) * kCluster + il] : 0;
+        const int sa = slot(ca), sb = slot(cb);
+        const PairGeo ga = geo(r, ca, sa, va), gb = geo(r, cb, sb, vb);
+        const JAtom ja = atom(sa), jb = atom(sb);
+        float fta, ela, eca, ftb, elb, ecb;
+        pair_math<NT, P0, S0, P1, S1>(p, ga, ia, ja, fta, ela, eca);
+        pair_math<NT, P0, S0, P1, S1>(p, gb, ia, jb, ftb, elb, ecb);
+        const float xa = ga.dx * fta, ya = ga.dy * fta, za = ga.dz * fta;
+        const float xb = gb.dx * ftb, yb = gb.dy * ftb, zb = gb.dz * ftb;
+        f[0] -= xa + xb; f[1] -= ya + yb; f[2] -= za + zb;
+        // (not below the limit: NaN too)
+        const bool ba = !(fmaxf(fabsf(xa), fmaxf(fabsf(ya), fabsf(za))) < kLimitJ) || isnan(fta);
+        const bool bb = !(fmaxf(fabsf(xb), fmaxf(fabsf(yb), fabsf(zb))) < kLimitJ) || isnan(ftb);
+        add_j(ca, sa, ba, va, xa, ya, za);
+        add_j(cb, sb, bb, vb, xb, yb, zb);
+        const bool na = va && ga.r2 < p.near2, nb = vb && gb.r2 < p.near2;     // near2 = 0: none
+        if (p.virial) {
+            const float ax = na ? 0.f : ga.dx, ay = na ? 0.f : ga.dy, az = na ? 0.f : ga.dz;
+            const float bx = nb ? 0.f : gb.dx, by = nb ? 0.f : gb.dy, bz = nb ? 0.f : gb.dz;
+            v[0] = fmaf(xa, ax, fmaf(xb, bx, v[0]));
+            v[1] = fmaf(xa, ay, fmaf(xb, by, v[1]));
+            v[2] = fmaf(xa, az, fmaf(xb, bz, v[2]));
+            v[3] = fmaf(ya, ay, fmaf(yb, by, v[3]));
+            v[4] = fmaf(ya, az, fmaf(yb, bz, v[4]));
+            v[5] = fmaf(za, az, fmaf(zb, bz, v[5]));
+        }
+        if (__any_sync(FULL, na || nb)) {
+            if (na) ela = eca = 0.f;
+            if (nb) elb = ecb = 0.f;
+            if (nq > kColNear - 64) { append_near(p, sh.near, nq, lane); nq = 0; }
+            const unsigned wa = __ballot_sync(FULL, na), wb = __ballot_sync(FULL, nb), lt = (1u << lane) - 1u;
+            if (na) sh.near[nq + __popc(wa & lt)] = make_int2(ia.m.x, ja.m.x | (ca & kCodeMod));
+            nq += __popc(wa);
+            if (nb) sh.near[nq + __popc(wb & lt)] = make_int2(ia.m.x, jb.m.x | (cb & kCodeMod));
+            nq += __popc(wb);
+        }
+        e[0] += ela + elb;
+        e[1] += eca + ecb;
         if (p.rec_pairs) {                             // diagnostic pair recording
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
-                const PairGeo& g = t ? gb : ga;
-                const JAtom& j = t ? jb : ja;
-                if (g.act) {
-                    const unsigned long long r = atomicAdd(p.rec_count, 1ull);
-                    if ((long long)r < p.rec_cap) {
-                        p.rec_pairs[2 * r] = min(ia.m.x, j.m.x);
-                        p.rec_pairs[2 * r + 1] = max(ia.m.x, j.m.x);
+                const int oj = t ? jb.m.x : ja.m.x;
+                if (t ? vb : va) {
+                    const unsigned long long k = atomicAdd(p.rec_count, 1ull);
+                    if ((long long)k < p.rec_cap) {
+                        p.rec_pairs[2 * k] = min(ia.m.x, oj);
+                        p.rec_pairs[2 * k + 1] = max(ia.m.x, oj);
                     }
                 }
             }
         }
+        if (++steps == kEnergyFlush) flush();
     }
-    el += (double)elf;
-    ec += (double)ecf;
-    // chunk end: i-forces (lanes jj = 0, 1, 2 hold component jj of i-atom il)
-    const float vi3 = i_reduce_scatter(fix, fiy, fiz, jj);
-    if (jj < 3 && vi && vi3 != 0.f) fixed_addf(p.facc + 3 * (size_t)si + jj, vi3, p.status);
-    if (nq > 0) append_near(p, s_near, nq, lane);
-    acc[0] += fixed_of(el, bad);
-    acc[1] += fixed_of(ec, bad);
-    if (p.virial) {
+    __device__ __forceinline__ void drain(ColRow& r, const int* ring, int keep)
+    {
+        // the ring's eights, each row atom from another one on: the rings of a
+        // row hold the same clusters in the same order, and the same j-atom in
+        // several lanes serialises their shared-memory adds
+        const int lane = threadIdx.x & 31, il = lane & 7, jj = lane >> 3;
+        const int cnt = r.tail - r.head;
+        int m = keep ? cnt >> 3 : (cnt + 7) >> 3;
+        int steps = __reduce_max_sync(0xffffffffu, m);
+        if (keep) steps = max(1, steps - 2);         // the fullest ring keeps two eights: fewer idle lanes
+        m = min(m, steps);
+        int b = m > 0 ? il % m : 0;
+        for (int s = 0; s < steps; ++s) {
+            const int at = 8 * b + jj;
+            step(r, ring, r.head + at, s < m && at < cnt, s < m && at + 4 < cnt);
+            b = b + 1 < m ? b + 1 : 0;
+        }
+        r.head += min(8 * m, cnt);
+    }
+    // One chunk of a row's entries
+    __device__ __forceinline__ void run(const ColTest& t, const int4& cd)
+    {
+        const int lane = threadIdx.x & 31;
+        const int n = min(cd.w, kColBlock);
+        if (n <= 0) return;
+        ColRow r;
+        col_row_begin(p, t, cd.x, r);
+        begin(r);
+        col_stage(p, p.clist + cd.z, n, sh.ent);
+        col_entries<false, kTwo>(p, t, r, sh.ring, sh.ent, n, true, *this);
+        // the chunk's j-forces
+        for (int k = lane; k < 4 * n; k += 32) {
+            unsigned long long* to = p.facc + 3 * (size_t)slot(k);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) acc[2 + a] += fixed_of(wv[a], bad);
+            for (int c = 0; c < 3; ++c) {
+                const int q = sh.fj[c][k];
+                if (q != 0) {
+                    sh.fj[c][k] = 0;
+                    atomicAdd(to + c, (unsigned long long)((long long)q * 1024));      // 2^-22 -> 2^-32
+                }
+            }
+        }
+        end(r);
     }
-    __syncwarp();
+    __device__ __forceinline__ void end(const ColRow& r)
+    {
+        flush();
+        const int lane = threadIdx.x & 31, jj = lane >> 3;
+        const double x = row_sum(fd[0]), y = row_sum(fd[1]), z = row_sum(fd[2]);
+        if (r.vi && jj < 3)
+            fixed_add(p.facc + 3 * (size_t)r.si + jj, jj == 0 ? x : (jj == 1 ? y : z), kScaleMixed, p.status);
+        double mine = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (k >= 2 && !p.virial) break;
+            double t = k < 2 ? ed[k] : vd[k - 2];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane == k) mine = t;
+        }
+        bool bad = false;
+        if (lane < 8) sh.acc[lane] += fixed_of(mine, bad);
+        if (bad) atomicOr(p.status, kStatusOverflow);
+        if (nq > 0) { append_near(p, sh.near, nq, lane); nq = 0; }
+    }
+    // the warp's sums into the system's energy words (LJ, Coulomb, virial row major)
+    __device__ __forceinline__ void store()
+    {
+        const int lane = threadIdx.x & 31;
+        __syncwarp();
+        if (lane < kERec) {
+            constexpr int at[kERec] = {0, 1, 2, 3, 4, 3, 5, 6, 4, 6, 7};
+            int k = 0;
+#pragma unroll
+            for (int c = 0; c < kERec; ++c) if (lane == c) k = at[c];
+            const long long v = sh.acc[k];
+            if (v != 0) atomicAdd(p.efix + lane, (unsigned long long)v);
+        }
+        __syncwarp();
+        if (lane < 8) sh.acc[lane] = 0;
+        __syncwarp();
+    }
+};
+
+// an incomplete list (capacity exceeded or the system refused, also when it
+// was built by an earlier evaluation and is reused) runs no pair
+__device__ __forceinline__ int col_chunks(const PairArgs& p, bool mark)
+{
+    const bool bad = (*p.status & (kStatusListFull | kStatusColumns)) || *p.plist_need != 0 || *p.chunk_need != 0;
+    if (bad && mark) atomicOr(p.status, kStatusListFull);
+    return bad ? 0 : min(*p.chunk_count, p.chunk_cap);
 }
 
-// Two 8 x 4 tiles (consecutive entries A and B of the chunk) per iteration:
-// two independent pair evaluations per lane interleave, and the per-tile
-// work -- votes, the j-force reduce-scatter of both tiles in one (7 shuffles
-// for 6 values), the fixed-point adds, the virial offsets, the energy sums --
-// is shared by the two.
 template <int NT, int P0, int S0, int P1, int S1>
-__global__ void __launch_bounds__(128, 5) k_pair_col(PairArgs p)
+__global__ void __launch_bounds__(128, 4) k_pair_col(const __grid_constant__ PairArgs p)
 {
     pdl_wait();
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, il = lane & 7, jj = lane >> 3;
-    __shared__ int2 s_near[4][kNearCap];
-    __shared__ unsigned long long s_e[kERec];
-    if (threadIdx.x < kERec) s_e[threadIdx.x] = 0ull;
-    __syncthreads();
-    // per-lane int64 sums over the chunks: LJ, Coulomb, and the tile-offset
-    // virial W[0..2][comp] of the lanes that hold a j-force component
-    long long acc[5] = {0, 0, 0, 0, 0};
-    bool bad = false;
-    // an incomplete list (capacity exceeded or the system refused, also when
-    // it was built by an earlier evaluation and is reused) runs no pair
-    const bool list_bad = (*p.status & (kStatusListFull | kStatusColumns)) || *p.plist_need != 0 || *p.chunk_need != 0;
-    if (list_bad && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(p.status, kStatusListFull);
-    const int nchunks = list_bad ? 0 : min(*p.chunk_count, p.chunk_cap);
-    // lane il (< 6) holds component il % 3 of a j-force (col_run)
-    const bool holds = il < 6;
-    const int comp = il < 3 ? il : il - 3;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __shared__ ColShared32 sh[4];
+    const int nchunks = col_chunks(p, blockIdx.x == 0 && threadIdx.x == 0);
+    const ColTest t = col_test(p);
+    ColForce32<NT, P0, S0, P1, S1> op{p, sh[w]};
+    op.init();
     while (true) {
         int ch = 0;
         if (lane == 0) ch = atomicAdd(p.chunk_next, 1);
-        ch = __shfl_sync(FULL, ch, 0);
+        ch = __shfl_sync(0xffffffffu, ch, 0);
         if (ch >= nchunks) break;
-        const int4 cd = p.chunks[ch];
-        col_run<false, NT, P0, S0, P1, S1>(p, cd.x, p.clist, cd.z, cd.z + cd.w, s_near[w], acc, bad);
+        op.run(t, p.chunks[ch]);
     }
-    if (bad) atomicOr(p.status, kStatusOverflow);
-#pragma unroll
-    for (int t = 0; t < 2; ++t)
-        for (int o = 16; o > 0; o >>= 1) acc[t] += __shfl_xor_sync(FULL, acc[t], o);
-    if (lane == 0) {
-        atomicAdd(&s_e[0], (unsigned long long)acc[0]);
-        atomicAdd(&s_e[1], (unsigned long long)acc[1]);
-    }
-    if (p.virial) {
-        // W[a][comp]: sum over the four j-atom groups (xor 8, 16; lanes that
-        // hold no component carry zeros), then lanes 0-5 of the first group
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            acc[2 + a] += __shfl_xor_sync(FULL, acc[2 + a], 8);
-            acc[2 + a] += __shfl_xor_sync(FULL, acc[2 + a], 16);
-        }
-        if (holds && jj == 0) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) atomicAdd(&s_e[2 + 3 * a + comp], (unsigned long long)acc[2 + a]);
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < kERec && s_e[threadIdx.x] != 0ull) atomicAdd(p.efix + threadIdx.x, s_e[threadIdx.x]);
-}
-
-// The lanes' int64 sums (acc) of one system into its energy words, at once
-// (the batch kernel: the warp leaves the system)
-__device__ __forceinline__ void col_warp_sums(const PairArgs& p, long long (&acc)[5], bool& bad)
-{
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, il = lane & 7, jj = lane >> 3;
-    const int comp = il < 3 ? il : il - 3;
-    if (bad && lane == 0) atomicOr(p.status, kStatusOverflow);
-    bad = __any_sync(FULL, bad) && false;
-#pragma unroll
-    for (int t = 0; t < 2; ++t)
-        for (int o = 16; o > 0; o >>= 1) acc[t] += __shfl_xor_sync(FULL, acc[t], o);
-    if (lane == 0) {
-        if (acc[0] != 0) atomicAdd(p.efix + 0, (unsigned long long)acc[0]);
-        if (acc[1] != 0) atomicAdd(p.efix + 1, (unsigned long long)acc[1]);
-    }
-    if (p.virial) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            acc[2 + a] += __shfl_xor_sync(FULL, acc[2 + a], 8);
-            acc[2 + a] += __shfl_xor_sync(FULL, acc[2 + a], 16);
-        }
-        if (il < 6 && jj == 0) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-                if (acc[2 + a] != 0) atomicAdd(p.efix + 2 + 3 * a + comp, (unsigned long long)acc[2 + a]);
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < 5; ++t) acc[t] = 0;
+    op.store();
 }
 
 // K11: the column-path pair kernels of a batch's members as one persistent
@@ -540,35 +692,32 @@ __device__ __forceinline__ void col_warp_sums(const PairArgs& p, long long (&acc
 // chunk counts in shared memory (a member whose list is incomplete counts
 // none and is marked as K2b' marks it); a warp takes items from one counter,
 // copies its member's arguments into shared memory when the member changes,
-// runs the chunk (col_run, the K2b' tile loop) and adds its sums to the
-// member's energy words when it leaves the member.  Nothing waits on
-// another launch: the graph orders this one after every member's list.
+// runs the chunk (as K2b') and adds its sums to the member's energy
+// words when it leaves the member.  Nothing waits on another launch: the
+// graph orders this one after every member's list.
 template <int NT, int P0, int S0, int P1, int S1>
 __global__ void __launch_bounds__(128, 4) k_pair_col_batch(BatchPairArgs b)
 {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __shared__ int2 s_near[4][kNearCap];
+    __shared__ ColShared32 sh[4];
     __shared__ int s_pre[kBatchPairMax + 1];
     __shared__ PairArgs s_args[4];
     if (threadIdx.x == 0) {
         int t = 0;
         for (int m = 0; m < b.n; ++m) {
-            const PairArgs& p = b.args[m];
             s_pre[m] = t;
-            const bool list_bad = (*p.status & (kStatusListFull | kStatusColumns)) || *p.plist_need != 0 ||
-                                  *p.chunk_need != 0;
-            if (list_bad && blockIdx.x == 0) atomicOr(p.status, kStatusListFull);
-            t += list_bad ? 0 : min(*p.chunk_count, p.chunk_cap);
+            t += col_chunks(b.args[m], blockIdx.x == 0);
         }
         s_pre[b.n] = t;
     }
     __syncthreads();
     const int total = s_pre[b.n];
-    long long acc[5] = {0, 0, 0, 0, 0};
-    bool bad = false;
     int cur = -1;
     const PairArgs& p = s_args[w];
+    ColForce32<NT, P0, S0, P1, S1> op{p, sh[w]};
+    op.init();
+    ColTest t;
     while (true) {
         int item = 0;
         if (lane == 0) item = atomicAdd(b.next, 1);
@@ -580,80 +729,81 @@ __global__ void __launch_bounds__(128, 4) k_pair_col_batch(BatchPairArgs b)
             if (s_pre[mid] <= item) lo = mid; else hi = mid;
         }
         if (lo != cur) {
-            if (cur >= 0) col_warp_sums(p, acc, bad);
+            if (cur >= 0) op.store();
             __syncwarp();
             const int* src = reinterpret_cast<const int*>(b.args + lo);
             int* dst = reinterpret_cast<int*>(&s_args[w]);
             for (int i = lane; i < (int)(sizeof(PairArgs) / sizeof(int)); i += 32) dst[i] = src[i];
             __syncwarp();
+            t = col_test(p);
             cur = lo;
         }
-        const int4 cd = p.chunks[item - s_pre[lo]];
-        col_run<false, NT, P0, S0, P1, S1>(p, cd.x, p.clist, cd.z, cd.z + cd.w, s_near[w], acc, bad);
+        op.run(t, p.chunks[item - s_pre[lo]]);
     }
-    if (cur >= 0) col_warp_sums(p, acc, bad);
+    if (cur >= 0) op.store();
 }
 
-// FP64 energies of one pair of atoms by original index: the FP64 kernel's
-// arithmetic (pot_f64, sw_f64) on the raw positions and the exact minimal
-// image
+// FP64 energies and force factor of one pair of atoms by original index: the
+// FP64 kernel's arithmetic (pair_f64) on the raw positions and the exact
+// minimal image (d)
 template <int NT, int P0, int S0, int P1, int S1>
-__device__ __forceinline__ void pair_energy_f64_orig(const PairArgs& p, int oi, int oj, int excl, double& el,
-                                                     double& ec)
+__device__ __forceinline__ void pair_f64_orig(const PairArgs& p, int oi, int oj, int excl, double& el, double& ec,
+                                              double& ft, double (&d)[3])
 {
-    constexpr bool kMod = sw_modifies(S0) || (NT > 1 && sw_modifies(S1));
     const double* pi = p.pos + 3 * (size_t)oi;
     const double* pj = p.pos + 3 * (size_t)oj;
-    double dx, dy, dz;
-    const double d2 = pbc_min_diff(p.pbc, pi[0], pi[1], pi[2], pj[0], pj[1], pj[2], dx, dy, dz);
-    const double rd2 = 1.0 / d2;
+    const double d2 = pbc_min_diff(p.pbc, pi[0], pi[1], pi[2], pj[0], pj[1], pj[2], d[0], d[1], d[2]);
     const double qi = p.qorig[oi], qj = p.qorig[oj];
     const int ti = p.torig[oi], tj = p.torig[oj];
-    double e0, f0, e1 = 0.0, f1 = 0.0;
-    pot_f64<P0>(p, p.td[0], d2, rd2, qi, qj, ti, tj, excl, e0, f0);
-    if (NT > 1) pot_f64<P1>(p, p.td[1], d2, rd2, qi, qj, ti, tj, excl, e1, f1);
-    if (kMod) {
-        double sv, sd;
-        sw_f64<S0>(p.td[0], d2, sv, sd);
-        e0 *= sv;
-        if (NT > 1) {
-            sw_f64<S1>(p.td[1], d2, sv, sd);
-            e1 *= sv;
-        }
-    }
-    el += (pot_lj_slot(P0) ? e0 : 0.0) + (NT > 1 && pot_lj_slot(P1) ? e1 : 0.0);
-    ec += (!pot_lj_slot(P0) ? e0 : 0.0) + (NT > 1 && !pot_lj_slot(P1) ? e1 : 0.0);
+    double e0, e1;
+    pair_f64<NT, P0, S0, P1, S1>(p, d2, qi, qj, ti, tj, excl, ft, e0, e1);
+    el = (pot_lj_slot(P0) ? e0 : 0.0) + (NT > 1 && pot_lj_slot(P1) ? e1 : 0.0);
+    ec = (!pot_lj_slot(P0) ? e0 : 0.0) + (NT > 1 && !pot_lj_slot(P1) ? e1 : 0.0);
 }
 
-// K2c': the FP64 energies of the near pairs K2b' listed (original indices),
-// each rounded to int64 fixed point on its own
+// K2c': the FP64 energies and virial of the near pairs K2b' listed (original
+// indices), each rounded to int64 fixed point on its own
 template <int NT, int P0, int S0, int P1, int S1>
-__global__ void __launch_bounds__(128) k_near_energy_col(PairArgs p)
+__global__ void __launch_bounds__(128) k_near_energy_col(const __grid_constant__ PairArgs p)
 {
     const unsigned FULL = 0xffffffffu;
-    __shared__ long long s_acc[2][4];
+    __shared__ long long s_acc[8][4];
     if (*p.status & (kStatusListFull | kStatusColumns)) return;   // block-uniform
     const int n = min(*p.near_count, p.near_cap);
-    long long al = 0, ac = 0;
+    long long acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};                   // LJ, Coulomb, virial xx xy xz yy yz zz
     bool bad = false;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const int2 e = p.near[k];
-        double el = 0.0, ec = 0.0;
-        pair_energy_f64_orig<NT, P0, S0, P1, S1>(p, e.x, e.y & 0x3fffffff,
-                                                 (e.y >> 30) ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE, el, ec);
-        al += fixed_of(el, bad);
-        ac += fixed_of(ec, bad);
+        double el, ec, ft, d[3];
+        pair_f64_orig<NT, P0, S0, P1, S1>(p, e.x, e.y & 0x3fffffff,
+                                          (e.y >> 30) ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE, el, ec, ft, d);
+        acc[0] += fixed_of(el, bad);
+        acc[1] += fixed_of(ec, bad);
+        if (p.virial) {
+            const double fx = ft * d[0], fy = ft * d[1], fz = ft * d[2];
+            acc[2] += fixed_of(fx * d[0], bad);
+            acc[3] += fixed_of(fx * d[1], bad);
+            acc[4] += fixed_of(fx * d[2], bad);
+            acc[5] += fixed_of(fy * d[1], bad);
+            acc[6] += fixed_of(fy * d[2], bad);
+            acc[7] += fixed_of(fz * d[2], bad);
+        }
     }
     if (bad) atomicOr(p.status, kStatusOverflow);
-    for (int o = 16; o > 0; o >>= 1) {
-        al += __shfl_xor_sync(FULL, al, o);
-        ac += __shfl_xor_sync(FULL, ac, o);
-    }
     const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) { s_acc[0][w] = al; s_acc[1][w] = ac; }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        if (c >= 2 && !p.virial) break;
+        for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(FULL, acc[c], o);
+        if ((threadIdx.x & 31) == 0) s_acc[c][w] = acc[c];
+    }
     __syncthreads();
-    if (threadIdx.x < 2) {
-        const long long t = s_acc[threadIdx.x][0] + s_acc[threadIdx.x][1] + s_acc[threadIdx.x][2] + s_acc[threadIdx.x][3];
+    if (threadIdx.x < kERec && (threadIdx.x < 2 || p.virial)) {
+        constexpr int at[kERec] = {0, 1, 2, 3, 4, 3, 5, 6, 4, 6, 7};
+        int c = 0;
+#pragma unroll
+        for (int k = 0; k < kERec; ++k) if (threadIdx.x == k) c = at[k];
+        const long long t = s_acc[c][0] + s_acc[c][1] + s_acc[c][2] + s_acc[c][3];
         if (t != 0) atomicAdd(p.efix + threadIdx.x, (unsigned long long)t);
     }
 }

@@ -1,5 +1,5 @@
 // pm_pair_mixed.cuh -- K2: mixed-precision cluster-pair force kernels
-// (included by pm_pair.cu, which provides the helpers).
+// (included by the pm_pair*.cu files after pm_pair_math.cuh).
 //
 // Clusters: inside a reference cell the atoms are ordered by the Morton key of
 // their position on an 8x8x8 sub-grid of the cell (k_bin_cells), so every run
@@ -116,7 +116,7 @@ __device__ __forceinline__ unsigned near_mask(const PairArgs& p, const Cand& c, 
     return m;
 }
 
-__global__ void __launch_bounds__(128) k_cluster_list(PairArgs p)
+static __global__ void __launch_bounds__(128) k_cluster_list(PairArgs p)
 {
     pdl_wait();
     // one warp per (cell, block of 32 half-shell cells): the warp's entries of
@@ -275,7 +275,8 @@ __device__ __forceinline__ void resolve_rare(const PairArgs& p, PairGeo& g, cons
 // the normal positive arguments of the pair kernel
 __device__ __forceinline__ float rsqrt_nr(float x)
 {
-    float y = rsqrtf(x);
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     float e = fmaf(-x * y, y, 1.0f);
     return fmaf(0.5f * y, e, y);
 }
@@ -296,11 +297,20 @@ __device__ __forceinline__ void pair_math(const PairArgs& p, const PairGeo& g, c
     pot_f32<P0>(p, p.tf[0], r2, rd2, rinv, qq, ia.m.y, ja.m.y, g.excl, e0, f0);
     if (NT > 1) pot_f32<P1>(p, p.tf[1], r2, rd2, rinv, qq, ia.m.y, ja.m.y, g.excl, e1, f1);
     if (kMod) {
+        // (a Cutoff switch is one inside, zero outside)
         float sv, sd;
-        sw_f32<S0>(p.tf[0], r2, rinv, g.in0, sv, sd);
-        f0 = f0 * sv - e0 * sd;
-        e0 = e0 * sv;
-        if (NT > 1) {
+        if (S0 == SCUT) {
+            f0 = g.in0 ? f0 : 0.f;
+            e0 = g.in0 ? e0 : 0.f;
+        } else {
+            sw_f32<S0>(p.tf[0], r2, rinv, g.in0, sv, sd);
+            f0 = f0 * sv - e0 * sd;
+            e0 = e0 * sv;
+        }
+        if (NT > 1 && S1 == SCUT) {
+            f1 = g.in1 ? f1 : 0.f;
+            e1 = g.in1 ? e1 : 0.f;
+        } else if (NT > 1) {
             sw_f32<S1>(p.tf[1], r2, rinv, g.in1, sv, sd);
             f1 = f1 * sv - e1 * sd;
             e1 = e1 * sv;
@@ -320,24 +330,12 @@ __device__ __forceinline__ void pair_math(const PairArgs& p, const PairGeo& g, c
 template <int NT, int P0, int S0, int P1, int S1>
 __device__ __forceinline__ void pair_energy_f64(const PairArgs& p, int si, int sj, int excl, double& el, double& ec)
 {
-    constexpr bool kMod = sw_modifies(S0) || (NT > 1 && sw_modifies(S1));
     const double4 pi = p.spos64[si], pj = p.spos64[sj];
     const int ti = p.smeta[si].y, tj = p.smeta[sj].y;
     double dx, dy, dz;
     const double d2 = pbc_min_diff(p.pbc, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z, dx, dy, dz);
-    const double rd2 = 1.0 / d2;
-    double e0, f0, e1 = 0.0, f1 = 0.0;
-    pot_f64<P0>(p, p.td[0], d2, rd2, pi.w, pj.w, ti, tj, excl, e0, f0);
-    if (NT > 1) pot_f64<P1>(p, p.td[1], d2, rd2, pi.w, pj.w, ti, tj, excl, e1, f1);
-    if (kMod) {
-        double sv, sd;
-        sw_f64<S0>(p.td[0], d2, sv, sd);
-        e0 *= sv;
-        if (NT > 1) {
-            sw_f64<S1>(p.td[1], d2, sv, sd);
-            e1 *= sv;
-        }
-    }
+    double ft, e0, e1;
+    pair_f64<NT, P0, S0, P1, S1>(p, d2, pi.w, pj.w, ti, tj, excl, ft, e0, e1);
     el += (pot_lj_slot(P0) ? e0 : 0.0) + (NT > 1 && pot_lj_slot(P1) ? e1 : 0.0);
     ec += (!pot_lj_slot(P0) ? e0 : 0.0) + (NT > 1 && !pot_lj_slot(P1) ? e1 : 0.0);
 }

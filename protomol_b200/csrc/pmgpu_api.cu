@@ -141,6 +141,7 @@ struct pmgpu_system {
     float4* d_slo = nullptr;
     int4* d_smeta = nullptr;
     double4* d_spos64 = nullptr;
+    int4* d_sfix = nullptr;
     // small per-evaluation scratch, zeroed by one memset: status word,
     // cluster-pair list and chunk counters, int64 energy/virial sums
     void* d_small = nullptr;
@@ -172,7 +173,8 @@ struct pmgpu_system {
     bool col_grid_stale = true;        // box or atom count changed since col_set_grid
     bool col_disabled = false;
     bool col_just_disabled = false;
-    bool eval_use_col = false;         // the evaluation being enqueued uses the column path
+    bool eval_use_col = false;         // the evaluation's mixed cutoff forces use the column path
+    bool eval_col64 = false;           // its FP64 cutoff forces (and molecular virials) do
     // reused pair lists (pmgpu_set_pair_list): the column list built with the
     // cutoff plus a skin is kept for rebuild_every evaluations while no atom
     // moves more than half the skin
@@ -200,11 +202,25 @@ struct pmgpu_system {
     float4* d_ibox = nullptr;
     float4* d_jbox = nullptr;
     int* d_ccol = nullptr;
-    int4* d_corg = nullptr;
+    double4* d_c64 = nullptr;          // raw position and charge per slot (FP64 row kernels)
+    int2* d_rowent = nullptr;          // the list's entries of every row
     unsigned long long* d_facc32c = nullptr;
+    unsigned long long* d_facc40c = nullptr;     // FP64 rows: wide sums (2^40) per slot, then fine ones (2^44)
     int col_ncl_cap = 0;
     double* d_acc0 = nullptr;          // 3N: the caller's force accumulator as pmgpu_evaluate received it
     double* h_fbuf = nullptr;          // pinned 3N: the forces' copy back for a pageable accumulator
+    // the backward pass's buffers, kept between calls: dq N, hv 3N, v 3N,
+    // energies 2 (doubles, one allocation); the LJ-table gradient T T 4 and its
+    // nonzero entries; pinned copies of the results (the entries' grown on demand)
+    double* d_adj = nullptr;
+    double* d_adj_lj = nullptr;
+    double* d_adj_val = nullptr;
+    unsigned* d_adj_idx = nullptr;
+    unsigned* d_adj_count = nullptr;
+    double* h_adj = nullptr;
+    double* h_adj_val = nullptr;
+    unsigned* h_adj_idx = nullptr;
+    size_t h_adj_cap = 0;
     bool binned = false;
     std::set<pmgpu_force*> forces;     // live forces made on this system
     int topo_version = 0;
@@ -379,6 +395,10 @@ extern "C" int pmgpu_system_create(int device, pmgpu_system** out)
 static void free_atom_buffers(pmgpu_system* s)
 {
     dfree(s->d_q); dfree(s->d_type); dfree(s->d_mol); dfree(s->d_ljn); dfree(s->d_ljm); dfree(s->d_ljd);
+    dfree(s->d_adj); dfree(s->d_adj_lj); dfree(s->d_adj_val); dfree(s->d_adj_idx); dfree(s->d_adj_count);
+    for (void* h : {(void*)s->h_adj, (void*)s->h_adj_val, (void*)s->h_adj_idx})
+        if (h) cudaFreeHost(h);
+    s->h_adj = s->h_adj_val = nullptr; s->h_adj_idx = nullptr; s->h_adj_cap = 0;
     dfree(s->d_molpos); s->molpos_set = false;
     dfree(s->d_slo); dfree(s->d_skey);
     dfree(s->d_xfull); dfree(s->d_xmod); dfree(s->d_xrow); dfree(s->d_xent);
@@ -386,7 +406,7 @@ static void free_atom_buffers(pmgpu_system* s)
     dfree(s->d_pos); dfree(s->d_fout); dfree(s->d_facc32); dfree(s->d_facc40); dfree(s->d_faccA);
     s->d_facc32p = nullptr;   // second half of d_facc32
     dfree(s->d_cell_lin); dfree(s->d_cell3); dfree(s->d_tmp); dfree(s->d_sorted); dfree(s->d_slot);
-    dfree(s->d_spos); dfree(s->d_smeta); dfree(s->d_spos64);
+    dfree(s->d_spos); dfree(s->d_smeta); dfree(s->d_spos64); dfree(s->d_sfix);
     dfree(s->d_qfix); dfree(s->d_colid); dfree(s->d_ctmp); dfree(s->d_cslot);
 }
 
@@ -394,7 +414,7 @@ static void free_col_buffers(pmgpu_system* s)
 {
     dfree(s->d_ccounts); dfree(s->d_colstart); dfree(s->d_ccstart); dfree(s->d_zidx);
     dfree(s->d_cq); dfree(s->d_cm); dfree(s->d_ibox); dfree(s->d_jbox); dfree(s->d_ccol); dfree(s->d_facc32c);
-    dfree(s->d_corg);
+    dfree(s->d_c64); dfree(s->d_rowent); dfree(s->d_facc40c);
     s->col_ncol_cap = 0;
     s->col_ncl_cap = 0;
 }
@@ -636,6 +656,7 @@ extern "C" int pmgpu_set_topology(pmgpu_system* sys, int n_atoms, const double* 
     CK(dalloc(&sys->d_cell_lin, n), "alloc"); CK(dalloc(&sys->d_cell3, 3 * (size_t)n), "alloc");
     CK(dalloc(&sys->d_tmp, n), "alloc"); CK(dalloc(&sys->d_sorted, n), "alloc"); CK(dalloc(&sys->d_slot, n), "alloc");
     CK(dalloc(&sys->d_spos, n), "alloc"); CK(dalloc(&sys->d_smeta, n), "alloc"); CK(dalloc(&sys->d_spos64, n), "alloc");
+    CK(dalloc(&sys->d_sfix, n), "alloc");
     CK(dalloc(&sys->d_slo, n), "alloc"); CK(dalloc(&sys->d_skey, n), "alloc");
     CK(dalloc(&sys->d_qfix, 3 * (size_t)n), "alloc"); CK(dalloc(&sys->d_colid, n), "alloc");
     CK(dalloc(&sys->d_ctmp, n), "alloc"); CK(dalloc(&sys->d_cslot, n), "alloc");
@@ -692,21 +713,20 @@ static int col_set_grid(pmgpu_system* sys)
 }
 
 // Reach of the column list for a pair test at cutoff rc, and whether the
-// column path applies: no column may be reached through two offsets, and the
-// z windows (an i-cluster's extent plus twice the list radius) must be
-// shorter than the box, so that every pair inside the cutoff lies in its
-// tile's image
+// column path applies: every edge at least twice the cutoff, so that a pair
+// inside it has one image (the fixed-point difference's).
 static bool col_reach(const pmgpu_system* sys, double rc, ColGrid& g)
 {
-    if (!sys->col_grid || sys->col_disabled) return false;
+    if (!sys->col_grid) return false;
     g = sys->cg;
     const double rl = std::sqrt(rc * rc * (1.0 + 8.0 * 2.0e-5) + 1e-3);
-    g.rx = (int)std::ceil(rl / g.sx) + 1;
-    g.ry = (int)std::ceil(rl / g.sy) + 1;
-    if (2 * g.rx + 1 > g.ncx || 2 * g.ry + 1 > g.ncy) return false;
+    if (!(std::min(g.lx, std::min(g.ly, g.lz)) >= 2.0 * rl)) return false;
+    g.rx = (int)std::min((double)g.ncx, std::ceil(rl / g.sx) + 1);
+    g.ry = (int)std::min((double)g.ncy, std::ceil(rl / g.sy) + 1);
+    // rows taller than the list's window prune too little: the mixed forces'
+    // cells take such a (dilute) system, where the box is wide enough for them
     const double zext = g.lz - 2.0 * rl - 0.5;
-    if (!(zext > 1.0)) return false;
-    g.zext = (float)zext;
+    g.zext = zext > 1.0 && 2 * g.rx + 1 <= g.ncx && 2 * g.ry + 1 <= g.ncy ? (float)zext : 3.0e38f;
     return true;
 }
 
@@ -1448,7 +1468,7 @@ static int bin(pmgpu_system* sys, const double* d_pos)
     a.pbc = sys->pbc; a.grid = sys->grid;
     a.cell_lin = sys->d_cell_lin; a.cell3 = sys->d_cell3; a.counts = sys->d_counts; a.done = sys->d_status + 8;
     a.start = sys->d_start; a.tmp = sys->d_tmp; a.sorted = sys->d_sorted; a.slot_of = sys->d_slot;
-    a.spos = sys->d_spos; a.slo = sys->d_slo; a.smeta = sys->d_smeta; a.spos64 = sys->d_spos64;
+    a.spos = sys->d_spos; a.slo = sys->d_slo; a.smeta = sys->d_smeta; a.spos64 = sys->d_spos64; a.sfix = sys->d_sfix;
     a.status = sys->d_status;
     int e = launch_bin(a, sys->stream, &sys->launches);
     if (e) return cuda_fail(sys, (cudaError_t)e, "binning");
@@ -1469,7 +1489,8 @@ static int col_bin(pmgpu_system* sys, const double* d_pos)
     a.colstart = sys->d_colstart; a.ccstart = sys->d_ccstart; a.tmp = sys->d_ctmp; a.zidx = sys->d_zidx;
     a.cq = sys->d_cq; a.cm = sys->d_cm; a.slot_of = sys->d_cslot;
     a.ibox = sys->d_ibox; a.jbox = sys->d_jbox; a.ccol = sys->d_ccol; a.ncl_cap = sys->col_ncl_cap;
-    a.corg = sys->d_corg;
+    a.c64 = sys->eval_col64 ? sys->d_c64 : nullptr;
+    a.refuse = sys->eval_use_col ? 1 : 0;
     a.status = sys->d_status;
     int e = launch_col_bin(a, sys->stream, &sys->launches);
     if (e) return cuda_fail(sys, (cudaError_t)e, "column binning");
@@ -1484,6 +1505,7 @@ static int col_refresh(pmgpu_system* sys, const double* d_pos)
     memset(&a, 0, sizeof(a));
     a.n = sys->n; a.pos = d_pos; a.pbc = sys->pbc; a.grid = sys->grid; a.cell3 = sys->d_cell3;
     a.g = sys->eval_cg; a.qfix = sys->d_qfix; a.cq = sys->d_cq; a.slot_of = sys->d_cslot; a.status = sys->d_status;
+    a.q = sys->d_q; a.c64 = sys->eval_col64 ? sys->d_c64 : nullptr;
     int e = launch_col_refresh(a, 0.5 * sys->list_skin, sys->stream, &sys->launches);
     if (e) return cuda_fail(sys, (cudaError_t)e, "pair list refresh");
     sys->binned = true;
@@ -1491,16 +1513,24 @@ static int col_refresh(pmgpu_system* sys, const double* d_pos)
 }
 
 // the column-path members of the pair arguments
-static void fill_col_args(pmgpu_system* sys, PairArgs& a)
+static void fill_col_args(pmgpu_system* sys, bool fp64, PairArgs& a, bool half)
 {
-    a.cq = sys->d_cq; a.cm = sys->d_cm; a.ibox = sys->d_ibox; a.jbox = sys->d_jbox;
-    a.ccstart = sys->d_ccstart; a.ccol = sys->d_ccol; a.icl_cap = sys->col_ncl_cap; a.corg = sys->d_corg;
-    a.zidx = sys->d_zidx;
-    a.clist = (int4*)sys->d_plist;          // entries of two int2 places each (plist_cap counts int2)
+    a.cq = sys->d_cq; a.cm = sys->d_cm; a.ibox = sys->d_ibox; a.jbox = sys->d_jbox; a.c64 = sys->d_c64;
+    a.ccstart = sys->d_ccstart; a.ccol = sys->d_ccol; a.icl_cap = sys->col_ncl_cap;
+    a.zidx = sys->d_zidx; a.rowent = sys->d_rowent;
+    a.clist = (int*)sys->d_plist;           // two entries in each int2 place
+    a.plist_cap = (int)std::min(2 * sys->plist_cap, (long long)INT_MAX);
     a.cg = sys->eval_cg;
     a.qorig = sys->d_q; a.torig = sys->d_type;
-    a.facc = sys->d_facc32c;
-    a.list_skin = sys->list_every > 1 ? (float)sys->list_skin : 0.0f;
+    a.facc = fp64 ? sys->d_facc40c : sys->d_facc32c;
+    a.faccj = fp64 ? sys->d_facc40c + 3 * kCluster * (size_t)(sys->col_ncl_cap + 1) : nullptr;
+    a.col_refuse = fp64 ? 0 : 1;
+    a.col_half = half ? 1 : 0;
+    a.col_none = 2 * sys->col_ncl_cap;
+    a.rows_split = col_rows_split(sys->n, sys->eval_cg, std::sqrt(a.cut2d));
+    const ColGrid& g = sys->eval_cg;
+    a.chunk = col_chunk_entries(sys->n, g, g.lx * g.ly * g.lz, std::sqrt(a.cut2d), 6 * sys->tuning.chunk_entries, half);
+    a.list_skin = !fp64 && sys->list_every > 1 ? (float)sys->list_skin : 0.0f;
 }
 
 // The pair kernels a force runs in this evaluation: the FP64 ones for an
@@ -1512,7 +1542,9 @@ static void fill_col_args(pmgpu_system* sys, PairArgs& a)
 // zero, set by the graph's zero kernel (pmgpu_evaluate's own buffers)
 constexpr unsigned kFlagZeroOut = 1u << 30;
 constexpr unsigned kFlagZeroForces = 1u << 29;
-constexpr unsigned kFlagsInternal = kFlagZeroOut | kFlagZeroForces;
+// the FP64 row kernels run whatever the forces' precision (the backward pass)
+constexpr unsigned kFlagNeeds64 = 1u << 28;
+constexpr unsigned kFlagsInternal = kFlagZeroOut | kFlagZeroForces | kFlagNeeds64;
 
 static inline bool pairs64(const pmgpu_system* sys, const pmgpu_force* f)
 {
@@ -1523,7 +1555,8 @@ static void fill_pair_args(pmgpu_system* sys, pmgpu_force* f, const double* d_po
 {
     memset(&a, 0, sizeof(a));
     a.start = sys->d_start; a.spos = sys->d_spos; a.slo = sys->d_slo; a.smeta = sys->d_smeta;
-    a.spos64 = sys->d_spos64; a.cstart = sys->d_cstart; a.cbox = sys->d_cbox;
+    a.spos64 = sys->d_spos64; a.sfix = sys->d_sfix; a.rows_split = rows_split(sys->n, sys->grid, f->nd);
+    a.cstart = sys->d_cstart; a.cbox = sys->d_cbox;
     a.pos = d_pos;
     a.xfull = sys->d_xfull; a.xmod = sys->d_xmod; a.xrow = sys->d_xrow; a.xent = sys->d_xent;
     a.ljn = sys->d_ljn; a.ljm = sys->d_ljm; a.ljd = sys->d_ljd; a.n_types = sys->t;
@@ -1571,17 +1604,56 @@ static int ensure_erec(pmgpu_system* sys, int need)
     return PMGPU_OK;
 }
 
+// blocks (records) of the FP64 row kernels of one cutoff force
+static int row_blocks(const pmgpu_system* sys, const pmgpu_force* f)
+{
+    return sys->eval_col64 ? col_row_blocks(sys->n, sys->eval_cg, std::sqrt(f->cut2)) : pair_blocks(sys->n, sys->grid, f->nd);
+}
+
 // energy records one cutoff force writes
 static int pair_records(pmgpu_system* sys, pmgpu_force* f)
 {
     // the mixed kernel sums energies in fixed point (d_efix), no records
     if (f->kind == 2) return adjoint_blocks(sys->n);
-    return pairs64(sys, f) ? pair_blocks(sys->grid, f->nd) : 0;
+    return pairs64(sys, f) ? row_blocks(sys, f) : 0;
 }
 
 // upper bound of the energy records of the fused x pass (one per CTA, at
 // least one x-line per CTA)
 static int pme_xblocks(const pmgpu_force* f) { return f->pp.grid[1] * f->kzh; }
+
+// The column-cluster path takes the cutoff forces of the group when the box
+// suits the largest of their cutoffs; the mixed ones not after it refused the
+// system.  Otherwise the cell layout takes them.
+static int choose_layout(pmgpu_system* sys, int nf, pmgpu_force* const* forces, unsigned flags)
+{
+    sys->eval_use_col = sys->eval_col64 = false;
+    double rc2 = 0.0;
+    bool any32 = false, any64 = (flags & kFlagNeeds64) != 0;
+    bool inside = true;
+    for (int k = 0; k < nf; ++k) {
+        if (forces[k]->kind != 0) continue;
+        (pairs64(sys, forces[k]) ? any64 : any32) = true;
+        rc2 = std::max(rc2, forces[k]->cut2);
+        // the cell pairs of the algorithm's cutoff hold every pair of the forces' own
+        inside = inside && forces[k]->cp.algorithm_cutoff * forces[k]->cp.algorithm_cutoff >= forces[k]->cut2;
+    }
+    if (!any32 && !any64) return PMGPU_OK;
+    if (flags & PMGPU_FLAG_MOLECULAR_VIRIAL) any64 = true;
+    if (sys->col_grid_stale) {
+        int rg = col_set_grid(sys);
+        if (rg) return rg;
+        sys->col_grid_stale = false;
+    }
+    ColGrid g;
+    if (!col_reach(sys, std::sqrt(rc2) + (any32 ? sys->list_skin : 0.0), g)) return PMGPU_OK;
+    if (any32 && !sys->col_disabled) sys->eval_use_col = true;
+    // one cell-pair rule for all FP64 rows: a force whose own cutoff reaches
+    // beyond the algorithm's keeps the cell layout
+    if (any64 && inside) sys->eval_col64 = true;
+    if (sys->eval_use_col || sys->eval_col64) sys->eval_cg = g;
+    return PMGPU_OK;
+}
 
 // Everything that allocates or copies synchronously: force tables, buffer
 // capacities.  Runs before an evaluation is enqueued (or captured).
@@ -1592,6 +1664,12 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
     for (int k = 0; k < nf; ++k) periodic |= forces[k] && forces[k]->kind != 2;
     if (periodic && !sys->box_set) return fail(sys, PMGPU_ERR_STATE, "box not set (pmgpu_set_box)");
     int need = 1;
+    for (int k = 0; k < nf; ++k)
+        if (!forces[k] || forces[k]->sys != sys) return fail(sys, PMGPU_ERR_ARG, "force belongs to another system");
+    {
+        int rc = choose_layout(sys, nf, forces, flags);
+        if (rc) return rc;
+    }
     for (int k = 0; k < nf; ++k) {
         pmgpu_force* f = forces[k];
         if (!f || f->sys != sys) return fail(sys, PMGPU_ERR_ARG, "force belongs to another system");
@@ -1613,7 +1691,7 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
             pmgpu_force* f = forces[k];
             if (f->kind == 2)
                 return fail(sys, PMGPU_ERR_UNSUPPORTED, "molecular virial of an all-pairs (vacuum) force");
-            if (f->kind == 0) mneed += pair_blocks(sys->grid, f->nd);
+            if (f->kind == 0) mneed += row_blocks(sys, f);
             if (f->kind == 1) {
                 ++n_pme;
                 if (f->pp.real && pme_needs_lattice(f)) mneed += 148 * 4;
@@ -1636,52 +1714,36 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
         sys->cbox_cap = ncl;
         sys->buf_version++;
     }
-    // the column-cluster path takes the mixed cutoff forces of the group when
-    // none of them is in the small-grid mode and the box suits the largest
-    // of their cutoffs; otherwise the cell-cluster path takes them all
-    sys->eval_use_col = false;
-    {
-        double rc2 = 0.0;
-        bool any = false, ok = true;
-        for (int k = 0; k < nf; ++k)
-            if (forces[k]->kind == 0 && !pairs64(sys, forces[k])) {
-                any = true;
-                ok = ok && !forces[k]->wrap;
-                rc2 = std::max(rc2, forces[k]->cut2);
-            }
-        if (any && ok) {
-            if (sys->col_grid_stale) {
-                int rg = col_set_grid(sys);
-                if (rg) return rg;
-                sys->col_grid_stale = false;
-            }
-            ColGrid g;
-            if (col_reach(sys, std::sqrt(rc2) + sys->list_skin, g)) {
-                sys->eval_use_col = true;
-                sys->eval_cg = g;
-            }
-        }
-    }
     long long lneed = 0, cneed = 0;
-    if (sys->eval_use_col) {
+    if (sys->eval_use_col || sys->eval_col64) {
         const ColGrid& g = sys->eval_cg;
         const int icl = sys->n / kCluster + g.ncol + 1;
         if (icl > sys->col_ncl_cap) {
-            const size_t slots = (size_t)kCluster * icl;
+            const size_t slots = (size_t)kCluster * (icl + 1);       // and a row of padding
             CK(dalloc(&sys->d_cq, slots), "alloc"); CK(dalloc(&sys->d_cm, slots), "alloc");
             CK(dalloc(&sys->d_ibox, 2 * (size_t)icl), "alloc"); CK(dalloc(&sys->d_jbox, 4 * (size_t)icl), "alloc");
             CK(dalloc(&sys->d_ccol, (size_t)icl), "alloc"); CK(dalloc(&sys->d_facc32c, 3 * slots), "alloc");
-            CK(dalloc(&sys->d_corg, (size_t)icl), "alloc");
+            CK(dalloc(&sys->d_rowent, (size_t)icl), "alloc");
+            dfree(sys->d_c64); dfree(sys->d_facc40c);
             sys->col_ncl_cap = icl;
             sys->buf_version++;
         }
-        double rc2 = 0.0;
-        for (int k = 0; k < nf; ++k)
-            if (forces[k]->kind == 0 && !pairs64(sys, forces[k])) rc2 = std::max(rc2, forces[k]->cut2);
-        const long long entries = col_list_estimate(sys->n, g, g.lx * g.ly * g.lz, std::sqrt(rc2) + sys->list_skin);
-        lneed = 2 * entries;                  // int4 entries in the int2 list buffer
-        cneed = col_chunk_estimate(entries, sys->n, g, sys->tuning.chunk_entries);
-    } else {
+        if (sys->eval_col64 && !sys->d_c64) {
+            const size_t slots = (size_t)kCluster * (sys->col_ncl_cap + 1);
+            CK(dalloc(&sys->d_c64, slots), "alloc"); CK(dalloc(&sys->d_facc40c, 6 * slots), "alloc");
+            sys->buf_version++;
+        }
+        for (int k = 0; k < nf; ++k) {
+            if (forces[k]->kind != 0) continue;
+            const double rc = std::sqrt(forces[k]->cut2);
+            const double rl = rc + (pairs64(sys, forces[k]) ? 0.0 : sys->list_skin), vol = g.lx * g.ly * g.lz;
+            const long long entries = col_list_estimate(sys->n, g, vol, rl);
+            const int chunk = col_chunk_entries(sys->n, g, vol, rc, 6 * sys->tuning.chunk_entries, true);
+            lneed = std::max(lneed, entries / 2);      // two entries in each int2 place of the list buffer
+            cneed = std::max(cneed, col_chunk_estimate(entries, sys->n, g, chunk));
+        }
+    }
+    if (!sys->eval_use_col) {
         for (int k = 0; k < nf; ++k)
             if (forces[k]->kind == 0 && !pairs64(sys, forces[k])) {
                 lneed = std::max(lneed, plist_estimate(sys->n, sys->grid, forces[k]->nh));
@@ -1777,7 +1839,10 @@ struct EvalRun {
     int used = 0;                       // energy records
     int last_mixed = -1;                // the last mixed cutoff force (its near pairs may go to the side stream)
     int lists = 0;
-    int pair_virial = 0, col_virial = 0;
+    float list_cut2 = -1.0f, list_skin = 0.0f;   // the column list in the buffer: its cutoff^2, skin, ...
+    int list_refuse = 0, list_chunk = 0;         // ... error status, chunk length ...
+    int list_half = 0;                           // ... and form (half or full)
+    int pair_virial = 0;
     int k_next = 0;                     // the next force run_cutoffs looks at
     int deferred = -1;                  // the force whose pair kernel a batch runs
     PairArgs dargs;                     // its arguments
@@ -1811,7 +1876,6 @@ struct EvalRun {
     [[maybe_unused]] int& last_mixed = (R).last_mixed;                                                   \
     [[maybe_unused]] int& lists = (R).lists;                                                             \
     [[maybe_unused]] int& pair_virial = (R).pair_virial;                                                 \
-    [[maybe_unused]] int& col_virial = (R).col_virial;                                                   \
     [[maybe_unused]] cudaStream_t s = sys->stream;                                                       \
     [[maybe_unused]] int r = PMGPU_OK;
 
@@ -2036,7 +2100,9 @@ static int run_begin(EvalRun& R)
     for (int k = 0; k < nf; ++k)
         if (forces[k]->kind == 0 && !pairs64(sys, forces[k]) && !use_col) mixed_cells = true;
     if (mixed_cells) zero(sys->d_facc32, 2 * sizeof(unsigned long long) * n3);
-    if (use40) zero(sys->d_facc40, sizeof(unsigned long long) * n3);
+    const bool cells64 = use40 && !sys->eval_col64;
+    if (cells64) zero(sys->d_facc40, sizeof(unsigned long long) * n3);
+    if (use40 && sys->eval_col64) zero(sys->d_facc40c, sizeof(unsigned long long) * 6 * kCluster * (size_t)(sys->col_ncl_cap + 1));
     if (atom_mixed) zero(sys->d_faccA, sizeof(unsigned long long) * n3);
     if (atom_fp64) zero(sys->d_faccA + n3, sizeof(unsigned long long) * n3);
     for (int k = 0; k < nf; ++k)
@@ -2054,10 +2120,10 @@ static int run_begin(EvalRun& R)
     // ones when the column path does not take them
     cell_sort = false;
     for (int k = 0; k < nf; ++k)
-        if (forces[k]->kind == 0 && (pairs64(sys, forces[k]) || !use_col)) cell_sort = true;
-    // the molecular virial kernels of the cutoff forces read the cell-sorted
-    // order too (binned for them alone on the column path)
-    mv_bin = molvir && any_cut && !cell_sort;
+        if (forces[k]->kind == 0 && !(pairs64(sys, forces[k]) ? sys->eval_col64 : use_col)) cell_sort = true;
+    // the molecular virial kernels of the cutoff forces read the column
+    // layout, or the cell-sorted order where the columns do not apply
+    mv_bin = molvir && any_cut && !sys->eval_col64 && !cell_sort;
     used = 0;
     // with cutoff forces too, PME runs on the side stream from the start,
     // beside binning, the list and the pair kernels, and is joined before
@@ -2074,7 +2140,7 @@ static int run_begin(EvalRun& R)
         r = bin(sys, d_pos);
         if (r) return r;
     }
-    if (use_col) {
+    if (use_col || sys->eval_col64) {
         r = sys->eval_reuse ? col_refresh(sys, d_pos) : col_bin(sys, d_pos);
         if (r) return r;
     }
@@ -2102,9 +2168,35 @@ static int run_begin(EvalRun& R)
         if (forces[k]->kind == 0 && !pairs64(sys, forces[k])) last_mixed = k;
     near_on_side = false;
     lists = 0;
-    pair_virial = col_virial = 0;
+    pair_virial = 0;
     R.k_next = 0;
     R.deferred = -1;
+    return PMGPU_OK;
+}
+
+// The pair list of the next cutoff force: the one in the buffer when it was
+// built for the same test (a group's forces of one cutoff share it; the work
+// counter and the near pairs start over), else a new one.
+static int run_list(EvalRun& R, const PairArgs& a, bool col)
+{
+    PM_EVAL_RUN_NAMES(R)
+    const bool same = col && lists > 0 && R.list_cut2 == a.cut2f && R.list_skin == a.list_skin &&
+                      R.list_refuse == a.col_refuse && R.list_chunk == a.chunk && R.list_half == a.col_half;
+    if (same) {
+        CK(cudaMemsetAsync(sys->d_chunk_next, 0, 2 * sizeof(int), s), "memset");    // and the near-pair count
+        return PMGPU_OK;
+    }
+    // list count and need, chunk count and need, work counter, near-pair count
+    if (lists++ > 0) CK(cudaMemsetAsync(sys->d_plist_count, 0, 6 * sizeof(int), s), "memset");
+    int ml = prof_begin(sys, kPhaseList);
+    int e = col ? launch_col_list(a, s, &sys->launches) : launch_cluster_list(a, s, &sys->launches);
+    if (e) return cuda_fail(sys, (cudaError_t)e, "pair list");
+    prof_end(sys, ml);
+    R.list_cut2 = col ? a.cut2f : -1.0f;
+    R.list_skin = a.list_skin;
+    R.list_refuse = a.col_refuse;
+    R.list_half = a.col_half;
+    R.list_chunk = a.chunk;
     return PMGPU_OK;
 }
 
@@ -2116,30 +2208,26 @@ static int run_cutoffs(EvalRun& R, bool may_defer)
         pmgpu_force* f = forces[k];
         if (f->kind != 0) continue;
         const bool fp64 = pairs64(sys, f);
-        const bool col = !fp64 && use_col;
+        const bool col = fp64 ? sys->eval_col64 : use_col;
         if (!fp64 && !col && !f->wrap && virial) pair_virial = 1;
-        if (col && virial) col_virial = 1;
         PairArgs a;
         fill_pair_args(sys, f, d_pos, a);
-        if (col) fill_col_args(sys, a);
+        if (col) fill_col_args(sys, fp64, a, true);
         a.virial = virial;
         a.erec = sys->d_erec + used;
-        if (!fp64 && !(col && sys->eval_reuse)) {
-            // list count and need, chunk count and need, work counter
-            if (lists++ > 0) CK(cudaMemsetAsync(sys->d_plist_count, 0, 6 * sizeof(int), s), "memset");
-            int ml = prof_begin(sys, kPhaseList);
-            int e = col ? launch_col_list(a, s, &sys->launches) : launch_cluster_list(a, s, &sys->launches);
-            if (e) return cuda_fail(sys, (cudaError_t)e, "cluster-pair list");
-            prof_end(sys, ml);
+        // the column list, or the cell-cluster list of the mixed forces
+        if (col ? !sys->eval_reuse : !fp64) {
+            r = run_list(R, a, col);
+            if (r) return r;
         }
-        if (may_defer && col && !sys->eval_reuse) {
+        if (may_defer && col && !fp64 && !sys->eval_reuse) {
             // a batch runs this pair kernel with its other members' (run_resume)
             R.deferred = k;
             R.dargs = a;
             return PMGPU_OK;
         }
         int m = prof_begin(sys, kPhasePair);
-        int e = fp64 ? launch_pair_fp64(a, f->combo, pair_blocks(sys->grid, f->nd), s, &sys->launches)
+        int e = fp64 ? launch_pair_fp64(a, f->combo, col, row_blocks(sys, f), s, &sys->launches)
                      : (col ? launch_pair_col(a, f->combo, s, &sys->launches)
                             : launch_pair_mixed(a, f->combo, s, &sys->launches));
         if (e) return cuda_fail(sys, (cudaError_t)e, "pair kernel");
@@ -2155,15 +2243,25 @@ static int run_end(EvalRun& R)
 {
     PM_EVAL_RUN_NAMES(R)
     if (molvir) {
-        // the cutoff forces' molecular virial over the cell-sorted order
+        // the cutoff forces' molecular virial: over the column list (the last
+        // force's, when it holds this one's pairs and no more), or the
+        // cell-sorted order
+        const bool col = sys->eval_col64;
         for (int k = 0; k < nf; ++k) {
             pmgpu_force* f = forces[k];
             if (f->kind != 0) continue;
             PairArgs a;
             fill_pair_args(sys, f, d_pos, a);
+            if (col) {
+                fill_col_args(sys, true, a, true);
+                if (!sys->eval_reuse && R.list_cut2 != a.cut2f) {
+                    r = run_list(R, a, true);
+                    if (r) return r;
+                }
+            }
             a.molpos = sys->d_molpos; a.mrec = sys->d_mrec + mused; a.mrec_stride = sys->mrec_cap;
-            const int blocks = pair_blocks(sys->grid, f->nd);
-            int e = launch_pair_molvir(a, f->combo, blocks, s, &sys->launches);
+            const int blocks = row_blocks(sys, f);
+            int e = launch_pair_molvir(a, f->combo, col, blocks, s, &sys->launches);
             if (e) return cuda_fail(sys, (cudaError_t)e, "molecular virial");
             mused += blocks;
         }
@@ -2182,14 +2280,13 @@ static int run_end(EvalRun& R)
         // the slot-ordered accumulators exist only with the cell-sorted order
         fa.f32 = mixed_cells ? sys->d_facc32 : nullptr;
         fa.f32p = mixed_cells ? sys->d_facc32p : nullptr;
-        fa.f40 = use40 && cell_sort ? sys->d_facc40 : nullptr;
-        if (use_col) {
-            fa.c32 = sys->d_facc32c; fa.c_slot_of = sys->d_cslot; fa.cq = sys->d_cq;
+        fa.f40 = use40 && cell_sort && !sys->eval_col64 ? sys->d_facc40 : nullptr;
+        if (use_col || sys->eval_col64) {
+            fa.c32 = use_col ? sys->d_facc32c : nullptr;
+            fa.c40 = use40 && sys->eval_col64 ? sys->d_facc40c : nullptr;
+            fa.c44 = fa.c40 ? sys->d_facc40c + 3 * kCluster * (size_t)(sys->col_ncl_cap + 1) : nullptr;
+            fa.c_slot_of = sys->d_cslot;
             fa.c_slots = kCluster * sys->col_ncl_cap;
-            fa.corg = sys->d_corg;
-            fa.cscale[0] = sys->eval_cg.lx / 4294967296.0;
-            fa.cscale[1] = sys->eval_cg.ly / 4294967296.0;
-            fa.cscale[2] = sys->eval_cg.lz / 4294967296.0;
         }
         for (int k = 0; k < nf; ++k)
             if (forces[k]->kind != 0) {
@@ -2197,7 +2294,7 @@ static int run_end(EvalRun& R)
                 else fa.a32 = sys->d_faccA;
             }
         fa.sorted = cell_sort ? sys->d_sorted : nullptr; fa.spos = sys->d_spos; fa.slo = sys->d_slo;
-        fa.pair_virial = pair_virial | (col_virial << 1);
+        fa.pair_virial = pair_virial;
         fa.fout = d_fout;
         fa.erec = sys->d_erec + used; fa.erec_stride = sys->erec_cap;
         int rec = 0;
@@ -2274,14 +2371,18 @@ static int eval_core(pmgpu_system* sys, int nf_in, pmgpu_force* const* forces_in
     // list is the system's only one), a rebuild period above one, a list
     // built for these forces, still valid and younger than the period
     std::vector<long long> ids;
-    int n_mixed_cut = 0;
+    int n_mixed_cut = 0, n_fp64_cut = 0;
     for (int k = 0; k < nf; ++k) {
         ids.push_back(forces[k]->id);
         if (forces[k]->kind == 0 && !pairs64(sys, forces[k])) ++n_mixed_cut;
+        if (forces[k]->kind == 0 && pairs64(sys, forces[k])) ++n_fp64_cut;
     }
-    const bool can_reuse = sys->eval_use_col && sys->list_every > 1 && n_mixed_cut == 1;
+    // (an FP64 force of the group on the columns lists its own pairs)
+    const bool can_reuse = sys->eval_use_col && sys->list_every > 1 && n_mixed_cut == 1 &&
+                           !(sys->eval_col64 && n_fp64_cut > 0);
     sys->eval_reuse = can_reuse && sys->list_valid && sys->list_ids == ids && sys->evals_since_build < sys->list_every;
     auto note_list = [&]() {
+        if (sys->eval_col64 && n_fp64_cut > 0) sys->list_valid = false;    // the FP64 forces' list took its place
         if (!sys->eval_use_col || n_mixed_cut == 0) return;
         if (sys->eval_reuse) {
             sys->evals_since_build++;
@@ -2481,13 +2582,14 @@ extern "C" int pmgpu_get_pairs(pmgpu_system* sys, pmgpu_force* f, const double* 
     CK(cudaMemsetAsync(sys->d_facc32, 0, 2 * sizeof(unsigned long long) * n3, s), "memset");
     CK(cudaMemsetAsync(sys->d_facc40, 0, sizeof(unsigned long long) * n3, s), "memset");
     bool fp64 = pairs64(sys, f);
-    const bool col = !fp64 && sys->eval_use_col;          // eval_prepare decided for this force alone
+    const bool col = fp64 ? sys->eval_col64 : sys->eval_use_col;   // eval_prepare decided for this force alone
     if (f->precision != PMGPU_PRECISION_FP64)
         sys->last_layout = fp64 ? PMGPU_LAYOUT_FP64 : (col ? PMGPU_LAYOUT_COLUMNS : PMGPU_LAYOUT_CELLS);
     if (col) {
-        CK(cudaMemsetAsync(sys->d_facc32c, 0, sizeof(unsigned long long) * 3 * kCluster * (size_t)sys->col_ncl_cap, s),
-           "memset");
+        CK(cudaMemsetAsync(fp64 ? sys->d_facc40c : sys->d_facc32c, 0, sizeof(unsigned long long) * (fp64 ? 6 : 3) *
+                           kCluster * (size_t)(sys->col_ncl_cap + (fp64 ? 1 : 0)), s), "memset");
         r = col_bin(sys, sys->d_pos);
+        sys->list_valid = false;
     } else {
         r = bin(sys, sys->d_pos);
     }
@@ -2502,14 +2604,14 @@ extern "C" int pmgpu_get_pairs(pmgpu_system* sys, pmgpu_force* f, const double* 
     CK(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), s), "memset");
     PairArgs a;
     fill_pair_args(sys, f, sys->d_pos, a);
-    if (col) fill_col_args(sys, a);
+    if (col) fill_col_args(sys, fp64, a, true);
     a.near2 = 0.0f;                                    // recording only: no near-pair list
     a.erec = sys->d_erec;
     a.rec_pairs = d_pairs; a.rec_count = d_count; a.rec_cap = dcap;
-    int e = fp64 ? launch_pair_fp64(a, f->combo, pair_blocks(sys->grid, f->nd), s, &sys->launches)
-                 : (col ? launch_col_list(a, s, &sys->launches) : launch_cluster_list(a, s, &sys->launches));
-    if (!e && !fp64) e = col ? launch_pair_col(a, f->combo, s, &sys->launches)
-                             : launch_pair_mixed(a, f->combo, s, &sys->launches);
+    int e = col ? launch_col_list(a, s, &sys->launches) : (fp64 ? 0 : launch_cluster_list(a, s, &sys->launches));
+    if (!e) e = fp64 ? launch_pair_fp64(a, f->combo, col, row_blocks(sys, f), s, &sys->launches)
+                     : (col ? launch_pair_col(a, f->combo, s, &sys->launches)
+                            : launch_pair_mixed(a, f->combo, s, &sys->launches));
     unsigned long long cnt = 0;
     int st = 0;
     if (!e) e = (int)cudaMemcpyAsync(&cnt, d_count, sizeof(cnt), cudaMemcpyDeviceToHost, s);
@@ -3428,7 +3530,7 @@ extern "C" int pmgpu_adjoint(pmgpu_system* sys, int n_forces, pmgpu_force* const
         fl.push_back(forces_in[k]);
     }
     if (hv && !v) return fail(sys, PMGPU_ERR_ARG, "Hessian-vector product needs v");
-    int r = eval_prepare(sys, (int)fl.size(), fl.data(), 0);
+    int r = eval_prepare(sys, (int)fl.size(), fl.data(), kFlagNeeds64);
     if (r) return r;
     if (hv)
         for (pmgpu_force* f : fl) {
@@ -3449,32 +3551,54 @@ extern "C" int pmgpu_adjoint(pmgpu_system* sys, int n_forces, pmgpu_force* const
     const int n = sys->n, T = sys->t;
     cudaStream_t s = sys->stream;
     size_t n3 = 3 * (size_t)n;
-    double *d_v = nullptr, *d_dq = nullptr, *d_lj = nullptr, *d_hv = nullptr, *d_e = nullptr;
-    auto cleanup = [&]() { dfree(d_v); dfree(d_dq); dfree(d_lj); dfree(d_hv); dfree(d_e); };
     cudaError_t e = cudaSuccess;
     auto ok = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
-    ok(cudaMemcpyAsync(sys->d_pos, positions, sizeof(double) * n3, cudaMemcpyHostToDevice, s));
-    ok(cudaMemsetAsync(sys->d_small, 0, kSmallBytes, s));
-    ok(dalloc(&d_dq, (size_t)n)); ok(dalloc(&d_lj, (size_t)T * T * 4)); ok(dalloc(&d_e, 2));
-    if (hv) { ok(dalloc(&d_v, n3)); ok(dalloc(&d_hv, n3)); }
-    if (e == cudaSuccess) {
-        ok(cudaMemsetAsync(d_dq, 0, sizeof(double) * n, s));
-        ok(cudaMemsetAsync(d_lj, 0, sizeof(double) * T * T * 4, s));
-        ok(cudaMemsetAsync(d_e, 0, sizeof(double) * 2, s));
-        if (hv) {
-            ok(cudaMemcpyAsync(d_v, v, sizeof(double) * n3, cudaMemcpyHostToDevice, s));
-            ok(cudaMemsetAsync(d_hv, 0, sizeof(double) * n3, s));
+    const size_t nlj = (size_t)T * T * 4;
+    const bool sparse = nlj < (1ull << 31);
+    if (!sys->d_adj) {
+        ok(dalloc(&sys->d_adj, 7 * (size_t)n + 2));
+        ok(cudaMallocHost((void**)&sys->h_adj, sizeof(double) * (4 * (size_t)n + 3)));
+    }
+    if (dE_dlj && !sys->d_adj_lj) {
+        ok(dalloc(&sys->d_adj_lj, nlj));
+        if (sparse) {
+            ok(dalloc(&sys->d_adj_val, nlj)); ok(dalloc(&sys->d_adj_idx, nlj)); ok(dalloc(&sys->d_adj_count, 1));
         }
     }
-    if (e != cudaSuccess) { cleanup(); return cuda_fail(sys, e, "adjoint setup"); }
+    if (e != cudaSuccess) {
+        dfree(sys->d_adj); dfree(sys->d_adj_lj);          // a half-made set is made again by the next call
+        dfree(sys->d_adj_val); dfree(sys->d_adj_idx); dfree(sys->d_adj_count);
+        if (sys->h_adj) { cudaFreeHost(sys->h_adj); sys->h_adj = nullptr; }
+        return cuda_fail(sys, e, "adjoint setup");
+    }
+    double* d_dq = sys->d_adj;
+    double* d_hv = hv ? d_dq + n : nullptr;
+    double* d_v = hv ? d_dq + 4 * (size_t)n : nullptr;
+    double* d_e = d_dq + 7 * (size_t)n;
+    double* d_lj = dE_dlj ? sys->d_adj_lj : nullptr;
+    ok(cudaMemcpyAsync(sys->d_pos, positions, sizeof(double) * n3, cudaMemcpyHostToDevice, s));
+    ok(cudaMemsetAsync(sys->d_small, 0, kSmallBytes, s));
+    ok(cudaMemsetAsync(sys->d_adj, 0, sizeof(double) * (hv ? 4 * (size_t)n : (size_t)n), s));
+    ok(cudaMemsetAsync(d_e, 0, sizeof(double) * 2, s));
+    if (d_lj) ok(cudaMemsetAsync(d_lj, 0, sizeof(double) * nlj, s));
+    if (d_lj && sparse) ok(cudaMemsetAsync(sys->d_adj_count, 0, sizeof(unsigned), s));
+    if (hv) ok(cudaMemcpyAsync(d_v, v, sizeof(double) * n3, cudaMemcpyHostToDevice, s));
+    if (e != cudaSuccess) return cuda_fail(sys, e, "adjoint setup");
     // cutoff forces run over the cell list of the positions (the forward
     // kernels' cell-sorted order)
     bool any_cut = false;
     for (pmgpu_force* f : fl) any_cut |= f->kind == 0;
     if (any_cut) {
-        r = bin(sys, sys->d_pos);
-        if (r) { cleanup(); return r; }
+        if (sys->eval_col64) {
+            sys->eval_use_col = false;               // no mixed forces here: nothing refuses the columns
+            sys->list_valid = false;
+            r = col_bin(sys, sys->d_pos);
+        } else {
+            r = bin(sys, sys->d_pos);
+        }
+        if (r) return r;
     }
+    float listed = -1.0f;
     std::vector<double> host_dq(n, 0.0);
     for (pmgpu_force* f : fl) {
         const bool fp64 = f->precision == PMGPU_PRECISION_FP64;
@@ -3485,8 +3609,16 @@ extern "C" int pmgpu_adjoint(pmgpu_system* sys, int n_forces, pmgpu_force* const
             if (f->kind == 0) {
                 PairArgs pa;
                 fill_pair_args(sys, f, sys->d_pos, pa);
-                ok((cudaError_t)launch_pair_adjoint_cells(pa, a, fp64 ? 1 : 0, pair_blocks(sys->grid, f->nd), s,
-                                                          &sys->launches));
+                if (sys->eval_col64) {
+                    fill_col_args(sys, true, pa, false);
+                    if (listed != pa.cut2f) {
+                        if (listed >= 0.0f) ok(cudaMemsetAsync(sys->d_plist_count, 0, 6 * sizeof(int), s));
+                        ok((cudaError_t)launch_col_list(pa, s, &sys->launches));
+                        listed = pa.cut2f;
+                    }
+                }
+                ok((cudaError_t)launch_pair_adjoint_rows(pa, a, fp64 ? 1 : 0, sys->eval_col64, row_blocks(sys, f), s,
+                                                         &sys->launches));
             } else {
                 ok((cudaError_t)launch_pair_adjoint(a, fp64 ? 1 : 0, s, &sys->launches));
             }
@@ -3538,17 +3670,44 @@ extern "C" int pmgpu_adjoint(pmgpu_system* sys, int n_forces, pmgpu_force* const
             }
         }
     }
-    std::vector<double> out_dq(n), out_lj((size_t)T * T * 4), out_hv(hv ? n3 : 0), out_e(2);
-    ok(cudaMemcpyAsync(out_dq.data(), d_dq, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-    ok(cudaMemcpyAsync(out_lj.data(), d_lj, sizeof(double) * out_lj.size(), cudaMemcpyDeviceToHost, s));
-    ok(cudaMemcpyAsync(out_e.data(), d_e, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
-    if (hv) ok(cudaMemcpyAsync(out_hv.data(), d_hv, sizeof(double) * n3, cudaMemcpyDeviceToHost, s));
+    // results: dq, hv and the energies to pinned memory, the LJ gradient as its
+    // nonzero entries (the whole table where their 32-bit index is too short)
+    double* h = sys->h_adj;
+    unsigned* h_count = reinterpret_cast<unsigned*>(h + 4 * (size_t)n + 2);
+    *h_count = 0;
+    ok(cudaMemcpyAsync(h, sys->d_adj, sizeof(double) * (hv ? 4 * (size_t)n : (size_t)n), cudaMemcpyDeviceToHost, s));
+    ok(cudaMemcpyAsync(h + 4 * (size_t)n, d_e, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
+    if (d_lj && sparse && e == cudaSuccess) {
+        ok((cudaError_t)launch_lj_entries(d_lj, (unsigned)nlj, sys->d_adj_idx, sys->d_adj_val, sys->d_adj_count, s,
+                                          &sys->launches));
+        ok(cudaMemcpyAsync(h_count, sys->d_adj_count, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    }
     ok(cudaStreamSynchronize(s));
-    cleanup();
+    const size_t nz = e == cudaSuccess ? *h_count : 0;
+    if (nz > sys->h_adj_cap) {
+        if (sys->h_adj_val) cudaFreeHost(sys->h_adj_val);
+        if (sys->h_adj_idx) cudaFreeHost(sys->h_adj_idx);
+        sys->h_adj_val = nullptr; sys->h_adj_idx = nullptr; sys->h_adj_cap = 0;
+        const size_t cap = std::min(nlj, nz + nz / 4);
+        ok(cudaMallocHost((void**)&sys->h_adj_val, sizeof(double) * cap));
+        ok(cudaMallocHost((void**)&sys->h_adj_idx, sizeof(unsigned) * cap));
+        if (e == cudaSuccess) sys->h_adj_cap = cap;
+    }
+    std::vector<double> dense;
+    if (e == cudaSuccess && nz > 0) {
+        ok(cudaMemcpyAsync(sys->h_adj_val, sys->d_adj_val, sizeof(double) * nz, cudaMemcpyDeviceToHost, s));
+        ok(cudaMemcpyAsync(sys->h_adj_idx, sys->d_adj_idx, sizeof(unsigned) * nz, cudaMemcpyDeviceToHost, s));
+        ok(cudaStreamSynchronize(s));
+    } else if (e == cudaSuccess && d_lj && !sparse) {
+        dense.resize(nlj);
+        ok(cudaMemcpyAsync(dense.data(), d_lj, sizeof(double) * nlj, cudaMemcpyDeviceToHost, s));
+        ok(cudaStreamSynchronize(s));
+    }
     if (e != cudaSuccess) return cuda_fail(sys, e, "adjoint");
-    if (dE_dq) for (int i = 0; i < n; ++i) dE_dq[i] += out_dq[i] + host_dq[i];
-    if (dE_dlj) for (size_t k = 0; k < out_lj.size(); ++k) dE_dlj[k] += out_lj[k];
-    if (hv) for (size_t k = 0; k < n3; ++k) hv[k] += out_hv[k];
-    if (energies) { energies[0] += out_e[0]; energies[1] += out_e[1]; }
+    if (dE_dq) for (int i = 0; i < n; ++i) dE_dq[i] += h[i] + host_dq[i];
+    if (hv) for (size_t k = 0; k < n3; ++k) hv[k] += h[n + k];
+    for (size_t k = 0; k < nz; ++k) dE_dlj[sys->h_adj_idx[k]] += sys->h_adj_val[k];
+    for (size_t k = 0; k < dense.size(); ++k) dE_dlj[k] += dense[k];
+    if (energies) { energies[0] += h[4 * (size_t)n]; energies[1] += h[4 * (size_t)n + 1]; }
     return PMGPU_OK;
 }

@@ -1,0 +1,172 @@
+"""The pair kernels over rows of column clusters where they can go wrong: small
+and flat boxes (the list's half by row parity instead of by half plane), two
+different cutoffs, j-forces too large for their 32-bit sums, and lists and
+columns that outgrow their estimates.
+
+Bounds, set before the first run: those of the parity suite (forces within 1e-5
+relative RMS mixed, 1e-11 of the RMS force FP64; pair sets equal; energies
+within 1e-6 of |E_LJ| + |E_C| on a few hundred atoms, 1e-11 FP64).
+"""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from oracle import oracle
+from protomol_b200 import forces as F
+from protomol_b200 import systems, workloads
+
+pytestmark = pytest.mark.gpu
+
+LJ9 = "LennardJones -switchingFunction C2 -algorithm NonbondedCutoff -switchon 8 -cutoff 9 -cutoff 9"
+CUTS_8_9 = ("LennardJones CoulombEwaldReal -switchingFunction C2 -switchingFunction Cutoff "
+            "-algorithm NonbondedCutoff -switchon 7 -cutoff 9 -alpha 0.35 -cutoff 8 -cutoff 9")
+
+
+def _box(lengths):
+    b = np.zeros((4, 3))
+    b[0, 0], b[1, 1], b[2, 2] = lengths
+    return b
+
+
+def _fluid(positions, lengths, charges=None):
+    """Oxygen-like atoms without molecules at the given places."""
+    base = systems.oxygen_fluid_216()
+    n = len(positions)
+    return dataclasses.replace(
+        base, positions=np.asarray(positions, float), scaled_charge=np.zeros(n) if charges is None else charges,
+        atom_type=np.zeros(n, np.int32), molecule=np.arange(n, dtype=np.int32), mass=np.full(n, 15.9994),
+        box=_box(lengths), cell_size=4.5)
+
+
+def _eval(s, defs, precision):
+    topo = F.Topology(s)
+    fs = [F.ForceFactory.make(topo, d, precision) for d in defs]
+    f, e = np.zeros((s.n_atoms, 3)), F.ScalarStructure()
+    F.evaluate_group(topo, fs, s.positions, f, e)
+    return topo, fs, f, e
+
+
+def _check(s, defs, precision, energy=None):
+    ref = oracle.evaluate(s, [F.parse_definition(d) for d in defs])
+    topo, fs, f, e = _eval(s, defs, precision)
+    rms = np.sqrt((ref["forces"] ** 2).mean())
+    scale = abs(ref["lennard_jones"]) + abs(ref["coulomb"])
+    if precision == "fp64":
+        assert np.abs(f - ref["forces"]).max() <= 1e-11 * max(rms, np.abs(ref["forces"]).max())
+        tol = 1e-11
+    else:
+        assert np.sqrt(((f - ref["forces"]) ** 2).mean()) <= 1e-5 * rms
+        tol = energy or 1e-6
+    assert abs(e.lennard_jones - ref["lennard_jones"]) <= tol * scale
+    assert abs(e.coulomb - ref["coulomb"]) <= tol * scale
+    assert np.abs(e.virial_tensor - ref["virial"]).max() <= tol * np.abs(ref["virial"]).max()
+    return topo, fs, ref
+
+
+def _same_pairs(s, d, force):
+    ref = oracle.evaluate(s, [F.parse_definition(d)], want_pairs=True)["pairs"]
+    key = lambda p: np.sort(p[:, 0].astype(np.int64) * s.n_atoms + p[:, 1])
+    assert np.array_equal(key(force.pairs(s.positions)), key(ref))
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("lengths", [(18.3, 18.3, 18.3), (19.1, 23.7, 40.9), (45.2, 18.5, 27.3), (37.0, 41.0, 18.2)])
+def test_small_and_flat_boxes(lengths, precision):
+    k = [int(x // 3.05) for x in lengths]
+    g = np.stack(np.meshgrid(*[np.arange(m) for m in k], indexing="ij"), -1).reshape(-1, 3)
+    sites = (g + 0.5) * (np.array(lengths) / k) - np.array(lengths) / 2
+    s = dataclasses.replace(systems.water_box(len(sites), 7), box=_box(lengths),
+                            positions=systems._water_atoms(np.random.default_rng(7), sites, jitter=0.1))
+    d = workloads.lj_ewald_split(8, 9, 0.35)
+    topo, fs, _ = _check(s, [d], precision)
+    if precision == "mixed":
+        assert topo.pair_layout() == "columns"
+    _same_pairs(s, d, fs[0])
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 8, 9, 33])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_a_few_atoms(n, precision):
+    rng = np.random.default_rng(n)
+    g = np.stack(np.meshgrid(*[np.arange(5)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = (g[rng.permutation(len(g))[:n]] + 0.5) * 4.1 - 10.2 + rng.uniform(-0.4, 0.4, (n, 3))
+    s = _fluid(pos, (20.5, 20.5, 20.5))
+    if n == 1:
+        _, _, f, e = _eval(s, [LJ9], precision)
+        assert not f.any() and e.lennard_jones == 0.0
+    else:
+        _check(s, [LJ9], precision)
+
+
+@pytest.mark.parametrize("lengths", [(18.3, 19.0, 21.0), (38.0, 38.0, 38.0)])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_two_cutoffs(lengths, precision):
+    """Pairs of the outer cutoff only, with distances at the inner one."""
+    rng = np.random.default_rng(5)
+    k = [int(x // 3.2) for x in lengths]
+    g = np.stack(np.meshgrid(*[np.arange(m) for m in k], indexing="ij"), -1).reshape(-1, 3)
+    pos = (g + 0.5) * (np.array(lengths) / k) - np.array(lengths) / 2 + rng.uniform(-0.2, 0.2, (len(g), 3))
+    for i in range(0, 60, 2):                           # partners at 8 A (1 +- 1e-9) of atom i
+        u = rng.normal(size=3)
+        pos[-1 - i] = pos[i] + u / np.linalg.norm(u) * 8.0 * (1.0 + (1e-9 if i % 4 else -1e-9))
+    d2 = pos[:, None] - pos[None]
+    d2 -= np.array(lengths) * np.rint(d2 / np.array(lengths))
+    r = np.sqrt((d2 ** 2).sum(-1)) + 10.0 * np.eye(len(pos))
+    keep = r.min(1) > 2.4                               # drop partners that landed on an atom
+    pos = pos[keep]
+    q = np.where(np.arange(len(pos)) % 2 == 0, 4.0, -4.0)
+    _check(_fluid(pos, lengths, q), [CUTS_8_9], precision, energy=2e-6)
+
+
+@pytest.mark.parametrize("r", [2.5, 2.25, 2.0])
+def test_forces_beyond_the_32_bit_sums(r):
+    """Pairs whose force exceeds the 60 kcal/mol/A that the j side holds in 32
+    bits, several of them on one atom, among ordinary ones."""
+    rng = np.random.default_rng(11)
+    g = np.stack(np.meshgrid(*[np.arange(8)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = (g + 0.5) * 5.2 - 20.8 + rng.uniform(-0.1, 0.1, (len(g), 3))
+    extra = []
+    for i in (0, 77, 300):
+        for axis in range(3):
+            u = np.zeros(3)
+            u[axis] = r
+            extra.append(pos[i] + u)
+    _check(_fluid(np.concatenate([pos, extra]), (41.6, 41.6, 41.6)), [LJ9], "mixed")
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_a_droplet_outgrows_the_list_estimate(precision):
+    """3,375 atoms in the middle of a 150 A box: the list estimate follows the
+    mean density.  The mixed evaluation is repeated with a grown list, the FP64
+    one needs none."""
+    rng = np.random.default_rng(2)
+    g = np.stack(np.meshgrid(*[np.arange(15)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = (g - 7.0) * 3.3 + rng.uniform(-0.2, 0.2, (len(g), 3))
+    s = _fluid(pos, (150.0, 150.0, 150.0))
+    _, fs, _ = _check(s, [LJ9], precision)
+    _same_pairs(s, LJ9, fs[0])
+
+
+def test_a_column_of_more_atoms_than_the_sort_holds():
+    """2,300 atoms on one line along z: one column holds them all.  The FP64
+    forces take the column unsorted."""
+    rng = np.random.default_rng(3)
+    z = (np.arange(2300) - 1150) * 3.9
+    pos = np.stack([0.3 + 0 * z, 0.4 + 0 * z, z], 1) + rng.uniform(-0.2, 0.2, (2300, 3))
+    _check(_fluid(pos, (30.0, 30.0, 2300 * 3.9)), [LJ9], "fp64")
+
+
+def test_reused_list_survives_an_fp64_evaluation_between():
+    """An FP64 evaluation (its own list, in the same buffers) between two
+    evaluations of a reused mixed list."""
+    s = systems.water_box(2100, 4)
+    d = workloads.lj_ewald_split(8, 9, 0.35)
+    topo = F.Topology(s)
+    mixed, fp64 = F.ForceFactory.make(topo, d, "mixed"), F.ForceFactory.make(topo, d, "fp64")
+    topo.set_pair_list(1.0, 10)
+    ref = oracle.evaluate(s, [F.parse_definition(d)])["forces"]
+    for fs in ([mixed], [fp64], [mixed], [mixed, fp64], [mixed]):
+        out = np.zeros((s.n_atoms, 3))
+        F.evaluate_group(topo, fs, s.positions, out, F.ScalarStructure())
+        assert np.sqrt(((out / len(fs) - ref) ** 2).mean()) <= 1e-5 * np.sqrt((ref ** 2).mean())
