@@ -532,6 +532,32 @@ struct ConsArgs {
     int* hits;                   // sweeps that ended at max_iter (+1 each)
 };
 int launch_shake(const ConsArgs& a, cudaStream_t s, long long* launches);
+// One Leapfrog step up to the next evaluation (kick [RATTLE, kick], drift,
+// SHAKE, forces and energies cleared), or the run's end (half kick, RATTLE),
+// in one launch, when every cluster of constraints has at most three atoms
+// (its constraints those of the atoms 0-1, 0-2, 1-2, in this order) and there
+// are at most kTriThreads of them.
+constexpr int kTriThreads = 512;
+struct RigidArgs {
+    int n_cons, n_clusters;
+    const int4* atoms;           // per cluster: its atoms (-1: none), number of constraints
+    const double* rest;          // 3 per cluster: rest lengths
+    int n_free;
+    const int* free_atoms;       // the atoms of no constraint
+    const double* mass;
+    double* pos;
+    double* vel;
+    double* force;
+    double* energy;              // kERec doubles
+    double h, hk, dt;
+    int first, drift;            // the run's first kick; a drift follows (else the run's end)
+    int rattle, shake;
+    double rattle_eps, shake_eps;
+    int rattle_iter, shake_iter;
+    double* virial;              // RATTLE's virial (+=) or null
+    int* hits;
+};
+int launch_rigid_step(const RigidArgs& a, cudaStream_t s, long long* launches);
 int launch_rattle(const ConsArgs& a, cudaStream_t s, long long* launches);
 
 }  // namespace pm

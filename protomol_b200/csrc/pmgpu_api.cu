@@ -91,6 +91,12 @@ struct pmgpu_system {
     // clusters of constraints sharing atoms, SHAKE's last positions
     int n_cons = 0, n_ccl = 0;
     int* d_cl_start = nullptr;
+    // clusters of at most three atoms each (k_rigid_step), and the free atoms
+    bool cons_tri = false;
+    int n_free = 0;
+    int4* d_tri_atoms = nullptr;
+    double* d_tri_rest = nullptr;
+    int* d_free = nullptr;
     int2* d_cons_atoms = nullptr;
     double* d_cons_rest = nullptr;
     double* d_cons_last = nullptr;
@@ -437,7 +443,7 @@ extern "C" int pmgpu_system_destroy(pmgpu_system* sys)
     free_col_buffers(sys);
     dfree(sys->d_counts); dfree(sys->d_start); dfree(sys->d_erec); dfree(sys->d_mrec);
     dfree(sys->d_cl_start); dfree(sys->d_cons_atoms); dfree(sys->d_cons_rest); dfree(sys->d_cons_last);
-    dfree(sys->d_cons_hits);
+    dfree(sys->d_cons_hits); dfree(sys->d_tri_atoms); dfree(sys->d_tri_rest); dfree(sys->d_free);
     dfree(sys->d_small); dfree(sys->d_energy);
     dfree(sys->d_cstart); dfree(sys->d_cbox); dfree(sys->d_ccell); dfree(sys->d_plist); dfree(sys->d_chunks);
     dfree(sys->d_near);
@@ -3337,6 +3343,33 @@ extern "C" int pmgpu_leapfrog_run(pmgpu_system* sys, int n_forces, pmgpu_force* 
         int e = launch_rattle(a, s, &sys->launches);
         return e ? cuda_fail(sys, (cudaError_t)e, "RATTLE") : PMGPU_OK;
     };
+    if ((shake || rattle) && sys->cons_tri) {
+        // small clusters: everything between two evaluations in one launch
+        RigidArgs ra;
+        memset(&ra, 0, sizeof(ra));
+        ra.n_cons = sys->n_cons; ra.n_clusters = sys->n_ccl; ra.atoms = sys->d_tri_atoms; ra.rest = sys->d_tri_rest;
+        ra.n_free = sys->n_free; ra.free_atoms = sys->d_free; ra.mass = d_mass;
+        ra.pos = d_positions; ra.vel = d_velocities; ra.force = d_forces; ra.energy = d_energies;
+        ra.h = h; ra.dt = ca.dt; ra.hits = ca.hits;
+        ra.shake = shake; ra.shake_eps = sys->shake_eps; ra.shake_iter = sys->shake_iter;
+        ra.rattle_eps = sys->rattle_eps; ra.rattle_iter = sys->rattle_iter;
+        for (int step = 0; step <= n_steps; ++step) {
+            ra.first = step == 0;
+            ra.drift = step < n_steps;
+            ra.rattle = step > 0 && rattle;
+            // a step without RATTLE kicks once by the whole step (k_leapfrog's
+            // middle form), one with it, and the run's end, by half steps
+            ra.hk = ra.drift && !ra.rattle ? h : hk;
+            // (a RATTLE before a drift leaves no virial: the evaluation clears it)
+            ra.virial = !ra.drift && (flags & PMGPU_FLAG_VIRIAL) ? d_energies + 2 : nullptr;
+            int e = launch_rigid_step(ra, s, &sys->launches);
+            if (e) return cuda_fail(sys, (cudaError_t)e, "constrained step");
+            if (!ra.drift) break;
+            int r = eval_core(sys, n_forces, forces, d_positions, d_forces, d_energies, flags);
+            if (r) return r;
+        }
+        return PMGPU_OK;
+    }
     // ModifierMetaRattleShake::doInitialize: the last positions start as the positions
     if (shake)
         CK(cudaMemcpyAsync(sys->d_cons_last, d_positions, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s), "copy");
@@ -3439,6 +3472,47 @@ extern "C" int pmgpu_set_constraints(pmgpu_system* sys, int n_constraints, const
     if (!sys->d_cons_hits) {
         CK(dalloc(&sys->d_cons_hits, 1), "alloc");
         CK(cudaMemset(sys->d_cons_hits, 0, sizeof(int)), "memset");
+    }
+    // clusters of at most three atoms, their constraints as k_rigid_step
+    // takes them (0-1, 0-2, 1-2: atom 0 is the one the first two share)
+    std::vector<int4> tri;
+    std::vector<double> tri_rest;
+    sys->cons_tri = n_constraints > 0 && members.size() <= (size_t)kTriThreads;
+    for (size_t c = 0; c < members.size() && sys->cons_tri; ++c) {
+        const std::vector<int>& m = members[c];
+        const int nk = (int)m.size();
+        if (nk > 3) { sys->cons_tri = false; break; }
+        int p[3][2];
+        for (int k = 0; k < nk; ++k) { p[k][0] = atoms[2 * m[k]]; p[k][1] = atoms[2 * m[k] + 1]; }
+        int a0 = p[0][0], a1 = p[0][1], a2 = -1;
+        if (nk > 1) {
+            if (p[1][0] == a1 || p[1][1] == a1) std::swap(a0, a1);
+            a2 = p[1][0] == a0 ? p[1][1] : p[1][0];
+            sys->cons_tri = (p[1][0] == a0 || p[1][1] == a0) && a2 != a1;
+        }
+        if (nk > 2)
+            sys->cons_tri = sys->cons_tri && ((p[2][0] == a1 && p[2][1] == a2) || (p[2][0] == a2 && p[2][1] == a1));
+        tri.push_back(make_int4(a0, a1, a2, nk));
+        for (int k = 0; k < 3; ++k) tri_rest.push_back(k < nk ? rest_length[m[k]] : 1.0);
+    }
+    dfree(sys->d_tri_atoms); dfree(sys->d_tri_rest); dfree(sys->d_free);
+    sys->n_free = 0;
+    if (sys->cons_tri) {
+        std::vector<char> held(n, 0);
+        for (const int4& t : tri)
+            for (int a : {t.x, t.y, t.z})
+                if (a >= 0) held[a] = 1;
+        std::vector<int> free_atoms;
+        for (int i = 0; i < n; ++i)
+            if (!held[i]) free_atoms.push_back(i);
+        CK(dalloc(&sys->d_tri_atoms, tri.size()), "alloc");
+        CK(dalloc(&sys->d_tri_rest, tri_rest.size()), "alloc");
+        CK(dalloc(&sys->d_free, std::max<size_t>(free_atoms.size(), 1)), "alloc");
+        CK(cudaMemcpy(sys->d_tri_atoms, tri.data(), sizeof(int4) * tri.size(), cudaMemcpyHostToDevice), "copy");
+        CK(cudaMemcpy(sys->d_tri_rest, tri_rest.data(), sizeof(double) * tri_rest.size(), cudaMemcpyHostToDevice), "copy");
+        if (!free_atoms.empty())
+            CK(cudaMemcpy(sys->d_free, free_atoms.data(), sizeof(int) * free_atoms.size(), cudaMemcpyHostToDevice), "copy");
+        sys->n_free = (int)free_atoms.size();
     }
     sys->n_cons = n_constraints;
     sys->n_ccl = (int)members.size();

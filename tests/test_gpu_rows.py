@@ -1,7 +1,7 @@
 """The pair kernels over rows of column clusters where they can go wrong: small
 and flat boxes (the list's half by row parity instead of by half plane), two
-different cutoffs, j-forces too large for their 32-bit sums, and lists and
-columns that outgrow their estimates.
+different cutoffs, j-forces too large for their 32-bit sums, lists and columns
+that outgrow their estimates, and the constrained step's clusters of every shape.
 
 Bounds, set before the first run: those of the parity suite (forces within 1e-5
 relative RMS mixed, 1e-11 of the RMS force FP64; pair sets equal; energies
@@ -14,7 +14,7 @@ import pytest
 
 from oracle import oracle
 from protomol_b200 import forces as F
-from protomol_b200 import systems, workloads
+from protomol_b200 import integrate, systems, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -170,3 +170,43 @@ def test_reused_list_survives_an_fp64_evaluation_between():
         out = np.zeros((s.n_atoms, 3))
         F.evaluate_group(topo, fs, s.positions, out, F.ScalarStructure())
         assert np.sqrt(((out / len(fs) - ref) ** 2).mean()) <= 1e-5 * np.sqrt((ref ** 2).mean())
+
+
+@pytest.mark.parametrize("shape", ["pairs", "stars", "triangles", "mixed_order", "chains", "many"])
+def test_constrained_steps(shape):
+    """Clusters of two and three atoms in any order of their constraints (the
+    one-launch step), four-atom chains and more clusters than it takes (the
+    separate kernels), free atoms beside them, against the oracle."""
+    m = 9 if shape == "many" else 6
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    length = 4.0 * m
+    pos = (g + 0.5) * 4.0 - length / 2
+    n0 = len(pos)
+    tri = np.array([[0.0, 0.0, 0.0], [0.95, 0.0, 0.0], [-0.3, 0.9, 0.0], [0.2, 0.3, 0.95]])
+    per = {"pairs": 2, "chains": 4}.get(shape, 3)
+    held = n0 - 5                                       # the last five sites hold single atoms
+    every = np.concatenate([(pos[:held, None] + tri[None, :per]).reshape(-1, 3), pos[held:]])
+    o = per * np.arange(held)
+    cons = {"pairs": [(0, 1)], "stars": [(1, 0), (0, 2)], "triangles": [(0, 1), (0, 2), (1, 2)],
+            "mixed_order": [(2, 1), (0, 2), (1, 0)], "chains": [(0, 1), (1, 2), (2, 3)],
+            "many": [(0, 1), (0, 2), (1, 2)]}[shape]
+    atoms = np.concatenate([np.stack([o + a, o + b], 1) for a, b in cons]).astype(np.int32)
+    s = _fluid(every, (length,) * 3)
+    mol = np.concatenate([np.repeat(np.arange(held), per), held + np.arange(5)])
+    # everything inside a molecule excluded
+    pairs = [(k + a, k + b) for k in o for a in range(per) for b in range(a + 1, per)]
+    excl = np.array([(a, b, systems.EXCLUSION_FULL) for a, b in pairs], np.int32)
+    s = dataclasses.replace(s, molecule=mol.astype(np.int32), exclusions=excl, exclusion_check=excl[:, 2].copy())
+    rest = np.linalg.norm(every[atoms[:, 0]] - every[atoms[:, 1]], axis=1)
+    con = {"atoms": atoms, "rest": rest, "shake": (1e-8, 100), "rattle": (1e-8, 100), "mass": s.mass}
+    v = integrate.maxwell_boltzmann(s.mass, 300.0, 3)
+    steps = 3
+    ref = oracle.leapfrog(s, [F.parse_definition(LJ9)], v, 1.0, steps, constraints=con)
+    topo = F.Topology(s)
+    lf = integrate.Leapfrog(topo, [F.ForceFactory.make(topo, LJ9, "fp64")], s.positions, v, s.mass, 1.0, virial=True,
+                            constraints=con).initialize()
+    lf.run(steps)
+    x, vel, f, e = lf.state()
+    assert np.abs(x - ref[0]).max() <= 1e-10
+    assert np.abs(vel - ref[1]).max() <= 1e-9 * np.abs(ref[1]).max()
+    assert lf.constraint_limit_hits() == 0
