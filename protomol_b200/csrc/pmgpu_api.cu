@@ -229,6 +229,9 @@ struct pmgpu_system {
     size_t h_adj_cap = 0;
     bool binned = false;
     std::set<pmgpu_force*> forces;     // live forces made on this system
+    // two one-term cutoff forces of a group evaluated as one (fuse_forces)
+    struct Fused { long long a, b; pmgpu_force* f; };
+    std::vector<Fused> fused;
     int topo_version = 0;
     int buf_version = 0;               // bumped when a per-evaluation buffer moves
     pmgpu_tuning tuning = {16, 0, 16, 1, 0, 0.0};   // launch shapes (pmgpu_set_tuning, pmgpu_autotune)
@@ -1446,12 +1449,68 @@ static void free_force(pmgpu_force* f)
     delete f;
 }
 
+// the fused forces that a force (or its real-space part) is in go with it
+static void drop_fused(pmgpu_system* sys, const pmgpu_force* f)
+{
+    for (size_t k = 0; k < sys->fused.size();) {
+        const pmgpu_system::Fused u = sys->fused[k];
+        const bool in = u.a == f->id || u.b == f->id ||
+                        (f->real_sub && (u.a == f->real_sub->id || u.b == f->real_sub->id));
+        if (!in) { ++k; continue; }
+        sys->forces.erase(u.f);
+        free_force(u.f);
+        sys->fused.erase(sys->fused.begin() + k);
+    }
+}
+
+// A group's one-term Lennard-Jones force and one-term electrostatic force with
+// the same cutoffs and precision, where the two terms are a registered pairing,
+// run as that pairing: every pair is found and loaded once instead of twice.
+// The pair set and the terms are the same (each switch acts on its own term;
+// a Cutoff switch is one inside the common cutoff), and so are the energy
+// slots.  Not with a reused pair list, which is kept for single forces.
+static int fuse_forces(pmgpu_system* sys, std::vector<pmgpu_force*>& all)
+{
+    if (sys->list_every > 1) return PMGPU_OK;
+    for (size_t i = 0; i < all.size(); ++i) {
+        pmgpu_force* a = all[i];
+        if (!a || a->sys != sys || a->kind != 0 || a->cp.n_terms != 1) continue;
+        for (size_t j = 0; j < all.size(); ++j) {
+            pmgpu_force* b = all[j];
+            if (!b || b->sys != sys || b == a || b->kind != 0 || b->cp.n_terms != 1) continue;
+            if (a->precision != b->precision || a->cut2 != b->cut2 ||
+                a->cp.algorithm_cutoff != b->cp.algorithm_cutoff)
+                continue;
+            const int pot[2] = {a->cp.pot[0], b->cp.pot[0]}, sw[2] = {a->cp.sw[0], b->cp.sw[0]};
+            if (pair_combo_id(2, pot, sw) < 0) continue;
+            pmgpu_force* f = nullptr;
+            for (const auto& u : sys->fused)
+                if (u.a == a->id && u.b == b->id) f = u.f;
+            if (!f) {
+                pmgpu_cutoff_params p = a->cp;
+                p.n_terms = 2;
+                p.pot[1] = pot[1]; p.sw[1] = sw[1];
+                p.switchon[1] = b->cp.switchon[0]; p.cutoff[1] = b->cp.cutoff[0]; p.alpha[1] = b->cp.alpha[0];
+                int r = pmgpu_cutoff_create(sys, &p, &f);
+                if (r) return r;
+                sys->fused.push_back({a->id, b->id, f});
+            }
+            all[std::min(i, j)] = f;
+            all.erase(all.begin() + std::max(i, j));
+            i = std::min(i, j);
+            break;
+        }
+    }
+    return PMGPU_OK;
+}
+
 extern "C" int pmgpu_force_destroy(pmgpu_force* f)
 {
     if (!f) return PMGPU_OK;
     pmgpu_system* sys = f->sys;
     cudaSetDevice(sys->device);
     cudaStreamSynchronize(sys->stream);
+    drop_fused(sys, f);
     sys->forces.erase(f);
     free_force(f);
     return PMGPU_OK;
@@ -2369,9 +2428,11 @@ static int eval_core(pmgpu_system* sys, int nf_in, pmgpu_force* const* forces_in
         if (forces_in[k]->real_sub && !pme_needs_lattice(forces_in[k])) all.push_back(forces_in[k]->real_sub);
         all.push_back(forces_in[k]);
     }
+    int r = fuse_forces(sys, all);
+    if (r) return r;
     const int nf = (int)all.size();
     pmgpu_force* const* forces = all.data();
-    int r = eval_prepare(sys, nf, forces, flags);
+    r = eval_prepare(sys, nf, forces, flags);
     if (r) return r;
     // a reused pair list: the column path with one mixed cutoff force (its
     // list is the system's only one), a rebuild period above one, a list
@@ -2820,6 +2881,7 @@ struct pmgpu_batch {
     struct Member {
         pmgpu_system* sys;
         std::vector<pmgpu_force*> forces;    // -real expanded
+        std::vector<pmgpu_force*> run;       // those, pairs of one-term forces as one (fuse_forces)
         const double* pos;
         double* fout;
         double* energy;
@@ -2910,10 +2972,12 @@ extern "C" int pmgpu_batch_evaluate(pmgpu_batch* b)
     std::vector<GraphKey> keys;
     for (auto& m : b->members) {
         if (m.sys->profiling) return batch_fail(b, PMGPU_ERR_STATE, "a member system is in profiling mode");
-        int r = eval_prepare(m.sys, (int)m.forces.size(), m.forces.data(), m.flags);
+        m.run = m.forces;
+        int r = fuse_forces(m.sys, m.run);
+        if (!r) r = eval_prepare(m.sys, (int)m.run.size(), m.run.data(), m.flags);
         if (r) return batch_fail(b, r, m.sys->err);
         GraphKey k;
-        for (pmgpu_force* f : m.forces) k.ids.push_back(f->id);
+        for (pmgpu_force* f : m.run) k.ids.push_back(f->id);
         k.pos = m.pos; k.fout = m.fout; k.energy = m.energy; k.flags = m.flags;
         k.box_version = m.sys->box_version; k.topo_version = m.sys->topo_version;
         k.buf_version = m.sys->buf_version;
@@ -2949,7 +3013,7 @@ extern "C" int pmgpu_batch_evaluate(pmgpu_batch* b)
             auto& m = b->members[k];
             e = cudaStreamWaitEvent(m.sys->stream, b->ev_start, 0);
             if (e != cudaSuccess) break;
-            run_init(runs[k], m.sys, (int)m.forces.size(), m.forces.data(), m.pos, m.fout, m.energy, m.flags);
+            run_init(runs[k], m.sys, (int)m.run.size(), m.run.data(), m.pos, m.fout, m.energy, m.flags);
             r = run_begin(runs[k]);
             if (!r) r = run_cutoffs(runs[k], one_launch);
             if (!r && runs[k].deferred < 0) r = run_end(runs[k]);

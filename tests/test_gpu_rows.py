@@ -1,7 +1,8 @@
 """The pair kernels over rows of column clusters where they can go wrong: small
 and flat boxes (the list's half by row parity instead of by half plane), two
 different cutoffs, j-forces too large for their 32-bit sums, lists and columns
-that outgrow their estimates, and the constrained step's clusters of every shape.
+that outgrow their estimates, one-term forces evaluated as a pair, and the
+constrained step's clusters of every shape.
 
 Bounds, set before the first run: those of the parity suite (forces within 1e-5
 relative RMS mixed, 1e-11 of the RMS force FP64; pair sets equal; energies
@@ -155,6 +156,29 @@ def test_a_column_of_more_atoms_than_the_sort_holds():
     z = (np.arange(2300) - 1150) * 3.9
     pos = np.stack([0.3 + 0 * z, 0.4 + 0 * z, z], 1) + rng.uniform(-0.2, 0.2, (2300, 3))
     _check(_fluid(pos, (30.0, 30.0, 2300 * 3.9)), [LJ9], "fp64")
+
+
+def test_one_term_forces_as_a_pair():
+    """LJ and Coulomb C2 as two forces of one group: their energies keep their
+    slots, each alone still evaluates alone, and the group goes on after one of
+    them is destroyed."""
+    s = systems.water_box(640, 9)
+    defs = workloads.lj_c2_coulomb_c2(8, 9)
+    topo, fs, ref = _check(s, defs, "fp64")
+    alone = []
+    for f, d in zip(fs, defs):
+        out, e = np.zeros((s.n_atoms, 3)), F.ScalarStructure()
+        F.evaluate_group(topo, [f], s.positions, out, e)
+        r = oracle.evaluate(s, [F.parse_definition(d)])
+        assert np.abs(out - r["forces"]).max() <= 1e-11 * np.abs(r["forces"]).max()
+        alone.append((e.lennard_jones, e.coulomb))
+    assert alone[0][1] == 0.0 and alone[1][0] == 0.0
+    fs[1].close()
+    again = F.ForceFactory.make(topo, defs[1], "fp64")
+    out, e = np.zeros((s.n_atoms, 3)), F.ScalarStructure()
+    F.evaluate_group(topo, [again, fs[0]], s.positions, out, e)
+    assert np.abs(out - ref["forces"]).max() <= 1e-11 * np.abs(ref["forces"]).max()
+    assert abs(e.lennard_jones - alone[0][0]) <= 1e-11 * abs(alone[0][0])
 
 
 def test_reused_list_survives_an_fp64_evaluation_between():
