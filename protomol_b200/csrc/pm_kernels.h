@@ -225,6 +225,7 @@ struct PairArgs {
     unsigned long long* efix;    // 11 int64 sums (scale 2^32): LJ, Coulomb, virial
     int blocks_per_sm;           // resident blocks of the mixed pair kernel per SM (0: the occupancy limit)
     int chunk;                   // cluster-list entries per chunk of pair work
+    int chunk_end;               // column lists: those of the last rows
     // column-cluster path (K2a' / K2b'): slot data, cluster boxes, grid
     const int4* cq;
     const int4* cm;
@@ -266,13 +267,14 @@ constexpr int kBatchPairMax = 1024;
 struct BatchPairArgs {
     const PairArgs* args;        // device copy of every member's pair arguments
     int n;
+    int two;                     // a member's terms have two different cutoffs
     int* next;                   // work counter (zero before the launch)
 };
 int launch_pair_col_batch(const BatchPairArgs& b, int combo, cudaStream_t s, long long* launches);
 int launch_near_energy_col(const PairArgs& a, int combo, int n_atoms, cudaStream_t s, long long* launches);
 long long col_list_estimate(int n_atoms, const ColGrid& g, double volume, double cutoff);
 long long col_chunk_estimate(long long entries, int n_atoms, const ColGrid& g, int chunk);
-int col_chunk_entries(int n_atoms, const ColGrid& g, double volume, double cutoff, int most, bool half);
+int col_chunk_entries(int n_atoms, const ColGrid& g, double volume, double cutoff, int most, bool last);
 int col_rows_split(int n_atoms, const ColGrid& g, double cutoff);
 int col_row_blocks(int n_atoms, const ColGrid& g, double cutoff);
 int launch_pair_fp64(const PairArgs& a, int combo, bool col, int blocks, cudaStream_t s, long long* launches);

@@ -19,17 +19,19 @@ long long col_list_estimate(int n_atoms, const ColGrid& g, double volume, double
     return (long long)(1.3 * rows * per) + 4096;
 }
 
-// Entries per chunk of the pair kernel: about four chunks for every resident
-// warp (148 SMs x 16), so that the last wave is short, but no more than
-// most (six tuned chunk units) or a block: every chunk ends with partly filled
-// rings.
-int col_chunk_entries(int n_atoms, const ColGrid& g, double volume, double cutoff, int most, bool half)
+// Entries per chunk of the pair kernel.  Every chunk ends with partly filled
+// rings (a fifth of its pair phase idle at 36 entries, an eighth at 75), and the
+// kernel ends with its last chunks (30 us each at 36 entries): the first five
+// eighths of the rows get chunks for about two of every resident warp (148 SMs
+// x 16), the rest (last) for about six, never more than most (six tuned chunk
+// units) or a block.
+int col_chunk_entries(int n_atoms, const ColGrid& g, double volume, double cutoff, int most, bool last)
 {
     const double rho = volume > 0.0 ? n_atoms / volume : 0.0;
     const double r = cutoff + 0.75 * std::max(g.sx, g.sy);
     const double rows = (double)n_atoms / kCluster + 0.5 * g.ncol + 1;
     const double per = std::min(rho * (4.0 / 3.0) * 3.14159265358979 * r * r * r / 4.0, 2.0 * rows);
-    const double want = rows * per * (half ? 0.5 : 1.0) / (4.0 * 148 * 16);
+    const double want = rows * per * 0.5 / ((last ? 6.0 : 2.0) * 148 * 16);
     return std::max(16, std::min(std::min(most, kColBlock), 2 * (int)(0.5 * std::min(want, 1e6) + 1.0)));
 }
 
@@ -46,22 +48,33 @@ int launch_col_list(const PairArgs& a, cudaStream_t s, long long* launches)
     return (int)cudaGetLastError();
 }
 
-template <int NT, int P0, int S0, int P1, int S1>
-static int run_col(const PairArgs& a, cudaStream_t s, long long* launches)
+template <int NT, int P0, int S0, int P1, int S1, bool TWO>
+static int run_col_t(const PairArgs& a, cudaStream_t s, long long* launches)
 {
     static int sms = 0, per_sm = 0;
     if (sms == 0) {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_col<NT, P0, S0, P1, S1>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_col<NT, P0, S0, P1, S1, TWO>, 128, 0);
         if (sms <= 0) sms = 148;
         if (per_sm <= 0) per_sm = 1;
     }
     const int bps = a.blocks_per_sm > 0 ? std::min(per_sm, a.blocks_per_sm) : per_sm;
-    launch_pdl(k_pair_col<NT, P0, S0, P1, S1>, sms * bps, 128, 0, s, a);
+    launch_pdl(k_pair_col<NT, P0, S0, P1, S1, TWO>, sms * bps, 128, 0, s, a);
     *launches += 1;
     return (int)cudaGetLastError();
+}
+
+// the terms' own cutoffs differ: a pair may be inside one of them only
+static bool two_cutoffs(const PairArgs& a) { return a.n_terms > 1 && a.tf[0].cut2 != a.tf[1].cut2; }
+
+template <int NT, int P0, int S0, int P1, int S1>
+static int run_col(const PairArgs& a, cudaStream_t s, long long* launches)
+{
+    if constexpr (NT > 1)
+        if (two_cutoffs(a)) return run_col_t<NT, P0, S0, P1, S1, true>(a, s, launches);
+    return run_col_t<NT, P0, S0, P1, S1, false>(a, s, launches);
 }
 
 int launch_pair_col(const PairArgs& a, int combo, cudaStream_t s, long long* launches)
@@ -98,21 +111,29 @@ int launch_pair_col(const PairArgs& a, int combo, cudaStream_t s, long long* lau
     }
 }
 
-template <int NT, int P0, int S0, int P1, int S1>
-static int run_col_batch(const BatchPairArgs& b, cudaStream_t s, long long* launches)
+template <int NT, int P0, int S0, int P1, int S1, bool TWO>
+static int run_col_batch_t(const BatchPairArgs& b, cudaStream_t s, long long* launches)
 {
     static int sms = 0, per_sm = 0;
     if (sms == 0) {
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_col_batch<NT, P0, S0, P1, S1>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_col_batch<NT, P0, S0, P1, S1, TWO>, 128, 0);
         if (sms <= 0) sms = 148;
         if (per_sm <= 0) per_sm = 1;
     }
-    k_pair_col_batch<NT, P0, S0, P1, S1><<<sms * per_sm, 128, 0, s>>>(b);
+    k_pair_col_batch<NT, P0, S0, P1, S1, TWO><<<sms * per_sm, 128, 0, s>>>(b);
     *launches += 1;
     return (int)cudaGetLastError();
+}
+
+template <int NT, int P0, int S0, int P1, int S1>
+static int run_col_batch(const BatchPairArgs& b, cudaStream_t s, long long* launches)
+{
+    if constexpr (NT > 1)
+        if (b.two) return run_col_batch_t<NT, P0, S0, P1, S1, true>(b, s, launches);
+    return run_col_batch_t<NT, P0, S0, P1, S1, false>(b, s, launches);
 }
 
 int launch_pair_col_batch(const BatchPairArgs& b, int combo, cudaStream_t s, long long* launches)

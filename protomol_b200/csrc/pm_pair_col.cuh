@@ -204,7 +204,8 @@ static __global__ void __launch_bounds__(128) k_col_list(const __grid_constant__
         return;
     }
     const ColGrid& g = p.cg;
-    if (row >= p.ccstart[g.ncol]) return;
+    const int rows = p.ccstart[g.ncol];
+    if (row >= rows) return;
     const float4 ic = p.ibox[2 * row], ih = p.ibox[2 * row + 1];
     if (p.col_refuse && 2.f * ih.z > g.zext) {                   // too tall to prune by: the cell layout
         if (lane == 0) { atomicOr(p.status, kStatusColumns); atomicMax(p.plist_need, 1); }
@@ -217,8 +218,10 @@ static __global__ void __launch_bounds__(128) k_col_list(const __grid_constant__
         if (lane == 0) p.rowent[row] = make_int2(0, 0);
         return;
     }
-    // equal chunks of a row, an even number of entries each
-    const int nch = (ne + p.chunk - 1) / p.chunk, per = ((ne + nch - 1) / nch + 1) & ~1;
+    // equal chunks of a row, an even number of entries each; the last rows'
+    // (about the last to run) are shorter, so that the kernel's end is
+    const int most = 8 * row < 5 * rows ? p.chunk : p.chunk_end;
+    const int nch = (ne + most - 1) / most, per = ((ne + nch - 1) / nch + 1) & ~1;
     int b0 = 0, b1 = 0;
     if (lane == 0) {
         b0 = atomicAdd(p.plist_count, ne);
@@ -252,7 +255,6 @@ struct ColTest {
     float far2, band2;
     float c0, c1;                // the terms' own cutoffs^2
     float g_lo, g_hi;
-    bool two;                    // they differ
 };
 
 __device__ __forceinline__ ColTest col_test(const PairArgs& p)
@@ -264,7 +266,6 @@ __device__ __forceinline__ ColTest col_test(const PairArgs& p)
     t.band2 = p.cut2f * t.g_lo;
     t.c0 = p.tf[0].cut2;
     t.c1 = p.n_terms > 1 ? p.tf[1].cut2 : p.tf[0].cut2;
-    t.two = t.c0 != t.c1;
     return t;
 }
 
@@ -288,7 +289,7 @@ __device__ __forceinline__ void col_resolve(const PairArgs& p, const ColTest& t,
     if (own ? j <= si : j == si) { in = false; return; }
     const int oi = p.cm[si].w, oj = p.cm[j].w;
     bool band = r2 >= t.band2;
-    if (TWO && t.two) band |= r2 >= fminf(t.c0, t.c1) * t.g_lo && r2 <= fminf(t.c0, t.c1) * t.g_hi;
+    if (TWO) band |= r2 >= fminf(t.c0, t.c1) * t.g_lo && r2 <= fminf(t.c0, t.c1) * t.g_hi;
     if (band) {
         const double d2 = exact_d2(p, oi, oj);
         if (d2 > p.cut2d) { in = false; return; }
@@ -350,7 +351,7 @@ __device__ __forceinline__ void col_entries(const PairArgs& p, const ColTest& t,
         int codeA = Op::kLocal ? 4 * k + jj : 4 * (e.x & 0x7fffffff) + jj;
         int codeB = Op::kLocal ? 4 * k + jj + 4 : 4 * (e.y & 0x7fffffff) + jj;
         bool rare = (inA & (sameA | (ra >= t.band2))) | (inB & (sameB | (rb >= t.band2))) | ((e.x | e.y) < 0);
-        if (TWO && t.two) {                           // two cutoffs: which terms the pair is inside of
+        if (TWO) {                                    // two cutoffs: which terms the pair is inside of
             codeA |= (ra <= t.c0 ? kCodeIn0 : 0) | (ra <= t.c1 ? kCodeIn1 : 0);
             codeB |= (rb <= t.c0 ? kCodeIn0 : 0) | (rb <= t.c1 ? kCodeIn1 : 0);
             const float lo = fminf(t.c0, t.c1);
@@ -422,11 +423,11 @@ constexpr float kLimitJ = 60.0f;         // a j-force component this large is ad
 // atoms' int64 sums once per chunk: everything is independent of the
 // chunk-to-warp assignment.  Near pairs (r < 5 A) go to the warp's queue for
 // K2c'; their FP32 energies and virial are left out.
-template <int NT, int P0, int S0, int P1, int S1>
+// TWO: the two terms' cutoffs differ (a pair may be inside one of them only).
+template <int NT, int P0, int S0, int P1, int S1, bool TWO>
 struct ColForce32 {
     static constexpr int kKeep = 16;     // a drain leaves rings below this (longer ones share the idle lanes)
     static constexpr bool kLocal = true;
-    static constexpr bool kTwo = NT > 1 && (S0 == SCUT || S1 == SCUT);
     const PairArgs& p;
     ColShared32& sh;
     int nq;
@@ -486,14 +487,13 @@ struct ColForce32 {
         const float qx = (float)(int)((unsigned)P.x - (unsigned)r.P.x);
         const float qy = (float)(int)((unsigned)P.y - (unsigned)r.P.y);
         const float qz = (float)(int)((unsigned)P.z - (unsigned)r.P.z);
-        g.dx = fmaf(qx, p.cg.sch[0], qx * p.cg.scl[0]);
-        g.dy = fmaf(qy, p.cg.sch[1], qy * p.cg.scl[1]);
-        g.dz = fmaf(qz, p.cg.sch[2], qz * p.cg.scl[2]);
-        g.r2 = fmaf(g.dz, g.dz, fmaf(g.dy, g.dy, g.dx * g.dx));
+        g.dx = fmaf(qx, p.cg.sch[0], __fmul_rn(qx, p.cg.scl[0]));
+        g.dy = fmaf(qy, p.cg.sch[1], __fmul_rn(qy, p.cg.scl[1]));
+        g.dz = fmaf(qz, p.cg.sch[2], __fmul_rn(qz, p.cg.scl[2]));
+        g.r2 = fmaf(g.dz, g.dz, fmaf(g.dy, g.dy, __fmul_rn(g.dx, g.dx)));
         g.act = valid;
-        const bool two = kTwo && p.tf[0].cut2 != p.tf[1].cut2;
-        g.in0 = !two || (code & kCodeIn0);
-        g.in1 = !two || (code & kCodeIn1);
+        g.in0 = !TWO || (code & kCodeIn0);
+        g.in1 = !TWO || (code & kCodeIn1);
         g.excl = (code & kCodeMod) ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE;
         g.near = g.same = false;
         return g;
@@ -525,10 +525,10 @@ struct ColForce32 {
         const PairGeo ga = geo(r, ca, sa, va), gb = geo(r, cb, sb, vb);
         const JAtom ja = atom(sa), jb = atom(sb);
         float fta, ela, eca, ftb, elb, ecb;
-        pair_math<NT, P0, S0, P1, S1>(p, ga, ia, ja, fta, ela, eca);
-        pair_math<NT, P0, S0, P1, S1>(p, gb, ia, jb, ftb, elb, ecb);
-        const float xa = ga.dx * fta, ya = ga.dy * fta, za = ga.dz * fta;
-        const float xb = gb.dx * ftb, yb = gb.dy * ftb, zb = gb.dz * ftb;
+        pair_math<NT, P0, S0, P1, S1, TWO>(p, ga, ia, ja, fta, ela, eca);
+        pair_math<NT, P0, S0, P1, S1, TWO>(p, gb, ia, jb, ftb, elb, ecb);
+        const float xa = __fmul_rn(ga.dx, fta), ya = __fmul_rn(ga.dy, fta), za = __fmul_rn(ga.dz, fta);
+        const float xb = __fmul_rn(gb.dx, ftb), yb = __fmul_rn(gb.dy, ftb), zb = __fmul_rn(gb.dz, ftb);
         f[0] -= xa + xb; f[1] -= ya + yb; f[2] -= za + zb;
         // (not below the limit: NaN too)
         const bool ba = !(fmaxf(fabsf(xa), fmaxf(fabsf(ya), fabsf(za))) < kLimitJ) || isnan(fta);
@@ -602,7 +602,7 @@ struct ColForce32 {
         col_row_begin(p, t, cd.x, r);
         begin(r);
         col_stage(p, p.clist + cd.z, n, sh.ent);
-        col_entries<false, kTwo>(p, t, r, sh.ring, sh.ent, n, true, *this);
+        col_entries<false, TWO>(p, t, r, sh.ring, sh.ent, n, true, *this);
         // the chunk's j-forces
         for (int k = lane; k < 4 * n; k += 32) {
             unsigned long long* to = p.facc + 3 * (size_t)slot(k);
@@ -624,17 +624,21 @@ struct ColForce32 {
         const double x = row_sum(fd[0]), y = row_sum(fd[1]), z = row_sum(fd[2]);
         if (r.vi && jj < 3)
             fixed_add(p.facc + 3 * (size_t)r.si + jj, jj == 0 ? x : (jj == 1 ? y : z), kScaleMixed, p.status);
-        double mine = 0.0;
+        // the eight sums over the warp, scattered: lane 4 k ends with sum k
+        double t[8] = {ed[0], ed[1], vd[0], vd[1], vd[2], vd[3], vd[4], vd[5]};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            if (k >= 2 && !p.virial) break;
-            double t = k < 2 ? ed[k] : vd[k - 2];
+        for (int w = 4; w > 0; w >>= 1) {
+            const bool up = lane & (4 * w);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (lane == k) mine = t;
+            for (int k = 0; k < w; ++k) {
+                const double give = up ? t[k] : t[k + w];
+                t[k] = (up ? t[k + w] : t[k]) + __shfl_xor_sync(0xffffffffu, give, 4 * w);
+            }
         }
+        t[0] += __shfl_xor_sync(0xffffffffu, t[0], 2);
+        t[0] += __shfl_xor_sync(0xffffffffu, t[0], 1);
         bool bad = false;
-        if (lane < 8) sh.acc[lane] += fixed_of(mine, bad);
+        if ((lane & 3) == 0) sh.acc[lane >> 2] += fixed_of(t[0], bad);
         if (bad) atomicOr(p.status, kStatusOverflow);
         if (nq > 0) { append_near(p, sh.near, nq, lane); nq = 0; }
     }
@@ -666,7 +670,7 @@ __device__ __forceinline__ int col_chunks(const PairArgs& p, bool mark)
     return bad ? 0 : min(*p.chunk_count, p.chunk_cap);
 }
 
-template <int NT, int P0, int S0, int P1, int S1>
+template <int NT, int P0, int S0, int P1, int S1, bool TWO>
 __global__ void __launch_bounds__(128, 4) k_pair_col(const __grid_constant__ PairArgs p)
 {
     pdl_wait();
@@ -674,7 +678,7 @@ __global__ void __launch_bounds__(128, 4) k_pair_col(const __grid_constant__ Pai
     __shared__ ColShared32 sh[4];
     const int nchunks = col_chunks(p, blockIdx.x == 0 && threadIdx.x == 0);
     const ColTest t = col_test(p);
-    ColForce32<NT, P0, S0, P1, S1> op{p, sh[w]};
+    ColForce32<NT, P0, S0, P1, S1, TWO> op{p, sh[w]};
     op.init();
     while (true) {
         int ch = 0;
@@ -695,7 +699,7 @@ __global__ void __launch_bounds__(128, 4) k_pair_col(const __grid_constant__ Pai
 // runs the chunk (as K2b') and adds its sums to the member's energy
 // words when it leaves the member.  Nothing waits on another launch: the
 // graph orders this one after every member's list.
-template <int NT, int P0, int S0, int P1, int S1>
+template <int NT, int P0, int S0, int P1, int S1, bool TWO>
 __global__ void __launch_bounds__(128, 4) k_pair_col_batch(BatchPairArgs b)
 {
     const unsigned FULL = 0xffffffffu;
@@ -715,7 +719,7 @@ __global__ void __launch_bounds__(128, 4) k_pair_col_batch(BatchPairArgs b)
     const int total = s_pre[b.n];
     int cur = -1;
     const PairArgs& p = s_args[w];
-    ColForce32<NT, P0, S0, P1, S1> op{p, sh[w]};
+    ColForce32<NT, P0, S0, P1, S1, TWO> op{p, sh[w]};
     op.init();
     ColTest t;
     while (true) {

@@ -112,18 +112,18 @@ __device__ __forceinline__ void pot_f32(const PairArgs& p, const TermF& t, float
         float r6B = fmaf(par.y, r6, par.w * r6);
         float r12A = fmaf(par.x, r12, par.z * r12);
         e = r12A - r6B;
-        f = (12.0f * r12A - 6.0f * r6B) * rd2;
+        f = __fmul_rn(fmaf(12.0f, r12A, -__fmul_rn(6.0f, r6B)), rd2);
     } else if (POT == CO) {
-        e = qq * rinv;
-        e = excl == PMGPU_EXCL_MODIFIED ? e * p.csf : e;
-        f = e * rd2;
+        e = __fmul_rn(qq, rinv);
+        e = excl == PMGPU_EXCL_MODIFIED ? __fmul_rn(e, p.csf) : e;
+        f = __fmul_rn(e, rd2);
     } else if (POT == EW) {
-        qq = (p.csfd != 1.0 && excl == PMGPU_EXCL_MODIFIED) ? qq * p.csf : qq;
+        qq = excl == PMGPU_EXCL_MODIFIED ? qq * p.csf : qq;
         float r = r2 * rinv;
         float ar = fmaf(t.alpha, r, t.alpha_lo * r);     // compensated alpha
         float ex = qq * exp_neg(ar * ar);
-        e = poly5f(ar) * ex * rinv;
-        f = fmaf(t.two_alpha_pi, ex, fmaf(t.two_alpha_pi_lo, ex, e)) * rinv * rinv;
+        e = __fmul_rn(poly5f(ar) * ex, rinv);
+        f = __fmul_rn(fmaf(t.two_alpha_pi, ex, fmaf(t.two_alpha_pi_lo, ex, e)) * rinv, rinv);
     } else if (pot_table(POT)) {
         // LookUpTableBase::index on the FP32 r^2 (its top exponent and PRE
         // mantissa bits pick the entry) and the cubic of ::interpolate
@@ -141,45 +141,45 @@ __device__ __forceinline__ void pot_f32(const PairArgs& p, const TermF& t, float
             const float4* tab = excl == PMGPU_EXCL_MODIFIED ? p.ljm : p.ljn;
             const float4 par = __ldg(tab + (ti * p.n_types + tj));   // A_hi, B_hi, A_lo, B_lo
             const float4 ta = __ldg(T), tb = __ldg(T + 1);
-            a = fmaf(par.x, ta.x, par.z * ta.x) + fmaf(par.y, tb.x, par.w * tb.x);
-            b = fmaf(par.x, ta.y, par.z * ta.y) + fmaf(par.y, tb.y, par.w * tb.y);
-            c = fmaf(par.x, ta.z, par.z * ta.z) + fmaf(par.y, tb.z, par.w * tb.z);
-            d = fmaf(par.x, ta.w, par.z * ta.w) + fmaf(par.y, tb.w, par.w * tb.w);
+            a = fmaf(par.x, ta.x, __fmul_rn(par.z, ta.x)) + fmaf(par.y, tb.x, __fmul_rn(par.w, tb.x));
+            b = fmaf(par.x, ta.y, __fmul_rn(par.z, ta.y)) + fmaf(par.y, tb.y, __fmul_rn(par.w, tb.y));
+            c = fmaf(par.x, ta.z, __fmul_rn(par.z, ta.z)) + fmaf(par.y, tb.z, __fmul_rn(par.w, tb.z));
+            d = fmaf(par.x, ta.w, __fmul_rn(par.z, ta.w)) + fmaf(par.y, tb.w, __fmul_rn(par.w, tb.w));
         } else {
-            const float q = (p.csfd != 1.0 && excl == PMGPU_EXCL_MODIFIED) ? qq * p.csf : qq;
+            const float q = excl == PMGPU_EXCL_MODIFIED ? qq * p.csf : qq;
             const float4 tc = __ldg(T);
-            a = tc.x * q; b = tc.y * q; c = tc.z * q; d = tc.w * q;
+            a = __fmul_rn(tc.x, q); b = __fmul_rn(tc.y, q); c = __fmul_rn(tc.z, q); d = __fmul_rn(tc.w, q);
         }
         e = fmaf(fmaf(fmaf(dt, d, c), dt, b), dt, a);
-        f = -2.0f * fmaf(fmaf(3.0f * dt, d, 2.0f * c), dt, b);
+        f = __fmul_rn(-2.0f, fmaf(fmaf(__fmul_rn(3.0f, dt), d, __fmul_rn(2.0f, c)), dt, b));
     } else {
         e = 0.f; f = 0.f;
     }
 }
 
 // switching functions as selects (no branches: the two pair evaluations of
-// a lane interleave)
-template <int SW>
+// a lane interleave); OUT: a pair may lie outside this term's cutoff
+template <int SW, bool OUT = true>
 __device__ __forceinline__ void sw_f32(const TermF& t, float r2, float rinv, bool inside, float& v, float& d)
 {
     if (SW == SC2) {
         const float c2 = t.cut2 - r2;
-        const float c4 = c2 * (t.s2 + 2.0f * r2);
-        const float c24 = c2 * c4;
-        const float dd = c2 * c2 - c4;
-        const bool out = r2 > t.cut2, mid = r2 >= t.on2;
-        v = out ? 0.f : (mid ? fmaf(t.s1, c24, t.s1_lo * c24) : 1.f);
-        d = (out || !mid) ? 0.f : fmaf(t.s3, dd, t.s3_lo * dd);
+        const float c4 = __fmul_rn(c2, fmaf(2.0f, r2, t.s2));
+        const float c24 = __fmul_rn(c2, c4);
+        const float dd = fmaf(c2, c2, -c4);
+        const bool out = OUT && r2 > t.cut2, mid = r2 >= t.on2;
+        v = out ? 0.f : (mid ? fmaf(t.s1, c24, __fmul_rn(t.s1_lo, c24)) : 1.f);
+        d = (out || !mid) ? 0.f : fmaf(t.s3, dd, __fmul_rn(t.s3_lo, dd));
     } else if (SW == SC1) {
         const float dist = r2 * rinv;
         const float in = fmaf(-r2, t.c1_05_3, t.c1_15_1) + fmaf(-r2, t.c1_05_3_lo, t.c1_15_1_lo);
-        const bool out = r2 > t.cut2;
+        const bool out = OUT && r2 > t.cut2;
         v = out ? 0.f : fmaf(-dist, in, 1.0f);
         d = out ? 0.f : fmaf(dist, t.c1_15_3, -t.c1_15_1 * rinv) + fmaf(dist, t.c1_15_3_lo, -t.c1_15_1_lo * rinv);
     } else if (SW == SSH) {
-        const float x = fmaf(-r2, t.sh_a, 1.0f) - r2 * t.sh_a_lo;
-        const bool out = r2 > t.cut2;
-        v = out ? 0.f : x * x;
+        const float x = fmaf(-r2, t.sh_a_lo, fmaf(-r2, t.sh_a, 1.0f));
+        const bool out = OUT && r2 > t.cut2;
+        v = out ? 0.f : __fmul_rn(x, x);
         d = out ? 0.f : fmaf(t.sh_b, x, t.sh_b_lo * x);
     } else if (SW == SCUT) {
         d = 0.f;

@@ -283,8 +283,13 @@ __device__ __forceinline__ float rsqrt_nr(float x)
 
 // the OneAtomPair[Two] terms of one pair (OneAtomPairTwo.h doOneAtomPair:
 // both switches are applied when either modifies): scalar force factor
-// (F_j = d * ft) and energies, zero for an inactive pair
-template <int NT, int P0, int S0, int P1, int S1>
+// (F_j = d * ft) and energies, zero for an inactive pair.  Every FMA is
+// written out and every other product rounded (__fmul_rn): a member of a batch
+// and the same system alone run two compilations of this code, and their
+// results are the same bit for bit.
+// OUT: the pair may lie outside one term's own cutoff (two different cutoffs,
+// or a pair that is only tested against a rounded one)
+template <int NT, int P0, int S0, int P1, int S1, bool OUT = true>
 __device__ __forceinline__ void pair_math(const PairArgs& p, const PairGeo& g, const JAtom& ia, const JAtom& ja,
                                           float& ft, float& el, float& ec)
 {
@@ -300,20 +305,24 @@ __device__ __forceinline__ void pair_math(const PairArgs& p, const PairGeo& g, c
         // (a Cutoff switch is one inside, zero outside)
         float sv, sd;
         if (S0 == SCUT) {
-            f0 = g.in0 ? f0 : 0.f;
-            e0 = g.in0 ? e0 : 0.f;
+            if (OUT) {
+                f0 = g.in0 ? f0 : 0.f;
+                e0 = g.in0 ? e0 : 0.f;
+            }
         } else {
-            sw_f32<S0>(p.tf[0], r2, rinv, g.in0, sv, sd);
-            f0 = f0 * sv - e0 * sd;
-            e0 = e0 * sv;
+            sw_f32<S0, OUT>(p.tf[0], r2, rinv, g.in0, sv, sd);
+            f0 = fmaf(f0, sv, -__fmul_rn(e0, sd));
+            e0 = __fmul_rn(e0, sv);
         }
         if (NT > 1 && S1 == SCUT) {
-            f1 = g.in1 ? f1 : 0.f;
-            e1 = g.in1 ? e1 : 0.f;
+            if (OUT) {
+                f1 = g.in1 ? f1 : 0.f;
+                e1 = g.in1 ? e1 : 0.f;
+            }
         } else if (NT > 1) {
-            sw_f32<S1>(p.tf[1], r2, rinv, g.in1, sv, sd);
-            f1 = f1 * sv - e1 * sd;
-            e1 = e1 * sv;
+            sw_f32<S1, OUT>(p.tf[1], r2, rinv, g.in1, sv, sd);
+            f1 = fmaf(f1, sv, -__fmul_rn(e1, sd));
+            e1 = __fmul_rn(e1, sv);
         }
     }
     float l = 0.f, c = 0.f;

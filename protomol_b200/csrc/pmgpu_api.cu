@@ -1594,7 +1594,8 @@ static void fill_col_args(pmgpu_system* sys, bool fp64, PairArgs& a, bool half)
     a.col_none = 2 * sys->col_ncl_cap;
     a.rows_split = col_rows_split(sys->n, sys->eval_cg, std::sqrt(a.cut2d));
     const ColGrid& g = sys->eval_cg;
-    a.chunk = col_chunk_entries(sys->n, g, g.lx * g.ly * g.lz, std::sqrt(a.cut2d), 6 * sys->tuning.chunk_entries, half);
+    a.chunk = col_chunk_entries(sys->n, g, g.lx * g.ly * g.lz, std::sqrt(a.cut2d), 6 * sys->tuning.chunk_entries, false);
+    a.chunk_end = col_chunk_entries(sys->n, g, g.lx * g.ly * g.lz, std::sqrt(a.cut2d), 6 * sys->tuning.chunk_entries, true);
     a.list_skin = !fp64 && sys->list_every > 1 ? (float)sys->list_skin : 0.0f;
 }
 
@@ -2877,7 +2878,7 @@ struct pmgpu_batch {
     int pair_launch = 1;                      // 1: the column-path pair kernels as one launch (K11)
     PairArgs* d_args = nullptr;               // the members' pair arguments for that launch
     size_t args_cap = 0;
-    int* d_next = nullptr;                    // its work counters, one per combination of terms
+    int* d_next = nullptr;                    // its work counters, one per combination of terms and one or two cutoffs
     struct Member {
         pmgpu_system* sys;
         std::vector<pmgpu_force*> forces;    // -real expanded
@@ -2912,7 +2913,7 @@ extern "C" int pmgpu_batch_create(int device, pmgpu_batch** out)
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_start, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_pairs, cudaEventDisableTiming) != cudaSuccess ||
-        cudaMalloc((void**)&b->d_next, 32 * sizeof(int)) != cudaSuccess) {
+        cudaMalloc((void**)&b->d_next, 64 * sizeof(int)) != cudaSuccess) {
         delete b;
         return PMGPU_ERR_CUDA;
     }
@@ -3027,24 +3028,30 @@ extern "C" int pmgpu_batch_evaluate(pmgpu_batch* b)
             }
         }
         if (r == PMGPU_OK && e == cudaSuccess && !deferred.empty()) {
-            // one persistent launch per combination of terms over the members'
-            // chunks, then every deferred member resumes after it
+            // one persistent launch per combination of terms (and one or two
+            // cutoffs, as the members' own launches tell them apart) over the
+            // members' chunks, then every deferred member resumes after it
             std::vector<int> combos;
+            auto kind_of = [&](size_t k) {
+                const PairArgs& a = runs[k].dargs;
+                return 2 * runs[k].forces[runs[k].deferred]->combo + (a.n_terms > 1 && a.tf[0].cut2 != a.tf[1].cut2 ? 1 : 0);
+            };
             for (size_t k : deferred) {
-                const int c = runs[k].forces[runs[k].deferred]->combo;
+                const int c = kind_of(k);
                 if (std::find(combos.begin(), combos.end(), c) == combos.end()) combos.push_back(c);
             }
             for (size_t g = 0; g < combos.size() && e == cudaSuccess && r == PMGPU_OK; ++g) {
                 const size_t off = hargs.size();
                 for (size_t k : deferred)
-                    if (runs[k].forces[runs[k].deferred]->combo == combos[g]) hargs.push_back(runs[k].dargs);
+                    if (kind_of(k) == combos[g]) hargs.push_back(runs[k].dargs);
                 e = cudaMemsetAsync(b->d_next + g, 0, sizeof(int), b->stream);
                 if (e != cudaSuccess) break;
                 BatchPairArgs ba;
                 ba.args = b->d_args + off;
                 ba.n = (int)(hargs.size() - off);
                 ba.next = b->d_next + g;
-                e = (cudaError_t)launch_pair_col_batch(ba, combos[g], b->stream, &b->members[deferred[0]].sys->launches);
+                ba.two = combos[g] & 1;
+                e = (cudaError_t)launch_pair_col_batch(ba, combos[g] >> 1, b->stream, &b->members[deferred[0]].sys->launches);
             }
             if (e == cudaSuccess) e = cudaEventRecord(b->ev_pairs, b->stream);
             for (size_t i = 0; i < deferred.size() && e == cudaSuccess && r == PMGPU_OK; ++i) {
