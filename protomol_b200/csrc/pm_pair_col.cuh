@@ -38,21 +38,21 @@
 //   pairs  the lanes of a row atom take the next pairs of its ring: the pair
 //          terms run on full warps.
 //
-// What bounds the mixed kernel: issue slots.  The pair terms are ~150 warp
-// instructions (LJ C2 + Ewald real) and 40% of an 8 x 4 tile's pairs lie inside
-// the cutoff; evaluated tile by tile they were two thirds of the kernel's 106 M
-// instructions on the 14,281-atom box.  The rings fill the lanes of the pair
-// phase (a tile's test is ~40 instructions).
-// Measured against the tile-by-tile kernel (each pair list's kernel alone): 106
-// -> 86 M instructions and 141 -> 139 us on the 14,281-atom box (894 atom types:
-// its Lennard-Jones table is an L2 gather, which neither form hides), 360 ->
-// 308 us for 61,233 atoms of water at 10 A, 8.10 -> 6.53 ms for 1,000,000 at
-// 12 A.  Tried: the full list with the rings and no j side (152 M
-// instructions, 217 us: the terms run twice); five blocks per SM (spills, 146
-// us); chunks twice and four times as long (within 1% from 61,233 atoms on,
-// 5% slower at 14,281).
+// What bounds the mixed kernel: issue slots and, at five blocks per SM, the
+// latency of the pair phase's chain.  An 8 x 4 tile's pairs are 40% inside the
+// cutoff; evaluated tile by tile, the terms (LJ C2 + Ewald real) at 40% of the
+// lanes were two thirds of the kernel's 106 M warp instructions on the
+// 14,281-atom box.  The rings fill the lanes of the pair phase, and its FP32
+// arithmetic is packed two pairs to an instruction: 67 M.
+// Measured against the tile-by-tile kernel, each kernel alone: 8.10 -> 5.62 ms
+// for 1,000,000 atoms at 12 A, 360 -> 270 us for 61,233 at 10 A, 141 -> 133 us
+// for 14,281 (where 47 us do not shrink with the cutoff: the near-pair kernel's
+// 13, the launch and the unevenness of the last chunks).  Tried: a full list
+// with rings and no j side (152 M instructions, 217 us: the terms run twice);
+// two or four times longer chunks (within 1% from 61,233 atoms on, 5% slower at
+// 14,281); short chunks taken last (132 us, but 3 to 8% slower at 20,001 and
+// 61,233 atoms).
 
-constexpr int kEnergyFlush = 8;          // pair-phase steps per FP32 partial sum
 constexpr int kColRing = 64;             // ring places per row atom
 constexpr int kColStageEntries = 1024;   // entries of one row staged in shared memory
 constexpr int kColBlock = 96;            // most entries of a chunk (and of a block of a longer row)
@@ -403,6 +403,189 @@ __device__ __forceinline__ double row_sum(double v)
     return v + __shfl_xor_sync(0xffffffffu, v, 16);
 }
 
+// ---------------------------------------------------------------- packed FP32
+// Two FP32 values in one 64-bit register: sm_100's packed add, multiply and FMA
+// do both in one issue slot, each rounded as the scalar operation.
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float lo, float hi)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float x) { return f2(x, x); }
+__device__ __forceinline__ void split(F2 a, float& lo, float& hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, f2(-1.f), a); }      // one rounding, as a - b
+__device__ __forceinline__ F2 sel2(bool lo, bool hi, F2 a, F2 b)
+{
+    float al, ah, bl, bh;
+    split(a, al, ah);
+    split(b, bl, bh);
+    return f2(lo ? al : bl, hi ? ah : bh);
+}
+__device__ __forceinline__ F2 rsqrt2(F2 x)          // rsqrt_nr of both
+{
+    float a, b, ya, yb;
+    split(x, a, b);
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ya) : "f"(a));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yb) : "f"(b));
+    const F2 y = f2(ya, yb);
+    const F2 e = fma2(mul2(x, y), y, f2(-1.f));      // the error, negated: so is the half below
+    return fma2(mul2(f2(-0.5f), y), e, y);
+}
+__device__ __forceinline__ F2 rcp2(F2 x)            // rcp_nr of both
+{
+    float a, b, ya, yb;
+    split(x, a, b);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ya) : "f"(a));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yb) : "f"(b));
+    const F2 y = f2(ya, yb);
+    const F2 e = fma2(x, y, f2(-1.f));
+    return fma2(mul2(f2(-1.f), y), e, y);
+}
+__device__ __forceinline__ F2 exp_neg2(F2 x)        // exp_neg of both
+{
+    float a, b, ya, yb;
+    split(mul2(x, f2(-1.4426950408889634f)), a, b);
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ya) : "f"(a));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(yb) : "f"(b));
+    return f2(ya, yb);
+}
+__device__ __forceinline__ F2 poly5_2(F2 ar)        // poly5f of both
+{
+    const double E1 = 0.254829592, E2 = -0.284496736, E3 = 1.421413741,
+                 E4 = -1.453152027, E5 = 1.061405429, PP = 0.3275911;
+    const F2 t = rcp2(fma2(f2(PM_HI(PP)), ar, fma2(f2(PM_LO(PP)), ar, f2(1.0f))));
+    F2 h = add2(fma2(t, f2(PM_HI(E5)), f2(PM_HI(E4))), fma2(t, f2(PM_LO(E5)), f2(PM_LO(E4))));
+    h = add2(fma2(t, h, f2(PM_HI(E3))), f2(PM_LO(E3)));
+    h = add2(fma2(t, h, f2(PM_HI(E2))), f2(PM_LO(E2)));
+    h = add2(fma2(t, h, f2(PM_HI(E1))), f2(PM_LO(E1)));
+    return mul2(t, h);
+}
+
+// pot_f32 of two pairs (no table potentials); m: 1-4 pairs
+template <int POT>
+__device__ __forceinline__ void pot2(const PairArgs& p, const TermF& t, F2 r2, F2 rd2, F2 rinv, F2 qq, int ti, int tja,
+                                     int tjb, bool ma, bool mb, F2& e, F2& f)
+{
+    if (POT == LJ) {
+        const float4 a = __ldg((ma ? p.ljm : p.ljn) + (ti * p.n_types + tja));   // A_hi, B_hi, A_lo, B_lo
+        const float4 b = __ldg((mb ? p.ljm : p.ljn) + (ti * p.n_types + tjb));
+        const F2 r6 = mul2(mul2(rd2, rd2), rd2), r12 = mul2(r6, r6);
+        float r6a, r6b, r12a, r12b;
+        split(r6, r6a, r6b);
+        split(r12, r12a, r12b);
+        const F2 r6B = f2(fmaf(a.y, r6a, __fmul_rn(a.w, r6a)), fmaf(b.y, r6b, __fmul_rn(b.w, r6b)));
+        const F2 r12A = f2(fmaf(a.x, r12a, __fmul_rn(a.z, r12a)), fmaf(b.x, r12b, __fmul_rn(b.z, r12b)));
+        e = sub2(r12A, r6B);
+        f = mul2(fma2(f2(12.0f), r12A, mul2(f2(-6.0f), r6B)), rd2);
+    } else if (POT == CO) {
+        e = mul2(qq, rinv);
+        e = sel2(ma, mb, mul2(e, f2(p.csf)), e);
+        f = mul2(e, rd2);
+    } else {
+        const F2 q = sel2(ma, mb, mul2(qq, f2(p.csf)), qq);
+        const F2 r = mul2(r2, rinv);
+        const F2 ar = fma2(f2(t.alpha), r, mul2(f2(t.alpha_lo), r));
+        const F2 ex = mul2(q, exp_neg2(mul2(ar, ar)));
+        e = mul2(mul2(poly5_2(ar), ex), rinv);
+        f = mul2(mul2(fma2(f2(t.two_alpha_pi), ex, fma2(f2(t.two_alpha_pi_lo), ex, e)), rinv), rinv);
+    }
+}
+
+// sw_f32 of two pairs applied to a term (f = f v - e d, e = e v); OUT as there,
+// ina / inb: inside a Cutoff switch
+template <int SW, bool OUT>
+__device__ __forceinline__ void switch2(const TermF& t, F2 r2, F2 rinv, bool ina, bool inb, F2& e, F2& f)
+{
+    if (SW == SUN || (SW == SCUT && !OUT)) return;
+    const F2 zero = f2(0.f);
+    if (SW == SCUT) {
+        f = sel2(ina, inb, f, zero);
+        e = sel2(ina, inb, e, zero);
+        return;
+    }
+    float ra, rb;
+    split(r2, ra, rb);
+    const bool oa = OUT && ra > t.cut2, ob = OUT && rb > t.cut2;
+    F2 v, d;                                         // the value, and its derivative negated
+    if (SW == SC2) {
+        const F2 c2 = sub2(f2(t.cut2), r2);
+        const F2 c4 = mul2(c2, fma2(f2(-2.0f), r2, f2(-t.s2)));          // negated
+        const F2 c24 = mul2(c2, c4);                                     // negated
+        const F2 dd = fma2(c2, c2, c4);
+        const bool ma = ra >= t.on2, mb = rb >= t.on2;
+        v = sel2(ma, mb, fma2(f2(-t.s1), c24, mul2(f2(-t.s1_lo), c24)), f2(1.f));
+        d = sel2(ma, mb, fma2(f2(-t.s3), dd, mul2(f2(-t.s3_lo), dd)), zero);
+    } else if (SW == SC1) {
+        const F2 dist = mul2(r2, rinv);
+        // -(fma(-r2, c05, c15) + fma(-r2, c05_lo, c15_lo)), then 1 + dist times it
+        const F2 in = add2(fma2(r2, f2(t.c1_05_3), f2(-t.c1_15_1)), fma2(r2, f2(t.c1_05_3_lo), f2(-t.c1_15_1_lo)));
+        v = fma2(dist, in, f2(1.f));
+        d = add2(fma2(dist, f2(-t.c1_15_3), mul2(f2(t.c1_15_1), rinv)),
+                 fma2(dist, f2(-t.c1_15_3_lo), mul2(f2(t.c1_15_1_lo), rinv)));
+    } else {                                         // Shift
+        const F2 x = fma2(r2, f2(-t.sh_a_lo), fma2(r2, f2(-t.sh_a), f2(1.f)));
+        v = mul2(x, x);
+        d = fma2(f2(-t.sh_b), x, mul2(f2(-t.sh_b_lo), x));
+    }
+    if (OUT) {
+        v = sel2(oa, ob, zero, v);
+        d = sel2(oa, ob, zero, d);
+    }
+    f = fma2(f, v, mul2(e, d));
+    e = mul2(e, v);
+}
+
+// pair_math of two pairs of one row atom (no table potentials): force factors
+// and energies, zero for an inactive pair
+template <int NT, int P0, int S0, int P1, int S1, bool OUT>
+__device__ __forceinline__ void pair_math2(const PairArgs& p, const JAtom& ia, const JAtom& ja, const JAtom& jb, F2 r2in,
+                                           bool va, bool vb, int ca, int cb, F2& ft, F2& el, F2& ec)
+{
+    constexpr bool kMod = sw_modifies(S0) || (NT > 1 && sw_modifies(S1));
+    const F2 zero = f2(0.f);
+    const F2 r2 = sel2(va, vb, r2in, f2(1.f));       // keeps inactive lanes finite
+    const F2 rinv = rsqrt2(r2), rd2 = mul2(rinv, rinv);
+    const bool ma = ca & kCodeMod, mb = cb & kCodeMod;
+    F2 qq = zero;
+    if (P0 != LJ || NT > 1)
+        qq = f2(fmaf(ia.p.w, ja.p.w, fmaf(ia.p.w, ja.l.w, __fmul_rn(ia.l.w, ja.p.w))),
+                fmaf(ia.p.w, jb.p.w, fmaf(ia.p.w, jb.l.w, __fmul_rn(ia.l.w, jb.p.w))));
+    F2 e0, f0, e1 = zero, f1 = zero;
+    pot2<P0>(p, p.tf[0], r2, rd2, rinv, qq, ia.m.y, ja.m.y, jb.m.y, ma, mb, e0, f0);
+    if (NT > 1) pot2<P1>(p, p.tf[1], r2, rd2, rinv, qq, ia.m.y, ja.m.y, jb.m.y, ma, mb, e1, f1);
+    if (kMod) {
+        switch2<S0, OUT>(p.tf[0], r2, rinv, ca & kCodeIn0, cb & kCodeIn0, e0, f0);
+        if (NT > 1) switch2<S1, OUT>(p.tf[1], r2, rinv, ca & kCodeIn1, cb & kCodeIn1, e1, f1);
+    }
+    ft = sel2(va, vb, NT > 1 ? add2(f0, f1) : f0, zero);
+    const F2 a = sel2(va, vb, e0, zero), b = NT > 1 ? sel2(va, vb, e1, zero) : zero;
+    el = pot_lj_slot(P0) ? a : zero;
+    ec = pot_lj_slot(P0) ? b : a;                    // (a second term is never Lennard-Jones)
+}
+
 // ---------------------------------------------------------------- K2b': FP32 pairs
 // A warp's shared memory in the mixed kernel
 struct ColShared32 {
@@ -415,9 +598,10 @@ struct ColShared32 {
 constexpr float kScaleJ = 4194304.0f;    // 2^22
 constexpr float kLimitJ = 60.0f;         // a j-force component this large is added in 64 bits at once (8 x 60 2^22 < 2^31)
 
-// Two pairs per lane and step (their instructions interleave).  i-forces, far
-// pairs' energies and virial in FP32 over kEnergyFlush steps, then in FP64 for
-// the chunk, then int64 fixed point.  j-forces are added up over the row's
+// Two pairs per lane and step, their FP32 arithmetic packed (one issue slot for
+// both: the kernel is bound by issue slots, not by the FMA pipe).  i-forces, far
+// pairs' energies and virial in FP32 over the chunk (at most 96 entries: about
+// 20 pairs in each half of a packed sum), then FP64 and int64 fixed point.  j-forces are added up over the row's
 // atoms in shared memory as 32-bit integers of 2^-22 (as fine as FP32 holds a
 // component of 1; each atom gets at most eight per chunk), and added to the
 // atoms' int64 sums once per chunk: everything is independent of the
@@ -432,9 +616,7 @@ struct ColForce32 {
     ColShared32& sh;
     int nq;
     JAtom ia;
-    float f[3], e[2], v[6];              // FP32 partial sums
-    double fd[3], ed[2], vd[6];
-    int steps;
+    F2 f[3], e[2], v[6];                 // FP32 sums, first and second pairs apart
 
     __device__ __forceinline__ void init()
     {
@@ -455,48 +637,24 @@ struct ColForce32 {
     __device__ __forceinline__ void begin(const ColRow& r)
     {
         ia = atom(r.si);
+        const F2 zero = f2(0.f);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) { f[k] = 0.f; fd[k] = 0.0; }
-        e[0] = e[1] = 0.f;
-        ed[0] = ed[1] = 0.0;
+        for (int k = 0; k < 3; ++k) f[k] = zero;
+        e[0] = e[1] = zero;
 #pragma unroll
-        for (int k = 0; k < 6; ++k) { v[k] = 0.f; vd[k] = 0.0; }
-        steps = 0;
+        for (int k = 0; k < 6; ++k) v[k] = zero;
     }
-    __device__ __forceinline__ void flush()
+    // both halves of a sum
+    static __device__ __forceinline__ double whole(F2 a)
     {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) { fd[k] += (double)f[k]; f[k] = 0.f; }
-        ed[0] += (double)e[0]; ed[1] += (double)e[1];
-        e[0] = e[1] = 0.f;
-        if (p.virial) {
-#pragma unroll
-            for (int k = 0; k < 6; ++k) { vd[k] += (double)v[k]; v[k] = 0.f; }
-        }
-        steps = 0;
+        float lo, hi;
+        split(a, lo, hi);
+        return (double)lo + (double)hi;
     }
     __device__ __forceinline__ int slot(int code) const
     {
         const int k = code & kCodeSlot;
         return 4 * (sh.ent[k >> 2] & 0x7fffffff) + (k & 3);
-    }
-    __device__ __forceinline__ PairGeo geo(const ColRow& r, int code, int slot, bool valid) const
-    {
-        PairGeo g;
-        const int4 P = __ldg(p.cq + slot);
-        const float qx = (float)(int)((unsigned)P.x - (unsigned)r.P.x);
-        const float qy = (float)(int)((unsigned)P.y - (unsigned)r.P.y);
-        const float qz = (float)(int)((unsigned)P.z - (unsigned)r.P.z);
-        g.dx = fmaf(qx, p.cg.sch[0], __fmul_rn(qx, p.cg.scl[0]));
-        g.dy = fmaf(qy, p.cg.sch[1], __fmul_rn(qy, p.cg.scl[1]));
-        g.dz = fmaf(qz, p.cg.sch[2], __fmul_rn(qz, p.cg.scl[2]));
-        g.r2 = fmaf(g.dz, g.dz, fmaf(g.dy, g.dy, __fmul_rn(g.dx, g.dx)));
-        g.act = valid;
-        g.in0 = !TWO || (code & kCodeIn0);
-        g.in1 = !TWO || (code & kCodeIn1);
-        g.excl = (code & kCodeMod) ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE;
-        g.near = g.same = false;
-        return g;
     }
     // the j-force of one pair
     __device__ __forceinline__ void add_j(int code, int slot, bool big, bool valid, float x, float y, float z)
@@ -522,33 +680,51 @@ struct ColForce32 {
         const int ca = va ? ring[(at & (kColRing - 1)) * kCluster + il] : 0;
         const int cb = vb ? ring[((at + 4) & (kColRing - 1)) * kCluster + il] : 0;
         const int sa = slot(ca), sb = slot(cb);
-        const PairGeo ga = geo(r, ca, sa, va), gb = geo(r, cb, sb, vb);
         const JAtom ja = atom(sa), jb = atom(sb);
-        float fta, ela, eca, ftb, elb, ecb;
-        pair_math<NT, P0, S0, P1, S1, TWO>(p, ga, ia, ja, fta, ela, eca);
-        pair_math<NT, P0, S0, P1, S1, TWO>(p, gb, ia, jb, ftb, elb, ecb);
-        const float xa = __fmul_rn(ga.dx, fta), ya = __fmul_rn(ga.dy, fta), za = __fmul_rn(ga.dz, fta);
-        const float xb = __fmul_rn(gb.dx, ftb), yb = __fmul_rn(gb.dy, ftb), zb = __fmul_rn(gb.dz, ftb);
-        f[0] -= xa + xb; f[1] -= ya + yb; f[2] -= za + zb;
-        // (not below the limit: NaN too)
-        const bool ba = !(fmaxf(fabsf(xa), fmaxf(fabsf(ya), fabsf(za))) < kLimitJ) || isnan(fta);
-        const bool bb = !(fmaxf(fabsf(xb), fmaxf(fabsf(yb), fabsf(zb))) < kLimitJ) || isnan(ftb);
+        // the pair vectors: exact in fixed point, one rounding to FP32, times
+        // the compensated L / 2^32
+        const int4 A = __ldg(p.cq + sa), B = __ldg(p.cq + sb);
+        const F2 qx = f2((float)(int)((unsigned)A.x - (unsigned)r.P.x), (float)(int)((unsigned)B.x - (unsigned)r.P.x));
+        const F2 qy = f2((float)(int)((unsigned)A.y - (unsigned)r.P.y), (float)(int)((unsigned)B.y - (unsigned)r.P.y));
+        const F2 qz = f2((float)(int)((unsigned)A.z - (unsigned)r.P.z), (float)(int)((unsigned)B.z - (unsigned)r.P.z));
+        const F2 dx = fma2(qx, f2(p.cg.sch[0]), mul2(qx, f2(p.cg.scl[0])));
+        const F2 dy = fma2(qy, f2(p.cg.sch[1]), mul2(qy, f2(p.cg.scl[1])));
+        const F2 dz = fma2(qz, f2(p.cg.sch[2]), mul2(qz, f2(p.cg.scl[2])));
+        const F2 r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+        float ra, rb;
+        split(r2, ra, rb);
+        F2 ft, el, ec;
+        if constexpr (pot_table(P0) || (NT > 1 && pot_table(P1))) {
+            PairGeo ga, gb;                            // (the look-ups do not pack)
+            ga.r2 = ra; ga.act = va;
+            gb.r2 = rb; gb.act = vb;
+            ga.in0 = !TWO || (ca & kCodeIn0); ga.in1 = !TWO || (ca & kCodeIn1);
+            gb.in0 = !TWO || (cb & kCodeIn0); gb.in1 = !TWO || (cb & kCodeIn1);
+            ga.excl = (ca & kCodeMod) ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE;
+            gb.excl = (cb & kCodeMod) ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE;
+            float fa, la, wa, fb, lb, wb;
+            pair_math<NT, P0, S0, P1, S1, TWO>(p, ga, ia, ja, fa, la, wa);
+            pair_math<NT, P0, S0, P1, S1, TWO>(p, gb, ia, jb, fb, lb, wb);
+            ft = f2(fa, fb); el = f2(la, lb); ec = f2(wa, wb);
+        } else {
+            pair_math2<NT, P0, S0, P1, S1, TWO>(p, ia, ja, jb, r2, va, vb, ca, cb, ft, el, ec);
+        }
+        const F2 x = mul2(dx, ft), y = mul2(dy, ft), z = mul2(dz, ft);
+        f[0] = sub2(f[0], x); f[1] = sub2(f[1], y); f[2] = sub2(f[2], z);
+        float xa, xb, ya, yb, za, zb;
+        split(x, xa, xb);
+        split(y, ya, yb);
+        split(z, za, zb);
+        // (not below the limit, and not NaN)
+        const bool ba = !(fabsf(xa) + fabsf(ya) + fabsf(za) < kLimitJ);
+        const bool bb = !(fabsf(xb) + fabsf(yb) + fabsf(zb) < kLimitJ);
         add_j(ca, sa, ba, va, xa, ya, za);
         add_j(cb, sb, bb, vb, xb, yb, zb);
-        const bool na = va && ga.r2 < p.near2, nb = vb && gb.r2 < p.near2;     // near2 = 0: none
-        if (p.virial) {
-            const float ax = na ? 0.f : ga.dx, ay = na ? 0.f : ga.dy, az = na ? 0.f : ga.dz;
-            const float bx = nb ? 0.f : gb.dx, by = nb ? 0.f : gb.dy, bz = nb ? 0.f : gb.dz;
-            v[0] = fmaf(xa, ax, fmaf(xb, bx, v[0]));
-            v[1] = fmaf(xa, ay, fmaf(xb, by, v[1]));
-            v[2] = fmaf(xa, az, fmaf(xb, bz, v[2]));
-            v[3] = fmaf(ya, ay, fmaf(yb, by, v[3]));
-            v[4] = fmaf(ya, az, fmaf(yb, bz, v[4]));
-            v[5] = fmaf(za, az, fmaf(zb, bz, v[5]));
-        }
+        const bool na = va && ra < p.near2, nb = vb && rb < p.near2;           // near2 = 0: none
         if (__any_sync(FULL, na || nb)) {
-            if (na) ela = eca = 0.f;
-            if (nb) elb = ecb = 0.f;
+            const F2 zero = f2(0.f);
+            el = sel2(na, nb, zero, el);
+            ec = sel2(na, nb, zero, ec);
             if (nq > kColNear - 64) { append_near(p, sh.near, nq, lane); nq = 0; }
             const unsigned wa = __ballot_sync(FULL, na), wb = __ballot_sync(FULL, nb), lt = (1u << lane) - 1u;
             if (na) sh.near[nq + __popc(wa & lt)] = make_int2(ia.m.x, ja.m.x | (ca & kCodeMod));
@@ -556,8 +732,18 @@ struct ColForce32 {
             if (nb) sh.near[nq + __popc(wb & lt)] = make_int2(ia.m.x, jb.m.x | (cb & kCodeMod));
             nq += __popc(wb);
         }
-        e[0] += ela + elb;
-        e[1] += eca + ecb;
+        e[0] = add2(e[0], el);
+        e[1] = add2(e[1], ec);
+        if (p.virial) {
+            const F2 w = f2(na ? 0.f : 1.f, nb ? 0.f : 1.f);                   // near pairs' in FP64
+            const F2 wx = mul2(x, w), wy = mul2(y, w), wz = mul2(z, w);
+            v[0] = fma2(wx, dx, v[0]);
+            v[1] = fma2(wx, dy, v[1]);
+            v[2] = fma2(wx, dz, v[2]);
+            v[3] = fma2(wy, dy, v[3]);
+            v[4] = fma2(wy, dz, v[4]);
+            v[5] = fma2(wz, dz, v[5]);
+        }
         if (p.rec_pairs) {                             // diagnostic pair recording
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
@@ -571,7 +757,6 @@ struct ColForce32 {
                 }
             }
         }
-        if (++steps == kEnergyFlush) flush();
     }
     __device__ __forceinline__ void drain(ColRow& r, const int* ring, int keep)
     {
@@ -619,13 +804,13 @@ struct ColForce32 {
     }
     __device__ __forceinline__ void end(const ColRow& r)
     {
-        flush();
         const int lane = threadIdx.x & 31, jj = lane >> 3;
-        const double x = row_sum(fd[0]), y = row_sum(fd[1]), z = row_sum(fd[2]);
+        const double x = row_sum(whole(f[0])), y = row_sum(whole(f[1])), z = row_sum(whole(f[2]));
         if (r.vi && jj < 3)
             fixed_add(p.facc + 3 * (size_t)r.si + jj, jj == 0 ? x : (jj == 1 ? y : z), kScaleMixed, p.status);
         // the eight sums over the warp, scattered: lane 4 k ends with sum k
-        double t[8] = {ed[0], ed[1], vd[0], vd[1], vd[2], vd[3], vd[4], vd[5]};
+        double t[8] = {whole(e[0]), whole(e[1]), whole(v[0]), whole(v[1]), whole(v[2]), whole(v[3]), whole(v[4]),
+                       whole(v[5])};
 #pragma unroll
         for (int w = 4; w > 0; w >>= 1) {
             const bool up = lane & (4 * w);
@@ -670,8 +855,13 @@ __device__ __forceinline__ int col_chunks(const PairArgs& p, bool mark)
     return bad ? 0 : min(*p.chunk_count, p.chunk_cap);
 }
 
+// Blocks per SM: five with an Ewald real term (96 registers, 32 bytes spilled:
+// 5.62 against 5.84 ms for 1,000,000 atoms, 270 against 278 us for 61,233), four
+// without (the fluid of 20,001 ions: 53 against 58 us a step with three systems
+// in flight, where the fifth block keeps the others' kernels waiting); six
+// spill 116 bytes and take 7.96 ms.
 template <int NT, int P0, int S0, int P1, int S1, bool TWO>
-__global__ void __launch_bounds__(128, 4) k_pair_col(const __grid_constant__ PairArgs p)
+__global__ void __launch_bounds__(128, P0 == EW || P1 == EW ? 5 : 4) k_pair_col(const __grid_constant__ PairArgs p)
 {
     pdl_wait();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
