@@ -599,9 +599,11 @@ constexpr float kScaleJ = 4194304.0f;    // 2^22
 constexpr float kLimitJ = 60.0f;         // a j-force component this large is added in 64 bits at once (8 x 60 2^22 < 2^31)
 
 // Two pairs per lane and step, their FP32 arithmetic packed (one issue slot for
-// both: the kernel is bound by issue slots, not by the FMA pipe).  i-forces, far
-// pairs' energies and virial in FP32 over the chunk (at most 96 entries: about
-// 20 pairs in each half of a packed sum), then FP64 and int64 fixed point.  j-forces are added up over the row's
+// both: the kernel is bound by issue slots, not by the FMA pipe).  i-forces
+// in FP32 over a drain (over a whole chunk their error against FP64 was 2-3%
+// larger), far pairs' energies and virial over the chunk (at most 96 entries:
+// about 20 pairs in each half of a packed sum), then FP64 and int64 fixed
+// point.  j-forces are added up over the row's
 // atoms in shared memory as 32-bit integers of 2^-22 (as fine as FP32 holds a
 // component of 1; each atom gets at most eight per chunk), and added to the
 // atoms' int64 sums once per chunk: everything is independent of the
@@ -617,6 +619,7 @@ struct ColForce32 {
     int nq;
     JAtom ia;
     F2 f[3], e[2], v[6];                 // FP32 sums, first and second pairs apart
+    double fs[3];                        // the row atom's force: the drains' sums
 
     __device__ __forceinline__ void init()
     {
@@ -639,7 +642,7 @@ struct ColForce32 {
         ia = atom(r.si);
         const F2 zero = f2(0.f);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) f[k] = zero;
+        for (int k = 0; k < 3; ++k) fs[k] = 0.0;
         e[0] = e[1] = zero;
 #pragma unroll
         for (int k = 0; k < 6; ++k) v[k] = zero;
@@ -770,12 +773,15 @@ struct ColForce32 {
         if (keep) steps = max(1, steps - 2);         // the fullest ring keeps two eights: fewer idle lanes
         m = min(m, steps);
         int b = m > 0 ? il % m : 0;
+        f[0] = f[1] = f[2] = f2(0.f);
         for (int s = 0; s < steps; ++s) {
             const int at = 8 * b + jj;
             step(r, ring, r.head + at, s < m && at < cnt, s < m && at + 4 < cnt);
             b = b + 1 < m ? b + 1 : 0;
         }
         r.head += min(8 * m, cnt);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) fs[k] += whole(f[k]);
     }
     // One chunk of a row's entries
     __device__ __forceinline__ void run(const ColTest& t, const int4& cd)
@@ -805,7 +811,7 @@ struct ColForce32 {
     __device__ __forceinline__ void end(const ColRow& r)
     {
         const int lane = threadIdx.x & 31, jj = lane >> 3;
-        const double x = row_sum(whole(f[0])), y = row_sum(whole(f[1])), z = row_sum(whole(f[2]));
+        const double x = row_sum(fs[0]), y = row_sum(fs[1]), z = row_sum(fs[2]);
         if (r.vi && jj < 3)
             fixed_add(p.facc + 3 * (size_t)r.si + jj, jj == 0 ? x : (jj == 1 ? y : z), kScaleMixed, p.status);
         // the eight sums over the warp, scattered: lane 4 k ends with sum k
