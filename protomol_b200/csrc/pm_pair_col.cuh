@@ -219,25 +219,31 @@ static __global__ void __launch_bounds__(128) k_col_list(const __grid_constant__
         return;
     }
     // equal chunks of a row, an even number of entries each; the last rows'
-    // (about the last to run) are shorter, so that the kernel's end is
+    // (about the last to run) are shorter, so that the kernel's end is even
     const int most = 8 * row < 5 * rows ? p.chunk : p.chunk_end;
     const int nch = (ne + most - 1) / most, per = ((ne + nch - 1) / nch + 1) & ~1;
     int b0 = 0, b1 = 0;
     if (lane == 0) {
         b0 = atomicAdd(p.plist_count, ne);
         b1 = atomicAdd(p.chunk_count, nch);
+        // (a count beyond 2^31 reads as negative)
+        const bool full0 = b0 < 0 || b0 > p.plist_cap - ne, full1 = b1 < 0 || b1 > p.chunk_cap - nch;
+        const bool full = full0 || full1;
         // the FP64 kernels take a row that did not fit without its entries
-        const bool full = b0 > p.plist_cap - ne || b1 > p.chunk_cap - nch;
         p.rowent[row] = full ? make_int2(-1, 0) : make_int2(b0, ne);
         if (full && p.col_refuse) {
             atomicOr(p.status, kStatusListFull);
             // the list buffer is counted in int2: two entries each
-            if (b0 > p.plist_cap - ne) atomicMax(p.plist_need, (b0 + ne) / 2 + 1);
-            if (b1 > p.chunk_cap - nch) atomicMax(p.chunk_need, b1 + nch);
+            if (full0) atomicMax(p.plist_need, (int)(((unsigned)b0 + (unsigned)ne) / 2) + 1);
+            if (full1) atomicMax(p.chunk_need, (int)min((unsigned)b1 + (unsigned)nch, 0x7fffffffu));
+        } else if (full) {                                       // (given back: the counts stay near their caps)
+            atomicSub(p.plist_count, ne);
+            atomicSub(p.chunk_count, nch);
         }
+        if (full) b0 = -1;
     }
     const int ebase = __shfl_sync(FULL, b0, 0), cbase = __shfl_sync(FULL, b1, 0);
-    if (ebase > p.plist_cap - ne || cbase > p.chunk_cap - nch) return;         // warp-uniform
+    if (ebase < 0) return;                                       // warp-uniform
     if (ne <= kColStageEntries) {
         for (int t = lane; t < ne; t += 32) p.clist[ebase + t] = s_ent[w][t];
     } else {                                              // more than the staging holds: list again, into place

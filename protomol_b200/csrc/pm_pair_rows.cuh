@@ -361,6 +361,24 @@ __device__ __forceinline__ void row_add(const PairArgs& p, int slot, int c, doub
         fixed_add(p.facc + 3 * (size_t)slot + c, v, p.scale, p.status);
 }
 
+// all three components, one test of their magnitudes (by the high words: 200
+// there is its bit pattern, and infinities and NaN are above)
+__device__ __forceinline__ void row_add3(const PairArgs& p, int slot, double x, double y, double z)
+{
+    const int lim = __double2hiint(200.0);
+    const int hx = __double2hiint(x) & 0x7fffffff, hy = __double2hiint(y) & 0x7fffffff, hz = __double2hiint(z) & 0x7fffffff;
+    if (max(hx, max(hy, hz)) < lim) {
+        unsigned long long* to = p.faccj + 3 * (size_t)slot;
+        atomicAdd(to, (unsigned long long)__double2ll_rn(x * kScaleRowJ));
+        atomicAdd(to + 1, (unsigned long long)__double2ll_rn(y * kScaleRowJ));
+        atomicAdd(to + 2, (unsigned long long)__double2ll_rn(z * kScaleRowJ));
+    } else {
+        row_add(p, slot, 0, x);
+        row_add(p, slot, 1, y);
+        row_add(p, slot, 2, z);
+    }
+}
+
 template <bool COL, int NT, int P0, int S0, int P1, int S1>
 struct ForceRow {
     const PairArgs& p;
@@ -396,9 +414,7 @@ struct ForceRow {
         if (!valid) { ft = 0.0; e0 = 0.0; e1 = 0.0; }
         if (COL && valid) {
             // the half list: the j side's force too
-            row_add(p, j, 0, dx * ft);
-            row_add(p, j, 1, dy * ft);
-            row_add(p, j, 2, dz * ft);
+            row_add3(p, j, dx * ft, dy * ft, dz * ft);
         }
         if (pot_lj_slot(P0)) el += e0; else ec += e0;
         if (NT > 1) { if (pot_lj_slot(P1)) el += e1; else ec += e1; }

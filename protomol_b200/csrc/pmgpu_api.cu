@@ -1781,6 +1781,7 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
         sys->buf_version++;
     }
     long long lneed = 0, cneed = 0;
+    bool mixed = false;                    // some force has the mixed kernels' near pairs
     if (sys->eval_use_col || sys->eval_col64) {
         const ColGrid& g = sys->eval_cg;
         const int icl = sys->n / kCluster + g.ncol + 1;
@@ -1802,6 +1803,7 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
         for (int k = 0; k < nf; ++k) {
             if (forces[k]->kind != 0) continue;
             const double rc = std::sqrt(forces[k]->cut2);
+            mixed |= !pairs64(sys, forces[k]);
             const double rl = rc + (pairs64(sys, forces[k]) ? 0.0 : sys->list_skin), vol = g.lx * g.ly * g.lz;
             const long long entries = col_list_estimate(sys->n, g, vol, rl);
             const int chunk = col_chunk_entries(sys->n, g, vol, rc, 6 * sys->tuning.chunk_entries, true);
@@ -1812,6 +1814,7 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
     if (!sys->eval_use_col) {
         for (int k = 0; k < nf; ++k)
             if (forces[k]->kind == 0 && !pairs64(sys, forces[k])) {
+                mixed = true;
                 lneed = std::max(lneed, plist_estimate(sys->n, sys->grid, forces[k]->nh));
                 cneed = std::max(cneed, chunk_estimate(sys->n, sys->grid, forces[k]->nh, sys->tuning.chunk_entries));
             }
@@ -1819,6 +1822,10 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
     if (lneed > 0) {
         lneed = std::max(lneed, sys->plist_need + sys->plist_need / 4);
         cneed = std::max(cneed, sys->chunk_need + sys->chunk_need / 4);
+        if (!mixed) {                        // a row without entries finds its pairs by itself
+            lneed = std::min(lneed, (long long)INT_MAX);
+            cneed = std::min(cneed, (long long)INT_MAX);
+        }
         if (lneed > INT_MAX || cneed > INT_MAX)
             return fail(sys, PMGPU_ERR_CAPACITY, "cluster-pair list above 2^31 entries");
         if (lneed > sys->plist_cap) {
@@ -1831,6 +1838,8 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
             sys->chunk_cap = cneed;
             sys->buf_version++;
         }
+    }
+    if (mixed) {
         // near pairs (< 5 A): ~26 per atom in water
         long long nneed = std::max(30LL * sys->n + 4096, sys->near_need + sys->near_need / 4);
         if (nneed > INT_MAX / 2) return fail(sys, PMGPU_ERR_CAPACITY, "near-pair list above 2^30 entries");
