@@ -275,8 +275,9 @@ int launch_near_energy_col(const PairArgs& a, int combo, int n_atoms, cudaStream
 long long col_list_estimate(int n_atoms, const ColGrid& g, double volume, double cutoff);
 long long col_chunk_estimate(long long entries, int n_atoms, const ColGrid& g, int chunk);
 int col_chunk_entries(int n_atoms, const ColGrid& g, double volume, double cutoff, int most, bool last);
-int col_rows_split(int n_atoms, const ColGrid& g, double cutoff);
-int col_row_blocks(int n_atoms, const ColGrid& g, double cutoff);
+int col_rows_split(int n_atoms, const ColGrid& g, double cutoff, int blocks_per_sm);
+int col_row_blocks(int n_atoms, const ColGrid& g, double cutoff, int blocks_per_sm);
+int fp64_col_blocks_per_sm(int combo);     // of launch_pair_fp64 over the columns (the other row kernels: 4)
 int launch_pair_fp64(const PairArgs& a, int combo, bool col, int blocks, cudaStream_t s, long long* launches);
 // the molecular virial records (kMRec) of a cutoff force over the cell-sorted
 // order, one per block (blocks as launch_pair_fp64), no forces or energies

@@ -49,6 +49,7 @@ __device__ __forceinline__ void lj_cache_add(LjCache& c, long long key, double p
 
 template <bool COL, typename R>
 struct AdjRow {
+    static constexpr bool kAhead = false;
     const PairArgs& p;
     const AdjArgs& aa;
     double* lj_tab;
@@ -187,11 +188,11 @@ int pair_blocks(int n_atoms, const CellGrid& g, int nd)
 }
 
 // Shares of a row of the FP64 row kernels over the columns.  The shares go to
-// the resident warps (148 SMs x 16) in a fixed order, so that a share count
+// the resident warps (148 SMs x 4 x blocks_per_sm) in a fixed order, so that a share count
 // just above a multiple of theirs leaves most of them idle in the last round;
 // a short share spends its end on partly filled rings (about twelve entries'
 // worth).  The share count of the best product is taken.
-int col_rows_split(int n_atoms, const ColGrid& g, double cutoff)
+int col_rows_split(int n_atoms, const ColGrid& g, double cutoff, int blocks_per_sm)
 {
     const double vol = g.lx * g.ly * g.lz, rho = vol > 0.0 ? n_atoms / vol : 0.0, r = cutoff + 3.0;
     const double rows = (double)n_atoms / kCluster + 0.5 * g.ncol + 1.0;
@@ -199,18 +200,21 @@ int col_rows_split(int n_atoms, const ColGrid& g, double cutoff)
     int best = 1;
     double top = 0.0;
     for (int s = 1; s <= 16; ++s) {
-        const double x = rows * s / (148.0 * 16.0), len = per / s;
+        const double x = rows * s / (148.0 * 4.0 * blocks_per_sm), len = per / s;
         const double score = x / std::ceil(x) * len / (len + 12.0);
         if (score > top) { top = score; best = s; }
     }
     return best;
 }
 
-int col_row_blocks(int n_atoms, const ColGrid& g, double cutoff)
+int col_row_blocks(int n_atoms, const ColGrid& g, double cutoff, int blocks_per_sm)
 {
-    const long long items = ((long long)n_atoms / kCluster + g.ncol + 1) * col_rows_split(n_atoms, g, cutoff);
-    return (int)std::max(1LL, std::min((items + 3) / 4, 148LL * 4));
+    const long long items = ((long long)n_atoms / kCluster + g.ncol + 1) * col_rows_split(n_atoms, g, cutoff, blocks_per_sm);
+    return (int)std::max(1LL, std::min((items + 3) / 4, 148LL * blocks_per_sm));
 }
+
+// (the combinations from 17 on have a table)
+int fp64_col_blocks_per_sm(int combo) { return combo >= 17 ? 4 : 5; }
 
 int launch_pair_fp64(const PairArgs& a, int combo, bool col, int blocks, cudaStream_t s, long long* launches)
 {

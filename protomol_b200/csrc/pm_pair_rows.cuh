@@ -263,11 +263,29 @@ struct ColOp64 {
         if (keep) steps = max(1, steps - 4);
         m = min(m, steps);
         int b = m > 0 ? (2 * il) % m : 0;
-        for (int s = 0; s < steps; ++s) {
+        bool valid = false;
+        auto code = [&](int s) {
             const int at = 4 * b + jj;
-            const bool valid = s < m && at < cnt;
-            op.pair(valid, valid ? ring[((r.head + at) & (kColRing - 1)) * kCluster + il] : r.si);
+            valid = s < m && at < cnt;
             b = b + 1 < m ? b + 1 : 0;
+            return valid ? ring[((r.head + at) & (kColRing - 1)) * kCluster + il] : r.si;
+        };
+        if constexpr (RowOp::kAhead) {
+            int next = code(0);
+            auto fetched = op.fetch(next);
+            for (int s = 0; s < steps; ++s) {
+                const int e = next;
+                const auto f = fetched;
+                const bool v = valid;
+                next = code(s + 1);
+                fetched = op.fetch(next);
+                op.pair(v, e, f);
+            }
+        } else {
+            for (int s = 0; s < steps; ++s) {
+                const int e = code(s);
+                op.pair(valid, e);
+            }
         }
         r.head += min(4 * m, cnt);
     }
@@ -381,6 +399,12 @@ __device__ __forceinline__ void row_add3(const PairArgs& p, int slot, double x, 
 
 template <bool COL, int NT, int P0, int S0, int P1, int S1>
 struct ForceRow {
+    // With a table every pair waits for its j-atom and then for its table row:
+    // the next pair's j-atom is loaded meanwhile (192k atoms, both terms from
+    // tables: 1337 -> 1269 us).  The other terms take the registers for a fifth
+    // block instead (14,281 atoms: 169 us, with the early load 177).
+    static constexpr bool kAhead = COL && (pot_table(P0) || (NT > 1 && pot_table(P1)));
+    struct Fetched { double4 P; int type; };
     const PairArgs& p;
     double4 Pi;
     int4 mi;
@@ -399,11 +423,17 @@ struct ForceRow {
         mi = row_meta<COL>(p, si);
         fx = fy = fz = 0.0;
     }
-    __device__ __forceinline__ void pair(bool valid, int e)
+    __device__ __forceinline__ Fetched fetch(int e) const
     {
         const int j = e & kCodeSlot;
-        const double4 Pj = row_pos<COL>(p, j);
-        const int tj = row_type<COL>(p, j);
+        return {row_pos<COL>(p, j), row_type<COL>(p, j)};
+    }
+    __device__ __forceinline__ void pair(bool valid, int e) { pair(valid, e, fetch(e)); }
+    __device__ __forceinline__ void pair(bool valid, int e, const Fetched& fe)
+    {
+        const int j = e & kCodeSlot;
+        const double4 Pj = fe.P;
+        const int tj = fe.type;
         const double dx = image_diff(Pi.x, Pj.x, p.pbc.e1x, p.pbc.e1rx);
         const double dy = image_diff(Pi.y, Pj.y, p.pbc.e2y, p.pbc.e2ry);
         const double dz = image_diff(Pi.z, Pj.z, p.pbc.e3z, p.pbc.e3rz);
@@ -470,8 +500,14 @@ __global__ void __launch_bounds__(128, 4) k_pair_fp64(const __grid_constant__ Pa
     force_record(p, op, 0.5);
 }
 
+// blocks an SM: with a table 4 (a fifth spills, and 192k atoms take 1334 us for
+// 1329), else 5 (the pair phase waits for its own results, 49% of the issue
+// slots used; 14,281 atoms: 191 -> 169 us)
+template <int NT, int P0, int P1>
+constexpr int kRow64Blocks = pot_table(P0) || (NT > 1 && pot_table(P1)) ? 4 : 5;
+
 template <int NT, int P0, int S0, int P1, int S1>
-__global__ void __launch_bounds__(128, 4) k_pair_fp64_col(const __grid_constant__ PairArgs p)
+__global__ void __launch_bounds__(128, kRow64Blocks<NT, P0, P1>) k_pair_fp64_col(const __grid_constant__ PairArgs p)
 {
     pdl_wait();
     __shared__ ColRowsShared sh[4];
@@ -492,6 +528,7 @@ __global__ void __launch_bounds__(128, 4) k_pair_fp64_col(const __grid_constant_
 // forces, no energies.
 template <bool COL, int NT, int P0, int S0, int P1, int S1>
 struct MolvirRow {
+    static constexpr bool kAhead = false;
     const PairArgs& p;
     double4 Pi;
     int4 mi;

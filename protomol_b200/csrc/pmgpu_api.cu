@@ -1592,7 +1592,7 @@ static void fill_col_args(pmgpu_system* sys, bool fp64, PairArgs& a, bool half)
     a.col_refuse = fp64 ? 0 : 1;
     a.col_half = half ? 1 : 0;
     a.col_none = 2 * sys->col_ncl_cap;
-    a.rows_split = col_rows_split(sys->n, sys->eval_cg, std::sqrt(a.cut2d));
+    a.rows_split = col_rows_split(sys->n, sys->eval_cg, std::sqrt(a.cut2d), 4);
     const ColGrid& g = sys->eval_cg;
     a.chunk = col_chunk_entries(sys->n, g, g.lx * g.ly * g.lz, std::sqrt(a.cut2d), 6 * sys->tuning.chunk_entries, false);
     a.chunk_end = col_chunk_entries(sys->n, g, g.lx * g.ly * g.lz, std::sqrt(a.cut2d), 6 * sys->tuning.chunk_entries, true);
@@ -1670,10 +1670,16 @@ static int ensure_erec(pmgpu_system* sys, int need)
     return PMGPU_OK;
 }
 
-// blocks (records) of the FP64 row kernels of one cutoff force
-static int row_blocks(const pmgpu_system* sys, const pmgpu_force* f)
+// blocks (records) of the FP64 row kernels of one cutoff force: the molecular
+// virial and the adjoint, and the force kernel
+static int row_blocks(const pmgpu_system* sys, const pmgpu_force* f, int per_sm = 4)
 {
-    return sys->eval_col64 ? col_row_blocks(sys->n, sys->eval_cg, std::sqrt(f->cut2)) : pair_blocks(sys->n, sys->grid, f->nd);
+    return sys->eval_col64 ? col_row_blocks(sys->n, sys->eval_cg, std::sqrt(f->cut2), per_sm)
+                           : pair_blocks(sys->n, sys->grid, f->nd);
+}
+static int force_row_blocks(const pmgpu_system* sys, const pmgpu_force* f)
+{
+    return row_blocks(sys, f, fp64_col_blocks_per_sm(f->combo));
 }
 
 // energy records one cutoff force writes
@@ -1681,7 +1687,7 @@ static int pair_records(pmgpu_system* sys, pmgpu_force* f)
 {
     // the mixed kernel sums energies in fixed point (d_efix), no records
     if (f->kind == 2) return adjoint_blocks(sys->n);
-    return pairs64(sys, f) ? row_blocks(sys, f) : 0;
+    return pairs64(sys, f) ? force_row_blocks(sys, f) : 0;
 }
 
 // upper bound of the energy records of the fused x pass (one per CTA, at
@@ -2288,6 +2294,8 @@ static int run_cutoffs(EvalRun& R, bool may_defer)
         PairArgs a;
         fill_pair_args(sys, f, d_pos, a);
         if (col) fill_col_args(sys, fp64, a, true);
+        if (col && fp64)
+            a.rows_split = col_rows_split(sys->n, sys->eval_cg, std::sqrt(a.cut2d), fp64_col_blocks_per_sm(f->combo));
         a.virial = virial;
         a.erec = sys->d_erec + used;
         // the column list, or the cell-cluster list of the mixed forces
@@ -2302,7 +2310,7 @@ static int run_cutoffs(EvalRun& R, bool may_defer)
             return PMGPU_OK;
         }
         int m = prof_begin(sys, kPhasePair);
-        int e = fp64 ? launch_pair_fp64(a, f->combo, col, row_blocks(sys, f), s, &sys->launches)
+        int e = fp64 ? launch_pair_fp64(a, f->combo, col, force_row_blocks(sys, f), s, &sys->launches)
                      : (col ? launch_pair_col(a, f->combo, s, &sys->launches)
                             : launch_pair_mixed(a, f->combo, s, &sys->launches));
         if (e) return cuda_fail(sys, (cudaError_t)e, "pair kernel");
