@@ -337,7 +337,9 @@ void* pmgpu_batch_stream(pmgpu_batch* batch);
  * block, whether PME runs on a second stream beside the pair kernels, and
  * whether mixed cutoff forces take the FP64 pair kernels.  Results do not
  * depend on the first four beyond the last bits of the fixed-point grouping
- * (a chunk's partial sums are rounded together); fp64_pairs gives the FP64
+ * (a chunk's partial sums are rounded together); over columns a chunk's length
+ * follows from the system's size and chunk_entries bounds it (at six times its
+ * value).  fp64_pairs gives the FP64
  * kernels' results, which hold every mixed-precision bound.  Defaults: 16, 0
  * (the occupancy limit), 16, 1, 0. */
 typedef struct pmgpu_tuning {
@@ -345,8 +347,8 @@ typedef struct pmgpu_tuning {
     int pair_blocks_per_sm;   /* resident blocks of the mixed pair kernel per SM: 0 (occupancy limit) or 1..8 */
     int fft_lines;            /* lines per block of the strided PME FFT passes, at most: 1..16 (z passes: twice) */
     int pme_concurrent;       /* 1: PME on a second stream beside the pair kernels; 0: after them */
-    int fp64_pairs;           /* 1: mixed cutoff forces run the FP64 pair kernels (no cluster list, no
-                                 near-pair pass: the shorter launch chain, faster on a few hundred atoms) */
+    int fp64_pairs;           /* 1: mixed cutoff forces run the FP64 pair kernels (no near-pair
+                                 pass: the shorter launch chain, faster on a few hundred atoms) */
     double ms_per_eval;       /* pmgpu_autotune: the measured time of the chosen tuning */
 } pmgpu_tuning;
 int pmgpu_get_tuning(pmgpu_system* sys, pmgpu_tuning* out);
@@ -448,7 +450,7 @@ int pmgpu_get_cells(pmgpu_system* sys, int* cells, int* dims);
 /* No counterpart in the reference (diagnostic).  The cluster layout the
  * mixed-precision cutoff forces of the last evaluation ran on:
  * PMGPU_LAYOUT_COLUMNS (fixed-point coordinates in z-sorted columns, boxes
- * well above twice the cutoff), PMGPU_LAYOUT_CELLS (clusters inside the
+ * of at least twice the cutoff), PMGPU_LAYOUT_CELLS (clusters inside the
  * reference cells: smaller boxes, the small-grid mode, or a system whose
  * columns or clusters exceeded the column layout's limits),
  * PMGPU_LAYOUT_FP64 (the FP64 pair kernels, tuning fp64_pairs), or 0 (none

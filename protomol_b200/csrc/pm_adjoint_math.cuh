@@ -1,5 +1,5 @@
 // pm_adjoint_math.cuh -- per-pair math of the backward pass (K10), shared by
-// the all-pairs kernel (pm_adjoint.cu) and the cell-list kernel (pm_pair.cu).
+// the all-pairs kernel (pm_adjoint.cu) and the row kernels (pm_pair_rows.cu).
 #pragma once
 
 #include "pm_kernels.h"

@@ -43,12 +43,11 @@ constexpr int kCluster = 8;     // atoms per cluster (z-sorted slab of a cell)
 int launch_bin(const BinArgs& a, cudaStream_t s, long long* launches);
 
 // ---------------------------------------------------------------- column clusters
-// The mixed pair path of boxes well above twice the cutoff: atoms in
+// The pair path of boxes of at least twice the cutoff: atoms in
 // unsigned 32-bit fixed point of the box (x / L * 2^32, so that the int32
 // difference of two atoms is their minimal-image displacement exactly), in
 // columns of an x-y grid (~4 A side) sorted by z; every run of 8 atoms of a
 // column is an i-cluster, each half of it a 4-atom j-cluster.
-constexpr int kColAtoms = 1024;  // atoms a column may hold (more: the cell-cluster path)
 struct ColGrid {
     int ncx, ncy, ncol;
     int rx, ry;                  // column reach of the list
@@ -226,7 +225,7 @@ struct PairArgs {
     int blocks_per_sm;           // resident blocks of the mixed pair kernel per SM (0: the occupancy limit)
     int chunk;                   // cluster-list entries per chunk of pair work
     int chunk_end;               // column lists: those of the last rows
-    // column-cluster path (K2a' / K2b'): slot data, cluster boxes, grid
+    // column-cluster path (K2a' / K2b' / K9'): slot data, cluster boxes, grid
     const int4* cq;
     const int4* cm;
     const float4* ibox;
@@ -238,7 +237,7 @@ struct PairArgs {
     int* clist;                  // column-path entries (the plist buffer): j-clusters, a row's contiguous
     int2* rowent;                // per row: first entry (< 0: not listed) and entries
     int col_none;                // a j-cluster of padding atoms (the last row's, written by the binning)
-    int col_half;                // the list names every unordered pair once (mixed forces), or every ordered one
+    int col_half;                // the list names every unordered pair once (forces, molecular virial), or every ordered one (adjoint)
     int col_refuse;              // 1: a list that does not fit (or a row too tall) is an error status (mixed forces)
     int icl_cap;                 // i-clusters the list kernel's grid covers
     ColGrid cg;

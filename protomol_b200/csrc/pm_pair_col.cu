@@ -31,8 +31,16 @@ int col_chunk_entries(int n_atoms, const ColGrid& g, double volume, double cutof
     const double r = cutoff + 0.75 * std::max(g.sx, g.sy);
     const double rows = (double)n_atoms / kCluster + 0.5 * g.ncol + 1;
     const double per = std::min(rho * (4.0 / 3.0) * 3.14159265358979 * r * r * r / 4.0, 2.0 * rows);
-    const double want = rows * per * 0.5 / ((last ? 6.0 : 2.0) * 148 * 16);
-    return std::max(16, std::min(std::min(most, kColBlock), 2 * (int)(0.5 * std::min(want, 1e6) + 1.0)));
+    const double all = rows * per * 0.5, warps = 148 * 16;
+    const double want = all / ((last ? 6.0 : 2.0) * warps);
+    // The shortest: 32 entries from about 2,000 atoms on (with 16 the partly
+    // filled rings at the chunks' ends cost more than the even end gives: with
+    // three 4,500-atom boxes in flight 40.8 us an evaluation for 43.6, 24 boxes
+    // of 300 to 9,000 atoms 874 us for 922), 16 below that (1,000 atoms: 22.0 us
+    // for 23.5, alone 56.9 for 60.5)
+    most = std::max(16, std::min(most, kColBlock));
+    const int least = std::min(most, all < 8.0 * warps ? 16 : 32);
+    return std::max(least, std::min(most, 2 * (int)(0.5 * std::min(want, 1e6) + 1.0)));
 }
 
 long long col_chunk_estimate(long long entries, int n_atoms, const ColGrid& g, int chunk)

@@ -18,9 +18,9 @@
 // K2a' k_col_list: one warp per row lists the j-clusters whose bounding box
 // comes within the cutoff (plus the FP32 guard band) of the row's box by the
 // nearest image.  Boxes are center and half extent; the gap of the nearest
-// centers is a bound in any box.  Two forms: the full list (FP64 kernels: every
-// ordered pair of atoms once) and the half list (mixed kernel, molecular
-// virial: every unordered pair once).  In the half list a pair of columns
+// centers is a bound in any box.  Two forms: the half list (the forces of both
+// precisions, the molecular virial: every unordered pair of atoms once) and the
+// full list (the backward pass: every ordered pair once).  In the half list a pair of columns
 // belongs to the one whose offset to the other is in the positive half plane
 // and, within a column, a pair of rows to the lower one; where the reach covers
 // the box (an offset is no longer unique) a pair of rows r < s belongs to r
@@ -44,7 +44,7 @@
 // lanes were two thirds of the kernel's 106 M warp instructions on the
 // 14,281-atom box.  The rings fill the lanes of the pair phase, and its FP32
 // arithmetic is packed two pairs to an instruction: 67 M.
-// Measured against the tile-by-tile kernel, each kernel alone: 8.10 -> 5.62 ms
+// Measured against the tile-by-tile kernel, each kernel alone: 8.10 -> 5.65 ms
 // for 1,000,000 atoms at 12 A, 360 -> 270 us for 61,233 at 10 A, 141 -> 133 us
 // for 14,281 (where 47 us do not shrink with the cutoff: the near-pair kernel's
 // 13, the launch and the unevenness of the last chunks).  Tried: a full list

@@ -39,10 +39,11 @@
 // sums, and the rings keep every lane of the pair phase busy.
 // Measured on the 14,281-atom box: 595 us over cell blocks, 479 us over these
 // rows (270 us of it the test phase: partly filled clusters of half-cutoff
-// cells, gathered in the kernel).  The column rows take 186 us: prebuilt
+// cells, gathered in the kernel).  The column rows take 169 us: prebuilt
 // entries of full clusters (half the test), and every pair once, the j side
 // added in 64-bit integers by the lane that has it (278 us with every pair from
-// both sides).  192,003 atoms with look-up tables: 5.32 -> 1.32 ms.
+// both sides, 191 us at four blocks per SM instead of five).  192,003 atoms with
+// look-up tables: 5.32 -> 1.27 ms.
 
 constexpr int kRing = 64;            // ring places per row atom
 constexpr int kRingDrain = 32;       // a drain stops when every ring is below this
