@@ -202,7 +202,7 @@ struct PairArgs {
     int virial;
     // outputs
     unsigned long long* facc;    // 3 per sorted slot
-    unsigned long long* faccj;   // FP64 rows over the columns: the fine sums (2^44), 3 per slot
+    unsigned long long* faccj;   // FP64 rows: the fine sums (2^44), 3 per slot
     double scale;
     double* erec;                // energy records (component-major, see kERec)
     int erec_stride;
@@ -465,6 +465,7 @@ struct FinArgs {
     const unsigned long long* f32;      // mixed pair forces (whole-cell shifts), 2^32
     const unsigned long long* f32p;     // other mixed forces (PME, per-pair minimal image), 2^32
     const unsigned long long* f40;      // FP64 forces, 2^40
+    const unsigned long long* f44;      // and their fine sums, 2^44 (with f40)
     const unsigned long long* a32;      // in atom order (PME): mixed, 2^32
     const unsigned long long* a40;      // in atom order (PME): FP64, 2^40
     const int* sorted;

@@ -368,7 +368,7 @@ __device__ __forceinline__ void col_rows64(const PairArgs& p, ColRowsShared& sh,
 }
 
 // ---------------------------------------------------------------- K9: forces
-// One force component of a slot over the columns.  Up to 200 kcal/mol/A it goes
+// One force component of a slot.  Up to 200 kcal/mol/A it goes
 // to the finer of the slot's two sums (2^44: the rounding of a pair's share is
 // a sixteenth of the other's quantum, and a few thousand such shares stay
 // inside 64 bits), above that (NaN too) to the wide one.
@@ -472,8 +472,7 @@ struct ForceRow {
         const int jj = (threadIdx.x & 31) >> 3;
         if (vi && jj < 3) {
             const double v = jj == 0 ? fx : (jj == 1 ? fy : fz);
-            if (COL) row_add(p, si, jj, v);
-            else fixed_add(p.facc + 3 * (size_t)si + jj, v, p.scale, p.status);
+            row_add(p, si, jj, v);
         }
     }
 };

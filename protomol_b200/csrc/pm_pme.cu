@@ -1271,7 +1271,9 @@ __global__ void __launch_bounds__(256) k_finalize(FinArgs a)
             if (a.f32) fp[c] = (double)(long long)a.f32[3 * (size_t)s + c] * (1.0 / kScaleMixed);
             double f = fp[c];
             if (a.f32p) f += (double)(long long)a.f32p[3 * (size_t)s + c] * (1.0 / kScaleMixed);
-            if (a.f40) f += (double)(long long)a.f40[3 * (size_t)s + c] * (1.0 / kScaleFp64);
+            if (a.f40)
+                f += (double)(long long)a.f40[3 * (size_t)s + c] * (1.0 / kScaleFp64) +
+                     (double)(long long)a.f44[3 * (size_t)s + c] * (1.0 / kScaleRowJ);
             if (a.a32) f += (double)(long long)a.a32[3 * (size_t)i + c] * (1.0 / kScaleMixed);
             if (a.a40) f += (double)(long long)a.a40[3 * (size_t)i + c] * (1.0 / kScaleFp64);
             ft[c] = f;

@@ -127,7 +127,7 @@ struct pmgpu_system {
     int* h_status = nullptr;           // pinned: the status word, copied back with the results
     unsigned long long* d_facc32 = nullptr;   // mixed (2^32): 3N pair forces + 3N other (d_facc32p)
     unsigned long long* d_facc32p = nullptr;
-    unsigned long long* d_facc40 = nullptr;   // FP64 (2^40)
+    unsigned long long* d_facc40 = nullptr;   // FP64 over cells: wide sums (2^40), then fine ones (2^44)
     // PME forces in atom order (PME needs no binning, so it runs beside it):
     // 3N mixed (2^32) then 3N FP64 (2^40)
     unsigned long long* d_faccA = nullptr;
@@ -659,7 +659,7 @@ extern "C" int pmgpu_set_topology(pmgpu_system* sys, int n_atoms, const double* 
     }
     // per-evaluation atom buffers
     CK(dalloc(&sys->d_pos, 3 * (size_t)n), "alloc"); CK(dalloc(&sys->d_fout, 3 * (size_t)n), "alloc");
-    CK(dalloc(&sys->d_facc32, 6 * (size_t)n), "alloc"); CK(dalloc(&sys->d_facc40, 3 * (size_t)n), "alloc");
+    CK(dalloc(&sys->d_facc32, 6 * (size_t)n), "alloc"); CK(dalloc(&sys->d_facc40, 6 * (size_t)n), "alloc");
     CK(dalloc(&sys->d_faccA, 6 * (size_t)n), "alloc");
     sys->d_facc32p = sys->d_facc32 + 3 * (size_t)n;
     CK(dalloc(&sys->d_cell_lin, n), "alloc"); CK(dalloc(&sys->d_cell3, 3 * (size_t)n), "alloc");
@@ -1656,7 +1656,7 @@ static void fill_pair_args(pmgpu_system* sys, pmgpu_force* f, const double* d_po
     a.status = sys->d_status;
     // mixed forces on whole-cell shifts go to the pair accumulator (their
     // virial is completed from it at finalize), the small-grid mode to the other
-    if (pairs64(sys, f)) { a.facc = sys->d_facc40; a.scale = kScaleFp64; }
+    if (pairs64(sys, f)) { a.facc = sys->d_facc40; a.faccj = sys->d_facc40 + 3 * (size_t)sys->n; a.scale = kScaleFp64; }
     else { a.facc = f->wrap ? sys->d_facc32p : sys->d_facc32; a.scale = kScaleMixed; }
 }
 
@@ -1694,6 +1694,8 @@ static int pair_records(pmgpu_system* sys, pmgpu_force* f)
 // least one x-line per CTA)
 static int pme_xblocks(const pmgpu_force* f) { return f->pp.grid[1] * f->kzh; }
 
+constexpr int kCol64Atoms = 900;       // FP64 forces of fewer atoms stay on the cells
+
 // The column-cluster path takes the cutoff forces of the group when the box
 // suits the largest of their cutoffs; the mixed ones not after it refused the
 // system.  Otherwise the cell layout takes them.
@@ -1722,7 +1724,11 @@ static int choose_layout(pmgpu_system* sys, int nf, pmgpu_force* const* forces, 
     if (any32 && !sys->col_disabled) sys->eval_use_col = true;
     // one cell-pair rule for all FP64 rows: a force whose own cutoff reaches
     // beyond the algorithm's keeps the cell layout
-    if (any64 && inside) sys->eval_col64 = true;
+    // few atoms, FP64: the cells are a chain of one launch less (steps/s of
+    // 216 atoms 28,300 for 25,500, of 648 rigid ones 31.0 k for 30.3 k; at 1,200
+    // atoms 27 us an evaluation for the columns' 21)
+    const bool few = sys->n < kCol64Atoms && !(flags & (PMGPU_FLAG_MOLECULAR_VIRIAL | kFlagNeeds64));
+    if (any64 && inside && !few) sys->eval_col64 = true;
     if (sys->eval_use_col || sys->eval_col64) sys->eval_cg = g;
     return PMGPU_OK;
 }
@@ -2182,7 +2188,7 @@ static int run_begin(EvalRun& R)
         if (forces[k]->kind == 0 && !pairs64(sys, forces[k]) && !use_col) mixed_cells = true;
     if (mixed_cells) zero(sys->d_facc32, 2 * sizeof(unsigned long long) * n3);
     const bool cells64 = use40 && !sys->eval_col64;
-    if (cells64) zero(sys->d_facc40, sizeof(unsigned long long) * n3);
+    if (cells64) zero(sys->d_facc40, sizeof(unsigned long long) * 2 * n3);
     if (use40 && sys->eval_col64) zero(sys->d_facc40c, sizeof(unsigned long long) * 6 * kCluster * (size_t)(sys->col_ncl_cap + 1));
     if (atom_mixed) zero(sys->d_faccA, sizeof(unsigned long long) * n3);
     if (atom_fp64) zero(sys->d_faccA + n3, sizeof(unsigned long long) * n3);
@@ -2364,6 +2370,7 @@ static int run_end(EvalRun& R)
         fa.f32 = mixed_cells ? sys->d_facc32 : nullptr;
         fa.f32p = mixed_cells ? sys->d_facc32p : nullptr;
         fa.f40 = use40 && cell_sort && !sys->eval_col64 ? sys->d_facc40 : nullptr;
+        fa.f44 = fa.f40 ? sys->d_facc40 + n3 : nullptr;
         if (use_col || sys->eval_col64) {
             fa.c32 = use_col ? sys->d_facc32c : nullptr;
             fa.c40 = use40 && sys->eval_col64 ? sys->d_facc40c : nullptr;
@@ -2665,7 +2672,7 @@ extern "C" int pmgpu_get_pairs(pmgpu_system* sys, pmgpu_force* f, const double* 
     CK(cudaMemcpyAsync(sys->d_pos, positions, sizeof(double) * n3, cudaMemcpyHostToDevice, s), "H2D");
     CK(cudaMemsetAsync(sys->d_small, 0, kSmallBytes, s), "memset");
     CK(cudaMemsetAsync(sys->d_facc32, 0, 2 * sizeof(unsigned long long) * n3, s), "memset");
-    CK(cudaMemsetAsync(sys->d_facc40, 0, sizeof(unsigned long long) * n3, s), "memset");
+    CK(cudaMemsetAsync(sys->d_facc40, 0, sizeof(unsigned long long) * 2 * n3, s), "memset");
     bool fp64 = pairs64(sys, f);
     const bool col = fp64 ? sys->eval_col64 : sys->eval_use_col;   // eval_prepare decided for this force alone
     if (f->precision != PMGPU_PRECISION_FP64)
