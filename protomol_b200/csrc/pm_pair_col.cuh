@@ -43,7 +43,7 @@
 // cutoff; evaluated tile by tile, the terms (LJ C2 + Ewald real) at 40% of the
 // lanes were two thirds of the kernel's 106 M warp instructions on the
 // 14,281-atom box.  The rings fill the lanes of the pair phase, and its FP32
-// arithmetic is packed two pairs to an instruction: 67 M.
+// arithmetic is packed two pairs to an instruction: 71 M.
 // Measured against the tile-by-tile kernel, each kernel alone: 8.10 -> 5.65 ms
 // for 1,000,000 atoms at 12 A, 360 -> 270 us for 61,233 at 10 A, 141 -> 133 us
 // for 14,281 (where 47 us do not shrink with the cutoff: the near-pair kernel's
