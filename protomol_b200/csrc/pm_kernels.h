@@ -236,6 +236,8 @@ struct PairArgs {
     const double4* c64;          // raw position and charge per slot
     int* clist;                  // column-path entries (the plist buffer): j-clusters, a row's contiguous
     int2* rowent;                // per row: first entry (< 0: not listed) and entries
+    unsigned long long* list_next;   // lists without an error status: entries so far ...
+    unsigned long long* list_short;  // ... and entries needed when they did not fit
     int col_none;                // a j-cluster of padding atoms (the last row's, written by the binning)
     int col_half;                // the list names every unordered pair once (forces, molecular virial), or every ordered one (adjoint)
     int col_refuse;              // 1: a list that does not fit (or a row too tall) is an error status (mixed forces)

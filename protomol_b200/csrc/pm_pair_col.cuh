@@ -54,7 +54,10 @@
 // 61,233 atoms).
 
 constexpr int kColRing = 64;             // ring places per row atom
-constexpr int kColStageEntries = 1024;   // entries of one row staged in shared memory
+// entries of one row staged in shared memory (512: with 1024 the list's blocks
+// held so much of it that the next kernel's first-level cache stayed small:
+// 192k atoms with tables 1755 us an evaluation, 1637 with this)
+constexpr int kColStageEntries = 512;
 constexpr int kColBlock = 96;            // most entries of a chunk (and of a block of a longer row)
 constexpr int kColNear = 256;            // near pairs a warp queues for FP64 energies
 constexpr int kCodeSlot = (1 << 27) - 1; // ring code: j (a slot, or 4 x entry + atom of the chunk) | flags
@@ -90,11 +93,14 @@ __device__ __forceinline__ int2 col_zrange(const PairArgs& p, const int* zi, int
 // The list of one row (one warp): the columns around its own (all of them
 // where the reach covers the box), in rounds of 32, one lane per column (x-y
 // gap, z window, at most two ranges of j-clusters), then the round's j-clusters
-// flattened over the lanes for the box tests.  Entries (j-clusters) are
-// written in a fixed order to out[0 .. cap); returns how many there are (also
-// when more than cap).
-static __device__ int col_gather(const PairArgs& p, int row, int col_i, const float4& ic, const float4& ih, float lim, int* out, int cap,
-                          int4* s_part, int* s_pre)
+// flattened over the lanes for the box tests.  The entries (j-clusters) have a
+// fixed order; those from `from` on are written to out[0 .. cap).  Returns how
+// many there are in all (ALL), or at least from + cap once that many are known.
+// ALL looks the lanes' columns up in shared memory, the other form by shuffles
+// (the FP64 kernels leave that space to the first-level cache).
+template <bool ALL>
+static __device__ int col_gather(const PairArgs& p, int row, int col_i, const float4& ic, const float4& ih, float lim,
+                                 int* out, int from, int cap, int4* s_part = nullptr, int* s_pre = nullptr)
 {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -105,7 +111,7 @@ static __device__ int col_gather(const PairArgs& p, int row, int col_i, const fl
     const bool half = p.col_half, plane = half && nxo == 2 * g.rx + 1 && nyo == 2 * g.ry + 1;
     const int cxi = col_i / g.ncy, cyi = col_i - cxi * g.ncy;
     int ne = 0;
-    for (int k0 = 0; k0 < ncand; k0 += 32) {
+    for (int k0 = 0; k0 < ncand && (ALL || ne < from + cap); k0 += 32) {
         const int k = k0 + lane;
         int4 part = make_int4(0, 0, 0, 0);            // {first, count} of up to two ranges
         if (k < ncand) {
@@ -137,28 +143,45 @@ static __device__ int col_gather(const PairArgs& p, int row, int col_i, const fl
             }
         }
         int incl = part.y + part.w;
-        s_part[lane] = part;
+        const int mine = incl;
+        if constexpr (ALL) s_part[lane] = part;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int v = __shfl_up_sync(FULL, incl, o);
             if (lane >= o) incl += v;
         }
-        s_pre[lane + 1] = incl;
-        if (lane == 0) s_pre[0] = 0;
-        __syncwarp();
+        if constexpr (ALL) {
+            s_pre[lane + 1] = incl;
+            if (lane == 0) s_pre[0] = 0;
+            __syncwarp();
+        }
         const int total = __shfl_sync(FULL, incl, 31);
         for (int f0 = 0; f0 < total; f0 += 32) {
             const int f = f0 + lane;
             bool take = false;
             int jc = 0;
+            int u = 0;
+            int4 pt = part;
+            if constexpr (!ALL) {                         // owner lane: the first whose sum is above f
+                int own = 0;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    if (__shfl_sync(FULL, incl, own + o - 1) <= min(f, total - 1)) own += o;
+                u = f - __shfl_sync(FULL, incl - mine, own);
+                pt.x = __shfl_sync(FULL, part.x, own);
+                pt.y = __shfl_sync(FULL, part.y, own);
+                pt.z = __shfl_sync(FULL, part.z, own);
+            }
             if (f < total) {
-                int lo = 0, hi = 32;                      // owner lane: s_pre[lo] <= f < s_pre[lo + 1]
-                while (hi - lo > 1) {
-                    const int mid = (lo + hi) >> 1;
-                    if (s_pre[mid] <= f) lo = mid; else hi = mid;
+                if constexpr (ALL) {
+                    int lo = 0, hi = 32;                  // owner lane: s_pre[lo] <= f < s_pre[lo + 1]
+                    while (hi - lo > 1) {
+                        const int mid = (lo + hi) >> 1;
+                        if (s_pre[mid] <= f) lo = mid; else hi = mid;
+                    }
+                    u = f - s_pre[lo];
+                    pt = s_part[lo];
                 }
-                const int u = f - s_pre[lo];
-                const int4 pt = s_part[lo];
                 jc = u < pt.y ? pt.x + u : pt.z + (u - pt.y);
                 const float4 bc = __ldg(p.jbox + 2 * jc), bh = __ldg(p.jbox + 2 * jc + 1);
                 const float bx = image_gap(bc.x - ic.x, g.lxf, ilx, bh.x + ih.x);
@@ -170,8 +193,8 @@ static __device__ int col_gather(const PairArgs& p, int row, int col_i, const fl
                 if (half && rj == row) jc |= 1 << 31;
             }
             const unsigned b = __ballot_sync(FULL, take);
-            const int at = ne + __popc(b & ((1u << lane) - 1u));
-            if (take && at < cap) out[at] = jc;
+            const int at = ne + __popc(b & ((1u << lane) - 1u)) - from;
+            if (take && at >= 0 && at < cap) out[at] = jc;
             ne += __popc(b);
         }
         __syncwarp();                                     // s_part / s_pre are rewritten next round
@@ -213,33 +236,43 @@ static __global__ void __launch_bounds__(128) k_col_list(const __grid_constant__
     }
     const float lim = col_list_lim(p);
     const int col_i = p.ccol[row];
-    const int ne = col_gather(p, row, col_i, ic, ih, lim, s_ent[w], kColStageEntries, s_part[w], s_pre[w]);
+    const int ne = col_gather<true>(p, row, col_i, ic, ih, lim, s_ent[w], 0, kColStageEntries, s_part[w], s_pre[w]);
     if (ne == 0) {                                               // not even its own cluster: cannot be
         if (lane == 0) p.rowent[row] = make_int2(0, 0);
         return;
     }
     // equal chunks of a row, an even number of entries each; the last rows'
-    // (about the last to run) are shorter, so that the kernel's end is even
+    // (about the last to run) are shorter, so that the kernel's end is even.
+    // Only the mixed kernels take chunks.
     const int most = 8 * row < 5 * rows ? p.chunk : p.chunk_end;
-    const int nch = (ne + most - 1) / most, per = ((ne + nch - 1) / nch + 1) & ~1;
+    const int nch = p.col_refuse ? (ne + most - 1) / most : 0;
     int b0 = 0, b1 = 0;
     if (lane == 0) {
-        b0 = atomicAdd(p.plist_count, ne);
-        b1 = atomicAdd(p.chunk_count, nch);
-        // (a count beyond 2^31 reads as negative)
-        const bool full0 = b0 < 0 || b0 > p.plist_cap - ne, full1 = b1 < 0 || b1 > p.chunk_cap - nch;
-        const bool full = full0 || full1;
-        // the FP64 kernels take a row that did not fit without its entries
-        p.rowent[row] = full ? make_int2(-1, 0) : make_int2(b0, ne);
-        if (full && p.col_refuse) {
-            atomicOr(p.status, kStatusListFull);
+        // A place once counted is never given back: another row may hold a
+        // later one, and would share its places with the next that asks.
+        bool full;
+        if (p.col_refuse) {
+            b0 = atomicAdd(p.plist_count, ne);
+            b1 = atomicAdd(p.chunk_count, nch);
+            // (a count beyond 2^31 reads as negative)
+            const bool full0 = b0 < 0 || b0 > p.plist_cap - ne, full1 = b1 < 0 || b1 > p.chunk_cap - nch;
+            full = full0 || full1;
+            if (full) atomicOr(p.status, kStatusListFull);
             // the list buffer is counted in int2: two entries each
             if (full0) atomicMax(p.plist_need, (int)(((unsigned)b0 + (unsigned)ne) / 2) + 1);
             if (full1) atomicMax(p.chunk_need, (int)min((unsigned)b1 + (unsigned)nch, 0x7fffffffu));
-        } else if (full) {                                       // (given back: the counts stay near their caps)
-            atomicSub(p.plist_count, ne);
-            atomicSub(p.chunk_count, nch);
+        } else {
+            // the FP64 kernels take a row that did not fit without its entries
+            // (the same ones, gathered again); a 64-bit count cannot come round
+            const unsigned long long at = atomicAdd(p.list_next, (unsigned long long)ne), end = at + ne;
+            full = end > (unsigned)p.plist_cap;
+            b0 = (int)at;
+            if (full) {
+                atomicOr(p.status, kStatusListShort);
+                atomicMax(p.list_short, end);
+            }
         }
+        p.rowent[row] = full ? make_int2(-1, ne) : make_int2(b0, ne);
         if (full) b0 = -1;
     }
     const int ebase = __shfl_sync(FULL, b0, 0), cbase = __shfl_sync(FULL, b1, 0);
@@ -247,8 +280,10 @@ static __global__ void __launch_bounds__(128) k_col_list(const __grid_constant__
     if (ne <= kColStageEntries) {
         for (int t = lane; t < ne; t += 32) p.clist[ebase + t] = s_ent[w][t];
     } else {                                              // more than the staging holds: list again, into place
-        col_gather(p, row, col_i, ic, ih, lim, p.clist + ebase, ne, s_part[w], s_pre[w]);
+        col_gather<true>(p, row, col_i, ic, ih, lim, p.clist + ebase, 0, ne, s_part[w], s_pre[w]);
     }
+    if (nch == 0) return;
+    const int per = ((ne + nch - 1) / nch + 1) & ~1;
     for (int t = lane; t < nch; t += 32)
         p.chunks[cbase + t] = make_int4(row, 0, ebase + t * per, max(0, min(per, ne - t * per)));
 }

@@ -8,8 +8,8 @@
 // pm_pair_col.cuh; a warp takes rows, or shares of their entries, in a fixed
 // order, so that the FP64 energy records do not depend on where the list
 // kernel placed a row's entries.  A row whose entries did not fit the list
-// is gathered again here, 32 j-clusters at a time: the FP64 forces need no
-// capacity.
+// gathers them again here, a block at a time: the FP64 forces need no
+// capacity, and their sums do not depend on it.
 //
 // A row is one 8-atom cluster of the cell-sorted order.  A warp takes a row
 // (or one of `rows_split` shares of its neighbour cells), and visits every
@@ -293,41 +293,16 @@ struct ColOp64 {
     __device__ __forceinline__ void end(const ColRow& r) { op.end(r.si, r.vi); }
 };
 
-// j-clusters [j0, j0 + n) (n <= 32) near the row's box into ent, followed by
-// three empty ones; returns how many there are
-static __device__ __noinline__ int col_near_block(const PairArgs& p, int row, int j0, int n, int* ent)
+// entries from, from + 1, .. from + n - 1 (n <= kColBlock) of a row that is not
+// in the list, in the list's order, followed by three empty ones
+static __device__ __noinline__ void col_gather_block(const PairArgs& p, int row, int from, int n, int* ent)
 {
-    const int lane = threadIdx.x & 31, jc = j0 + lane;
     const float4 ic = p.ibox[2 * row], ih = p.ibox[2 * row + 1];
-    bool take = false;
-    if (lane < n) {
-        const float4 bc = __ldg(p.jbox + 2 * jc), bh = __ldg(p.jbox + 2 * jc + 1);
-        const float bx = image_gap(bc.x - ic.x, p.cg.lxf, 1.0f / p.cg.lxf, bh.x + ih.x);
-        const float by = image_gap(bc.y - ic.y, p.cg.lyf, 1.0f / p.cg.lyf, bh.y + ih.y);
-        const float bz = image_gap(bc.z - ic.z, p.cg.lzf, 1.0f / p.cg.lzf, bh.z + ih.z);
-        take = bh.w == 0.f && bx * bx + by * by + bz * bz <= col_list_lim(p);
-        if (p.col_half && take) {                     // the list's half
-            const int rj = jc >> 1;
-            const ColGrid& g = p.cg;
-            if (2 * g.rx + 1 <= g.ncx && 2 * g.ry + 1 <= g.ncy) {
-                const int ci = p.ccol[row], cj = p.ccol[rj];
-                int ox = cj / g.ncy - ci / g.ncy, oy = cj % g.ncy - ci % g.ncy;
-                ox += 2 * ox <= -g.ncx ? g.ncx : 0; ox -= 2 * ox > g.ncx ? g.ncx : 0;
-                oy += 2 * oy <= -g.ncy ? g.ncy : 0; oy -= 2 * oy > g.ncy ? g.ncy : 0;
-                take = cj == ci ? rj >= row : ox > 0 || (ox == 0 && oy > 0);
-            } else if (rj != row) {
-                take = (((row + rj) & 1) == 0) == (row < rj);
-            }
-        }
-    }
-    const bool own = p.col_half && (jc >> 1) == row;
-    const unsigned m = __ballot_sync(0xffffffffu, take);
-    const int k = __popc(m);
     __syncwarp();
-    if (take) ent[__popc(m & ((1u << lane) - 1u))] = jc | (own ? 1 << 31 : 0);
-    if (lane < 3) ent[k + lane] = p.col_none;
+    col_gather<false>(p, row, p.ccol[row], ic, ih, col_list_lim(p), ent, from, n);
+    const int lane = threadIdx.x & 31;
+    if (lane < 3) ent[n + lane] = p.col_none;
     __syncwarp();
-    return k;
 }
 
 // the rows (p.rows_split shares of each) in a fixed order
@@ -345,20 +320,19 @@ __device__ __forceinline__ void col_rows64(const PairArgs& p, ColRowsShared& sh,
     ColOp64<RowOp> op{rop};
     for (int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < n_items; item += warps) {
         const int row = item / split, part = item - row * split;
-        const int2 re = p.rowent[row];                // first entry, entries (first < 0: not listed)
+        const int2 re = p.rowent[row];                // first entry (< 0: not listed), entries
+        const int b = (int)((long long)re.y * part / split), e = (int)((long long)re.y * (part + 1) / split);
         ColRow r;
         col_row_begin(p, t, row, r);
         op.begin(r);
         // the entries in blocks: of the list, or, for a row that is not in it,
-        // the j-clusters whose box is near, 32 at a time
-        const bool listed = re.x >= 0;
-        const int all = listed ? re.y : 2 * rows;
-        const int b = (int)((long long)all * part / split), e = (int)((long long)all * (part + 1) / split);
+        // gathered again (the same in the same order: the results do not
+        // depend on which rows fitted)
         for (int k = b;;) {
-            int n = min(listed ? kColBlock : 32, e - k);
-            if (listed) col_stage(p, p.clist + re.x + k, n, sh.ent);
+            const int n = min(kColBlock, e - k);
+            if (re.x >= 0) col_stage(p, p.clist + re.x + k, n, sh.ent);
+            else col_gather_block(p, row, k, n, sh.ent);
             k += n;
-            if (!listed) n = col_near_block(p, row, k - n, n, sh.ent);
             col_entries<DIFFMOL, false>(p, t, r, sh.ring, sh.ent, n, k >= e, op);
             if (k >= e) break;
         }

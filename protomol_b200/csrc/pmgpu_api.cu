@@ -157,11 +157,14 @@ struct pmgpu_system {
     int* d_chunk_count = nullptr;
     int* d_chunk_need = nullptr;
     int* d_chunk_next = nullptr;
+    unsigned long long* d_list_short = nullptr;
+    unsigned long long* d_list_next = nullptr;
     unsigned long long* d_efix = nullptr;
     // cluster-pair list and chunks of the mixed kernel
     int2* d_plist = nullptr;
     long long plist_cap = 0;
     long long plist_need = 0;          // reported by the last evaluation that overflowed
+    long long plist_short = 0;         // places an FP64 column list needs (as many as there is memory for)
     int4* d_chunks = nullptr;
     long long chunk_cap = 0;
     long long chunk_need = 0;
@@ -396,7 +399,9 @@ extern "C" int pmgpu_system_create(int device, pmgpu_system** out)
     sys->d_chunk_count = sys->d_status + 3;
     sys->d_chunk_need = sys->d_status + 4;
     sys->d_chunk_next = sys->d_status + 5;
-    sys->d_efix = (unsigned long long*)((char*)sys->d_small + 64);   // ints 8..15: binning
+    sys->d_list_short = (unsigned long long*)(sys->d_status + 10);   // (8 and 9: binning)
+    sys->d_list_next = sys->d_list_short + 1;
+    sys->d_efix = (unsigned long long*)((char*)sys->d_small + 64);
     *out = sys;
     return PMGPU_OK;
 }
@@ -545,6 +550,12 @@ static int status_result(pmgpu_system* sys, int st)
         sys->near_need = std::max<long long>(sys->near_need, need[5]);
         sys->list_valid = false;
         return fail(sys, PMGPU_ERR_CAPACITY, "cluster-pair list capacity exceeded (grown for the next evaluation)");
+    }
+    if (st & kStatusListShort) {
+        // no error: the next FP64 evaluation's list holds these rows too
+        unsigned long long entries = 0;
+        CK(cudaMemcpy(&entries, sys->d_list_short, sizeof(entries), cudaMemcpyDeviceToHost), "status");
+        sys->plist_short = std::max(sys->plist_short, (long long)std::min(entries, 1ull << 40) / 2 + 1);
     }
     return PMGPU_OK;
 }
@@ -1582,7 +1593,7 @@ static void fill_col_args(pmgpu_system* sys, bool fp64, PairArgs& a, bool half)
 {
     a.cq = sys->d_cq; a.cm = sys->d_cm; a.ibox = sys->d_ibox; a.jbox = sys->d_jbox; a.c64 = sys->d_c64;
     a.ccstart = sys->d_ccstart; a.ccol = sys->d_ccol; a.icl_cap = sys->col_ncl_cap;
-    a.zidx = sys->d_zidx; a.rowent = sys->d_rowent;
+    a.zidx = sys->d_zidx; a.rowent = sys->d_rowent; a.list_next = sys->d_list_next; a.list_short = sys->d_list_short;
     a.clist = (int*)sys->d_plist;           // two entries in each int2 place
     a.plist_cap = (int)std::min(2 * sys->plist_cap, (long long)INT_MAX);
     a.cg = sys->eval_cg;
@@ -1820,7 +1831,7 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
             const long long entries = col_list_estimate(sys->n, g, vol, rl);
             const int chunk = col_chunk_entries(sys->n, g, vol, rc, 6 * sys->tuning.chunk_entries, true);
             lneed = std::max(lneed, entries / 2);      // two entries in each int2 place of the list buffer
-            cneed = std::max(cneed, col_chunk_estimate(entries, sys->n, g, chunk));
+            if (!pairs64(sys, forces[k])) cneed = std::max(cneed, col_chunk_estimate(entries, sys->n, g, chunk));
         }
     }
     if (!sys->eval_use_col) {
@@ -1835,15 +1846,26 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
         lneed = std::max(lneed, sys->plist_need + sys->plist_need / 4);
         cneed = std::max(cneed, sys->chunk_need + sys->chunk_need / 4);
         if (!mixed) {                        // a row without entries finds its pairs by itself
+            lneed = std::max(lneed, sys->plist_short + sys->plist_short / 4);
             lneed = std::min(lneed, (long long)INT_MAX);
-            cneed = std::min(cneed, (long long)INT_MAX);
+            cneed = 0;
         }
         if (lneed > INT_MAX || cneed > INT_MAX)
             return fail(sys, PMGPU_ERR_CAPACITY, "cluster-pair list above 2^31 entries");
         if (lneed > sys->plist_cap) {
-            CK(dalloc(&sys->d_plist, (size_t)lneed), "alloc");
-            sys->plist_cap = lneed;
+            const long long had = sys->plist_cap;
+            sys->plist_cap = 0;
+            sys->list_valid = false;
             sys->buf_version++;
+            cudaError_t e = dalloc(&sys->d_plist, (size_t)lneed);
+            if (e != cudaSuccess && !mixed) {        // as many places as before, and no more asked for
+                cudaGetLastError();
+                sys->plist_short = 0;
+                lneed = had;
+                e = lneed > 0 ? dalloc(&sys->d_plist, (size_t)lneed) : cudaSuccess;
+            }
+            CK(e, "alloc");
+            sys->plist_cap = lneed;
         }
         if (cneed > sys->chunk_cap) {
             CK(dalloc(&sys->d_chunks, (size_t)cneed), "alloc");
@@ -2274,7 +2296,10 @@ static int run_list(EvalRun& R, const PairArgs& a, bool col)
         return PMGPU_OK;
     }
     // list count and need, chunk count and need, work counter, near-pair count
-    if (lists++ > 0) CK(cudaMemsetAsync(sys->d_plist_count, 0, 6 * sizeof(int), s), "memset");
+    if (lists++ > 0) {
+        CK(cudaMemsetAsync(sys->d_plist_count, 0, 6 * sizeof(int), s), "memset");
+        CK(cudaMemsetAsync(sys->d_list_next, 0, sizeof(unsigned long long), s), "memset");
+    }
     int ml = prof_begin(sys, kPhaseList);
     int e = col ? launch_col_list(a, s, &sys->launches) : launch_cluster_list(a, s, &sys->launches);
     if (e) return cuda_fail(sys, (cudaError_t)e, "pair list");
@@ -3781,7 +3806,7 @@ extern "C" int pmgpu_adjoint(pmgpu_system* sys, int n_forces, pmgpu_force* const
                 if (sys->eval_col64) {
                     fill_col_args(sys, true, pa, false);
                     if (listed != pa.cut2f) {
-                        if (listed >= 0.0f) ok(cudaMemsetAsync(sys->d_plist_count, 0, 6 * sizeof(int), s));
+                        if (listed >= 0.0f) ok(cudaMemsetAsync(sys->d_list_next, 0, sizeof(unsigned long long), s));
                         ok((cudaError_t)launch_col_list(pa, s, &sys->launches));
                         listed = pa.cut2f;
                     }
@@ -3851,7 +3876,9 @@ extern "C" int pmgpu_adjoint(pmgpu_system* sys, int n_forces, pmgpu_force* const
                                           &sys->launches));
         ok(cudaMemcpyAsync(h_count, sys->d_adj_count, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     }
+    ok(cudaMemcpyAsync(sys->h_status, sys->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
     ok(cudaStreamSynchronize(s));
+    if (e == cudaSuccess && (*sys->h_status & kStatusListShort)) status_result(sys, kStatusListShort);
     const size_t nz = e == cudaSuccess ? *h_count : 0;
     if (nz > sys->h_adj_cap) {
         if (sys->h_adj_val) cudaFreeHost(sys->h_adj_val);

@@ -12,6 +12,7 @@ import dataclasses
 
 import numpy as np
 import pytest
+from scipy.spatial import cKDTree
 
 from oracle import oracle
 from protomol_b200 import forces as F
@@ -69,6 +70,24 @@ def _same_pairs(s, d, force):
     ref = oracle.evaluate(s, [F.parse_definition(d)], want_pairs=True)["pairs"]
     key = lambda p: np.sort(p[:, 0].astype(np.int64) * s.n_atoms + p[:, 1])
     assert np.array_equal(key(force.pairs(s.positions)), key(ref))
+
+
+def _lj9_hessian_v(pos, v, A, B):
+    """LJ9's Hessian times v for atoms of one type and no periodic image, in
+    a = r^2: E = (A / a^6 - B / a^3) S(a), S the C2 switch from 8 to 9 A."""
+    i, j = cKDTree(pos).query_pairs(9.0, output_type="ndarray").T
+    d, u = pos[i] - pos[j], v[i] - v[j]
+    a, on, c = (d * d).sum(1), 64.0, 81.0
+    e, e1, e2 = A / a ** 6 - B / a ** 3, -6 * A / a ** 7 + 3 * B / a ** 4, 42 * A / a ** 8 - 12 * B / a ** 5
+    k = np.where(a >= on, 1.0 / (c - on) ** 3, 0.0)
+    s0 = np.where(a >= on, k * (c - a) ** 2 * (c - 3 * on + 2 * a), 1.0)
+    s1, s2 = 6 * k * (c - a) * (on - a), 6 * k * (2 * a - on - c)
+    E1, E2 = e1 * s0 + e * s1, e2 * s0 + 2 * e1 * s1 + e * s2
+    w = 2 * E1[:, None] * u + (4 * E2 * (d * u).sum(1))[:, None] * d
+    out = np.zeros_like(pos)
+    np.add.at(out, i, w)
+    np.add.at(out, j, -w)
+    return out
 
 
 @pytest.mark.parametrize("precision", ["mixed", "fp64"])
@@ -147,6 +166,38 @@ def test_a_droplet_outgrows_the_list_estimate(precision):
     s = _fluid(pos, (150.0, 150.0, 150.0))
     _, fs, _ = _check(s, [LJ9], precision)
     _same_pairs(s, LJ9, fs[0])
+
+
+def test_a_list_far_beyond_its_estimate():
+    """13,824 atoms in a 28th of their box, whose list is many times the
+    estimate: forces, both virials and the backward pass, over and over, with
+    the same energies to the last bit whichever rows found a place."""
+    rng = np.random.default_rng(8)
+    g = np.stack(np.meshgrid(*[np.arange(24)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = (g - 11.5) * 3.3 + rng.uniform(-0.2, 0.2, (len(g), 3))
+    s = _fluid(pos, (240.0, 240.0, 240.0))
+    ref = oracle.evaluate(s, [F.parse_definition(LJ9)])
+    topo = F.Topology(s)
+    force = F.ForceFactory.make(topo, LJ9, "fp64")
+    topo.set_molecule_positions(pos)
+    seen = set()
+    scale = np.abs(ref["forces"]).max()
+    v = rng.normal(size=pos.shape)
+    for k in range(20):
+        out, e = np.zeros((s.n_atoms, 3)), F.ScalarStructure(virial=True, molecular_virial=k % 2 == 1)
+        F.evaluate_group(topo, [force], s.positions, out, e)
+        seen.add(e.lennard_jones)
+        assert np.abs(out - ref["forces"]).max() <= 1e-11 * scale
+        assert np.abs(e.virial_tensor - ref["virial"]).max() <= 1e-11 * np.abs(ref["virial"]).max()
+        if k % 2:                                       # every atom is its own molecule
+            assert np.abs(e.molecular_virial_tensor - ref["virial"]).max() <= 1e-11 * np.abs(ref["virial"]).max()
+        r = F.adjoint(topo, [force], s.positions, v)
+        assert abs(r["lennard_jones"] - ref["lennard_jones"]) <= 1e-11 * abs(ref["lennard_jones"])
+        # the energy is linear in the table
+        assert abs((r["dE_dlj"] * s.lj_table).sum() - ref["lennard_jones"]) <= 1e-9 * abs(ref["lennard_jones"])
+    assert len(seen) == 1 and abs(seen.pop() - ref["lennard_jones"]) <= 1e-11 * abs(ref["lennard_jones"])
+    hv = _lj9_hessian_v(pos, v, *s.lj_table[0, 0, :2])
+    assert np.abs(r["hv"] - hv).max() <= 1e-11 * np.abs(hv).max()
 
 
 def test_a_column_of_more_atoms_than_the_sort_holds():
