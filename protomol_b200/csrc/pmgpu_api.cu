@@ -394,10 +394,13 @@ extern "C" int pmgpu_system_create(int device, pmgpu_system** out)
         return PMGPU_ERR_NOMEM;
     }
     sys->d_status = (int*)sys->d_small;
-    sys->d_plist_count = sys->d_status + 1;
-    sys->d_plist_need = sys->d_status + 2;
-    sys->d_chunk_count = sys->d_status + 3;
-    sys->d_chunk_need = sys->d_status + 4;
+    // what an evaluation's lists needed (kept through all of them), the counts
+    // of the list in the buffer (run_list starts them over), then the near
+    // pairs' (ints 6 and 7)
+    sys->d_plist_need = sys->d_status + 1;
+    sys->d_chunk_need = sys->d_status + 2;
+    sys->d_plist_count = sys->d_status + 3;
+    sys->d_chunk_count = sys->d_status + 4;
     sys->d_chunk_next = sys->d_status + 5;
     sys->d_list_short = (unsigned long long*)(sys->d_status + 10);   // (8 and 9: binning)
     sys->d_list_next = sys->d_list_short + 1;
@@ -542,12 +545,12 @@ static int status_result(pmgpu_system* sys, int st)
                                              "built (it is rebuilt at the next evaluation)");
     }
     if (st & kStatusListFull) {
-        // list need, chunk count, chunk need, work counter, near count, near need
-        int need[6] = {0, 0, 0, 0, 0, 0};
+        // list and chunk need, list and chunk count, work counter, near count, near need
+        int need[7] = {0, 0, 0, 0, 0, 0, 0};
         CK(cudaMemcpy(need, sys->d_plist_need, sizeof(need), cudaMemcpyDeviceToHost), "status");
         sys->plist_need = std::max<long long>(sys->plist_need, need[0]);
-        sys->chunk_need = std::max<long long>(sys->chunk_need, need[2]);
-        sys->near_need = std::max<long long>(sys->near_need, need[5]);
+        sys->chunk_need = std::max<long long>(sys->chunk_need, need[1]);
+        sys->near_need = std::max<long long>(sys->near_need, need[6]);
         sys->list_valid = false;
         return fail(sys, PMGPU_ERR_CAPACITY, "cluster-pair list capacity exceeded (grown for the next evaluation)");
     }
@@ -2186,7 +2189,7 @@ static int run_begin(EvalRun& R)
         zr.words[zr.count++] = (long long)(bytes / sizeof(unsigned));
     };
     if (sys->eval_reuse) {
-        // the list's counts (ints 1-4) stay; the status, the work counter,
+        // the list's needs and counts (ints 1-4) stay; the status, the work counter,
         // the near-pair counts, the binning counters and the sums start at zero
         zero(sys->d_small, sizeof(int));
         zero((char*)sys->d_small + 5 * sizeof(int), kSmallBytes - 5 * sizeof(int));
@@ -2284,20 +2287,21 @@ static int run_begin(EvalRun& R)
 }
 
 // The pair list of the next cutoff force: the one in the buffer when it was
-// built for the same test (a group's forces of one cutoff share it; the work
-// counter and the near pairs start over), else a new one.
-static int run_list(EvalRun& R, const PairArgs& a, bool col)
+// built for the same test (a group's forces of one cutoff share it), else a new
+// one.  near: a mixed force, whose work counter and near pairs start over (an
+// earlier mixed force's near pairs were evaluated on this stream; the last
+// one's may still be in work on the side stream when another list follows).
+static int run_list(EvalRun& R, const PairArgs& a, bool col, bool near)
 {
     PM_EVAL_RUN_NAMES(R)
     const bool same = col && lists > 0 && R.list_cut2 == a.cut2f && R.list_skin == a.list_skin &&
                       R.list_refuse == a.col_refuse && R.list_chunk == a.chunk && R.list_half == a.col_half;
     if (same) {
-        CK(cudaMemsetAsync(sys->d_chunk_next, 0, 2 * sizeof(int), s), "memset");    // and the near-pair count
+        if (near) CK(cudaMemsetAsync(sys->d_chunk_next, 0, 2 * sizeof(int), s), "memset");
         return PMGPU_OK;
     }
-    // list count and need, chunk count and need, work counter, near-pair count
     if (lists++ > 0) {
-        CK(cudaMemsetAsync(sys->d_plist_count, 0, 6 * sizeof(int), s), "memset");
+        CK(cudaMemsetAsync(sys->d_plist_count, 0, (near ? 4 : 3) * sizeof(int), s), "memset");
         CK(cudaMemsetAsync(sys->d_list_next, 0, sizeof(unsigned long long), s), "memset");
     }
     int ml = prof_begin(sys, kPhaseList);
@@ -2331,7 +2335,7 @@ static int run_cutoffs(EvalRun& R, bool may_defer)
         a.erec = sys->d_erec + used;
         // the column list, or the cell-cluster list of the mixed forces
         if (col ? !sys->eval_reuse : !fp64) {
-            r = run_list(R, a, col);
+            r = run_list(R, a, col, !fp64);
             if (r) return r;
         }
         if (may_defer && col && !fp64 && !sys->eval_reuse) {
@@ -2369,7 +2373,7 @@ static int run_end(EvalRun& R)
             if (col) {
                 fill_col_args(sys, true, a, true);
                 if (!sys->eval_reuse && R.list_cut2 != a.cut2f) {
-                    r = run_list(R, a, true);
+                    r = run_list(R, a, true, false);
                     if (r) return r;
                 }
             }

@@ -200,6 +200,53 @@ def test_a_list_far_beyond_its_estimate():
     assert np.abs(r["hv"] - hv).max() <= 1e-11 * np.abs(hv).max()
 
 
+EWALD12 = "CoulombEwaldReal -switchingFunction Cutoff -algorithm NonbondedCutoff -alpha 0.3 -cutoff 12 -cutoff 12"
+
+
+@pytest.mark.parametrize("concurrent", [0, 1])
+@pytest.mark.parametrize("group", ["fp64_after_mixed", "two_cutoffs_molecular_virial"])
+def test_a_list_after_the_last_near_pairs(group, concurrent):
+    """A list made after the last mixed force, whose near pairs may still be in
+    work beside PME: the group's sums are those of its forces alone."""
+    s = systems.water_box(2100, 4)
+    split = workloads.lj_ewald_split(8, 9, 0.35)
+    pme = workloads.pme_reciprocal((40, 40, 40), 9, 0.35)
+    defs, mol = (([(split, "mixed"), (split, "fp64"), (pme, "mixed")], False) if group == "fp64_after_mixed" else
+                 ([(LJ9, "mixed"), (EWALD12, "mixed"), (pme, "mixed")], True))
+    topo = F.Topology(s)
+    topo.set_tuning(pme_concurrent=concurrent)
+    topo.set_molecule_positions(F.molecular_centers(s.molecule, s.positions, s.mass))
+    fs = [F.ForceFactory.make(topo, d, p) for d, p in defs]
+
+    def evaluate(which):
+        f, e = np.zeros((s.n_atoms, 3)), F.ScalarStructure(virial=True, molecular_virial=mol)
+        F.evaluate_group(topo, which, s.positions, f, e)
+        return f, np.array([e.lennard_jones, e.coulomb]), e.virial_tensor, e.molecular_virial_tensor if mol else 0 * e.virial_tensor
+
+    alone = [evaluate([f]) for f in fs]
+    f, e, v, m = [sum(a[k] for a in alone) for k in range(4)]
+    scale = sum(np.abs(a[1]).sum() for a in alone)
+    for _ in range(10):
+        g = evaluate(fs)
+        assert np.sqrt(((g[0] - f) ** 2).mean()) <= 1e-5 * np.sqrt((f ** 2).mean())
+        assert np.abs(g[1] - e).max() <= 1e-6 * scale
+        assert np.abs(g[2] - v).max() <= 1e-6 * np.abs(v).max()
+        assert np.abs(g[3] - m).max() <= 1e-6 * max(np.abs(m).max(), 1.0)
+
+
+def test_an_overflowing_mixed_list_beside_an_fp64_one_grows():
+    rng = np.random.default_rng(2)
+    g = np.stack(np.meshgrid(*[np.arange(15)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    s = _fluid((g - 7.0) * 3.3 + rng.uniform(-0.2, 0.2, (len(g), 3)), (150.0, 150.0, 150.0))
+    ref = oracle.evaluate(s, [F.parse_definition(LJ9)])
+    topo = F.Topology(s)
+    fs = [F.ForceFactory.make(topo, LJ9, p) for p in ("mixed", "fp64")]
+    out, e = np.zeros((s.n_atoms, 3)), F.ScalarStructure()
+    F.evaluate_group(topo, fs, s.positions, out, e)
+    assert np.sqrt(((out / 2 - ref["forces"]) ** 2).mean()) <= 1e-5 * np.sqrt((ref["forces"] ** 2).mean())
+    assert abs(e.lennard_jones / 2 - ref["lennard_jones"]) <= 1e-6 * abs(ref["lennard_jones"])
+
+
 def test_a_column_of_more_atoms_than_the_sort_holds():
     """2,300 atoms on one line along z: one column holds them all.  The FP64
     forces take the column unsorted."""
