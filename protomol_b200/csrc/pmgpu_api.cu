@@ -190,6 +190,7 @@ struct pmgpu_system {
     double list_skin = 0.0;
     int list_every = 1;
     bool list_valid = false;
+    bool list_c64 = false;             // it was built with the slots' FP64 positions (d_c64, its padding too)
     bool list_just_invalidated = false;
     int evals_since_build = 0;
     std::vector<long long> list_ids;   // the forces the list was built for
@@ -2501,7 +2502,10 @@ static int eval_core(pmgpu_system* sys, int nf_in, pmgpu_force* const* forces_in
     // (an FP64 force of the group on the columns lists its own pairs)
     const bool can_reuse = sys->eval_use_col && sys->list_every > 1 && n_mixed_cut == 1 &&
                            !(sys->eval_col64 && n_fp64_cut > 0);
-    sys->eval_reuse = can_reuse && sys->list_valid && sys->list_ids == ids && sys->evals_since_build < sys->list_every;
+    // (a molecular virial needs the FP64 positions of the list's padding slots,
+    // which only the build writes)
+    sys->eval_reuse = can_reuse && sys->list_valid && sys->list_ids == ids && sys->evals_since_build < sys->list_every &&
+                      (!sys->eval_col64 || sys->list_c64);
     auto note_list = [&]() {
         if (sys->eval_col64 && n_fp64_cut > 0) sys->list_valid = false;    // the FP64 forces' list took its place
         if (!sys->eval_use_col || n_mixed_cut == 0) return;
@@ -2510,6 +2514,7 @@ static int eval_core(pmgpu_system* sys, int nf_in, pmgpu_force* const* forces_in
         } else {
             sys->list_builds++;
             sys->list_valid = can_reuse;
+            sys->list_c64 = sys->eval_col64;
             sys->list_ids = ids;
             sys->evals_since_build = 1;
         }

@@ -294,6 +294,27 @@ def test_reused_list_survives_an_fp64_evaluation_between():
         assert np.sqrt(((out / len(fs) - ref) ** 2).mean()) <= 1e-5 * np.sqrt((ref ** 2).mean())
 
 
+def test_reused_list_and_a_first_molecular_virial():
+    """The molecular virial asked for while the pair list of an evaluation
+    without it is kept: that of a system that never kept one."""
+    s = systems.water_box(2100, 4)
+    d = workloads.lj_ewald_split(8, 9, 0.35)
+    centers = F.molecular_centers(s.molecule, s.positions, s.mass)
+    got = []
+    for every in (1, 10):
+        topo = F.Topology(s)
+        topo.set_molecule_positions(centers)
+        force = F.ForceFactory.make(topo, d, "mixed")
+        topo.set_pair_list(1.0, every)
+        for mol in (False, True, True):
+            f, e = np.zeros((s.n_atoms, 3)), F.ScalarStructure(virial=True, molecular_virial=mol)
+            F.evaluate_group(topo, [force], s.positions, f, e)
+        got.append(e.molecular_virial_tensor)
+        if every > 1:
+            assert topo.pair_list_builds() == 2         # the second has the slots the virial reads
+    assert np.abs(got[0] - got[1]).max() <= 1e-11 * np.abs(got[0]).max()
+
+
 @pytest.mark.parametrize("shape", ["pairs", "stars", "triangles", "mixed_order", "chains", "many"])
 def test_constrained_steps(shape):
     """Clusters of two and three atoms in any order of their constraints (the
