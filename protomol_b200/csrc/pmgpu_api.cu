@@ -2494,8 +2494,10 @@ static int eval_core(pmgpu_system* sys, int nf_in, pmgpu_force* const* forces_in
     // built for these forces, still valid and younger than the period
     std::vector<long long> ids;
     int n_mixed_cut = 0, n_fp64_cut = 0;
+    bool any_cut = false;
     for (int k = 0; k < nf; ++k) {
         ids.push_back(forces[k]->id);
+        any_cut |= forces[k]->kind == 0;
         if (forces[k]->kind == 0 && !pairs64(sys, forces[k])) ++n_mixed_cut;
         if (forces[k]->kind == 0 && pairs64(sys, forces[k])) ++n_fp64_cut;
     }
@@ -2507,7 +2509,8 @@ static int eval_core(pmgpu_system* sys, int nf_in, pmgpu_force* const* forces_in
     sys->eval_reuse = can_reuse && sys->list_valid && sys->list_ids == ids && sys->evals_since_build < sys->list_every &&
                       (!sys->eval_col64 || sys->list_c64);
     auto note_list = [&]() {
-        if (sys->eval_col64 && n_fp64_cut > 0) sys->list_valid = false;    // the FP64 forces' list took its place
+        // every other evaluation with a list of its own has it in the same buffers
+        if (!sys->eval_reuse && (n_mixed_cut > 0 || (sys->eval_col64 && any_cut))) sys->list_valid = false;
         if (!sys->eval_use_col || n_mixed_cut == 0) return;
         if (sys->eval_reuse) {
             sys->evals_since_build++;
@@ -2715,10 +2718,10 @@ extern "C" int pmgpu_get_pairs(pmgpu_system* sys, pmgpu_force* f, const double* 
         CK(cudaMemsetAsync(fp64 ? sys->d_facc40c : sys->d_facc32c, 0, sizeof(unsigned long long) * (fp64 ? 6 : 3) *
                            kCluster * (size_t)(sys->col_ncl_cap + (fp64 ? 1 : 0)), s), "memset");
         r = col_bin(sys, sys->d_pos);
-        sys->list_valid = false;
     } else {
         r = bin(sys, sys->d_pos);
     }
+    sys->list_valid = false;
     if (r) return r;
     r = ensure_erec(sys, std::max(1, pair_records(sys, f)));
     if (r) return r;
@@ -3072,8 +3075,12 @@ extern "C" int pmgpu_batch_evaluate(pmgpu_batch* b)
             auto& m = b->members[k];
             e = cudaStreamWaitEvent(m.sys->stream, b->ev_start, 0);
             if (e != cudaSuccess) break;
+            // the layout of this member's forces (its system may be another's
+            // too), with a list of its own
+            r = choose_layout(m.sys, (int)m.run.size(), m.run.data(), m.flags);
+            m.sys->eval_reuse = false;
             run_init(runs[k], m.sys, (int)m.run.size(), m.run.data(), m.pos, m.fout, m.energy, m.flags);
-            r = run_begin(runs[k]);
+            if (!r) r = run_begin(runs[k]);
             if (!r) r = run_cutoffs(runs[k], one_launch);
             if (!r && runs[k].deferred < 0) r = run_end(runs[k]);
             if (r) { b->err = m.sys->err; break; }
@@ -3155,7 +3162,10 @@ extern "C" int pmgpu_batch_evaluate(pmgpu_batch* b)
     }
     cudaError_t e = cudaGraphLaunch(b->exec, b->stream);
     if (e != cudaSuccess) return batch_fail(b, PMGPU_ERR_CUDA, std::string("batch graph launch: ") + cudaGetErrorString(e));
-    for (size_t k = 0; k < b->members.size(); ++k) b->members[k].sys->launches += b->member_launches[k];
+    for (size_t k = 0; k < b->members.size(); ++k) {
+        b->members[k].sys->launches += b->member_launches[k];
+        b->members[k].sys->list_valid = false;           // in the same buffers as a list kept by the system
+    }
     return PMGPU_OK;
 }
 

@@ -12,11 +12,13 @@ import dataclasses
 
 import numpy as np
 import pytest
+import torch
 from scipy.spatial import cKDTree
 
 from oracle import oracle
 from protomol_b200 import forces as F
 from protomol_b200 import integrate, systems, workloads
+from protomol_b200.batch import Batch
 
 pytestmark = pytest.mark.gpu
 
@@ -292,6 +294,43 @@ def test_reused_list_survives_an_fp64_evaluation_between():
         out = np.zeros((s.n_atoms, 3))
         F.evaluate_group(topo, fs, s.positions, out, F.ScalarStructure())
         assert np.sqrt(((out / len(fs) - ref) ** 2).mean()) <= 1e-5 * np.sqrt((ref ** 2).mean())
+
+
+@pytest.mark.parametrize("other", ["cells", "pairs", "batch"])
+def test_a_kept_list_that_another_call_overwrote(other):
+    """A reused pair list shares its buffers with every other list of its
+    system: a force on the cell layout (a cutoff beyond half the box), a pair
+    recording, a batch with the system as a member."""
+    s = systems.water_box(700, 4)                       # 27.6 A
+    d = workloads.lj_ewald_split(8, 9, 0.35)
+    ref = oracle.evaluate(s, [F.parse_definition(d)])["forces"]
+    topo = F.Topology(s)
+    kept = F.ForceFactory.make(topo, d, "mixed")
+    wide = F.ForceFactory.make(topo, LJ9.replace("cutoff 9", "cutoff 14.5"), "mixed")
+    topo.set_pair_list(1.0, 10)
+
+    def check(forces):
+        assert np.sqrt(((forces - ref) ** 2).mean()) <= 1e-5 * np.sqrt((ref ** 2).mean())
+
+    for _ in range(3):
+        out = np.zeros((s.n_atoms, 3))
+        F.evaluate_group(topo, [kept], s.positions, out, F.ScalarStructure())
+        check(out)
+        if other == "cells":
+            F.evaluate_group(topo, [wide], s.positions, np.zeros((s.n_atoms, 3)), F.ScalarStructure())
+        elif other == "pairs":
+            wide.pairs(s.positions)
+        else:
+            b = Batch()
+            moved = systems.perturbed(s, 0.3, 5)
+            b.add(topo, [kept], moved.positions)
+            torch.cuda.synchronize()
+            b.evaluate()
+            b.synchronize()
+            m = oracle.evaluate(moved, [F.parse_definition(d)])["forces"]
+            got = b.members[0][3].cpu().numpy()
+            assert np.sqrt(((got - m) ** 2).mean()) <= 1e-5 * np.sqrt((m ** 2).mean())
+    assert topo.pair_list_builds() == 3
 
 
 def test_reused_list_and_a_first_molecular_virial():
