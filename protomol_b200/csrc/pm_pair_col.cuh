@@ -203,10 +203,12 @@ static __device__ int col_gather(const PairArgs& p, int row, int col_i, const fl
 }
 
 // box distance^2 within which a j-cluster is listed; a reused list holds the
-// pairs within the cutoff plus the skin
+// pairs within the cutoff plus the skin.  The FP32 boxes: every corner, center
+// and difference of centers is rounded by up to 2^-24 of the edge, 6.7 such
+// errors in a gap and sqrt(3) of that over the axes: 7e-7 of the edge.
 __device__ __forceinline__ float col_list_lim(const PairArgs& p)
 {
-    const float rl = sqrtf(p.cut2f) + p.list_skin;
+    const float rl = sqrtf(p.cut2f) + p.list_skin + 7e-7f * fmaxf(p.cg.lxf, fmaxf(p.cg.lyf, p.cg.lzf));
     return rl * rl * (1.0f + 8.0f * p.guard) + 1e-3f;
 }
 

@@ -1662,7 +1662,13 @@ static void fill_pair_args(pmgpu_system* sys, pmgpu_force* f, const double* d_po
     a.n_terms = f->cp.n_terms;
     a.tf[0] = f->tf[0]; a.tf[1] = f->tf[1]; a.td[0] = f->td[0]; a.td[1] = f->td[1];
     a.cut2f = (float)f->cut2; a.cut2d = f->cut2;
-    a.guard = 2.0e-5f;
+    // the FP32 distance test's error, and that of fixed-point coordinates (steps
+    // of L / 2^32: 2 sqrt(3) of one, relative to the smallest cutoff)
+    double rmin2 = f->cut2;
+    for (int t = 0; t < a.n_terms; ++t)
+        if (f->td[t].cut2 > 0.0) rmin2 = std::min(rmin2, f->td[t].cut2);
+    a.guard = (float)(2.0e-5 + 4.0 / 4294967296.0 * std::max(sys->box[0], std::max(sys->box[4], sys->box[8])) /
+                                   std::sqrt(rmin2));
     // the energies of pairs closer than 5 A are recomputed in FP64: they hold
     // nearly all of the FP32 energy rounding (|e| up to ~30 kcal/mol each on
     // water, where the total is a ~1e-3 cancellation of the sum of |e|)

@@ -202,6 +202,26 @@ def test_a_list_far_beyond_its_estimate():
     assert np.abs(r["hv"] - hv).max() <= 1e-11 * np.abs(hv).max()
 
 
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("length", [2500.0, 60000.0])
+def test_pairs_at_the_cutoff_in_a_long_box(length, precision):
+    """Pairs just inside the cutoff along a long edge, where the list's FP32
+    cluster boxes are coarse (a step of 4e-3 A at 60,000 A)."""
+    rng = np.random.default_rng(4)
+    n = int(length / 80)                                # pairs on each of two lines
+    pos = []
+    for x in (-7.5, 7.5):
+        # a single atom first: every fourth pair has its atoms in two rows
+        z = (np.arange(n) + 0.5) * (length - 100) / n - length / 2 + 50 + rng.uniform(-20, 20, n)
+        z = np.concatenate([[-length / 2 + 1.0], np.stack([z, z + 9.0 * (1 - 1e-10)], 1).ravel()])
+        pos.append(np.stack([np.full_like(z, x), np.full_like(z, x), z], 1))
+    s = _fluid(np.concatenate(pos), (30.0, 30.0, length))
+    force = F.ForceFactory.make(F.Topology(s), LJ9, precision)
+    got = force.pairs(s.positions)
+    assert len(got) >= 2 * n
+    _same_pairs(s, LJ9, force)
+
+
 EWALD12 = "CoulombEwaldReal -switchingFunction Cutoff -algorithm NonbondedCutoff -alpha 0.3 -cutoff 12 -cutoff 12"
 
 
