@@ -38,7 +38,7 @@ int col_chunk_entries(int n_atoms, const ColGrid& g, double volume, double cutof
     // three 4,500-atom boxes in flight 40.8 us an evaluation for 43.6, 24 boxes
     // of 300 to 9,000 atoms 874 us for 922), 16 below that (1,000 atoms: 22.0 us
     // for 23.5, alone 56.9 for 60.5)
-    most = std::max(16, std::min(most, kColBlock));
+    most = std::max(16, std::min(most, kColChunk));
     const int least = std::min(most, all < 8.0 * warps ? 16 : 32);
     return std::max(least, std::min(most, 2 * (int)(0.5 * std::min(want, 1e6) + 1.0)));
 }

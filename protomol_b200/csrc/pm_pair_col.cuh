@@ -44,8 +44,8 @@
 // lanes were two thirds of the kernel's 106 M warp instructions on the
 // 14,281-atom box.  The rings fill the lanes of the pair phase, and its FP32
 // arithmetic is packed two pairs to an instruction: 71 M.
-// Measured against the tile-by-tile kernel, each kernel alone: 8.10 -> 5.65 ms
-// for 1,000,000 atoms at 12 A, 360 -> 270 us for 61,233 at 10 A, 141 -> 133 us
+// Measured against the tile-by-tile kernel, each kernel alone: 8.10 -> 6.05 ms
+// for 1,000,000 atoms at 12 A, 360 -> 286 us for 61,233 at 10 A, 141 -> 138 us
 // for 14,281 (where 47 us do not shrink with the cutoff: the near-pair kernel's
 // 13, the launch and the unevenness of the last chunks).  Tried: a full list
 // with rings and no j side (152 M instructions, 217 us: the terms run twice);
@@ -58,8 +58,9 @@ constexpr int kColRing = 64;             // ring places per row atom
 // held so much of it that the next kernel's first-level cache stayed small:
 // 192k atoms with tables 1755 us an evaluation, 1637 with this)
 constexpr int kColStageEntries = 512;
-constexpr int kColBlock = 96;            // most entries of a chunk (and of a block of a longer row)
-constexpr int kColNear = 256;            // near pairs a warp queues for FP64 energies
+constexpr int kColBlock = 96;            // entries of a row the FP64 kernels stage at a time
+constexpr int kColChunk = 64;            // most entries of a chunk of the mixed kernels
+constexpr int kColNear = 128;            // near pairs a warp queues for FP64 energies
 constexpr int kCodeSlot = (1 << 27) - 1; // ring code: j (a slot, or 4 x entry + atom of the chunk) | flags
 constexpr int kCodeIn0 = 1 << 28, kCodeIn1 = 1 << 29, kCodeMod = 1 << 30;
 
@@ -633,26 +634,31 @@ __device__ __forceinline__ void pair_math2(const PairArgs& p, const JAtom& ia, c
 // A warp's shared memory in the mixed kernel
 struct ColShared32 {
     int ring[kColRing * kCluster];
-    int ent[kColBlock + 4];
-    int fj[3][4 * kColBlock];            // the chunk's j-forces (2^23 per kcal/mol/A), zero between chunks
+    int ent[kColChunk + 4];
+    int fj[6][4 * kColChunk];            // the chunk's j-forces: steps of 2^-11, then of 2^-34; zero between chunks
     int2 near[kColNear];
     long long acc[8];                    // sums: LJ, Coulomb, virial xx xy xz yy yz zz
 };
-constexpr float kScaleJ = 8388608.0f;    // 2^23
-constexpr float kLimitJ = 30.0f;         // a j-force this large is added in 64 bits at once (8 x 30 2^23 < 2^31)
+// An FP32 value in two integers without a conversion: added to 1.5 x 2^12 it is
+// rounded to steps of 2^-11, in the sum's low bits, and what is left (exact, at
+// most 2^-12) to steps of 2^-34 by 1.5 x 2^-11.
+constexpr float kJHigh = 6144.0f, kJLow = 7.32421875e-4f;
+constexpr int kJHighBits = 0x45c00000, kJLowBits = 0x3a400000;
+constexpr float kLimitJ = 2047.0f;       // a j-force this large is added in 64 bits at once
 
 // Two pairs per lane and step, their FP32 arithmetic packed (one issue slot for
 // both: the kernel is bound by issue slots, not by the FMA pipe).  i-forces
 // in FP32 over a drain (over a whole chunk their error against FP64 was 2-3%
-// larger), far pairs' energies and virial over the chunk (at most 96 entries:
-// about 20 pairs in each half of a packed sum), then FP64 and int64 fixed
-// point.  j-forces are added up over the row's
-// atoms in shared memory as 32-bit integers of 2^-23 (as fine as FP32 holds a
-// component of 2; with 2^-22 the force error of 1,000,000 atoms was 9.47e-7
-// instead of 9.39e-7; each atom gets at most eight per chunk), and added to the
-// atoms' int64 sums once per chunk: everything is independent of the
-// chunk-to-warp assignment.  Near pairs (r < 5 A) go to the warp's queue for
-// K2c'; their FP32 energies and virial are left out.
+// larger), far pairs' energies and virial over the chunk (at most 64 entries:
+// about 15 pairs in each half of a packed sum), then FP64 and int64 fixed
+// point.  j-forces are added up over the row's atoms in shared memory, each FP32
+// value whole in two 32-bit integers (each atom gets at most eight per chunk:
+// 2^25 in each), and added to the atoms' int64 sums once per chunk: everything
+// is independent of the chunk-to-warp assignment.  One integer of 2^-23 took
+// 5.65 ms instead of 6.05 for 1,000,000 atoms (133 us instead of 138 for 14,281),
+// but its step is fixed: forces of 0.008 kcal/mol/A had a relative error of 5e-5,
+// with two 6.5e-7, as forces of 10 have.  Near pairs (r < 5 A) go to the
+// warp's queue for K2c'; their FP32 energies and virial are left out.
 // TWO: the two terms' cutoffs differ (a pair may be inside one of them only).
 template <int NT, int P0, int S0, int P1, int S1, bool TWO>
 struct ColForce32 {
@@ -669,7 +675,7 @@ struct ColForce32 {
     {
         const int lane = threadIdx.x & 31;
         if (lane < 8) sh.acc[lane] = 0;
-        for (int k = lane; k < 12 * kColBlock; k += 32) (&sh.fj[0][0])[k] = 0;
+        for (int k = lane; k < 24 * kColChunk; k += 32) (&sh.fj[0][0])[k] = 0;
         nq = 0;
     }
     __device__ __forceinline__ JAtom atom(int slot) const
@@ -703,20 +709,22 @@ struct ColForce32 {
         const int k = code & kCodeSlot;
         return 4 * (sh.ent[k >> 2] & 0x7fffffff) + (k & 3);
     }
-    // the j-force of one pair
-    __device__ __forceinline__ void add_j(int code, int slot, bool big, bool valid, float x, float y, float z)
+    // the j-force of one pair: its two parts (t, u: sums with kJHigh, kJLow)
+    __device__ __forceinline__ void add_j(int code, int slot, bool big, bool valid, const float (&v)[3],
+                                          const float (&t)[3], const float (&u)[3])
     {
         if (!valid) return;
-        const int k = code & kCodeSlot;
         if (!big) {
-            atomicAdd(&sh.fj[0][k], __float2int_rn(x * kScaleJ));
-            atomicAdd(&sh.fj[1][k], __float2int_rn(y * kScaleJ));
-            atomicAdd(&sh.fj[2][k], __float2int_rn(z * kScaleJ));
+            int* to = &sh.fj[0][code & kCodeSlot];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                atomicAdd(to + c * 4 * kColChunk, __float_as_int(t[c]) - kJHighBits);
+                atomicAdd(to + (3 + c) * 4 * kColChunk, __float_as_int(u[c]) - kJLowBits);
+            }
         } else {
             unsigned long long* to = p.facc + 3 * (size_t)slot;
-            fixed_addf(to, x, p.status);
-            fixed_addf(to + 1, y, p.status);
-            fixed_addf(to + 2, z, p.status);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) fixed_addf(to + c, v[c], p.status);
         }
     }
     // the pairs from places at and at + 4 of the lane's ring
@@ -758,15 +766,20 @@ struct ColForce32 {
         }
         const F2 x = mul2(dx, ft), y = mul2(dy, ft), z = mul2(dz, ft);
         f[0] = sub2(f[0], x); f[1] = sub2(f[1], y); f[2] = sub2(f[2], z);
-        float xa, xb, ya, yb, za, zb;
-        split(x, xa, xb);
-        split(y, ya, yb);
-        split(z, za, zb);
+        float ga[3], gb[3], ta[3], tb[3], ua[3], ub[3];
+        const F2 g[3] = {x, y, z};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            split(g[c], ga[c], gb[c]);
+            const F2 t = add2(g[c], f2(kJHigh));
+            split(t, ta[c], tb[c]);
+            split(add2(sub2(g[c], add2(t, f2(-kJHigh))), f2(kJLow)), ua[c], ub[c]);
+        }
         // (not below the limit, and not NaN)
-        const bool ba = !(fabsf(xa) + fabsf(ya) + fabsf(za) < kLimitJ);
-        const bool bb = !(fabsf(xb) + fabsf(yb) + fabsf(zb) < kLimitJ);
-        add_j(ca, sa, ba, va, xa, ya, za);
-        add_j(cb, sb, bb, vb, xb, yb, zb);
+        const bool ba = !(fabsf(ga[0]) + fabsf(ga[1]) + fabsf(ga[2]) < kLimitJ);
+        const bool bb = !(fabsf(gb[0]) + fabsf(gb[1]) + fabsf(gb[2]) < kLimitJ);
+        add_j(ca, sa, ba, va, ga, ta, ua);
+        add_j(cb, sb, bb, vb, gb, tb, ub);
         const bool na = va && ra < p.near2, nb = vb && rb < p.near2;           // near2 = 0: none
         if (__any_sync(FULL, na || nb)) {
             const F2 zero = f2(0.f);
@@ -831,7 +844,7 @@ struct ColForce32 {
     __device__ __forceinline__ void run(const ColTest& t, const int4& cd)
     {
         const int lane = threadIdx.x & 31;
-        const int n = min(cd.w, kColBlock);
+        const int n = min(cd.w, kColChunk);
         if (n <= 0) return;
         ColRow r;
         col_row_begin(p, t, cd.x, r);
@@ -843,10 +856,10 @@ struct ColForce32 {
             unsigned long long* to = p.facc + 3 * (size_t)slot(k);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const int q = sh.fj[c][k];
-                if (q != 0) {
-                    sh.fj[c][k] = 0;
-                    atomicAdd(to + c, (unsigned long long)((long long)q * 512));       // 2^-23 -> 2^-32
+                const int q = sh.fj[c][k], l = sh.fj[3 + c][k];
+                if ((q | l) != 0) {
+                    sh.fj[c][k] = sh.fj[3 + c][k] = 0;
+                    atomicAdd(to + c, (unsigned long long)((long long)q * 2097152 + ((l + 1 + ((l >> 2) & 1)) >> 2)));  // 2^-32, ties to even
                 }
             }
         }

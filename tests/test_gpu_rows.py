@@ -141,10 +141,11 @@ def test_two_cutoffs(lengths, precision):
     _check(_fluid(pos, lengths, q), [CUTS_8_9], precision, energy=2e-6)
 
 
-@pytest.mark.parametrize("r", [2.5, 2.25, 2.0])
+@pytest.mark.parametrize("r", [2.5, 2.25, 2.0, 1.7])
 def test_forces_beyond_the_32_bit_sums(r):
-    """Pairs whose force exceeds the 60 kcal/mol/A that the j side holds in 32
-    bits, several of them on one atom, among ordinary ones."""
+    """Pairs whose force is large, or (at 1.7 A) exceeds the 2,047 kcal/mol/A
+    that the j side holds in 32-bit words, several of them on one atom, among
+    ordinary ones."""
     rng = np.random.default_rng(11)
     g = np.stack(np.meshgrid(*[np.arange(8)] * 3, indexing="ij"), -1).reshape(-1, 3)
     pos = (g + 0.5) * 5.2 - 20.8 + rng.uniform(-0.1, 0.1, (len(g), 3))
@@ -155,6 +156,22 @@ def test_forces_beyond_the_32_bit_sums(r):
             u[axis] = r
             extra.append(pos[i] + u)
     _check(_fluid(np.concatenate([pos, extra]), (41.6, 41.6, 41.6)), [LJ9], "mixed")
+
+
+@pytest.mark.parametrize("scale", [1e-1, 1e-3])
+def test_weak_forces(scale):
+    """Energies scaled down, as in a weakly bound fluid: forces keep their
+    relative error, and the sum over the atoms its zero (6,300 independent FP32
+    errors of 6.5e-7: 5e-5 of the RMS force; 3e-4 allowed)."""
+    s = systems.water_box(2100, 5)
+    s = dataclasses.replace(s, scaled_charge=s.scaled_charge * np.sqrt(scale), lj_table=s.lj_table * scale)
+    d = workloads.lj_ewald_split(8, 9, 0.35)
+    ref = oracle.evaluate(s, [F.parse_definition(d)])["forces"]
+    topo, _, f, _ = _eval(s, [d], "mixed")
+    rms = np.sqrt((ref ** 2).mean())
+    assert topo.pair_layout() == "columns"
+    assert np.sqrt(((f - ref) ** 2).mean()) <= 1e-6 * rms
+    assert np.abs(f.sum(0)).max() <= 3e-4 * rms
 
 
 @pytest.mark.parametrize("precision", ["mixed", "fp64"])
