@@ -225,7 +225,9 @@ __device__ __forceinline__ void pot_f64(const PairArgs& p, const TermD& t, doubl
         double qq = qi * qj;
         if (p.csfd != 1.0 && excl == PMGPU_EXCL_MODIFIED) qq *= p.csfd;
         double rr = rinv;
-        double ar = t.alpha * (d2 * rr);
+        // r from the reciprocal root, with its rounding put right
+        const double h = d2 * rr;
+        double ar = t.alpha * fma(0.5 * rr, fma(-h, h, d2), h);
         double ex = qq * exp(-ar * ar);
         const double E1 = 0.254829592, E2 = -0.284496736, E3 = 1.421413741,
                      E4 = -1.453152027, E5 = 1.061405429, PP = 0.3275911;
@@ -306,7 +308,10 @@ __device__ __forceinline__ void pair_f64(const PairArgs& p, double d2, double qi
     constexpr bool kRoot = P0 == CO || P0 == EW || (NT > 1 && (P1 == CO || P1 == EW));
     constexpr bool kR2 = pot_r2(P0) || (NT > 1 && pot_r2(P1));
     const double rinv = kRoot ? rsqrt(d2) : 0.0;
-    const double rd2 = kRoot ? rinv * rinv : (kR2 ? 1.0 / d2 : 1.0);
+    double rd2 = kRoot ? rinv * rinv : (kR2 ? 1.0 / d2 : 1.0);
+    // (one Newton step: the square of a rounded root alone is 2.5 ulp off, and a
+    // Lennard-Jones term takes its sixth power)
+    if (kRoot && kR2) rd2 = fma(rd2, fma(-d2, rd2, 1.0), rd2);
     double f0, f1 = 0.0;
     e1 = 0.0;
     pot_f64<P0>(p, p.td[0], d2, rd2, rinv, qi, qj, ti, tj, excl, e0, f0);

@@ -187,6 +187,30 @@ def test_a_droplet_outgrows_the_list_estimate(precision):
     _same_pairs(s, LJ9, fs[0])
 
 
+def test_fp64_pair_energies_to_the_last_bits():
+    """Repulsive Lennard-Jones pairs beside an electrostatic term, whose 1/r^2
+    comes from the reciprocal root both share, have the errors against extended
+    precision of the same pairs alone, whose 1/r^2 is a division: both half a
+    unit (rms 0.43 to 0.45 of 2^-53), so their energies' within 1.3 (the square
+    of a rounded root, 0.92: about 2)."""
+    s = _fluid(np.zeros((2, 3)), (30.0, 30.0, 30.0))
+    topo = F.Topology(s)
+    both = F.ForceFactory.make(topo, "LennardJones Coulomb -switchingFunction C2 -switchingFunction C2 -algorithm "
+                               "NonbondedCutoff -switchon 8 -cutoff 9 -switchon 8 -cutoff 9 -cutoff 9", "fp64")
+    alone = F.ForceFactory.make(topo, LJ9, "fp64")
+    A, B = (np.longdouble(x) for x in s.lj_table[0, 0, :2])
+    err = {both: [], alone: []}
+    for r in np.random.default_rng(6).integers(int(2.2 * 2 ** 20), int(2.8 * 2 ** 20), 200) / 2.0 ** 20:
+        a = np.longdouble(r) ** 2                       # (exact: so is the kernels' r^2)
+        ref = A / a ** 6 - B / a ** 3
+        for force, out in err.items():
+            e = F.ScalarStructure()
+            F.evaluate_group(topo, [force], np.array([[0.0, 0, 0], [r, 0, 0]]), np.zeros((2, 3)), e)
+            out.append(float((e.lennard_jones - ref) / ref) * 2.0 ** 53)
+    rms = {f: np.sqrt(np.mean(np.square(x))) for f, x in err.items()}
+    assert rms[both] <= 1.3 * rms[alone]
+
+
 def test_a_list_far_beyond_its_estimate():
     """13,824 atoms in a 28th of their box, whose list is many times the
     estimate: forces, both virials and the backward pass, over and over, with
