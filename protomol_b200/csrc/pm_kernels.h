@@ -56,6 +56,7 @@ struct ColGrid {
     float sx, sy;                // column side
     float lxf, lyf, lzf;         // box edges (FP32)
     float sch[3], scl[3];        // L / 2^32 per axis, FP32 hi + lo
+    int fine;                    // small boxes: pair vectors rounded once (fixed_diff)
     float zext;                  // largest z extent of an i-cluster of the mixed path (taller ones prune too little)
 };
 

@@ -56,7 +56,7 @@ int launch_col_list(const PairArgs& a, cudaStream_t s, long long* launches)
     return (int)cudaGetLastError();
 }
 
-template <int NT, int P0, int S0, int P1, int S1, bool TWO>
+template <int NT, int P0, int S0, int P1, int S1, bool TWO, int FINE>
 static int run_col_t(const PairArgs& a, cudaStream_t s, long long* launches)
 {
     static int sms = 0, per_sm = 0;
@@ -64,12 +64,12 @@ static int run_col_t(const PairArgs& a, cudaStream_t s, long long* launches)
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_col<NT, P0, S0, P1, S1, TWO>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_col<NT, P0, S0, P1, S1, TWO, FINE>, 128, 0);
         if (sms <= 0) sms = 148;
         if (per_sm <= 0) per_sm = 1;
     }
     const int bps = a.blocks_per_sm > 0 ? std::min(per_sm, a.blocks_per_sm) : per_sm;
-    launch_pdl(k_pair_col<NT, P0, S0, P1, S1, TWO>, sms * bps, 128, 0, s, a);
+    launch_pdl(k_pair_col<NT, P0, S0, P1, S1, TWO, FINE>, sms * bps, 128, 0, s, a);
     *launches += 1;
     return (int)cudaGetLastError();
 }
@@ -80,9 +80,13 @@ static bool two_cutoffs(const PairArgs& a) { return a.n_terms > 1 && a.tf[0].cut
 template <int NT, int P0, int S0, int P1, int S1>
 static int run_col(const PairArgs& a, cudaStream_t s, long long* launches)
 {
+    const bool fine = a.cg.fine != 0;
     if constexpr (NT > 1)
-        if (two_cutoffs(a)) return run_col_t<NT, P0, S0, P1, S1, true>(a, s, launches);
-    return run_col_t<NT, P0, S0, P1, S1, false>(a, s, launches);
+        if (two_cutoffs(a))
+            return fine ? run_col_t<NT, P0, S0, P1, S1, true, 1>(a, s, launches)
+                        : run_col_t<NT, P0, S0, P1, S1, true, 0>(a, s, launches);
+    return fine ? run_col_t<NT, P0, S0, P1, S1, false, 1>(a, s, launches)
+                : run_col_t<NT, P0, S0, P1, S1, false, 0>(a, s, launches);
 }
 
 int launch_pair_col(const PairArgs& a, int combo, cudaStream_t s, long long* launches)

@@ -8,8 +8,8 @@
 // displacement in units of L / 2^32, exactly: no cell offset and no rounding
 // shared by the pairs of an atom or of a cell pair enters the pair vector.
 // The only roundings are the conversion of that integer to FP32 and its
-// product with the FP32 hi + lo of L / 2^32, both unbiased, so the FP32 pair
-// energies carry no systematic error into the sums.
+// product with the FP32 hi + lo of L / 2^32 (in small boxes the product's alone:
+// fixed_diff).
 //
 // Clusters: the atoms of one column of an x-y grid (~4 A side), sorted by z,
 // cut into runs of 8; each run is a row (the i side), each half of it a 4-atom
@@ -481,6 +481,53 @@ __device__ __forceinline__ F2 add2(F2 a, F2 b)
     return r;
 }
 __device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(b, f2(-1.f), a); }      // one rounding, as a - b
+// (a - c, b - c) x (hi + lo) of fixed-point coordinates.  fine: rounded once,
+// the difference's low byte beside its upper three (a byte in a float's mantissa
+// is 32768 + byte; the 32768 is taken off before), and what the rounding left
+// out in rest, for r^2.  Otherwise the 32-bit difference is rounded to FP32
+// first, which errs alike for all pairs of a lattice that divides the box.  Such
+// errors count in small boxes: the energies of 216 waters at 24 spacings were
+// off by 1.1e-5 of their sum, and fine by 1.3e-6 (on the cell layout by 2.3e-6);
+// C2 forces of random configurations by 1.1e-6, and fine by 2.0e-7.  The first 15
+// of the 50 instructions a step took 5% of the kernel of 1,000,000 atoms: fine
+// where the reach covers the box, whose evaluations take no longer for it (216
+// waters 18.6 us).
+__device__ __forceinline__ F2 fixed_diff(bool fine, int a, int b, int c, float hi, float lo, F2& rest)
+{
+    unsigned u = (unsigned)a - (unsigned)c, v = (unsigned)b - (unsigned)c;
+    if (!fine) {
+        const F2 d = f2((float)(int)u, (float)(int)v);
+        return fma2(d, f2(hi), mul2(d, f2(lo)));
+    }
+    u -= 32768u;
+    v -= 32768u;
+    const F2 up = f2((float)(int)(u & 0xffffff00u), (float)(int)(v & 0xffffff00u));
+    const F2 low = f2(__uint_as_float(__byte_perm(u, 0x47000000u, 0x7404)),
+                      __uint_as_float(__byte_perm(v, 0x47000000u, 0x7404)));
+    const F2 t = fma2(low, f2(hi), mul2(up, f2(lo)));
+    const F2 d = fma2(up, f2(hi), t);
+    rest = add2(fma2(up, f2(hi), fma2(d, f2(-1.f), f2(0.f))), t);
+    return d;
+}
+// r^2 of fine pair vectors to the last bit, and what its rounding left out (rem):
+// the squares added largest first, so that every difference below is exact
+__device__ __forceinline__ F2 fine_norm2(F2 x, F2 y, F2 z, const F2 (&rest)[3], F2& rem)
+{
+    float x0, x1, y0, y1, z0, z1;
+    split(x, x0, x1);
+    split(y, y0, y1);
+    split(z, z0, z1);
+    const float m0 = fmaxf(fabsf(x0), fabsf(y0)), m1 = fmaxf(fabsf(x1), fabsf(y1));
+    const F2 a = f2(fmaxf(m0, fabsf(z0)), fmaxf(m1, fabsf(z1)));
+    const F2 b = f2(fminf(m0, fabsf(z0)), fminf(m1, fabsf(z1)));
+    const F2 c = f2(fminf(fabsf(x0), fabsf(y0)), fminf(fabsf(x1), fabsf(y1)));
+    const F2 s0 = mul2(a, a), s1 = fma2(b, b, s0), s2 = fma2(c, c, s1);
+    const F2 e = add2(fma2(a, a, mul2(s0, f2(-1.f))), add2(fma2(b, b, sub2(s0, s1)), fma2(c, c, sub2(s1, s2))));
+    const F2 low = fma2(f2(2.f), fma2(z, rest[2], fma2(y, rest[1], mul2(x, rest[0]))), e);
+    const F2 r2 = add2(s2, low);
+    rem = sub2(low, sub2(r2, s2));
+    return r2;
+}
 __device__ __forceinline__ F2 sel2(bool lo, bool hi, F2 a, F2 b)
 {
     float al, ah, bl, bh;
@@ -559,9 +606,11 @@ __device__ __forceinline__ void pot2(const PairArgs& p, const TermF& t, F2 r2, F
 }
 
 // sw_f32 of two pairs applied to a term (f = f v - e d, e = e v); OUT as there,
-// ina / inb: inside a Cutoff switch
-template <int SW, bool OUT>
-__device__ __forceinline__ void switch2(const TermF& t, F2 r2, F2 rinv, bool ina, bool inb, F2& e, F2& f)
+// ina / inb: inside a Cutoff switch.  FINE: r^2 is r2 + rem (the C2 switch's
+// polynomials in rc^2 - r^2 lose most of the bits of r^2: their rounding was
+// 85% of the virial's error of a lattice box).
+template <int SW, bool OUT, bool FINE>
+__device__ __forceinline__ void switch2(const TermF& t, F2 r2, F2 rem, F2 rinv, bool ina, bool inb, F2& e, F2& f)
 {
     if (SW == SUN || (SW == SCUT && !OUT)) return;
     const F2 zero = f2(0.f);
@@ -575,8 +624,12 @@ __device__ __forceinline__ void switch2(const TermF& t, F2 r2, F2 rinv, bool ina
     const bool oa = OUT && ra > t.cut2, ob = OUT && rb > t.cut2;
     F2 v, d;                                         // the value, and its derivative negated
     if (SW == SC2) {
-        const F2 c2 = sub2(f2(t.cut2), r2);
-        const F2 c4 = mul2(c2, fma2(f2(-2.0f), r2, f2(-t.s2)));          // negated
+        F2 c2 = sub2(f2(t.cut2), r2), u = fma2(f2(-2.0f), r2, f2(-t.s2));
+        if (FINE) {
+            c2 = sub2(c2, rem);
+            u = fma2(f2(-2.0f), rem, u);
+        }
+        const F2 c4 = mul2(c2, u);                                       // negated
         const F2 c24 = mul2(c2, c4);                                     // negated
         const F2 dd = fma2(c2, c2, c4);
         const bool ma = ra >= t.on2, mb = rb >= t.on2;
@@ -590,7 +643,8 @@ __device__ __forceinline__ void switch2(const TermF& t, F2 r2, F2 rinv, bool ina
         d = add2(fma2(dist, f2(-t.c1_15_3), mul2(f2(t.c1_15_1), rinv)),
                  fma2(dist, f2(-t.c1_15_3_lo), mul2(f2(t.c1_15_1_lo), rinv)));
     } else {                                         // Shift
-        const F2 x = fma2(r2, f2(-t.sh_a_lo), fma2(r2, f2(-t.sh_a), f2(1.f)));
+        F2 x = fma2(r2, f2(-t.sh_a_lo), fma2(r2, f2(-t.sh_a), f2(1.f)));
+        if (FINE) x = fma2(rem, f2(-t.sh_a), x);
         v = mul2(x, x);
         d = fma2(f2(-t.sh_b), x, mul2(f2(-t.sh_b_lo), x));
     }
@@ -604,9 +658,9 @@ __device__ __forceinline__ void switch2(const TermF& t, F2 r2, F2 rinv, bool ina
 
 // pair_math of two pairs of one row atom (no table potentials): force factors
 // and energies, zero for an inactive pair
-template <int NT, int P0, int S0, int P1, int S1, bool OUT>
+template <int NT, int P0, int S0, int P1, int S1, bool OUT, bool FINE>
 __device__ __forceinline__ void pair_math2(const PairArgs& p, const JAtom& ia, const JAtom& ja, const JAtom& jb, F2 r2in,
-                                           bool va, bool vb, int ca, int cb, F2& ft, F2& el, F2& ec)
+                                           F2 rem, bool va, bool vb, int ca, int cb, F2& ft, F2& el, F2& ec)
 {
     constexpr bool kMod = sw_modifies(S0) || (NT > 1 && sw_modifies(S1));
     const F2 zero = f2(0.f);
@@ -621,8 +675,8 @@ __device__ __forceinline__ void pair_math2(const PairArgs& p, const JAtom& ia, c
     pot2<P0>(p, p.tf[0], r2, rd2, rinv, qq, ia.m.y, ja.m.y, jb.m.y, ma, mb, e0, f0);
     if (NT > 1) pot2<P1>(p, p.tf[1], r2, rd2, rinv, qq, ia.m.y, ja.m.y, jb.m.y, ma, mb, e1, f1);
     if (kMod) {
-        switch2<S0, OUT>(p.tf[0], r2, rinv, ca & kCodeIn0, cb & kCodeIn0, e0, f0);
-        if (NT > 1) switch2<S1, OUT>(p.tf[1], r2, rinv, ca & kCodeIn1, cb & kCodeIn1, e1, f1);
+        switch2<S0, OUT, FINE>(p.tf[0], r2, rem, rinv, ca & kCodeIn0, cb & kCodeIn0, e0, f0);
+        if (NT > 1) switch2<S1, OUT, FINE>(p.tf[1], r2, rem, rinv, ca & kCodeIn1, cb & kCodeIn1, e1, f1);
     }
     ft = sel2(va, vb, NT > 1 ? add2(f0, f1) : f0, zero);
     const F2 a = sel2(va, vb, e0, zero), b = NT > 1 ? sel2(va, vb, e1, zero) : zero;
@@ -660,7 +714,9 @@ constexpr float kLimitJ = 2047.0f;       // a j-force this large is added in 64 
 // with two 6.5e-7, as forces of 10 have.  Near pairs (r < 5 A) go to the
 // warp's queue for K2c'; their FP32 energies and virial are left out.
 // TWO: the two terms' cutoffs differ (a pair may be inside one of them only).
-template <int NT, int P0, int S0, int P1, int S1, bool TWO>
+// FINE: the grid's fine, 0 or 1, or (2, a batch's boxes) as it comes: a test a step
+// costs 3% of the kernel.
+template <int NT, int P0, int S0, int P1, int S1, bool TWO, int FINE>
 struct ColForce32 {
     static constexpr int kKeep = 16;     // a drain leaves rings below this (longer ones share the idle lanes)
     static constexpr bool kLocal = true;
@@ -736,16 +792,14 @@ struct ColForce32 {
         const int cb = vb ? ring[((at + 4) & (kColRing - 1)) * kCluster + il] : 0;
         const int sa = slot(ca), sb = slot(cb);
         const JAtom ja = atom(sa), jb = atom(sb);
-        // the pair vectors: exact in fixed point, one rounding to FP32, times
-        // the compensated L / 2^32
         const int4 A = __ldg(p.cq + sa), B = __ldg(p.cq + sb);
-        const F2 qx = f2((float)(int)((unsigned)A.x - (unsigned)r.P.x), (float)(int)((unsigned)B.x - (unsigned)r.P.x));
-        const F2 qy = f2((float)(int)((unsigned)A.y - (unsigned)r.P.y), (float)(int)((unsigned)B.y - (unsigned)r.P.y));
-        const F2 qz = f2((float)(int)((unsigned)A.z - (unsigned)r.P.z), (float)(int)((unsigned)B.z - (unsigned)r.P.z));
-        const F2 dx = fma2(qx, f2(p.cg.sch[0]), mul2(qx, f2(p.cg.scl[0])));
-        const F2 dy = fma2(qy, f2(p.cg.sch[1]), mul2(qy, f2(p.cg.scl[1])));
-        const F2 dz = fma2(qz, f2(p.cg.sch[2]), mul2(qz, f2(p.cg.scl[2])));
-        const F2 r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+        const bool fine = FINE == 2 ? p.cg.fine != 0 : FINE == 1;
+        F2 rest[3];
+        const F2 dx = fixed_diff(fine, A.x, B.x, r.P.x, p.cg.sch[0], p.cg.scl[0], rest[0]);
+        const F2 dy = fixed_diff(fine, A.y, B.y, r.P.y, p.cg.sch[1], p.cg.scl[1], rest[1]);
+        const F2 dz = fixed_diff(fine, A.z, B.z, r.P.z, p.cg.sch[2], p.cg.scl[2], rest[2]);
+        F2 rem = f2(0.f);
+        const F2 r2 = fine ? fine_norm2(dx, dy, dz, rest, rem) : fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
         float ra, rb;
         split(r2, ra, rb);
         F2 ft, el, ec;
@@ -762,7 +816,7 @@ struct ColForce32 {
             pair_math<NT, P0, S0, P1, S1, TWO>(p, gb, ia, jb, fb, lb, wb);
             ft = f2(fa, fb); el = f2(la, lb); ec = f2(wa, wb);
         } else {
-            pair_math2<NT, P0, S0, P1, S1, TWO>(p, ia, ja, jb, r2, va, vb, ca, cb, ft, el, ec);
+            pair_math2<NT, P0, S0, P1, S1, TWO, FINE != 0>(p, ia, ja, jb, r2, rem, va, vb, ca, cb, ft, el, ec);
         }
         const F2 x = mul2(dx, ft), y = mul2(dy, ft), z = mul2(dz, ft);
         f[0] = sub2(f[0], x); f[1] = sub2(f[1], y); f[2] = sub2(f[2], z);
@@ -923,7 +977,7 @@ __device__ __forceinline__ int col_chunks(const PairArgs& p, bool mark)
 // without (the fluid of 20,001 ions: 53 against 58 us a step with three systems
 // in flight, where the fifth block keeps the others' kernels waiting); six
 // spill 116 bytes and take 7.96 ms.
-template <int NT, int P0, int S0, int P1, int S1, bool TWO>
+template <int NT, int P0, int S0, int P1, int S1, bool TWO, int FINE>
 __global__ void __launch_bounds__(128, P0 == EW || P1 == EW ? 5 : 4) k_pair_col(const __grid_constant__ PairArgs p)
 {
     pdl_wait();
@@ -931,7 +985,7 @@ __global__ void __launch_bounds__(128, P0 == EW || P1 == EW ? 5 : 4) k_pair_col(
     __shared__ ColShared32 sh[4];
     const int nchunks = col_chunks(p, blockIdx.x == 0 && threadIdx.x == 0);
     const ColTest t = col_test(p);
-    ColForce32<NT, P0, S0, P1, S1, TWO> op{p, sh[w]};
+    ColForce32<NT, P0, S0, P1, S1, TWO, FINE> op{p, sh[w]};
     op.init();
     while (true) {
         int ch = 0;
@@ -972,7 +1026,7 @@ __global__ void __launch_bounds__(128, 4) k_pair_col_batch(BatchPairArgs b)
     const int total = s_pre[b.n];
     int cur = -1;
     const PairArgs& p = s_args[w];
-    ColForce32<NT, P0, S0, P1, S1, TWO> op{p, sh[w]};
+    ColForce32<NT, P0, S0, P1, S1, TWO, 2> op{p, sh[w]};
     op.init();
     ColTest t;
     while (true) {

@@ -750,7 +750,8 @@ static bool col_reach(const pmgpu_system* sys, double rc, ColGrid& g)
     // rows taller than the list's window prune too little: the mixed forces'
     // cells take such a (dilute) system, where the box is wide enough for them
     const double zext = g.lz - 2.0 * rl - 0.5;
-    g.zext = zext > 1.0 && 2 * g.rx + 1 <= g.ncx && 2 * g.ry + 1 <= g.ncy ? (float)zext : 3.0e38f;
+    g.fine = !(zext > 1.0 && 2 * g.rx + 1 <= g.ncx && 2 * g.ry + 1 <= g.ncy);
+    g.zext = g.fine ? 3.0e38f : (float)zext;
     return true;
 }
 

@@ -158,6 +158,23 @@ def test_forces_beyond_the_32_bit_sums(r):
     _check(_fluid(np.concatenate([pos, extra]), (41.6, 41.6, 41.6)), [LJ9], "mixed")
 
 
+@pytest.mark.parametrize("spacing", [3.07, 3.1, 3.15, 3.2])
+def test_lattice_boxes(spacing):
+    """216 waters on a lattice that divides the box: thousands of pairs at a few
+    distances, whose FP32 roundings add up instead of averaging out.  Pair
+    vectors and r^2 to the last bit leave about ten roundings of 2^-25 in a
+    force, 1e-7 to 2e-7: 5e-7 allowed (1.3e-6 when the fixed-point difference is
+    rounded first)."""
+    length = 6 * spacing
+    pos = systems._water_atoms(np.random.default_rng(1), systems._lattice(6, length))
+    s = dataclasses.replace(systems.water_box_216(), positions=pos, box=_box((length,) * 3))
+    defs = workloads.lj_c2_coulomb_c2(8, 9)
+    ref = oracle.evaluate(s, [F.parse_definition(d) for d in defs])["forces"]
+    topo, _, f, _ = _eval(s, defs, "mixed")
+    assert topo.pair_layout() == "columns"
+    assert np.sqrt(((f - ref) ** 2).mean()) <= 5e-7 * np.sqrt((ref ** 2).mean())
+
+
 @pytest.mark.parametrize("scale", [1e-1, 1e-3])
 def test_weak_forces(scale):
     """Energies scaled down, as in a weakly bound fluid: forces keep their
