@@ -432,6 +432,35 @@ def test_reused_list_and_a_first_molecular_virial():
     assert np.abs(got[0] - got[1]).max() <= 1e-11 * np.abs(got[0]).max()
 
 
+def test_constrained_step_with_many_free_atoms():
+    """A few constrained triangles among thousands of free atoms, every one of
+    them advanced as the oracle does."""
+    m = 14
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    length = 4.0 * m
+    pos = (g + 0.5) * 4.0 - length / 2
+    held = 7
+    tri = np.array([[0.0, 0.0, 0.0], [0.95, 0.0, 0.0], [-0.3, 0.9, 0.0]])
+    every = np.concatenate([(pos[:held, None] + tri).reshape(-1, 3), pos[held:]])
+    o = 3 * np.arange(held)
+    atoms = np.concatenate([np.stack([o + a, o + b], 1) for a, b in ((0, 1), (0, 2), (1, 2))]).astype(np.int32)
+    excl = np.array([(a, b, systems.EXCLUSION_FULL) for a, b in atoms], np.int32)
+    s = dataclasses.replace(_fluid(every, (length,) * 3), exclusions=excl, exclusion_check=excl[:, 2].copy(),
+                            molecule=np.concatenate([np.repeat(np.arange(held), 3),
+                                                     held + np.arange(len(pos) - held)]).astype(np.int32))
+    con = {"atoms": atoms, "rest": np.linalg.norm(every[atoms[:, 0]] - every[atoms[:, 1]], axis=1),
+           "shake": (1e-8, 100), "rattle": (1e-8, 100), "mass": s.mass}
+    v = integrate.maxwell_boltzmann(s.mass, 300.0, 3)
+    ref = oracle.leapfrog(s, [F.parse_definition(LJ9)], v, 1.0, 3, constraints=con)
+    topo = F.Topology(s)
+    lf = integrate.Leapfrog(topo, [F.ForceFactory.make(topo, LJ9, "fp64")], s.positions, v, s.mass, 1.0, virial=True,
+                            constraints=con).initialize()
+    lf.run(3)
+    x, vel, f, e = lf.state()
+    assert np.abs(x - ref[0]).max() <= 1e-10
+    assert np.abs(vel - ref[1]).max() <= 1e-9 * np.abs(ref[1]).max()
+
+
 @pytest.mark.parametrize("shape", ["pairs", "stars", "triangles", "mixed_order", "chains", "many"])
 def test_constrained_steps(shape):
     """Clusters of two and three atoms in any order of their constraints (the
