@@ -575,7 +575,7 @@ __device__ __forceinline__ F2 poly5_2(F2 ar)        // poly5f of both
     return mul2(t, h);
 }
 
-// pot_f32 of two pairs (no table potentials); m: 1-4 pairs
+// pot_f32 of two pairs; m: 1-4 pairs
 template <int POT>
 __device__ __forceinline__ void pot2(const PairArgs& p, const TermF& t, F2 r2, F2 rd2, F2 rinv, F2 qq, int ti, int tja,
                                      int tjb, bool ma, bool mb, F2& e, F2& f)
@@ -595,6 +595,14 @@ __device__ __forceinline__ void pot2(const PairArgs& p, const TermF& t, F2 r2, F
         e = mul2(qq, rinv);
         e = sel2(ma, mb, mul2(e, f2(p.csf)), e);
         f = mul2(e, rd2);
+    } else if (pot_table(POT)) {                     // (the look-ups do not pack)
+        float ra, rb, qa, qb, ea, eb, fa, fb;
+        split(r2, ra, rb);
+        split(qq, qa, qb);
+        pot_f32<POT>(p, t, ra, 0.f, 0.f, qa, ti, tja, ma ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE, ea, fa);
+        pot_f32<POT>(p, t, rb, 0.f, 0.f, qb, ti, tjb, mb ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE, eb, fb);
+        e = f2(ea, eb);
+        f = f2(fa, fb);
     } else {
         const F2 q = sel2(ma, mb, mul2(qq, f2(p.csf)), qq);
         const F2 r = mul2(r2, rinv);
@@ -656,8 +664,8 @@ __device__ __forceinline__ void switch2(const TermF& t, F2 r2, F2 rem, F2 rinv, 
     e = mul2(e, v);
 }
 
-// pair_math of two pairs of one row atom (no table potentials): force factors
-// and energies, zero for an inactive pair
+// pair_math of two pairs of one row atom: force factors and energies, zero for an
+// inactive pair
 template <int NT, int P0, int S0, int P1, int S1, bool OUT, bool FINE>
 __device__ __forceinline__ void pair_math2(const PairArgs& p, const JAtom& ia, const JAtom& ja, const JAtom& jb, F2 r2in,
                                            F2 rem, bool va, bool vb, int ca, int cb, F2& ft, F2& el, F2& ec)
@@ -803,21 +811,7 @@ struct ColForce32 {
         float ra, rb;
         split(r2, ra, rb);
         F2 ft, el, ec;
-        if constexpr (pot_table(P0) || (NT > 1 && pot_table(P1))) {
-            PairGeo ga, gb;                            // (the look-ups do not pack)
-            ga.r2 = ra; ga.act = va;
-            gb.r2 = rb; gb.act = vb;
-            ga.in0 = !TWO || (ca & kCodeIn0); ga.in1 = !TWO || (ca & kCodeIn1);
-            gb.in0 = !TWO || (cb & kCodeIn0); gb.in1 = !TWO || (cb & kCodeIn1);
-            ga.excl = (ca & kCodeMod) ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE;
-            gb.excl = (cb & kCodeMod) ? PMGPU_EXCL_MODIFIED : PMGPU_EXCL_NONE;
-            float fa, la, wa, fb, lb, wb;
-            pair_math<NT, P0, S0, P1, S1, TWO>(p, ga, ia, ja, fa, la, wa);
-            pair_math<NT, P0, S0, P1, S1, TWO>(p, gb, ia, jb, fb, lb, wb);
-            ft = f2(fa, fb); el = f2(la, lb); ec = f2(wa, wb);
-        } else {
-            pair_math2<NT, P0, S0, P1, S1, TWO, FINE != 0>(p, ia, ja, jb, r2, rem, va, vb, ca, cb, ft, el, ec);
-        }
+        pair_math2<NT, P0, S0, P1, S1, TWO, FINE != 0>(p, ia, ja, jb, r2, rem, va, vb, ca, cb, ft, el, ec);
         const F2 x = mul2(dx, ft), y = mul2(dy, ft), z = mul2(dz, ft);
         f[0] = sub2(f[0], x); f[1] = sub2(f[1], y); f[2] = sub2(f[2], z);
         float ga[3], gb[3], ta[3], tb[3], ua[3], ub[3];
