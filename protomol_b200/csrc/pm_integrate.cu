@@ -241,12 +241,11 @@ __global__ void __launch_bounds__(kConsThreads) k_rattle(ConsArgs a)
 // with a common atom): one thread keeps its cluster's positions and velocities
 // in registers through the step's half kick, RATTLE, half kick, drift and
 // SHAKE, all of them in block 0; the other blocks take the atoms without
-// constraints (10 pairs in a fluid of 20,001 atoms: 101 us a step, 779 when block 0 took
-// these too).  The
-// arithmetic is k_leapfrog's, rattle_one's and shake_one's, operation by
-// operation; SHAKE's bond vectors are the positions before the drift (what the
-// last SHAKE left), so no copy of them is kept.  A constraint's two atoms may
-// change places: every product keeps its bits.
+// constraints (10 pairs in a fluid of 20,001 atoms: 101 us a step, 779 when block
+// 0 took these too).  The arithmetic is k_leapfrog's, rattle_one's and
+// shake_one's, operation by operation; SHAKE's bond vectors are the positions
+// before the drift (what the last SHAKE left), so no copy of them is kept.  A
+// constraint's two atoms may change places: every product keeps its bits.
 //
 // What bounds it: the serial chain of FP64 operations (a division per
 // constraint and sweep), one CTA.  In global memory with eight divisions per

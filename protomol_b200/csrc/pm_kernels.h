@@ -281,8 +281,8 @@ int col_rows_split(int n_atoms, const ColGrid& g, double cutoff, int blocks_per_
 int col_row_blocks(int n_atoms, const ColGrid& g, double cutoff, int blocks_per_sm);
 int fp64_col_blocks_per_sm(int combo);     // of launch_pair_fp64 over the columns (the other row kernels: 4)
 int launch_pair_fp64(const PairArgs& a, int combo, bool col, int blocks, cudaStream_t s, long long* launches);
-// the molecular virial records (kMRec) of a cutoff force over the cell-sorted
-// order, one per block (blocks as launch_pair_fp64), no forces or energies
+// the molecular virial records (kMRec) of a cutoff force over the column list
+// (col) or the cell-sorted order, one per block, no forces or energies
 int launch_pair_molvir(const PairArgs& a, int combo, bool col, int blocks, cudaStream_t s, long long* launches);
 // shares of a row and blocks of the FP64 row kernels (records: one per block)
 int rows_split(int n_atoms, const CellGrid& g, int nd);

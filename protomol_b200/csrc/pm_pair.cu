@@ -11,16 +11,10 @@ struct Combo { int n, p0, s0, p1, s1; };
 // (factories/registerForceExemplarsCutoff.cpp:36-137) plus the fused
 // LennardJones Coulomb -switchingFunction C2 -switchingFunction C2.  A table
 // potential's own switching function is inside its table; the pair applies
-// UniversalSwitchingFunction to it (combos 17-24).
+// UniversalSwitchingFunction to it (combos 17-24).  Their list: PM_COMBOS.
+#define PM_COMBO_ROW(_, ID, ...) {__VA_ARGS__},
 static const Combo kCombos[] = {
-    {1, CO, SC1, NP, SUN}, {1, CO, SC2, NP, SUN}, {1, CO, SCUT, NP, SUN}, {1, CO, SSH, NP, SUN},
-    {1, EW, SCUT, NP, SUN}, {1, LJ, SC1, NP, SUN}, {1, LJ, SC2, NP, SUN}, {1, LJ, SCUT, NP, SUN},
-    {1, LJ, SSH, NP, SUN},
-    {2, LJ, SC1, EW, SCUT}, {2, LJ, SC1, CO, SSH}, {2, LJ, SC2, CO, SC1}, {2, LJ, SC2, EW, SCUT},
-    {2, LJ, SC2, CO, SCUT}, {2, LJ, SC2, CO, SSH}, {2, LJ, SCUT, EW, SCUT}, {2, LJ, SC2, CO, SC2},
-    {1, LJT, SUN, NP, SUN}, {1, COT, SUN, NP, SUN}, {1, EWT, SUN, NP, SUN},
-    {2, LJ, SC1, EWT, SUN}, {2, LJ, SC2, EWT, SUN}, {2, LJ, SCUT, EWT, SUN},
-    {2, LJT, SUN, EWT, SUN}, {2, LJT, SUN, COT, SUN},
+    PM_COMBOS(PM_COMBO_ROW, 0)
 };
 constexpr int kNumCombos = sizeof(kCombos) / sizeof(kCombos[0]);
 
@@ -97,36 +91,7 @@ int launch_cluster_list(const PairArgs& a, cudaStream_t s, long long* launches)
 
 int launch_pair_mixed(const PairArgs& a, int combo, cudaStream_t s, long long* launches)
 {
-    switch (combo) {
-#define PM_MIXED_CASE(ID, ...) case ID: return run_mixed<__VA_ARGS__>(a, s, launches);
-    PM_MIXED_CASE(0, 1, CO, SC1, NP, SUN)
-    PM_MIXED_CASE(1, 1, CO, SC2, NP, SUN)
-    PM_MIXED_CASE(2, 1, CO, SCUT, NP, SUN)
-    PM_MIXED_CASE(3, 1, CO, SSH, NP, SUN)
-    PM_MIXED_CASE(4, 1, EW, SCUT, NP, SUN)
-    PM_MIXED_CASE(5, 1, LJ, SC1, NP, SUN)
-    PM_MIXED_CASE(6, 1, LJ, SC2, NP, SUN)
-    PM_MIXED_CASE(7, 1, LJ, SCUT, NP, SUN)
-    PM_MIXED_CASE(8, 1, LJ, SSH, NP, SUN)
-    PM_MIXED_CASE(9, 2, LJ, SC1, EW, SCUT)
-    PM_MIXED_CASE(10, 2, LJ, SC1, CO, SSH)
-    PM_MIXED_CASE(11, 2, LJ, SC2, CO, SC1)
-    PM_MIXED_CASE(12, 2, LJ, SC2, EW, SCUT)
-    PM_MIXED_CASE(13, 2, LJ, SC2, CO, SCUT)
-    PM_MIXED_CASE(14, 2, LJ, SC2, CO, SSH)
-    PM_MIXED_CASE(15, 2, LJ, SCUT, EW, SCUT)
-    PM_MIXED_CASE(16, 2, LJ, SC2, CO, SC2)
-    PM_MIXED_CASE(17, 1, LJT, SUN, NP, SUN)
-    PM_MIXED_CASE(18, 1, COT, SUN, NP, SUN)
-    PM_MIXED_CASE(19, 1, EWT, SUN, NP, SUN)
-    PM_MIXED_CASE(20, 2, LJ, SC1, EWT, SUN)
-    PM_MIXED_CASE(21, 2, LJ, SC2, EWT, SUN)
-    PM_MIXED_CASE(22, 2, LJ, SCUT, EWT, SUN)
-    PM_MIXED_CASE(23, 2, LJT, SUN, EWT, SUN)
-    PM_MIXED_CASE(24, 2, LJT, SUN, COT, SUN)
-#undef PM_MIXED_CASE
-    default: return (int)cudaErrorInvalidValue;
-    }
+    PM_COMBO_SWITCH(PM_COMBO_RETURN, run_mixed)
 }
 
 int launch_near_energy(const PairArgs& a, int combo, int n_atoms, cudaStream_t s, long long* launches)
@@ -142,7 +107,7 @@ int launch_near_energy(const PairArgs& a, int combo, int n_atoms, cudaStream_t s
     // resident wave (16 blocks per SM; the kernel is grid-stride)
     long long want = (30LL * n_atoms + 127) / 128;
     const int blocks = (int)std::max(1LL, std::min<long long>(want, 16LL * sms));
-    PM_COMBO_SWITCH(k_near_energy)
+    PM_COMBO_SWITCH(PM_COMBO_LAUNCH, k_near_energy)
     *launches += 1;
     return (int)cudaGetLastError();
 }

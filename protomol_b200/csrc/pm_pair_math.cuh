@@ -45,9 +45,6 @@ __host__ __device__ constexpr bool pot_lj_slot(int p) { return p == LJ || p == L
 
 __host__ __device__ constexpr bool sw_modifies(int s) { return s == SC1 || s == SC2 || s == SSH; }
 __host__ __device__ constexpr bool pot_r2(int p) { return p == LJ || p == CO; }
-// the pair's rough cutoff test runs when a switching function is used or the
-// potential has its own cutoff (OneAtomPair.h:141, OneAtomPairTwo.h:145)
-__host__ __device__ constexpr bool term_cut(int p, int s) { return s != SUN || pot_table(p); }
 
 // ---------------------------------------------------------------- shared
 // ExclusionTable::check for a pair of the same molecule; returns the class
@@ -330,34 +327,43 @@ __device__ __forceinline__ void pair_f64(const PairArgs& p, double d2, double qi
     ft = NT > 1 ? f0 + f1 : f0;
 }
 
-#define PM_COMBO_SWITCH(KERNEL)                                                                        \
-    switch (combo) {                                                                                   \
-    case 0: KERNEL<1, CO, SC1, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                               \
-    case 1: KERNEL<1, CO, SC2, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                               \
-    case 2: KERNEL<1, CO, SCUT, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                              \
-    case 3: KERNEL<1, CO, SSH, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                               \
-    case 4: KERNEL<1, EW, SCUT, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                              \
-    case 5: KERNEL<1, LJ, SC1, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                               \
-    case 6: KERNEL<1, LJ, SC2, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                               \
-    case 7: KERNEL<1, LJ, SCUT, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                              \
-    case 8: KERNEL<1, LJ, SSH, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                               \
-    case 9: KERNEL<2, LJ, SC1, EW, SCUT><<<blocks, 128, 0, s>>>(a); break;                              \
-    case 10: KERNEL<2, LJ, SC1, CO, SSH><<<blocks, 128, 0, s>>>(a); break;                              \
-    case 11: KERNEL<2, LJ, SC2, CO, SC1><<<blocks, 128, 0, s>>>(a); break;                              \
-    case 12: KERNEL<2, LJ, SC2, EW, SCUT><<<blocks, 128, 0, s>>>(a); break;                             \
-    case 13: KERNEL<2, LJ, SC2, CO, SCUT><<<blocks, 128, 0, s>>>(a); break;                             \
-    case 14: KERNEL<2, LJ, SC2, CO, SSH><<<blocks, 128, 0, s>>>(a); break;                              \
-    case 15: KERNEL<2, LJ, SCUT, EW, SCUT><<<blocks, 128, 0, s>>>(a); break;                            \
-    case 16: KERNEL<2, LJ, SC2, CO, SC2><<<blocks, 128, 0, s>>>(a); break;                              \
-    case 17: KERNEL<1, LJT, SUN, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                             \
-    case 18: KERNEL<1, COT, SUN, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                             \
-    case 19: KERNEL<1, EWT, SUN, NP, SUN><<<blocks, 128, 0, s>>>(a); break;                             \
-    case 20: KERNEL<2, LJ, SC1, EWT, SUN><<<blocks, 128, 0, s>>>(a); break;                             \
-    case 21: KERNEL<2, LJ, SC2, EWT, SUN><<<blocks, 128, 0, s>>>(a); break;                             \
-    case 22: KERNEL<2, LJ, SCUT, EWT, SUN><<<blocks, 128, 0, s>>>(a); break;                            \
-    case 23: KERNEL<2, LJT, SUN, EWT, SUN><<<blocks, 128, 0, s>>>(a); break;                            \
-    case 24: KERNEL<2, LJT, SUN, COT, SUN><<<blocks, 128, 0, s>>>(a); break;                            \
-    default: return (int)cudaErrorInvalidValue;                                                        \
+// the registered combinations: X(ARG, id, number of terms, potential and switch
+// of each), the ids in order from 0
+#define PM_COMBOS(X, ARG) \
+    X(ARG, 0, 1, CO, SC1, NP, SUN) \
+    X(ARG, 1, 1, CO, SC2, NP, SUN) \
+    X(ARG, 2, 1, CO, SCUT, NP, SUN) \
+    X(ARG, 3, 1, CO, SSH, NP, SUN) \
+    X(ARG, 4, 1, EW, SCUT, NP, SUN) \
+    X(ARG, 5, 1, LJ, SC1, NP, SUN) \
+    X(ARG, 6, 1, LJ, SC2, NP, SUN) \
+    X(ARG, 7, 1, LJ, SCUT, NP, SUN) \
+    X(ARG, 8, 1, LJ, SSH, NP, SUN) \
+    X(ARG, 9, 2, LJ, SC1, EW, SCUT) \
+    X(ARG, 10, 2, LJ, SC1, CO, SSH) \
+    X(ARG, 11, 2, LJ, SC2, CO, SC1) \
+    X(ARG, 12, 2, LJ, SC2, EW, SCUT) \
+    X(ARG, 13, 2, LJ, SC2, CO, SCUT) \
+    X(ARG, 14, 2, LJ, SC2, CO, SSH) \
+    X(ARG, 15, 2, LJ, SCUT, EW, SCUT) \
+    X(ARG, 16, 2, LJ, SC2, CO, SC2) \
+    X(ARG, 17, 1, LJT, SUN, NP, SUN) \
+    X(ARG, 18, 1, COT, SUN, NP, SUN) \
+    X(ARG, 19, 1, EWT, SUN, NP, SUN) \
+    X(ARG, 20, 2, LJ, SC1, EWT, SUN) \
+    X(ARG, 21, 2, LJ, SC2, EWT, SUN) \
+    X(ARG, 22, 2, LJ, SCUT, EWT, SUN) \
+    X(ARG, 23, 2, LJT, SUN, EWT, SUN) \
+    X(ARG, 24, 2, LJT, SUN, COT, SUN)
+
+// inside switch (combo): a kernel of the combination launched on its blocks, or
+// a function of it called
+#define PM_COMBO_LAUNCH(KERNEL, ID, ...) case ID: KERNEL<__VA_ARGS__><<<blocks, 128, 0, s>>>(a); break;
+#define PM_COMBO_RETURN(FUNCTION, ID, ...) case ID: return FUNCTION<__VA_ARGS__>(a, s, launches);
+#define PM_COMBO_SWITCH(CASE, WHAT) \
+    switch (combo) { \
+    PM_COMBOS(CASE, WHAT) \
+    default: return (int)cudaErrorInvalidValue; \
     }
 
 }  // namespace pm

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(128) k_pair_adjoint_rows(const __grid_constant
     for (int k = 0; k < kLjCache; ++k) { op.cache.key[k] = -1; op.cache.a[k] = 0.0; op.cache.b[k] = 0.0; op.cache.hits[k] = 0; }
     op.mi = make_int4(-1, -1, -1, 0);
     if (COL) col_rows64<false>(p, sh_cols[COL ? threadIdx.x >> 5 : 0], op);
-    else cell_rows<true, false>(p, sh_cells[COL ? 0 : threadIdx.x >> 5], op);
+    else cell_rows<false>(p, sh_cells[COL ? 0 : threadIdx.x >> 5], op);
 #pragma unroll
     for (int k = 0; k < kLjCache; ++k)
         if (op.cache.key[k] >= 0) {
@@ -163,14 +163,12 @@ __global__ void __launch_bounds__(128) k_pair_adjoint_rows(const __grid_constant
 int launch_pair_adjoint_rows(const PairArgs& p, const AdjArgs& a, int fp64, bool col, int blocks, cudaStream_t s,
                              long long* launches)
 {
-    PairArgs q = p;
-    if (!a.use_cut) { q.cut2f = 3.0e38f; q.cut2d = 1.0e300; }      // no pair test
     if (col) {
-        if (fp64) k_pair_adjoint_rows<true, double><<<blocks, 128, 0, s>>>(q, a);
-        else k_pair_adjoint_rows<true, float><<<blocks, 128, 0, s>>>(q, a);
+        if (fp64) k_pair_adjoint_rows<true, double><<<blocks, 128, 0, s>>>(p, a);
+        else k_pair_adjoint_rows<true, float><<<blocks, 128, 0, s>>>(p, a);
     } else {
-        if (fp64) k_pair_adjoint_rows<false, double><<<blocks, 128, 0, s>>>(q, a);
-        else k_pair_adjoint_rows<false, float><<<blocks, 128, 0, s>>>(q, a);
+        if (fp64) k_pair_adjoint_rows<false, double><<<blocks, 128, 0, s>>>(p, a);
+        else k_pair_adjoint_rows<false, float><<<blocks, 128, 0, s>>>(p, a);
     }
     *launches += 1;
     return (int)cudaGetLastError();
@@ -226,16 +224,16 @@ int fp64_col_blocks_per_sm(int combo) { return combo >= 17 ? 4 : 5; }
 
 int launch_pair_fp64(const PairArgs& a, int combo, bool col, int blocks, cudaStream_t s, long long* launches)
 {
-    if (col) { PM_COMBO_SWITCH(k_pair_fp64_col) }
-    else { PM_COMBO_SWITCH(k_pair_fp64) }
+    if (col) { PM_COMBO_SWITCH(PM_COMBO_LAUNCH, k_pair_fp64_col) }
+    else { PM_COMBO_SWITCH(PM_COMBO_LAUNCH, k_pair_fp64) }
     *launches += 1;
     return (int)cudaGetLastError();
 }
 
 int launch_pair_molvir(const PairArgs& a, int combo, bool col, int blocks, cudaStream_t s, long long* launches)
 {
-    if (col) { PM_COMBO_SWITCH(k_pair_molvir_col) }
-    else { PM_COMBO_SWITCH(k_pair_molvir) }
+    if (col) { PM_COMBO_SWITCH(PM_COMBO_LAUNCH, k_pair_molvir_col) }
+    else { PM_COMBO_SWITCH(PM_COMBO_LAUNCH, k_pair_molvir) }
     *launches += 1;
     return (int)cudaGetLastError();
 }

@@ -62,7 +62,7 @@ struct RowTile { int4 a, b; };       // a lane's two candidates of a cluster
 // the row loop: op.begin(slot, valid), op.pair(valid, slot | modified << 30),
 // op.end(slot, valid) for every share of a row.  DIFFMOL: pairs of different
 // molecules only.
-template <bool CUT, bool DIFFMOL, class Op>
+template <bool DIFFMOL, class Op>
 __device__ __forceinline__ void cell_rows(const PairArgs& p, RowsShared& sh, Op& op)
 {
     const unsigned FULL = 0xffffffffu;
@@ -97,13 +97,13 @@ __device__ __forceinline__ void cell_rows(const PairArgs& p, RowsShared& sh, Op&
             const float dz = (float)(int)((unsigned)Pj.z - (unsigned)Pi.z) * sz;
             const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
             const bool same = Pj.w == Pi.w;
-            bool in = valid && j != si && (!CUT || r2 <= far2) && !(DIFFMOL && same);
+            bool in = valid && j != si && r2 <= far2 && !(DIFFMOL && same);
             int code = j;
-            const bool rare = in && ((CUT && r2 >= band2) || (!DIFFMOL && same));
+            const bool rare = in && (r2 >= band2 || (!DIFFMOL && same));
             if (__any_sync(FULL, rare)) {
                 if (rare) {
                     const int oi = p.smeta[si].x, oj = p.smeta[j].x;
-                    if (CUT && r2 >= band2) in = !(exact_d2(p, min(oi, oj), max(oi, oj)) > p.cut2d);
+                    if (r2 >= band2) in = !(exact_d2(p, min(oi, oj), max(oi, oj)) > p.cut2d);
                     if (!DIFFMOL && same) {
                         const int x = excl_class(p, oi, oj);
                         if (x == PMGPU_EXCL_FULL) in = false;
@@ -172,7 +172,7 @@ __device__ __forceinline__ void cell_rows(const PairArgs& p, RowsShared& sh, Op&
                     jfirst = c.y + kCluster * u;
                     nj = min(kCluster, c.z - jfirst);
                     near = true;
-                    if (CUT && !p.wrap) {
+                    if (!p.wrap) {
                         const float4 o = c.w > 0 ? p.doff[c.w - 1] : make_float4(0.f, 0.f, 0.f, 0.f);
                         near = box_near(ilo, ihi, p.cbox[2 * (c.x + u)], p.cbox[2 * (c.x + u) + 1], o.x, o.y, o.z, lim);
                     }
@@ -309,8 +309,6 @@ static __device__ __noinline__ void col_gather_block(const PairArgs& p, int row,
 template <bool DIFFMOL, class RowOp>
 __device__ __forceinline__ void col_rows64(const PairArgs& p, ColRowsShared& sh, RowOp& rop)
 {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
     const int split = p.rows_split;
     const int rows = p.ccstart[p.cg.ncol];
     // a refused system (another force of the group) has no whole list
@@ -469,8 +467,7 @@ __global__ void __launch_bounds__(128, 4) k_pair_fp64(const __grid_constant__ Pa
     __shared__ RowsShared sh[4];
     ForceRow<false, NT, P0, S0, P1, S1> op{p};
     op.init();
-    constexpr bool kUse = term_cut(P0, S0) || (NT > 1 && term_cut(P1, S1));
-    cell_rows<kUse, false>(p, sh[threadIdx.x >> 5], op);
+    cell_rows<false>(p, sh[threadIdx.x >> 5], op);
     force_record(p, op, 0.5);
 }
 
@@ -561,8 +558,7 @@ __global__ void __launch_bounds__(128, 4) k_pair_molvir(const __grid_constant__ 
     __shared__ RowsShared sh[4];
     MolvirRow<false, NT, P0, S0, P1, S1> op{p};
     op.init();
-    constexpr bool kUse = term_cut(P0, S0) || (NT > 1 && term_cut(P1, S1));
-    cell_rows<kUse, true>(p, sh[threadIdx.x >> 5], op);
+    cell_rows<true>(p, sh[threadIdx.x >> 5], op);
     molvir_record(p, op, 0.5);
 }
 

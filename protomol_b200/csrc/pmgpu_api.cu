@@ -1593,8 +1593,9 @@ static int col_refresh(pmgpu_system* sys, const double* d_pos)
     return PMGPU_OK;
 }
 
-// the column-path members of the pair arguments
-static void fill_col_args(pmgpu_system* sys, bool fp64, PairArgs& a, bool half)
+// the column-path members of the pair arguments (per_sm: blocks per SM of the
+// FP64 row kernel, which its shares of a row follow)
+static void fill_col_args(pmgpu_system* sys, bool fp64, PairArgs& a, bool half, int per_sm = 4)
 {
     a.cq = sys->d_cq; a.cm = sys->d_cm; a.ibox = sys->d_ibox; a.jbox = sys->d_jbox; a.c64 = sys->d_c64;
     a.ccstart = sys->d_ccstart; a.ccol = sys->d_ccol; a.icl_cap = sys->col_ncl_cap;
@@ -1608,7 +1609,7 @@ static void fill_col_args(pmgpu_system* sys, bool fp64, PairArgs& a, bool half)
     a.col_refuse = fp64 ? 0 : 1;
     a.col_half = half ? 1 : 0;
     a.col_none = 2 * sys->col_ncl_cap;
-    a.rows_split = col_rows_split(sys->n, sys->eval_cg, std::sqrt(a.cut2d), 4);
+    a.rows_split = col_rows_split(sys->n, sys->eval_cg, std::sqrt(a.cut2d), per_sm);
     const ColGrid& g = sys->eval_cg;
     a.chunk = col_chunk_entries(sys->n, g, g.lx * g.ly * g.lz, std::sqrt(a.cut2d), 6 * sys->tuning.chunk_entries, false);
     a.chunk_end = col_chunk_entries(sys->n, g, g.lx * g.ly * g.lz, std::sqrt(a.cut2d), 6 * sys->tuning.chunk_entries, true);
@@ -2336,9 +2337,7 @@ static int run_cutoffs(EvalRun& R, bool may_defer)
         if (!fp64 && !col && !f->wrap && virial) pair_virial = 1;
         PairArgs a;
         fill_pair_args(sys, f, d_pos, a);
-        if (col) fill_col_args(sys, fp64, a, true);
-        if (col && fp64)
-            a.rows_split = col_rows_split(sys->n, sys->eval_cg, std::sqrt(a.cut2d), fp64_col_blocks_per_sm(f->combo));
+        if (col) fill_col_args(sys, fp64, a, true, fp64_col_blocks_per_sm(f->combo));
         a.virial = virial;
         a.erec = sys->d_erec + used;
         // the column list, or the cell-cluster list of the mixed forces
@@ -2740,12 +2739,12 @@ extern "C" int pmgpu_get_pairs(pmgpu_system* sys, pmgpu_force* f, const double* 
     CK(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), s), "memset");
     PairArgs a;
     fill_pair_args(sys, f, sys->d_pos, a);
-    if (col) fill_col_args(sys, fp64, a, true);
+    if (col) fill_col_args(sys, fp64, a, true, fp64_col_blocks_per_sm(f->combo));
     a.near2 = 0.0f;                                    // recording only: no near-pair list
     a.erec = sys->d_erec;
     a.rec_pairs = d_pairs; a.rec_count = d_count; a.rec_cap = dcap;
     int e = col ? launch_col_list(a, s, &sys->launches) : (fp64 ? 0 : launch_cluster_list(a, s, &sys->launches));
-    if (!e) e = fp64 ? launch_pair_fp64(a, f->combo, col, row_blocks(sys, f), s, &sys->launches)
+    if (!e) e = fp64 ? launch_pair_fp64(a, f->combo, col, force_row_blocks(sys, f), s, &sys->launches)
                      : (col ? launch_pair_col(a, f->combo, s, &sys->launches)
                             : launch_pair_mixed(a, f->combo, s, &sys->launches));
     unsigned long long cnt = 0;
