@@ -1717,6 +1717,7 @@ static int pair_records(pmgpu_system* sys, pmgpu_force* f)
 // least one x-line per CTA)
 static int pme_xblocks(const pmgpu_force* f) { return f->pp.grid[1] * f->kzh; }
 
+constexpr int kSlotCodes = 1 << 27;    // atom slots the pair kernels' ring codes tell apart
 constexpr int kCol64Atoms = 900;       // FP64 forces of fewer atoms stay on the cells
 
 // The column-cluster path takes the cutoff forces of the group when the box
@@ -1744,6 +1745,7 @@ static int choose_layout(pmgpu_system* sys, int nf, pmgpu_force* const* forces, 
     }
     ColGrid g;
     if (!col_reach(sys, std::sqrt(rc2) + (any32 ? sys->list_skin : 0.0), g)) return PMGPU_OK;
+    if (sys->n / kCluster + g.ncol + 1 >= kSlotCodes / kCluster) return PMGPU_OK;
     if (any32 && !sys->col_disabled) sys->eval_use_col = true;
     // one cell-pair rule for all FP64 rows: a force whose own cutoff reaches
     // beyond the algorithm's keeps the cell layout
@@ -1773,7 +1775,8 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
     }
     for (int k = 0; k < nf; ++k) {
         pmgpu_force* f = forces[k];
-        if (!f || f->sys != sys) return fail(sys, PMGPU_ERR_ARG, "force belongs to another system");
+        if (f->kind == 0 && sys->n >= kSlotCodes)
+            return fail(sys, PMGPU_ERR_CAPACITY, "cutoff forces of 2^27 atoms or more");
         int r = f->kind == 0 ? prepare_cutoff(f) : (f->kind == 1 ? prepare_pme(f) : PMGPU_OK);
         if (r) return r;
         if (f->kind != 1) need += pair_records(sys, f);
