@@ -339,7 +339,7 @@ void* pmgpu_batch_stream(pmgpu_batch* batch);
  * depend on the first four beyond the last bits of the fixed-point grouping
  * (a chunk's partial sums are rounded together); over columns a chunk's length
  * follows from the system's size and chunk_entries bounds it (at six times its
- * value).  fp64_pairs gives the FP64
+ * value, and never more than 64).  fp64_pairs gives the FP64
  * kernels' results, which hold every mixed-precision bound.  Defaults: 16, 0
  * (the occupancy limit), 16, 1, 0. */
 typedef struct pmgpu_tuning {

@@ -24,7 +24,7 @@ long long col_list_estimate(int n_atoms, const ColGrid& g, double volume, double
 // kernel ends with its last chunks (30 us each at 36 entries): the first five
 // eighths of the rows get chunks for about two of every resident warp (148 SMs
 // x 16), the rest (last) for about six, never more than most (six tuned chunk
-// units) or a block.
+// units) or a chunk's shared memory.
 int col_chunk_entries(int n_atoms, const ColGrid& g, double volume, double cutoff, int most, bool last)
 {
     const double rho = volume > 0.0 ? n_atoms / volume : 0.0;

@@ -43,7 +43,7 @@
 // cutoff; evaluated tile by tile, the terms (LJ C2 + Ewald real) at 40% of the
 // lanes were two thirds of the kernel's 106 M warp instructions on the
 // 14,281-atom box.  The rings fill the lanes of the pair phase, and its FP32
-// arithmetic is packed two pairs to an instruction: 71 M.
+// arithmetic is packed two pairs to an instruction: 75 M.
 // Measured against the tile-by-tile kernel, each kernel alone: 8.10 -> 6.05 ms
 // for 1,000,000 atoms at 12 A, 360 -> 286 us for 61,233 at 10 A, 141 -> 138 us
 // for 14,281 (where 47 us do not shrink with the cutoff: the near-pair kernel's
@@ -907,7 +907,9 @@ struct ColForce32 {
                 const int q = sh.fj[c][k], l = sh.fj[3 + c][k];
                 if ((q | l) != 0) {
                     sh.fj[c][k] = sh.fj[3 + c][k] = 0;
-                    atomicAdd(to + c, (unsigned long long)((long long)q * 2097152 + ((l + 1 + ((l >> 2) & 1)) >> 2)));  // 2^-32, ties to even
+                    // to steps of 2^-32, ties to even
+                    const long long v = (long long)q * 2097152 + ((l + 1 + ((l >> 2) & 1)) >> 2);
+                    atomicAdd(to + c, (unsigned long long)v);
                 }
             }
         }
@@ -966,8 +968,9 @@ __device__ __forceinline__ int col_chunks(const PairArgs& p, bool mark)
     return bad ? 0 : min(*p.chunk_count, p.chunk_cap);
 }
 
-// Blocks per SM: five with an Ewald real term (96 registers, 32 bytes spilled:
-// 5.62 against 5.84 ms for 1,000,000 atoms, 270 against 278 us for 61,233), four
+// Blocks per SM (measured with the j-forces in one integer): five with an Ewald
+// real term (96 registers, 32 bytes spilled: 5.62 against 5.84 ms for 1,000,000
+// atoms, 270 against 278 us for 61,233), four
 // without (the fluid of 20,001 ions: 53 against 58 us a step with three systems
 // in flight, where the fifth block keeps the others' kernels waiting); six
 // spill 116 bytes and take 7.96 ms.
