@@ -164,7 +164,8 @@ struct pmgpu_system {
     int2* d_plist = nullptr;
     long long plist_cap = 0;
     long long plist_need = 0;          // reported by the last evaluation that overflowed
-    long long plist_short = 0;         // places an FP64 column list needs (as many as there is memory for)
+    long long plist_short = 0;         // places an FP64 column list needs ...
+    long long plist_most = INT_MAX;    // ... and those there was memory for
     int4* d_chunks = nullptr;
     long long chunk_cap = 0;
     long long chunk_need = 0;
@@ -1820,6 +1821,7 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
     }
     long long lneed = 0, cneed = 0;
     bool mixed = false;                    // some force has the mixed kernels' near pairs
+    const bool backward = (flags & kFlagNeeds64) != 0;     // (which runs none of them)
     if (sys->eval_use_col || sys->eval_col64) {
         const ColGrid& g = sys->eval_cg;
         const int icl = sys->n / kCluster + g.ncol + 1;
@@ -1841,15 +1843,15 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
         for (int k = 0; k < nf; ++k) {
             if (forces[k]->kind != 0) continue;
             const double rc = std::sqrt(forces[k]->cut2);
-            mixed |= !pairs64(sys, forces[k]);
+            mixed |= !pairs64(sys, forces[k]) && !backward;
             const double rl = rc + (pairs64(sys, forces[k]) ? 0.0 : sys->list_skin), vol = g.lx * g.ly * g.lz;
             const long long entries = col_list_estimate(sys->n, g, vol, rl);
             const int chunk = col_chunk_entries(sys->n, g, vol, rc, 6 * sys->tuning.chunk_entries, true);
             lneed = std::max(lneed, entries / 2);      // two entries in each int2 place of the list buffer
-            if (!pairs64(sys, forces[k])) cneed = std::max(cneed, col_chunk_estimate(entries, sys->n, g, chunk));
+            if (mixed) cneed = std::max(cneed, col_chunk_estimate(entries, sys->n, g, chunk));
         }
     }
-    if (!sys->eval_use_col) {
+    if (!sys->eval_use_col && !backward) {
         for (int k = 0; k < nf; ++k)
             if (forces[k]->kind == 0 && !pairs64(sys, forces[k])) {
                 mixed = true;
@@ -1862,7 +1864,7 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
         cneed = std::max(cneed, sys->chunk_need + sys->chunk_need / 4);
         if (!mixed) {                        // a row without entries finds its pairs by itself
             lneed = std::max(lneed, sys->plist_short + sys->plist_short / 4);
-            lneed = std::min(lneed, (long long)INT_MAX);
+            lneed = std::min(lneed, sys->plist_most);
             cneed = 0;
         }
         if (lneed > INT_MAX || cneed > INT_MAX)
@@ -1875,8 +1877,7 @@ static int eval_prepare(pmgpu_system* sys, int nf, pmgpu_force* const* forces, u
             cudaError_t e = dalloc(&sys->d_plist, (size_t)lneed);
             if (e != cudaSuccess && !mixed) {        // as many places as before, and no more asked for
                 cudaGetLastError();
-                sys->plist_short = 0;
-                lneed = had;
+                sys->plist_most = lneed = had;
                 e = lneed > 0 ? dalloc(&sys->d_plist, (size_t)lneed) : cudaSuccess;
             }
             CK(e, "alloc");

@@ -258,6 +258,10 @@ def test_a_list_far_beyond_its_estimate():
     assert len(seen) == 1 and abs(seen.pop() - ref["lennard_jones"]) <= 1e-11 * abs(ref["lennard_jones"])
     hv = _lj9_hessian_v(pos, v, *s.lj_table[0, 0, :2])
     assert np.abs(r["hv"] - hv).max() <= 1e-11 * np.abs(hv).max()
+    mixed = F.ForceFactory.make(topo, LJ9, "mixed")
+    for _ in range(2):
+        r = F.adjoint(topo, [mixed], s.positions, v)
+        assert np.linalg.norm(r["hv"] - hv) <= 1e-5 * np.linalg.norm(hv)
 
 
 @pytest.mark.parametrize("precision", ["mixed", "fp64"])
