@@ -24,9 +24,11 @@ using namespace pm;
 
 static const double kPi = 3.14159265358979323846;   // Constant::M_PI (base/pmconstants.cpp:56)
 static const double kEpsilon = 1.0e-14;              // Constant::EPSILON (base/pmconstants.cpp:45)
-// status word, list count and need, chunk count and need, work counter, pad,
-// then 11 int64 energy/virial sums
+// ints: status word, list and chunk need, list and chunk count, work counter,
+// near-pair count and need, two of the binning, the FP64 lists' need and count
+// (64 bits each), LJ entries, pad; then 11 int64 energy/virial sums
 static const size_t kSmallBytes = 64 + 8 * kERec;
+static const int kAdjCount = 14;       // its int that counts a backward pass's LJ entries
 // the evaluation's output slots: pmgpu_energies_mol (LJ, Coulomb, virial,
 // molecular virial)
 static const int kEOut = 20;
@@ -124,7 +126,7 @@ struct pmgpu_system {
     double* d_fout = nullptr;
     double* d_energy = nullptr;        // kEOut
     double* h_energy = nullptr;        // pinned kEOut
-    int* h_status = nullptr;           // pinned: the status word, copied back with the results
+    int* h_status = nullptr;           // pinned: the status word (16 ints), copied back with the results
     unsigned long long* d_facc32 = nullptr;   // mixed (2^32): 3N pair forces + 3N other (d_facc32p)
     unsigned long long* d_facc32p = nullptr;
     unsigned long long* d_facc40 = nullptr;   // FP64 over cells: wide sums (2^40), then fine ones (2^44)
@@ -227,7 +229,6 @@ struct pmgpu_system {
     double* d_adj_lj = nullptr;
     double* d_adj_val = nullptr;
     unsigned* d_adj_idx = nullptr;
-    unsigned* d_adj_count = nullptr;
     double* h_adj = nullptr;
     double* h_adj_val = nullptr;
     unsigned* h_adj_idx = nullptr;
@@ -391,7 +392,7 @@ extern "C" int pmgpu_system_create(int device, pmgpu_system** out)
     if (cudaMalloc(&sys->d_small, kSmallBytes) != cudaSuccess ||
         cudaMalloc((void**)&sys->d_energy, sizeof(double) * kEOut) != cudaSuccess ||
         cudaMallocHost((void**)&sys->h_energy, sizeof(double) * kEOut) != cudaSuccess ||
-        cudaMallocHost((void**)&sys->h_status, sizeof(int)) != cudaSuccess) {
+        cudaMallocHost((void**)&sys->h_status, 16 * sizeof(int)) != cudaSuccess) {
         delete sys;
         return PMGPU_ERR_NOMEM;
     }
@@ -405,7 +406,7 @@ extern "C" int pmgpu_system_create(int device, pmgpu_system** out)
     sys->d_chunk_count = sys->d_status + 4;
     sys->d_chunk_next = sys->d_status + 5;
     sys->d_list_short = (unsigned long long*)(sys->d_status + 10);   // (8 and 9: binning)
-    sys->d_list_next = sys->d_list_short + 1;
+    sys->d_list_next = sys->d_list_short + 1;                        // (14: kAdjCount)
     sys->d_efix = (unsigned long long*)((char*)sys->d_small + 64);
     *out = sys;
     return PMGPU_OK;
@@ -414,7 +415,7 @@ extern "C" int pmgpu_system_create(int device, pmgpu_system** out)
 static void free_atom_buffers(pmgpu_system* s)
 {
     dfree(s->d_q); dfree(s->d_type); dfree(s->d_mol); dfree(s->d_ljn); dfree(s->d_ljm); dfree(s->d_ljd);
-    dfree(s->d_adj); dfree(s->d_adj_lj); dfree(s->d_adj_val); dfree(s->d_adj_idx); dfree(s->d_adj_count);
+    dfree(s->d_adj); dfree(s->d_adj_lj); dfree(s->d_adj_val); dfree(s->d_adj_idx);
     for (void* h : {(void*)s->h_adj, (void*)s->h_adj_val, (void*)s->h_adj_idx})
         if (h) cudaFreeHost(h);
     s->h_adj = s->h_adj_val = nullptr; s->h_adj_idx = nullptr; s->h_adj_cap = 0;
@@ -3780,17 +3781,17 @@ extern "C" int pmgpu_adjoint(pmgpu_system* sys, int n_forces, pmgpu_force* const
     const bool sparse = nlj < (1ull << 31);
     if (!sys->d_adj) {
         ok(dalloc(&sys->d_adj, 7 * (size_t)n + 2));
-        ok(cudaMallocHost((void**)&sys->h_adj, sizeof(double) * (4 * (size_t)n + 3)));
+        ok(cudaMallocHost((void**)&sys->h_adj, sizeof(double) * (4 * (size_t)n + 2)));
     }
     if (dE_dlj && !sys->d_adj_lj) {
         ok(dalloc(&sys->d_adj_lj, nlj));
         if (sparse) {
-            ok(dalloc(&sys->d_adj_val, nlj)); ok(dalloc(&sys->d_adj_idx, nlj)); ok(dalloc(&sys->d_adj_count, 1));
+            ok(dalloc(&sys->d_adj_val, nlj)); ok(dalloc(&sys->d_adj_idx, nlj));
         }
     }
     if (e != cudaSuccess) {
         dfree(sys->d_adj); dfree(sys->d_adj_lj);          // a half-made set is made again by the next call
-        dfree(sys->d_adj_val); dfree(sys->d_adj_idx); dfree(sys->d_adj_count);
+        dfree(sys->d_adj_val); dfree(sys->d_adj_idx);
         if (sys->h_adj) { cudaFreeHost(sys->h_adj); sys->h_adj = nullptr; }
         return cuda_fail(sys, e, "adjoint setup");
     }
@@ -3804,7 +3805,6 @@ extern "C" int pmgpu_adjoint(pmgpu_system* sys, int n_forces, pmgpu_force* const
     ok(cudaMemsetAsync(sys->d_adj, 0, sizeof(double) * (hv ? 4 * (size_t)n : (size_t)n), s));
     ok(cudaMemsetAsync(d_e, 0, sizeof(double) * 2, s));
     if (d_lj) ok(cudaMemsetAsync(d_lj, 0, sizeof(double) * nlj, s));
-    if (d_lj && sparse) ok(cudaMemsetAsync(sys->d_adj_count, 0, sizeof(unsigned), s));
     if (hv) ok(cudaMemcpyAsync(d_v, v, sizeof(double) * n3, cudaMemcpyHostToDevice, s));
     if (e != cudaSuccess) return cuda_fail(sys, e, "adjoint setup");
     // cutoff forces run over the cell list of the positions (the forward
@@ -3896,19 +3896,16 @@ extern "C" int pmgpu_adjoint(pmgpu_system* sys, int n_forces, pmgpu_force* const
     // results: dq, hv and the energies to pinned memory, the LJ gradient as its
     // nonzero entries (the whole table where their 32-bit index is too short)
     double* h = sys->h_adj;
-    unsigned* h_count = reinterpret_cast<unsigned*>(h + 4 * (size_t)n + 2);
-    *h_count = 0;
     ok(cudaMemcpyAsync(h, sys->d_adj, sizeof(double) * (hv ? 4 * (size_t)n : (size_t)n), cudaMemcpyDeviceToHost, s));
     ok(cudaMemcpyAsync(h + 4 * (size_t)n, d_e, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
     if (d_lj && sparse && e == cudaSuccess) {
-        ok((cudaError_t)launch_lj_entries(d_lj, (unsigned)nlj, sys->d_adj_idx, sys->d_adj_val, sys->d_adj_count, s,
-                                          &sys->launches));
-        ok(cudaMemcpyAsync(h_count, sys->d_adj_count, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+        ok((cudaError_t)launch_lj_entries(d_lj, (unsigned)nlj, sys->d_adj_idx, sys->d_adj_val,
+                                          (unsigned*)sys->d_status + kAdjCount, s, &sys->launches));
     }
-    ok(cudaMemcpyAsync(sys->h_status, sys->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
+    ok(cudaMemcpyAsync(sys->h_status, sys->d_status, 16 * sizeof(int), cudaMemcpyDeviceToHost, s));
     ok(cudaStreamSynchronize(s));
     if (e == cudaSuccess && (*sys->h_status & kStatusListShort)) status_result(sys, kStatusListShort);
-    const size_t nz = e == cudaSuccess ? *h_count : 0;
+    const size_t nz = e == cudaSuccess ? (unsigned)sys->h_status[kAdjCount] : 0;
     if (nz > sys->h_adj_cap) {
         if (sys->h_adj_val) cudaFreeHost(sys->h_adj_val);
         if (sys->h_adj_idx) cudaFreeHost(sys->h_adj_idx);
